@@ -2,6 +2,7 @@
 // (hits per bin) obtained from the sorted keys instead of from atomics.
 #include "common.cuh"
 #include "binning.cuh"
+#include "binning_device.cuh"
 
 namespace hgc {
 
@@ -96,123 +97,16 @@ __global__ void __launch_bounds__(256)
 range_partial_kernel(const float *__restrict__ coords, int coord_stride, int n_dims, int n_vert,
                      float *__restrict__ partial /* [gridDim.x][2][kMaxBinDims] */)
 {
-    float mn[kMaxBinDims], mx[kMaxBinDims];
-#pragma unroll
-    for (int c = 0; c < kMaxBinDims; c++) { mn[c] = INFINITY; mx[c] = -INFINITY; }
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n_vert; v += gridDim.x * blockDim.x) {
-#pragma unroll
-        for (int c = 0; c < kMaxBinDims; c++)
-            if (c < n_dims) {
-                const float x = coords[(size_t)v * coord_stride + c];
-                mn[c] = fminf(mn[c], x);
-                mx[c] = fmaxf(mx[c], x);
-            }
-    }
-    __shared__ float s_mn[8][kMaxBinDims], s_mx[8][kMaxBinDims];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int c = 0; c < kMaxBinDims; c++) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            mn[c] = fminf(mn[c], __shfl_xor_sync(0xffffffffu, mn[c], o));
-            mx[c] = fmaxf(mx[c], __shfl_xor_sync(0xffffffffu, mx[c], o));
-        }
-        if (lane == 0) { s_mn[warp][c] = mn[c]; s_mx[warp][c] = mx[c]; }
-    }
-    __syncthreads();
-    if (threadIdx.x < kMaxBinDims) {
-        const int c = threadIdx.x;
-        float a = s_mn[0][c], b = s_mx[0][c];
-        for (int w = 1; w < 8; w++) { a = fminf(a, s_mn[w][c]); b = fmaxf(b, s_mx[w][c]); }
-        partial[((size_t)blockIdx.x * 2 + 0) * kMaxBinDims + c] = a;
-        partial[((size_t)blockIdx.x * 2 + 1) * kMaxBinDims + c] = b;
-    }
+    range_of_block(coords, coord_stride, n_dims, n_vert, partial);
 }
 
-constexpr int kGridSetupThreads = 256;
-
-// One block: finishes the min/max reduction and derives the grid exactly as the Python wrappers do
-// (modules/bin_by_coordinates_op.py:49-71, modules/binned_select_knn_op.py:57-63), in float32.
+// One block: finishes the min/max reduction and derives the grid.
 __global__ void __launch_bounds__(kGridSetupThreads)
 grid_setup_kernel(const float *__restrict__ partial, int n_partials, int n_dims, int n_all,
                   const int *__restrict__ row_splits, int n_rs, int n_bins_arg, int n_neigh,
                   int pre_normalized, GridParams *__restrict__ g)
 {
-    // min / max over the per-block partial results: thread t looks at coordinate t % 8 of every
-    // (kGridSetupThreads / 8)-th partial, a shared-memory pass combines the threads of a coordinate
-    static_assert(kMaxBinDims == 8 && kGridSetupThreads % 8 == 0, "layout of the reduction");
-    __shared__ float s_mn[kGridSetupThreads], s_mx[kGridSetupThreads];
-    {
-        const int cc = threadIdx.x & 7;
-        float a = INFINITY, b = -INFINITY;
-        for (int p = threadIdx.x >> 3; p < n_partials; p += kGridSetupThreads / 8) {
-            a = fminf(a, partial[((size_t)p * 2 + 0) * kMaxBinDims + cc]);
-            b = fmaxf(b, partial[((size_t)p * 2 + 1) * kMaxBinDims + cc]);
-        }
-        s_mn[threadIdx.x] = a;
-        s_mx[threadIdx.x] = b;
-    }
-    __syncthreads();
-    if (threadIdx.x >= 32) return;  // the rest is one warp's work
-    const int c = threadIdx.x;
-    float mn = 0.f, mx = 0.f;
-    if (c < n_all) {
-        mn = INFINITY; mx = -INFINITY;
-        for (int t = c; t < kGridSetupThreads; t += 8) {
-            mn = fminf(mn, s_mn[t]);
-            mx = fmaxf(mx, s_mx[t]);
-        }
-    }
-    // The wrapper shifts by the minimum first; x -> x - mn is monotone, so the shifted extremes
-    // are the extremes shifted.
-    const float shift = pre_normalized ? 0.f : mn;
-    const float smin = __fsub_rn(mn, shift);
-    float dmax = __fsub_rn(mx, shift);
-    if (smin == dmax) dmax = __fadd_rn(dmax, 1.f);
-    dmax = __fadd_rn(dmax, 1e-3f);
-    if (!isfinite(dmax)) dmax = 1.f;
-
-    int n_bins = n_bins_arg;
-    if (n_bins <= 0) {
-        const float first_event = n_rs > 1 ? (float)row_splits[1] : 1.f;
-        const float t = powf(__fdiv_rn(first_event, (float)n_neigh / 32.f), 1.f / (float)n_dims);
-        n_bins = (int)t;
-        n_bins = n_bins < 5 ? 5 : (n_bins > 30 ? 30 : n_bins);
-    }
-    float bw = c < n_dims ? __fdiv_rn(dmax, (float)n_bins) : -INFINITY;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) bw = fmaxf(bw, __shfl_xor_sync(0xffffffffu, bw, o));
-    int nb = 1;
-    if (c < n_dims) nb = (int)__fadd_rn(__fdiv_rn(dmax, bw), 1.f);
-    int prod = nb;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) prod *= __shfl_xor_sync(0xffffffffu, prod, o);
-    if (c < n_dims) { g->shift[c] = shift; g->n_bins[c] = nb; }
-    if (c == 0) {
-        g->bin_width = bw;
-        g->bins_per_event = prod;
-        g->n_total_bins = prod * (n_rs - 1);
-    }
-    // within-bin ordering code: start from the bin width (binned) or the batch range (others)
-    float ext = 0.f;
-    if (c < n_dims) ext = bw;
-    else if (c < n_all) { ext = mx - mn; if (!isfinite(ext)) ext = 0.f; }
-    if (c < kMaxBinDims) { g->all_min[c] = mn; g->all_ext[c] = ext; }
-    float cell[kMaxBinDims];
-#pragma unroll
-    for (int k = 0; k < kMaxBinDims; k++) cell[k] = __shfl_sync(0xffffffffu, ext, k);
-    if (c == 0) {
-        for (int k = 0; k < kSubBits; k++) {
-            int best = 0;
-#pragma unroll
-            for (int q = 1; q < kMaxBinDims; q++)
-                if (cell[q] > cell[best]) best = q;
-            g->sub_seq[k] = best;
-#pragma unroll
-            for (int q = 0; q < kMaxBinDims; q++)
-                if (q == best) cell[q] *= 0.5f;
-        }
-    }
+    grid_from_partials(partial, n_partials, n_dims, n_all, row_splits, n_rs, n_bins_arg, n_neigh, pre_normalized, g);
 }
 
 int compute_grid(const float *coords, int coord_stride, int n_dims, int n_all, int n_vert,

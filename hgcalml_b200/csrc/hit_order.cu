@@ -1,0 +1,339 @@
+// Ordering of a ragged batch for the neighbour search: by grid bin (the reference's argsort) and along a Hilbert
+// curve, both inside every event.
+//
+// Events are contiguous in the input, so both sorts run event by event: a block works on a tile of up to 2048
+// hits of one event and the event needs no key bits.  Both are stable sorts of 32-bit keys, least significant
+// digit first, four passes of 8 bits, and every pass does both orders in one launch (blockIdx.y).  A pass is
+// one kernel: the digits of every tile have been counted by the kernel before it (the keys kernel for
+// the first pass; a scattering block adds the next digit of every hit to the count of the tile the hit lands in),
+// the digits of the whole event by the keys kernel for all passes at once.  A block adds up the counts of
+// the tiles before its own, which takes no waiting for other blocks.  Counts are sums of integers, so the
+// result does not depend on the order of the atomic additions.
+//
+// At 200k hits a pass is bound by latency (about 100 blocks): what counts is the number of launches, seven
+// here for grid, keys and both orders, against 43 with separate count, scan and scatter kernels per digit and
+// order.
+#include "common.cuh"
+#include "binning_device.cuh"
+#include "hit_order.cuh"
+
+namespace hgc {
+namespace {
+
+constexpr int kThreads = 256;
+constexpr int kWarps = kThreads / kWarp;
+constexpr int kRounds = kOrderTile / kThreads;
+
+template <typename Op>
+__device__ __forceinline__ int block_scan_inclusive(int v, Op op, int identity, int *s_warp)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v = op(v, t);
+    }
+    __syncthreads();  // s_warp may still be read by the previous scan
+    if (lane == 31) s_warp[warp] = v;
+    __syncthreads();
+    int before = identity;
+    for (int w = 0; w < warp; w++) before = op(before, s_warp[w]);
+    return op(before, v);
+}
+
+// First position, tile, chunk and super-chunk of every event, and of the run of hits that lie beyond the last
+// event.  Row splits are clamped to an ascending sequence inside [0, n_vert], so the layout stays
+// inside its arrays whatever they hold.  One block of kThreads.
+__device__ void event_layout(const int *__restrict__ row_splits, int n_events, int n_vert, const HitOrder &o)
+{
+    __shared__ int s_warp[kWarps];
+    __shared__ int s_last[4];
+    auto add = [](int a, int b) { return a + b; };
+    auto mx = [](int a, int b) { return a > b ? a : b; };
+    int pos = 0, tile = 0, chunk = 0, super = 0;  // carried over from the events before
+    for (int base = 0; base <= n_events; base += kThreads) {
+        const int e = base + threadIdx.x;
+        // end of event e; the last entry (the hits beyond the last event) ends with the batch
+        int end = e < n_events ? min(max(row_splits[e + 1], 0), n_vert) : n_vert;
+        end = mx(pos, block_scan_inclusive(end, mx, 0, s_warp));
+        int begin = __shfl_up_sync(0xffffffffu, end, 1);
+        __syncthreads();
+        if ((threadIdx.x & 31) == 31) s_warp[threadIdx.x >> 5] = end;
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0) begin = threadIdx.x == 0 ? pos : s_warp[(threadIdx.x >> 5) - 1];
+        const int n = e <= n_events ? end - begin : 0;
+        const int nt = (n + kOrderTile - 1) / kOrderTile, nc = (n + 31) / 32, ns = (nc + 31) / 32;
+        const int ti = tile + block_scan_inclusive(nt, add, 0, s_warp);
+        const int ci = chunk + block_scan_inclusive(nc, add, 0, s_warp);
+        const int si = super + block_scan_inclusive(ns, add, 0, s_warp);
+        if (e <= n_events) {
+            o.event_pos[e] = begin;
+            o.event_tile[e] = ti - nt;
+            o.event_chunk[e] = ci - nc;
+            o.event_super[e] = si - ns;
+            if (e == n_events) {
+                o.event_pos[e + 1] = end;
+                o.event_tile[e + 1] = ti;
+                o.event_chunk[e + 1] = ci;
+                o.event_super[e + 1] = si;
+            }
+        }
+        __syncthreads();
+        if (threadIdx.x == kThreads - 1) { s_last[0] = end; s_last[1] = ti; s_last[2] = ci; s_last[3] = si; }
+        __syncthreads();
+        pos = s_last[0]; tile = s_last[1]; chunk = s_last[2]; super = s_last[3];
+    }
+}
+
+// Range of the coordinates over the batch; the first block also lays out the events, the last one to
+// finish derives the grid.
+__global__ void __launch_bounds__(kThreads)
+range_and_layout_kernel(const float *__restrict__ coords, int C, int n_dims, int n_all, int n_vert,
+                        const int *__restrict__ row_splits, int n_rs, int n_bins, int n_neigh, HitOrder o,
+                        unsigned *arrived)
+{
+    __shared__ bool s_last;
+    range_of_block(coords, C, n_all, n_vert, o.partial);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(arrived, 1u) == gridDim.x - 1;
+    }
+    if (blockIdx.x == 0) event_layout(row_splits, n_rs - 1, n_vert, o);
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    grid_from_partials(o.partial, gridDim.x, n_dims, n_all, row_splits, n_rs, n_bins, n_neigh, 0, o.grid);
+}
+
+__device__ __forceinline__ int event_of_tile(const int *__restrict__ event_tile, int n_events, int tile)
+{
+    int lo = 0, hi = n_events;  // last event whose first tile is <= tile (events without hits share one)
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (event_tile[mid] <= tile) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
+struct Tile { int event, first, n; };  // positions [first, first + n)
+
+__device__ __forceinline__ bool find_tile(const HitOrder &o, int n_events, int tile, Tile *t)
+{
+    if (tile >= o.event_tile[n_events + 1]) return false;
+    t->event = event_of_tile(o.event_tile, n_events, tile);
+    t->first = o.event_pos[t->event] + (tile - o.event_tile[t->event]) * kOrderTile;
+    t->n = min(o.event_pos[t->event + 1] - t->first, kOrderTile);
+    return true;
+}
+
+// Keys of both orders, digit counts of the tile (first pass) and of the event (all passes).
+//   order 0: bin number inside the event (as modules/compiled/bin_by_coordinates_kernel.cc:64-113: truncating float
+//            division, last dimension fastest, out-of-range bins forced to 0), then the 16-bit locality code
+//   order 1: position on a Hilbert curve of B bits per coordinate
+template <int D, int B>
+__global__ void __launch_bounds__(kThreads)
+order_keys_kernel(const float *__restrict__ coords, int C, int n_dims, HitOrder o, int n_events, int tiles_cap,
+                  unsigned *status)
+{
+    __shared__ int s_hist[2][kOrderPasses][256];
+    __shared__ unsigned short s_frac[kMaxBinDims][kThreads];
+    Tile t;
+    if (!find_tile(o, n_events, blockIdx.x, &t)) return;
+    for (int i = threadIdx.x; i < 2 * kOrderPasses * 256; i += kThreads) (&s_hist[0][0][0])[i] = 0;
+    __syncthreads();
+    if (t.event == n_events && threadIdx.x == 0) flag_status(status, HGC_STATUS_FLAT_BIN_OVERFLOW);
+    const GridParams *__restrict__ g = o.grid;
+    const float bw = g->bin_width, scale = g->curve_scale * (float)(1u << B);
+    for (int r = 0; r < kRounds; r++) {
+        const int i = r * kThreads + threadIdx.x;
+        if (i >= t.n) break;
+        const int v = t.first + i;
+        float x[D];
+#pragma unroll
+        for (int c = 0; c < D; c++) x[c] = coords[(size_t)v * C + c];
+        unsigned flat = 0u, curve[D];
+        int stride = 1;
+#pragma unroll
+        for (int c = D - 1; c >= 0; c--) {
+            unsigned f;
+            if (c < n_dims) {
+                const float u = __fdiv_rn(__fsub_rn(x[c], g->shift[c]), bw);
+                int ci = __float2int_rz(u);
+                f = (unsigned)fminf(fmaxf((u - (float)ci) * 65536.f, 0.f), 65535.f);
+                const int nb = g->n_bins[c];
+                if (ci < 0 || ci >= nb) {
+                    ci = 0;
+                    flag_status(status, HGC_STATUS_BIN_OUT_OF_RANGE);
+                }
+                flat += (unsigned)(ci * stride);
+                stride *= nb;
+            } else {
+                const float ext = g->all_ext[c];
+                const float u = ext > 0.f ? (x[c] - g->all_min[c]) / ext : 0.f;
+                f = (unsigned)fminf(fmaxf(u * 65536.f, 0.f), 65535.f);
+            }
+            s_frac[c][threadIdx.x] = (unsigned short)f;
+            curve[c] = (unsigned)fminf(fmaxf((x[c] - g->all_min[c]) * scale, 0.f), (float)((1u << B) - 1u));
+        }
+        unsigned code = 0u;
+#pragma unroll
+        for (int k = 0; k < kSubBits; k++) {
+            const int c = g->sub_seq[k];  // the same for all threads
+            code = (code << 1) | ((unsigned)(s_frac[c][threadIdx.x] >> g->sub_bit[k]) & 1u);
+        }
+        const unsigned key[2] = {(flat << kSubBits) | code, hilbert_code<D, B>(curve)};
+#pragma unroll
+        for (int s = 0; s < 2; s++) {
+            o.key[s][0][v] = key[s];
+#pragma unroll
+            for (int p = 0; p < kOrderPasses; p++) atomicAdd(&s_hist[s][p][(key[s] >> (8 * p)) & 255u], 1);
+        }
+    }
+    __syncthreads();
+    const int d = threadIdx.x;  // kThreads == 256 digits
+#pragma unroll
+    for (int s = 0; s < 2; s++) {
+        o.tile_hist[((size_t)(s * kOrderPasses) * tiles_cap + blockIdx.x) * 256 + d] = s_hist[s][0][d];
+#pragma unroll
+        for (int p = 0; p < kOrderPasses; p++) {
+            const int c = s_hist[s][p][d];
+            if (c) atomicAdd(&o.event_hist[((size_t)(s * kOrderPasses + p) * (n_events + 2) + t.event) * 256 + d], c);
+        }
+    }
+}
+
+// One pass of both sorts.  LAST: the permutation (and, for order 0, its inverse) is written instead of keys and values.
+template <bool FIRST, bool LAST>
+__global__ void __launch_bounds__(kThreads)
+order_pass_kernel(HitOrder o, int n_events, int tiles_cap, int pass, int *__restrict__ bin_perm,
+                  int *__restrict__ rank, int *__restrict__ curve_perm)
+{
+    __shared__ int s_count[kWarps][256];
+    __shared__ int s_warp[kWarps];
+    const int order = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d = threadIdx.x;
+    Tile t;
+    if (!find_tile(o, n_events, blockIdx.x, &t)) return;
+    const unsigned *__restrict__ key_in = o.key[order][pass & 1];
+    const int *__restrict__ val_in = o.val[order][pass & 1];
+    const int shift = 8 * pass;
+
+    // this tile's items: a warp owns 32 * kRounds consecutive ones, so that equal digits keep their order
+    unsigned key[kRounds];
+    int val[kRounds];
+    const int warp_base = warp * (kRounds * kWarp);
+#pragma unroll
+    for (int r = 0; r < kRounds; r++) {
+        const int i = warp_base + r * kWarp + lane;
+        key[r] = 0u;
+        val[r] = 0;
+        if (i < t.n) {
+            key[r] = key_in[t.first + i];
+            val[r] = FIRST ? t.first + i : val_in[t.first + i];
+        }
+    }
+    // where the digit starts: smaller digits of the event, and the same digit in the tiles before
+    int start = o.event_pos[t.event];
+    {
+        const int mine = o.event_hist[((size_t)(order * kOrderPasses + pass) * (n_events + 2) + t.event) * 256 + d];
+        start += block_scan_inclusive(mine, [](int a, int b) { return a + b; }, 0, s_warp) - mine;
+        const int *__restrict__ h = o.tile_hist + (size_t)(order * kOrderPasses + pass) * tiles_cap * 256 + d;
+        int sum = 0;
+#pragma unroll 8
+        for (int q = o.event_tile[t.event]; q < (int)blockIdx.x; q++) sum += h[(size_t)q * 256];
+        start += sum;
+    }
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) s_count[w][d] = 0;
+    unsigned peers[kRounds];
+#pragma unroll
+    for (int r = 0; r < kRounds; r++) {
+        // places beyond the tile take a digit of their own
+        const unsigned dg = warp_base + r * kWarp + lane < t.n ? (key[r] >> shift) & 255u : 256u;
+        peers[r] = __match_any_sync(0xffffffffu, dg);
+    }
+    __syncthreads();
+    int place[kRounds];  // inside the run of this digit in this warp
+#pragma unroll
+    for (int r = 0; r < kRounds; r++) {
+        const bool ok = warp_base + r * kWarp + lane < t.n;
+        const unsigned dg = (key[r] >> shift) & 255u, before = peers[r] & ((1u << lane) - 1u);
+        const int seen = ok ? s_count[warp][dg] : 0;
+        place[r] = seen + __popc(before);
+        __syncwarp();
+        if (ok && before == 0u) s_count[warp][dg] = seen + __popc(peers[r]);
+        __syncwarp();
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) {
+        const int c = s_count[w][d];
+        s_count[w][d] = start;
+        start += c;
+    }
+    __syncthreads();
+    int *__restrict__ next_hist = o.tile_hist + (size_t)(order * kOrderPasses + pass + 1) * tiles_cap * 256;
+    const int pos0 = o.event_pos[t.event], tile0 = o.event_tile[t.event];
+#pragma unroll
+    for (int r = 0; r < kRounds; r++) {
+        if (warp_base + r * kWarp + lane < t.n) {
+            const int dst = s_count[warp][(key[r] >> shift) & 255u] + place[r];
+            if (LAST) {
+                if (order == 0) {
+                    bin_perm[dst] = val[r];
+                    rank[val[r]] = dst;
+                } else {
+                    curve_perm[dst] = val[r];
+                }
+            } else {
+                o.key[order][(pass + 1) & 1][dst] = key[r];
+                o.val[order][(pass + 1) & 1][dst] = val[r];
+                const int q = tile0 + (dst - pos0) / kOrderTile;
+                atomicAdd(&next_hist[(size_t)q * 256 + ((key[r] >> (shift + 8)) & 255u)], 1);
+            }
+        }
+    }
+}
+
+}  // namespace
+
+int order_hits(const float *coords, int n_coords, int n_bin_dims, const int *row_splits, int n_rs, int n_bins, int n_neigh,
+               int n_vert, int bin_bits, const HitOrder &o, int *bin_perm, int *rank, int *curve_perm,
+               unsigned *status, cudaStream_t stream)
+{
+    if (n_vert <= 0) return HGC_OK;
+    if (bin_bits + kSubBits > 32) return HGC_ERR_UNSUPPORTED;
+    const int n_events = n_rs - 1;
+    const int n_all = n_coords < kMaxBinDims ? n_coords : kMaxBinDims;
+    range_and_layout_kernel<<<range_partial_blocks(n_vert), kThreads, 0, stream>>>(
+            coords, n_coords, n_bin_dims, n_all, n_vert, row_splits, n_rs, n_bins, n_neigh, o, status + 8);
+    HGC_LAUNCH_CHECK();
+    const int tiles = (int)order_tiles_cap(n_vert, n_events);
+#define HGC_KEYS(D, B)                                                                                            \
+    case D: order_keys_kernel<D, B><<<tiles, kThreads, 0, stream>>>(coords, n_coords, n_bin_dims, o, n_events, tiles, status); break
+    switch (n_all) {
+        HGC_KEYS(2, 16);
+        HGC_KEYS(3, 10);
+        HGC_KEYS(4, 8);
+        HGC_KEYS(5, 6);
+        HGC_KEYS(6, 5);
+        HGC_KEYS(7, 4);
+        HGC_KEYS(8, 4);
+        default: return HGC_ERR_UNSUPPORTED;
+    }
+#undef HGC_KEYS
+    HGC_LAUNCH_CHECK();
+    const dim3 grid(tiles, 2);
+    for (int p = 0; p < kOrderPasses; p++) {
+        if (p == 0)
+            order_pass_kernel<true, false><<<grid, kThreads, 0, stream>>>(o, n_events, tiles, p, bin_perm, rank, curve_perm);
+        else if (p + 1 < kOrderPasses)
+            order_pass_kernel<false, false><<<grid, kThreads, 0, stream>>>(o, n_events, tiles, p, bin_perm, rank, curve_perm);
+        else
+            order_pass_kernel<false, true><<<grid, kThreads, 0, stream>>>(o, n_events, tiles, p, bin_perm, rank, curve_perm);
+        HGC_LAUNCH_CHECK();
+    }
+    return HGC_OK;
+}
+
+}  // namespace hgc

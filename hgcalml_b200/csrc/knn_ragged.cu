@@ -5,18 +5,22 @@
 // replaces IndexReplacer and the two scatter_nd calls.
 #include "common.cuh"
 #include "binning.cuh"
-#include "select_knn.cuh"
+#include "hit_order.cuh"
+#include "select_knn_tile_api.cuh"
 
 namespace hgc {
 namespace {
 
-__global__ void gather_rows_kernel(const int *__restrict__ src, int width, const int *__restrict__ perm,
-                                   int *__restrict__ dst, int n)
+__global__ void gather_kernel(const int *__restrict__ src, const int *__restrict__ perm, int *__restrict__ dst, int n)
 {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)n * width) return;
-    const int i = (int)(t / width), c = (int)(t % width);
-    dst[t] = src[(size_t)perm[i] * width + c];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) dst[i] = src[perm[i]];
+}
+
+__global__ void invert_perm_kernel(const int *__restrict__ perm, int *__restrict__ inv, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) inv[perm[i]] = i;
 }
 
 struct RaggedPlan {
@@ -47,34 +51,38 @@ using namespace hgc;
 namespace {
 
 struct RaggedBuffers {
-    GridParams *grid;
-    float *partial;
-    int *keys, *subkeys, *skeys, *perm, *k1, *v1, *tkeys, *tvals, *hist, *assigned, *sassigned, *bounds, *sdir;
-    KnnScratch knn;
+    HitOrder order;
+    TileScratch tiles;
+    int *bin_perm, *curve_perm, *rank;
+    // orders by bin whose keys do not fit 32 bits (see wide_bins)
+    int *keys, *subkeys, *k1, *v1, *tkeys, *tvals, *hist;
 };
+
+// A bin number inside an event and the 16-bit locality code make a 32-bit sort key up to 2^16 bins per event; finer
+// grids (a bin count asked for by the caller, or four and five binned dimensions) are sorted in two steps.
+bool wide_bins(const RaggedPlan &p, int n_events) { return p.max_bins / (n_events > 0 ? n_events : 1) > (1LL << 16); }
 
 // One definition of the layout serves both the size query (Sizer) and the real carve (Carver).
 template <typename W>
-void layout(W &ws, int n_vert, int n_coords, const RaggedPlan &p, bool use_dir, RaggedBuffers *b)
+void layout(W &ws, int n_vert, int n_coords, int n_rs, const RaggedPlan &p, RaggedBuffers *b)
 {
     const size_t n = n_vert > 0 ? n_vert : 0;
+    const int n_events = n_rs > 1 ? n_rs - 1 : 0;
     RaggedBuffers t;
-    t.grid = ws.template take<GridParams>(1);
-    t.partial = ws.template take<float>((size_t)range_partial_blocks(n_vert) * 2 * kMaxBinDims);
-    t.keys = ws.template take<int>(n);
-    t.subkeys = ws.template take<int>(n);
-    t.k1 = ws.template take<int>(n);
-    t.v1 = ws.template take<int>(n);
-    t.skeys = ws.template take<int>(n);
-    t.perm = ws.template take<int>(n);
-    t.tkeys = ws.template take<int>(n);
-    t.tvals = ws.template take<int>(n);
-    t.hist = ws.template take<int>(sort_hist_ints(n_vert));
-    t.assigned = ws.template take<int>(n * (p.cb + 1));
-    t.sassigned = ws.template take<int>(n * (p.cb + 1));
-    t.bounds = ws.template take<int>((size_t)p.max_bins + 1);
-    t.knn = knn_scratch_layout(ws, n_vert, n_coords);
-    t.sdir = ws.template take<int>(use_dir ? n : 0);
+    t.order = hit_order_layout(ws, n_vert, n_events);
+    t.tiles = tile_scratch_layout(ws, n_vert, n_coords, n_events);
+    t.bin_perm = ws.template take<int>(n);
+    t.curve_perm = ws.template take<int>(n);
+    t.rank = ws.template take<int>(n);
+    if (wide_bins(p, n_events)) {
+        t.keys = ws.template take<int>(n);
+        t.subkeys = ws.template take<int>(n);
+        t.k1 = ws.template take<int>(n);
+        t.v1 = ws.template take<int>(n);
+        t.tkeys = ws.template take<int>(n);
+        t.tvals = ws.template take<int>(n);
+        t.hist = ws.template take<int>(sort_hist_ints(n_vert));
+    }
     if (b) *b = t;
 }
 
@@ -92,7 +100,7 @@ extern "C" size_t hgc_binned_select_knn_ragged_workspace_bytes(int n_vert, int n
     RaggedPlan p;
     if (n_coords < 1 || !make_plan(n_coords, n_rs, n_bins, max_bin_dims, &p)) return 0;
     SizerW w;
-    layout(w, n_vert, n_coords, p, true, nullptr);
+    layout(w, n_vert, n_coords, n_rs, p, nullptr);
     return w.s.used;
 }
 
@@ -118,46 +126,36 @@ extern "C" int hgc_binned_select_knn_ragged(
 
     Carver ws(workspace);
     RaggedBuffers b;
-    layout(ws, n_vert, n_coords, p, use_direction != 0, &b);
-    HGC_CUDA_TRY(cudaMemsetAsync(ws.status(), 0, kAlign, stream));
-
-    if (int rc = compute_grid(d_coords, n_coords, p.cb, n_coords, n_vert, d_row_splits, n_rs, n_bins, n_neigh,
-                              /*pre_normalized=*/0, b.partial, b.grid, stream))
+    layout(ws, n_vert, n_coords, n_rs, p, &b);
+    const int n_events = n_rs - 1;
+    // the status word and the histograms of the sorts, which follow it
+    HGC_CUDA_TRY(cudaMemsetAsync(ws.status(), 0, hit_order_zeroed_bytes(n_vert, n_events), stream));
+    int *perm = d_sorting_out ? d_sorting_out : b.bin_perm;
+    const bool wide = wide_bins(p, n_events);
+    if (int rc = order_hits(d_coords, n_coords, p.cb, d_row_splits, n_rs, n_bins, n_neigh, n_vert,
+                            wide ? 16 : bits_for(p.max_bins / (n_events > 0 ? n_events : 1) - 1), b.order, perm, b.rank,
+                            b.curve_perm, ws.status(), stream))
         return rc;
-    if (int rc = launch_bin_keys(d_coords, n_coords, p.cb, b.grid->shift, d_row_splits, n_rs,
-                                 &b.grid->bin_width, b.grid->n_bins, b.assigned, nullptr, b.keys, n_vert,
-                                 0, &b.grid->n_total_bins, ws.status(), stream, b.grid, n_coords, b.subkeys))
-        return rc;
-    // Order: by bin (what the reference's argsort gives), and inside a bin by the locality code
-    // instead of by original index -- a free choice, since results do not depend on it.  Two stable
-    // counting sorts, least significant key first.
-    if (int rc = sort_pairs(b.subkeys, nullptr, b.k1, b.v1, b.tkeys, b.tvals, b.hist, n_vert, kSubBits, stream))
-        return rc;
-    {
-        gather_rows_kernel<<<div_up(n_vert, 256), 256, 0, stream>>>(b.keys, 1, b.v1, b.k1, n_vert);
+    if (wide) {
+        // two stable counting sorts, least significant key first
+        const GridParams *g = b.order.grid;
+        if (int rc = launch_bin_keys(d_coords, n_coords, p.cb, g->shift, d_row_splits, n_rs, &g->bin_width, g->n_bins,
+                                     nullptr, nullptr, b.keys, n_vert, 0, &g->n_total_bins, ws.status(), stream, g,
+                                     n_coords, b.subkeys))
+            return rc;
+        if (int rc = sort_pairs(b.subkeys, nullptr, b.k1, b.v1, b.tkeys, b.tvals, b.hist, n_vert, kSubBits, stream))
+            return rc;
+        gather_kernel<<<div_up(n_vert, 256), 256, 0, stream>>>(b.keys, b.v1, b.k1, n_vert);
+        HGC_LAUNCH_CHECK();
+        if (int rc = sort_pairs(b.k1, b.v1, b.keys, perm, b.tkeys, b.tvals, b.hist, n_vert, bits_for(p.max_bins), stream))
+            return rc;
+        invert_perm_kernel<<<div_up(n_vert, 256), 256, 0, stream>>>(perm, b.rank, n_vert);
         HGC_LAUNCH_CHECK();
     }
-    if (int rc = sort_pairs(b.k1, b.v1, b.skeys, b.perm, b.tkeys, b.tvals, b.hist, n_vert,
-                            bits_for(p.max_bins), stream))
+    const int *direction = use_direction ? d_direction : nullptr;
+    if (int rc = build_tiles(d_coords, n_coords, b.curve_perm, b.rank, b.order, n_events, direction, b.tiles, n_vert, stream)) return rc;
+    if (int rc = search_tiles(b.tiles, b.order, perm, d_coords, n_coords, direction, d_indices, d_dist, n_vert, n_rs - 1, n_neigh,
+                              tf_compat, stream))
         return rc;
-    if (int rc = boundaries_from_sorted_keys(b.skeys, n_vert, b.bounds, (int)p.max_bins, stream)) return rc;
-    if (int rc = pack_points(d_coords, n_coords, b.perm, b.knn, n_vert, stream)) return rc;
-    {
-        const long long total = (long long)n_vert * (p.cb + 1);
-        gather_rows_kernel<<<div_up(total, 256), 256, 0, stream>>>(b.assigned, p.cb + 1, b.perm, b.sassigned, n_vert);
-        HGC_LAUNCH_CHECK();
-        if (use_direction) {
-            gather_rows_kernel<<<div_up(n_vert, 256), 256, 0, stream>>>(d_direction, 1, b.perm, b.sdir, n_vert);
-            HGC_LAUNCH_CHECK();
-        }
-    }
-    if (int rc = launch_select_knn(b.knn, n_coords, b.skeys, b.sassigned, b.bounds, b.grid->n_bins,
-                                   &b.grid->bin_width, use_direction ? b.sdir : nullptr, d_indices, d_dist,
-                                   b.perm, b.perm, n_vert, n_neigh, p.cb, (int)p.max_bins + 1, tf_compat,
-                                   use_direction != 0, ws.status(), stream))
-        return rc;
-    if (d_sorting_out)
-        HGC_CUDA_TRY(cudaMemcpyAsync(d_sorting_out, b.perm, sizeof(int) * (size_t)n_vert,
-                                     cudaMemcpyDeviceToDevice, stream));
     return HGC_OK;
 }

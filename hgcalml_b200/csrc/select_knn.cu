@@ -19,14 +19,14 @@ namespace {
 __device__ unsigned long long g_knn_stats[96];
 #endif
 
-// [n_vert, n_coords] floats (optionally gathered through perm) -> zero-padded float4 records
+// [n_vert, n_coords] floats -> zero-padded float4 records
 __global__ void pack_points_kernel(const float *__restrict__ coords, int n_coords, int nv4,
-                                   const int *__restrict__ perm, float4 *__restrict__ out, int n_vert)
+                                   float4 *__restrict__ out, int n_vert)
 {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)n_vert * nv4) return;
     const int i = (int)(t / nv4), u = (int)(t % nv4);
-    const float *src = coords + (size_t)(perm ? perm[i] : i) * n_coords;
+    const float *src = coords + (size_t)i * n_coords;
     float c[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) c[k] = (u * 4 + k < n_coords) ? src[u * 4 + k] : 0.f;
@@ -66,13 +66,13 @@ chunk_aabb_kernel(const float4 *__restrict__ pts, int nv4, int n_vert, float4 *_
 
 }  // namespace
 
-int pack_points(const float *coords, int n_coords, const int *perm, const KnnScratch &s, int n_vert,
+int pack_points(const float *coords, int n_coords, const KnnScratch &s, int n_vert,
                 cudaStream_t stream)
 {
     if (n_vert <= 0) return HGC_OK;
     const int nv4 = knn_nv4(n_coords);
     const long long total = (long long)n_vert * nv4;
-    pack_points_kernel<<<div_up(total, 256), 256, 0, stream>>>(coords, n_coords, nv4, perm, s.pts, n_vert);
+    pack_points_kernel<<<div_up(total, 256), 256, 0, stream>>>(coords, n_coords, nv4, s.pts, n_vert);
     HGC_LAUNCH_CHECK();
     chunk_aabb_kernel<<<div_up((long long)knn_chunks(n_vert), 8), 256, 0, stream>>>(s.pts, nv4, n_vert,
                                                                                     s.chunk_lo, s.chunk_hi);
@@ -82,8 +82,7 @@ int pack_points(const float *coords, int n_coords, const int *perm, const KnnScr
 
 int launch_select_knn(const KnnScratch &s, int n_coords, const int *bin_idx, const int *dim_bin_idx,
                       const int *bin_boundaries, const int *n_bins, const float *bin_width,
-                      const int *direction, int *out_idx, float *out_dist, const int *row_map,
-                      const int *id_map, int n_vert, int K, int n_bin_dim, int n_bboundaries,
+                      const int *direction, int *out_idx, float *out_dist, int n_vert, int K, int n_bin_dim, int n_bboundaries,
                       int tf_compat, bool use_dir, unsigned *status, cudaStream_t stream)
 {
     if (n_vert <= 0) return HGC_OK;
@@ -91,7 +90,7 @@ int launch_select_knn(const KnnScratch &s, int n_coords, const int *bin_idx, con
     a.pts = s.pts; a.chunk_lo = s.chunk_lo; a.chunk_hi = s.chunk_hi;
     a.bin_idx = bin_idx; a.dim_bin_idx = dim_bin_idx; a.bin_boundaries = bin_boundaries;
     a.n_bins = n_bins; a.bin_width = bin_width; a.direction = direction;
-    a.out_idx = out_idx; a.out_dist = out_dist; a.row_map = row_map; a.id_map = id_map;
+    a.out_idx = out_idx; a.out_dist = out_dist;
     a.n_vert = n_vert; a.K = K; a.n_bboundaries = n_bboundaries; a.tf_compat = tf_compat;
     a.status = status;
     a.work_counter = status + 16;  // inside the 256 zeroed bytes that start every workspace
@@ -171,9 +170,9 @@ extern "C" int hgc_binned_select_knn(
     Carver ws(workspace);
     HGC_CUDA_TRY(cudaMemsetAsync(ws.status(), 0, kAlign, stream));
     const KnnScratch s = knn_scratch_layout(ws, n_vert, n_coords);
-    if (int rc = pack_points(d_coord, n_coords, nullptr, s, n_vert, stream)) return rc;
+    if (int rc = pack_points(d_coord, n_coords, s, n_vert, stream)) return rc;
     return launch_select_knn(s, n_coords, d_bin_idx, d_dim_bin_idx, d_bin_boundaries, d_n_bins,
-                             d_bin_width, d_direction, d_indices, d_dist, nullptr, nullptr, n_vert,
+                             d_bin_width, d_direction, d_indices, d_dist, n_vert,
                              n_neigh, n_bin_dim, n_bboundaries, tf_compat, use_direction != 0,
                              ws.status(), stream);
 }

@@ -16,8 +16,6 @@ struct KnnArgs {
     const int *direction;       // [n_vert] or null
     int *out_idx;               // [n_vert][K]
     float *out_dist;            // [n_vert][K]
-    const int *row_map;         // output row of bin-sorted query i (null: i)
-    const int *id_map;          // output id of bin-sorted hit j (null: j)
     int n_vert, K, n_bboundaries;
     int tf_compat;
     int fetch, blocks_per_sm;   // queries a warp takes at a time; grid size per SM
@@ -49,17 +47,15 @@ inline KnnScratch knn_scratch_layout(W &ws, int n_vert, int n_coords)
     return s;
 }
 
-// coords [n_vert, n_coords] (row perm[i] when perm is given) -> packed float4 records, plus the
+// coords [n_vert, n_coords] -> packed float4 records, plus the
 // bounding boxes of every 32 consecutive records
-int pack_points(const float *coords, int n_coords, const int *perm, const KnnScratch &s, int n_vert,
+int pack_points(const float *coords, int n_coords, const KnnScratch &s, int n_vert,
                 cudaStream_t stream);
 
-// The neighbour search on bin-sorted, packed points.  Row i of the result is written to output
-// row row_map[i] and neighbour ids are translated through id_map (both may be null = identity).
+// The neighbour search on bin-sorted, packed points, in the caller's bins.
 int launch_select_knn(const KnnScratch &s, int n_coords, const int *bin_idx, const int *dim_bin_idx,
                       const int *bin_boundaries, const int *n_bins, const float *bin_width,
-                      const int *direction, int *out_idx, float *out_dist, const int *row_map,
-                      const int *id_map, int n_vert, int K, int n_bin_dim, int n_bboundaries,
+                      const int *direction, int *out_idx, float *out_dist, int n_vert, int K, int n_bin_dim, int n_bboundaries,
                       int tf_compat, bool use_dir, unsigned *status, cudaStream_t stream);
 
 }  // namespace hgc

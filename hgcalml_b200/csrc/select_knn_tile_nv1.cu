@@ -1,0 +1,5 @@
+// Instantiates the tile search for hits of 1 packed float4 record(s).
+#include "select_knn_tile.cuh"
+namespace hgc {
+template int launch_tile_nv<1>(const TileKnnArgs &, int, cudaStream_t);
+}

@@ -1,0 +1,5 @@
+// Instantiates the tile search for hits of 4 packed float4 record(s).
+#include "select_knn_tile.cuh"
+namespace hgc {
+template int launch_tile_nv<4>(const TileKnnArgs &, int, cudaStream_t);
+}

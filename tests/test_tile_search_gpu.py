@@ -1,0 +1,82 @@
+"""The wrapper-level neighbour search (tiles of queries over boxed chunks) against the CPU checker where its
+shapes change: list lengths, chunk / super-chunk / sort-tile remainders, many events, direction, bins that do
+not fit the sort key, lists of chunks that do not fit the tile, and points that coincide."""
+import numpy as np
+import pytest
+
+from conftest import assert_knn_equal
+from hgcalml_b200 import synth
+from test_ops_gpu import T, N
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(cuda, oracle, K, c, rs, direction=None, **kw):
+    from hgcalml_b200.binned_select_knn_op import BinnedSelectKnn
+    d = None if direction is None else T(direction, cuda)
+    gi, gd, sorting = BinnedSelectKnn(K, T(c, cuda), T(rs, cuda), direction=d, return_sorting=True, **kw)
+    ri, rd = oracle.BinnedSelectKnn(K, c, rs, direction=direction, **kw)
+    assert_knn_equal(N(gi), N(gd), ri, rd)
+    assert np.array_equal(np.sort(N(sorting)), np.arange(len(c)))
+    return N(sorting)
+
+
+@pytest.mark.parametrize("K", [1, 2, 32, 33, 34, 64, 65, 66, 129, 257, 513])
+def test_list_lengths(cuda, oracle, K):
+    c, _, rs = synth.shower_batch([1500, 40], dims=4, n_feat=0, seed=11, with_features=False)
+    _check(cuda, oracle, K, c, rs)
+
+
+@pytest.mark.parametrize("dims", [2, 3, 5, 6, 7, 8, 9, 13])
+def test_coordinate_counts(cuda, oracle, dims):
+    c, _, rs = synth.shower_batch([900, 33, 700], dims=dims, with_features=False, seed=dims)
+    _check(cuda, oracle, 17, c, rs)
+
+
+@pytest.mark.parametrize("sizes", [[31], [32], [33, 1, 0, 31], [1023, 1025], [1024], [2047, 2049, 2048, 5], [4097]])
+def test_event_sizes(cuda, oracle, sizes):
+    c, _, rs = synth.shower_batch(sizes, dims=3, with_features=False, seed=len(sizes))
+    _check(cuda, oracle, 20, c, rs)
+
+
+def test_many_small_events(cuda, oracle):
+    sizes = np.random.default_rng(5).integers(0, 25, 700)
+    rng = np.random.default_rng(6)
+    rs = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
+    _check(cuda, oracle, 12, rng.random((int(rs[-1]), 3), dtype=np.float32), rs)
+
+
+@pytest.mark.parametrize("kw", [dict(n_bins=80), dict(n_bins=12, max_bin_dims=5), dict(n_bins=39, max_bin_dims=3)])
+def test_bins_beyond_the_sort_key(cuda, oracle, kw):
+    c, _, rs = synth.shower_batch([3000, 500], dims=5, with_features=False, seed=9)
+    sorting = _check(cuda, oracle, 10, c, rs, **kw)
+    assert np.array_equal(np.sort(sorting[:3000]), np.arange(3000))  # events stay together
+
+
+def test_sorting_is_by_bin(cuda, oracle):
+    from hgcalml_b200.bin_by_coordinates_op import BinByCoordinates
+    c, _, rs = synth.shower_batch([5000, 70, 2500], dims=4, with_features=False, seed=19)
+    sorting = _check(cuda, oracle, 8, c, rs, n_bins=9)
+    _, flat, _, _, _ = BinByCoordinates(T(c[:, :3], cuda), T(rs, cuda), n_bins=9)
+    assert (np.diff(N(flat)[sorting]) >= 0).all()
+
+
+def test_direction_over_chunks(cuda, oracle):
+    c, _, rs = synth.shower_batch([2100, 64], dims=4, with_features=False, seed=23)
+    d = np.random.default_rng(24).integers(0, 4, len(c)).astype(np.int32)
+    d[:1200] = 1  # whole chunks without a possible neighbour
+    _check(cuda, oracle, 25, c, rs, direction=d)
+
+
+def test_more_chunks_than_the_list_holds(cuda, oracle):
+    rng = np.random.default_rng(31)
+    c = rng.random((36000, 6), dtype=np.float32)
+    _check(cuda, oracle, 40, c, np.array([0, 36000], np.int32))
+
+
+@pytest.mark.parametrize("K", [16, 64])
+def test_coinciding_points(cuda, oracle, K):
+    rng = np.random.default_rng(41)
+    c = rng.integers(0, 3, (2500, 3)).astype(np.float32)
+    c[:400] = 1.5
+    _check(cuda, oracle, K, c, np.array([0, 1300, 2500], np.int32))
