@@ -62,7 +62,9 @@ def collect_neighbours(features, neighbour_indices, distancesq, *, first_slot: i
             out_column < 0 or out_column + 2 * f > out.shape[1]:
         raise C.HgcError("collect_neighbours: out must be a row-major float32 [N, >= out_column + 2F] buffer")
     maxidx = torch.empty((n, f), dtype=torch.int32, device=feat.device) if with_max_idxs else None
-    if order is not None:
+    if order is None:
+        order = C.order_of(neighbour_indices, n)
+    else:
         C.require_cuda(order)
         order = C.i32(order)
     view = out[:, out_column:out_column + 2 * f]

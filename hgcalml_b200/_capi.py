@@ -44,6 +44,7 @@ def _load():
         "hgc_binned_select_knn_static_status": (I, [P, ctypes.POINTER(ctypes.c_uint)]),
         "hgc_index_replacer": (I, [P, P, P, I, I, P, P]),
         "hgc_accumulate_knn": (I, [P] * 5 + [I] * 6 + [P]),
+        "hgc_accumulate_knn_ordered": (I, [P] * 5 + [I] * 6 + [P, P]),
         "hgc_accumulate_knn_exp": (I, [P] * 5 + [I] * 5 + [ctypes.c_float, P, P]),
         "hgc_gravnet_collect": (I, [P, P, I, I, I, P, P, I, P, I, I, ctypes.c_float, I, P, P]),
         "hgc_binned_select_knn_ragged_workspace_bytes": (S, [I] * 6),
@@ -52,11 +53,14 @@ def _load():
         "hgc_build_and_assign_condensates": (I, [P] * 11 + [I] * 3 + [ctypes.c_float] * 2 + [I] * 2 + [P, S, P]),
         "hgc_local_distance": (I, [P, P, P, I, I, I, I, P]),
         "hgc_push_knn": (I, [P, P, P, P, I, I, I, P, S, P]),
+        "hgc_push_knn_ordered": (I, [P, P, P, P, I, I, I, P, P, S, P]),
         "hgc_push_knn_grad": (I, [P] * 6 + [I] * 3 + [P]),
+        "hgc_push_knn_grad_ordered": (I, [P] * 6 + [I] * 3 + [P, P]),
         "hgc_knn_grad_workspace_bytes": (S, [I, I]),
         "hgc_accumulate_knn_grad": (I, [P] * 7 + [I] * 6 + [P, S, P]),
         "hgc_accumulate_knn_grad_ordered": (I, [P] * 7 + [I] * 6 + [P, P, S, P]),
         "hgc_select_knn_grad": (I, [P] * 5 + [I] * 3 + [P, S, P]),
+        "hgc_select_knn_grad_ordered": (I, [P] * 5 + [I] * 3 + [P, P, S, P]),
         "hgc_binned_assign_to_condensates_workspace_bytes": (S, [I] * 4),
         "hgc_binned_assign_to_condensates": (I, [I, I] + [P] * 4 + [P] + [P] * 2 + [P] * 4 + [P] * 4 + [P] * 3
                                              + [P, I, I, I, I] + [P, S, P]),
@@ -82,19 +86,22 @@ def check(rc: int, what: str) -> None:
 
 def ptr(t):
     """Device pointer of a tensor (None -> NULL)."""
-    if t is None:
-        return None
-    return c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
+
+
+_raw_stream = torch._C._cuda_getCurrentRawStream if hasattr(torch._C, "_cuda_getCurrentRawStream") else \
+    lambda index: torch.cuda.current_stream(index).cuda_stream
 
 
 def stream_of(t: torch.Tensor):
     """The current stream of the tensor's device.  The library launches on the calling thread's
     current device, so that device must be the tensor's."""
-    if t.device.index is not None and t.device.index != torch.cuda.current_device():
+    index = t.get_device()
+    if index != torch.cuda.current_device():
         raise HgcError(f"tensors live on {t.device} but the current CUDA device is "
                        f"cuda:{torch.cuda.current_device()}: call torch.cuda.set_device (or use "
                        "torch.cuda.device) before calling hgcalml_b200 ops")
-    return c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+    return _raw_stream(index)
 
 
 def workspace(nbytes: int, device) -> torch.Tensor:
@@ -113,14 +120,33 @@ def read_status(ws: torch.Tensor, raise_on_flag: bool = True) -> int:
     return out.value
 
 
+def _as(t, dtype, device):
+    # the usual argument is a dense tensor of the right type and needs no call into torch
+    if isinstance(t, torch.Tensor) and t.dtype is dtype and t.is_contiguous() and (device is None or t.device == device):
+        return t
+    return torch.as_tensor(t, device=device).to(dtype).contiguous()
+
+
 def f32(t, device=None):
-    t = torch.as_tensor(t, device=device)
-    return t.to(torch.float32).contiguous()
+    return _as(t, torch.float32, device)
 
 
 def i32(t, device=None):
-    t = torch.as_tensor(t, device=device)
-    return t.to(torch.int32).contiguous()
+    return _as(t, torch.int32, device)
+
+
+def set_order(idx: torch.Tensor, order: torch.Tensor):
+    """Notes with a neighbour table the order in which its rows are best processed (the search's sorting of the
+    hits).  Ops that gather or scatter along the table look it up when the caller names no order; results do
+    not depend on it, and a table without one (a slice, a copy) is processed row by row."""
+    idx._hgc_order = order
+
+
+def order_of(idx, n: int):
+    order = getattr(idx, "_hgc_order", None)
+    if order is None or order.shape[0] != n or idx.shape[0] != n or order.device != idx.device:
+        return None
+    return order
 
 
 def require_cuda(*tensors):

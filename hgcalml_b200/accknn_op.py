@@ -26,15 +26,24 @@ def _prepare(weights, features, indices, mean_and_max, with_max_idxs):
     return weights, features, indices, out, maxidx, n, k, f, n_out
 
 
-def AccumulateLinKnn(weights, features, indices, mean_and_max=True, force_tf=False, with_max_idxs=True):
+def _order(order, indices, n):
+    """The processing order the caller names, else the one noted with the neighbour table, if any."""
+    if order is None:
+        return C.order_of(indices, n)
+    C.require_cuda(order)
+    return C.i32(order)
+
+
+def AccumulateLinKnn(weights, features, indices, mean_and_max=True, force_tf=False, with_max_idxs=True, order=None):
     """Accumulates neighbour features with linear weights: the registered op ``AccumulateKnn``
     as is (modules/accknn_op.py:17-36, modules/compiled/accumulate_knn_module.cc:7-14).
     Returns ``(out_features [N, 2F or F], out_max_idxs [N, F])``."""
     del force_tf
     w, feat, idx, out, maxidx, n, k, f, n_out = _prepare(weights, features, indices, mean_and_max,
                                                         with_max_idxs)
-    C.check(C.lib.hgc_accumulate_knn(C.ptr(w), C.ptr(feat), C.ptr(idx), C.ptr(out), C.ptr(maxidx),
-                                     n, k, f, n_out, 0, int(bool(mean_and_max)), C.stream_of(feat)),
+    C.check(C.lib.hgc_accumulate_knn_ordered(C.ptr(w), C.ptr(feat), C.ptr(idx), C.ptr(out), C.ptr(maxidx),
+                                             n, k, f, n_out, 0, int(bool(mean_and_max)),
+                                             C.ptr(_order(order, indices, n)), C.stream_of(feat)),
             "AccumulateKnn")
     return out, maxidx
 
@@ -51,9 +60,7 @@ def AccumulateKnn(distances, features, indices, mean_and_max=True, force_tf=Fals
     del force_tf
     d, feat, idx, out, maxidx, n, k, f, n_out = _prepare(distances, features, indices, mean_and_max,
                                                         with_max_idxs)
-    if order is not None:
-        C.require_cuda(order)
-        order = C.i32(order)
+    order = _order(order, indices, n)
     C.check(C.lib.hgc_accumulate_knn_exp(C.ptr(d), C.ptr(feat), C.ptr(idx), C.ptr(out), C.ptr(maxidx),
                                          n, k, f, n_out, int(bool(mean_and_max)), float(distance_scale),
                                          C.ptr(order),
@@ -83,9 +90,7 @@ def AccumulateKnnGrad(grad_from_out_features, distances, features, neigh_indices
     gw = torch.empty((n, k), dtype=torch.float32, device=dev)
     gf = torch.empty((n, f), dtype=torch.float32, device=dev)
     ws = C.workspace(C.lib.hgc_knn_grad_workspace_bytes(n, k), dev)
-    if order is not None:
-        C.require_cuda(order)
-        order = C.i32(order)
+    order = _order(order, neigh_indices, n)
     C.check(C.lib.hgc_accumulate_knn_grad_ordered(C.ptr(g), C.ptr(w), C.ptr(feat), C.ptr(maxidx), C.ptr(idx),
                                                   C.ptr(gw), C.ptr(gf), n, k, f, g.shape[1], 0, int(mean_and_max),
                                                   C.ptr(order), C.ptr(ws), ws.numel(), C.stream_of(feat)),
@@ -98,16 +103,20 @@ class _AccumulateLinKnnFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, weights, features, indices, mean_and_max, order):
-        out, maxidx = AccumulateLinKnn(weights, features, indices, mean_and_max=mean_and_max)
+        order = _order(order, indices, indices.shape[0])
+        out, maxidx = AccumulateLinKnn(weights, features, indices, mean_and_max=mean_and_max, order=order)
         ctx.save_for_backward(weights, features, indices, maxidx)
         ctx.order = order
         ctx.mark_non_differentiable(maxidx)
+        ctx.set_materialize_grads(False)  # no zeros for the arg-max output
         return out, maxidx
 
     @staticmethod
     def backward(ctx, grad_out, _grad_maxidx):
+        if grad_out is None:
+            return None, None, None, None, None
         weights, features, indices, maxidx = ctx.saved_tensors
-        gw, gf = AccumulateKnnGrad(grad_out.contiguous(), weights, features, indices, maxidx, order=ctx.order)
+        gw, gf = AccumulateKnnGrad(grad_out, weights, features, indices, maxidx, order=ctx.order)
         return gw, gf, None, None, None
 
 

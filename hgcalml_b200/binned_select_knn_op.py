@@ -69,7 +69,7 @@ def BinnedSelectKnn(K: int, coords, row_splits, direction=None, n_bins=None, max
     dev = coords.device
     idx = torch.empty((n, K), dtype=torch.int32, device=dev)
     dist = torch.empty((n, K), dtype=torch.float32, device=dev)
-    sorting = torch.empty((n,), dtype=torch.int32, device=dev) if return_sorting else None
+    sorting = torch.empty((n,), dtype=torch.int32, device=dev)
     nbytes = C.lib.hgc_binned_select_knn_ragged_workspace_bytes(n, K, c, n_rs, nb, max_bin_dims)
     if nbytes == 0:
         raise C.HgcError("BinnedSelectKnn: unsupported combination of sizes")
@@ -78,24 +78,27 @@ def BinnedSelectKnn(K: int, coords, row_splits, direction=None, n_bins=None, max
         C.ptr(coords), C.ptr(row_splits), C.ptr(direction), C.ptr(idx), C.ptr(dist), C.ptr(sorting),
         n, K, c, n_rs, nb, int(max_bin_dims), int(bool(tf_compatible)), int(use_direction),
         C.ptr(ws), ws.numel(), C.stream_of(coords)), "BinnedSelectKnn")
+    C.set_order(idx, sorting)
     if return_sorting:
         return idx, dist, sorting
     return idx, dist
 
 
-def SelectKnnGrad(grad_distances, indices, distances, coordinates):
+def SelectKnnGrad(grad_distances, indices, distances, coordinates, order=None):
     """The registered op ``SelectKnnGrad`` (modules/compiled/select_knn_grad_module.cc), which the
     reference attaches as the gradient of ``BinnedSelectKnn`` (modules/binned_select_knn_op.py:107-118):
-    gradient of the squared neighbour distances with respect to the coordinates, ``[N, C]``."""
+    gradient of the squared neighbour distances with respect to the coordinates, ``[N, C]``.
+    ``order`` (optional int32 permutation of the hits) only sets the order in which hits are processed."""
     C.require_cuda(grad_distances, indices, coordinates)
     g, idx, coords = C.f32(grad_distances), C.i32(indices), C.f32(coordinates)
     d = None if distances is None else C.f32(distances)
     n, k = idx.shape
     out = torch.empty_like(coords)
     ws = C.workspace(C.lib.hgc_knn_grad_workspace_bytes(n, k), coords.device)
-    C.check(C.lib.hgc_select_knn_grad(C.ptr(g), C.ptr(idx), C.ptr(d), C.ptr(coords), C.ptr(out),
-                                      n, k, coords.shape[1], C.ptr(ws), ws.numel(), C.stream_of(coords)),
-            "SelectKnnGrad")
+    order = C.order_of(indices, n) if order is None else C.i32(order)
+    C.check(C.lib.hgc_select_knn_grad_ordered(C.ptr(g), C.ptr(idx), C.ptr(d), C.ptr(coords), C.ptr(out),
+                                              n, k, coords.shape[1], C.ptr(order), C.ptr(ws), ws.numel(),
+                                              C.stream_of(coords)), "SelectKnnGrad")
     return out
 
 
@@ -105,13 +108,17 @@ class _BinnedSelectKnnFunction(torch.autograd.Function):
         idx, dist = BinnedSelectKnn(K, coords, row_splits, n_bins=n_bins, max_bin_dims=max_bin_dims,
                                     tf_compatible=tf_compatible)
         ctx.save_for_backward(coords, idx, dist)
+        ctx.order = C.order_of(idx, idx.shape[0])
         ctx.mark_non_differentiable(idx)
+        ctx.set_materialize_grads(False)  # no zeros for the index output
         return idx, dist
 
     @staticmethod
     def backward(ctx, _grad_idx, grad_dist):
+        if grad_dist is None:
+            return None, None, None, None, None, None
         coords, idx, dist = ctx.saved_tensors
-        return SelectKnnGrad(grad_dist.contiguous(), idx, dist, coords), None, None, None, None, None
+        return SelectKnnGrad(grad_dist, idx, dist, coords, order=ctx.order), None, None, None, None, None
 
 
 def BinnedSelectKnnDifferentiable(K, coords, row_splits, n_bins=None, max_bin_dims=3, tf_compatible=False):

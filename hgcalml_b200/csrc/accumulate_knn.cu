@@ -383,10 +383,20 @@ extern "C" int hgc_accumulate_knn(
         int n_vert, int n_neigh, int n_feat, int n_out_feat, int n_moments, int mean_and_max,
         hgc_stream_t stream)
 {
+    return hgc_accumulate_knn_ordered(d_weights, d_feat, d_idxs, d_out_feat, d_out_maxidxs, n_vert, n_neigh, n_feat,
+                                      n_out_feat, n_moments, mean_and_max, nullptr, stream);
+}
+
+extern "C" int hgc_accumulate_knn_ordered(
+        const float *d_weights, const float *d_feat, const int *d_idxs,
+        float *d_out_feat, int *d_out_maxidxs,
+        int n_vert, int n_neigh, int n_feat, int n_out_feat, int n_moments, int mean_and_max,
+        const int *d_order, hgc_stream_t stream)
+{
     (void)n_moments;  // read and ignored by the reference too (accumulate_knn_kernel.cc:44)
     if (n_out_feat != (mean_and_max ? 2 * n_feat : n_feat)) return HGC_ERR_INVALID_ARGUMENT;
     return hgc::accumulate_dispatch(false, d_weights, d_feat, d_idxs, d_out_feat, d_out_maxidxs, n_vert,
-                                    n_neigh, n_neigh, n_feat, n_out_feat, mean_and_max, nullptr, 1.f, false,
+                                    n_neigh, n_neigh, n_feat, n_out_feat, mean_and_max, d_order, 1.f, false,
                                     static_cast<cudaStream_t>(stream));
 }
 

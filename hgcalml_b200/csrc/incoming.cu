@@ -1,0 +1,166 @@
+// Transposition of the neighbour table: a counting sort of the edges by target.
+//
+// Targets are counted with integer atomics, which also hand every edge a place in its target's list; a prefix sum
+// gives the lists their room, the edges are written to their places, and every list is then sorted by edge id,
+// which takes out the order in which the atomics happened: the result is the same on every run.  Lists hold about
+// as many edges as a hit has neighbours, so a warp sorts one in registers; lists of more than 128 edges go to a
+// block of their own.
+//
+// 12.8 M edges (200k hits, K = 64): 0.25 ms, against 0.75 ms with three passes of the stable radix sort over
+// (target, edge) pairs and a search for the list bounds, and 7 launches instead of 17.  Bound by the scattered
+// accesses to L2 (one atomic and one 4-byte write per edge).
+#include "incoming.cuh"
+#include "knn_device.cuh"
+
+namespace hgc {
+namespace {
+
+__global__ void __launch_bounds__(256)
+count_targets_kernel(const int *__restrict__ nidx, long long n_edges, int n_vert, int *__restrict__ count,
+                     int *__restrict__ place)
+{
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n_edges) return;
+    const int m = nidx[e];
+    if (m >= 0 && m < n_vert) place[e] = atomicAdd(count + m, 1);  // others belong to no list
+}
+
+__global__ void __launch_bounds__(256)
+place_edges_kernel(const int *__restrict__ nidx, const int *__restrict__ place, long long n_edges, int n_vert,
+                   const int *__restrict__ bounds, int *__restrict__ edges)
+{
+    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n_edges) return;
+    const int m = nidx[e];
+    if (m >= 0 && m < n_vert) edges[bounds[m] + place[e]] = (int)e;
+}
+
+// Sorts 32 * R ids held by a warp (striped) and writes back the first n.
+template <int R>
+__device__ __forceinline__ void sort_list(int *list, int n, int lane)
+{
+    unsigned v[R];
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        v[r] = warp_sort_u32(r * 32 + lane < n ? (unsigned)list[r * 32 + lane] : 0xffffffffu, lane);
+    // merge runs of 1, then 2 registers: compare with the mirrored run, then clean both bitonic halves
+#pragma unroll
+    for (int m = 1; m < R; m <<= 1)
+#pragma unroll
+        for (int g = 0; g < R; g += 2 * m) {
+#pragma unroll
+            for (int i = 0; i < m; i++) {
+                const unsigned lo = v[g + i], hi = __shfl_xor_sync(0xffffffffu, v[g + 2 * m - 1 - i], 31);
+                v[g + i] = min(lo, hi);
+                v[g + 2 * m - 1 - i] = __shfl_xor_sync(0xffffffffu, max(lo, hi), 31);
+            }
+            if (m == 2)
+#pragma unroll
+                for (int h = 0; h < 4; h += 2) {
+                    const unsigned lo = v[g + h], hi = v[g + h + 1];
+                    v[g + h] = min(lo, hi);
+                    v[g + h + 1] = max(lo, hi);
+                }
+#pragma unroll
+            for (int i = 0; i < 2 * m; i++) v[g + i] = warp_bitonic_merge_u32(v[g + i], lane);
+        }
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        if (r * 32 + lane < n) list[r * 32 + lane] = (int)v[r];
+}
+
+__global__ void __launch_bounds__(256)
+sort_lists_kernel(const int *__restrict__ bounds, int *__restrict__ edges, int n_vert, int *__restrict__ long_lists)
+{
+    const int m = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (m >= n_vert) return;
+    const int begin = bounds[m], n = bounds[m + 1] - begin;
+    if (n <= 1) return;
+    if (n <= 32) sort_list<1>(edges + begin, n, lane);
+    else if (n <= 64) sort_list<2>(edges + begin, n, lane);
+    else if (n <= 128) sort_list<4>(edges + begin, n, lane);
+    else if (lane == 0) long_lists[1 + atomicAdd(long_lists, 1)] = m;
+}
+
+// Lists of more than 128 edges: a block per list, radix sort of 8-bit digits through global memory.
+__global__ void __launch_bounds__(256)
+sort_long_lists_kernel(const int *__restrict__ bounds, int *edges, int *tmp, const int *__restrict__ long_lists,
+                       int n_passes)
+{
+    __shared__ int s_run[256], s_count[8][256], s_warp[8];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int n_long = long_lists[0];
+    for (int l = blockIdx.x; l < n_long; l += gridDim.x) {
+        const int m = long_lists[1 + l], begin = bounds[m], n = bounds[m + 1] - begin;
+        int *src = edges + begin, *dst = tmp + begin;
+        for (int p = 0; p < n_passes; p++) {
+            const int shift = 8 * p;
+            __syncthreads();
+            s_run[t] = 0;
+            __syncthreads();
+            for (int i = t; i < n; i += 256) atomicAdd(&s_run[(src[i] >> shift) & 255], 1);
+            __syncthreads();
+            const int c = s_run[t];
+            int incl = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            if (lane == 31) s_warp[warp] = incl;
+            __syncthreads();
+            for (int w = 0; w < warp; w++) incl += s_warp[w];
+            s_run[t] = incl - c;
+            // 256 ids at a time, warp by warp in order
+            for (int base = 0; base < n; base += 256) {
+                for (int w = 0; w < 8; w++) s_count[w][t] = 0;
+                __syncthreads();
+                const bool ok = base + t < n;
+                const int id = ok ? src[base + t] : 0;
+                const unsigned dg = ok ? (unsigned)(id >> shift) & 255u : 256u;
+                const unsigned peers = __match_any_sync(0xffffffffu, dg), before = peers & ((1u << lane) - 1u);
+                if (ok && before == 0u) s_count[warp][dg] = __popc(peers);
+                __syncthreads();
+                int run = s_run[t];
+                for (int w = 0; w < 8; w++) {
+                    const int k = s_count[w][t];
+                    s_count[w][t] = run;
+                    run += k;
+                }
+                s_run[t] = run;
+                __syncthreads();
+                if (ok) dst[s_count[warp][dg] + __popc(before)] = id;
+                __syncthreads();
+            }
+            int *x = src; src = dst; dst = x;
+        }
+        if (n_passes & 1)
+            for (int i = t; i < n; i += 256) edges[begin + i] = tmp[begin + i];
+    }
+}
+
+}  // namespace
+
+int build_incoming(const int *nidx, int n_vert, int n_neigh, const Incoming &b, unsigned *status, cudaStream_t stream)
+{
+    const long long ne = (long long)n_vert * n_neigh;
+    // the status word, the counts (bounds) and the number of long lists lie one after another
+    HGC_CUDA_TRY(cudaMemsetAsync(status, 0, (size_t)(reinterpret_cast<char *>(b.long_lists + 1) - reinterpret_cast<char *>(status)), stream));
+    count_targets_kernel<<<div_up(ne, 256), 256, 0, stream>>>(nidx, ne, n_vert, b.bounds, b.place);
+    HGC_LAUNCH_CHECK();
+    if (int rc = exclusive_scan_ints(b.bounds, n_vert + 1, b.scan, stream)) return rc;
+    place_edges_kernel<<<div_up(ne, 256), 256, 0, stream>>>(nidx, b.place, ne, n_vert, b.bounds, b.edges);
+    HGC_LAUNCH_CHECK();
+    sort_lists_kernel<<<div_up(n_vert, 8), 256, 0, stream>>>(b.bounds, b.edges, n_vert, b.long_lists);
+    HGC_LAUNCH_CHECK();
+    if (ne > 128) {
+        int blocks = sm_count();
+        if (blocks > ne / 129) blocks = (int)(ne / 129);
+        if (blocks < 1) blocks = 1;
+        sort_long_lists_kernel<<<blocks, 256, 0, stream>>>(b.bounds, b.edges, b.place, b.long_lists, (bits_for(ne) + 7) / 8);
+        HGC_LAUNCH_CHECK();
+    }
+    return HGC_OK;
+}
+
+}  // namespace hgc

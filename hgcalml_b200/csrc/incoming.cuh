@@ -1,27 +1,31 @@
 // Transposed neighbour lists: for every hit, the (hit, slot) edges that point at it, in ascending
-// (hit, slot) order.  Built with the stable counting sort, used by the ops that push values from a
-// hit to its neighbours (backward ops, PushKnn) so that they need no atomics.
+// (hit, slot) order.  Used by the ops that push values from a hit to its neighbours (backward ops,
+// PushKnn) so that they need no floating-point atomics and sum in a fixed order.
 #pragma once
 #include "common.cuh"
 
 namespace hgc {
 
 struct Incoming {
-    int *keys, *skeys, *sedges, *tkeys, *tvals, *hist, *bounds;
+    int *bounds;          // [n_vert + 2] incoming edges of hit m are edges[bounds[m] .. bounds[m + 1])
+    int *long_lists;      // [1 + n_edges / 129 + 1] number of hits with more than 128 incoming edges, and the hits
+    int *scan;            // scratch of the prefix sum
+    int *edges;           // [n_edges] edge ids e = hit * n_neigh + slot
+    int *place;           // [n_edges] place of an edge in its target's list; scratch of the long sort afterwards
+    unsigned *flags;      // [n_edges][2] scratch of the op: one bit per feature of a slab of 64
 };
 
 template <typename W>
 Incoming incoming_layout(W &ws, int n_vert, int n_neigh)
 {
-    const size_t ne = (size_t)(n_vert > 0 ? n_vert : 0) * (size_t)(n_neigh > 0 ? n_neigh : 0);
+    const size_t n = n_vert > 0 ? n_vert : 0, ne = n * (size_t)(n_neigh > 0 ? n_neigh : 0);
     Incoming b;
-    b.keys = ws.template take<int>(ne);
-    b.skeys = ws.template take<int>(ne);
-    b.sedges = ws.template take<int>(ne);
-    b.tkeys = ws.template take<int>(ne);
-    b.tvals = ws.template take<int>(ne);
-    b.hist = ws.template take<int>(sort_hist_ints((int)ne));
-    b.bounds = ws.template take<int>((size_t)(n_vert > 0 ? n_vert : 0) + 2);
+    b.bounds = ws.template take<int>(n + 2);  // first, with long_lists: one memset clears both and the status word
+    b.long_lists = ws.template take<int>(ne / 129 + 2);
+    b.scan = ws.template take<int>(scan_scratch_ints((int)n + 1));
+    b.edges = ws.template take<int>(ne);
+    b.place = ws.template take<int>(ne);
+    b.flags = ws.template take<unsigned>(2 * ne);
     return b;
 }
 
@@ -30,8 +34,7 @@ struct IncomingSizer {
     template <typename T> T *take(size_t n) { s.take<T>(n); return nullptr; }
 };
 
-// bounds[m] .. bounds[m+1]: positions in sedges of the edges whose neighbour is hit m; sedges holds
-// edge ids e = hit * n_neigh + slot.
-int build_incoming(const int *nidx, int n_vert, int n_neigh, const Incoming &b, cudaStream_t stream);
+// Builds the lists; also clears the workspace's status word.
+int build_incoming(const int *nidx, int n_vert, int n_neigh, const Incoming &b, unsigned *status, cudaStream_t stream);
 
 }  // namespace hgc

@@ -4,8 +4,7 @@
 //   1. digit_count_kernel   : every block counts the digits of its tile (per-warp counters,
 //                             warp peers found with __match_any_sync, no atomics)
 //   2. scan_*_kernel        : exclusive scan of the [digit][block] table (digit-major, so a
-//                             digit's blocks are contiguous and block order = input order);
-//                             long tables are scanned tile-wise by many blocks
+//                             digit's blocks are contiguous and block order = input order)
 //   3. digit_scatter_kernel : every block recomputes the rank of each item inside its
 //                             (warp, digit) run and scatters to its final place.
 // A warp owns a contiguous run of its block's tile and walks it 32 items at a time, so equal
@@ -57,46 +56,8 @@ digit_count_kernel(const int *__restrict__ keys, int n_max, const int *__restric
     block_hist[(size_t)dg * n_blocks + blockIdx.x] = total;
 }
 
-// Single-block exclusive scan over `len` ints, in place.
-__global__ void __launch_bounds__(1024) scan_hist_kernel(int *__restrict__ data, int len)
-{
-    __shared__ int warp_sums[32];
-    __shared__ int carry_s;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) carry_s = 0;
-    __syncthreads();
-    for (int base = 0; base < len; base += 1024) {
-        const int i = base + threadIdx.x;
-        const int v = i < len ? data[i] : 0;
-        int incl = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
-        }
-        if (lane == 31) warp_sums[warp] = incl;
-        __syncthreads();
-        if (warp == 0) {
-            int s = warp_sums[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, s, o);
-                if (lane >= o) s += t;
-            }
-            warp_sums[lane] = s;  // inclusive over warps
-        }
-        __syncthreads();
-        const int carry = carry_s;
-        const int warp_excl = warp == 0 ? 0 : warp_sums[warp - 1];
-        if (i < len) data[i] = carry + warp_excl + incl - v;
-        __syncthreads();
-        if (threadIdx.x == 1023) carry_s = carry + warp_excl + incl;
-        __syncthreads();
-    }
-}
-
-// Exclusive scan of a long table in three steps: every block scans its own tile of kScanTile ints
-// and records the tile total, one block scans the totals (scan_hist_kernel), the totals are added back.
+// Exclusive scan in two steps: every block scans its own tile of kScanTile ints and records the tile total,
+// then the totals of the tiles before are added to every tile.
 constexpr int kScanTile = 4096;
 
 __global__ void __launch_bounds__(1024) scan_tiles_kernel(int *__restrict__ data, int len, int *__restrict__ tile_sums)
@@ -135,10 +96,23 @@ __global__ void __launch_bounds__(1024) scan_tiles_kernel(int *__restrict__ data
     if (threadIdx.x == 1023) tile_sums[blockIdx.x] = warp_sums[31];
 }
 
-__global__ void add_tile_offsets_kernel(int *__restrict__ data, int len, const int *__restrict__ tile_sums)
+// Adds the sum of the tiles before its own to every entry of a block's tile: a block adds those totals up itself,
+// which for a few thousand tiles costs less than a launch that scans them.
+__global__ void __launch_bounds__(1024) add_tile_offsets_kernel(int *__restrict__ data, int len,
+                                                                const int *__restrict__ tile_sums)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < len) data[i] += tile_sums[i / kScanTile];
+    __shared__ int warp_sums[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int sum = 0;
+    for (int t = threadIdx.x; t < (int)blockIdx.x; t += 1024) sum += tile_sums[t];
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) warp_sums[warp] = sum;
+    __syncthreads();
+    sum = __reduce_add_sync(0xffffffffu, warp_sums[lane]);
+    const int base = blockIdx.x * kScanTile + threadIdx.x;
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        if (base + q * 1024 < len) data[base + q * 1024] += sum;
 }
 
 __global__ void __launch_bounds__(kSortThreads)
@@ -233,18 +207,13 @@ size_t scan_scratch_ints(int len) { return (size_t)div_up(len > 0 ? len : 1, kSc
 int exclusive_scan_ints(int *data, int len, int *tile_sums, cudaStream_t stream)
 {
     if (len <= 0) return HGC_OK;
-    if (len <= 4 * kScanTile) {
-        scan_hist_kernel<<<1, 1024, 0, stream>>>(data, len);
-        HGC_LAUNCH_CHECK();
-        return HGC_OK;
-    }
     const int n_tiles = div_up(len, kScanTile);
     scan_tiles_kernel<<<n_tiles, 1024, 0, stream>>>(data, len, tile_sums);
     HGC_LAUNCH_CHECK();
-    scan_hist_kernel<<<1, 1024, 0, stream>>>(tile_sums, n_tiles);
-    HGC_LAUNCH_CHECK();
-    add_tile_offsets_kernel<<<div_up(len, 256), 256, 0, stream>>>(data, len, tile_sums);
-    HGC_LAUNCH_CHECK();
+    if (n_tiles > 1) {
+        add_tile_offsets_kernel<<<n_tiles, 1024, 0, stream>>>(data, len, tile_sums);
+        HGC_LAUNCH_CHECK();
+    }
     return HGC_OK;
 }
 

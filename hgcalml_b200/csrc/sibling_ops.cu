@@ -1,6 +1,7 @@
 // Two small ops that live on the same neighbour tables as the main path and are used by the
 // graph-condensation layers: LocalDistance and PushKnn.
 #include "common.cuh"
+#include "edge_kernels.cuh"
 #include "incoming.cuh"
 
 namespace hgc {
@@ -25,65 +26,48 @@ __global__ void local_distance_kernel(const int *__restrict__ nidx, const float 
     dist[e] = s;
 }
 
-// out[m,f] = sum over the edges (i,k) that point at m, in (i,k) order, of feat[i,f] * w[i,k]
-// (modules/compiled/push_knn_kernel.cc:35-71; the reference's GPU kernel scatters with atomicAdd,
-// push_knn_kernel.cu.cc:61).  One warp per target hit, lanes over the features.
-__global__ void __launch_bounds__(256)
-push_knn_kernel(const float *__restrict__ weights, const float *__restrict__ feat,
-                const int *__restrict__ bounds, const int *__restrict__ sedges, float *__restrict__ out,
-                int n_vert, int K, int F)
-{
-    const int lane = threadIdx.x & 31;
-    const int m = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (m >= n_vert) return;
-    const int e_begin = bounds[m], e_end = bounds[m + 1];
-    for (int f = lane; f < F; f += 32) {
-        float acc = 0.f;
-        for (int p = e_begin; p < e_end; p++) {
-            const int e = sedges[p];
-            const int i = e / K;
-            acc = __fadd_rn(acc, __fmul_rn(feat[(size_t)i * F + f], weights[e]));
-        }
-        out[(size_t)m * F + f] = acc;
-    }
-}
-
-// PushKnnGrad (modules/compiled/push_knn_grad_kernel.cc:22-95): both parts are gathers.
+// PushKnnGrad (modules/compiled/push_knn_grad_kernel.cc:22-95): both parts are gathers.  The part w.r.t. the weights,
+// w_grad[i,k] = sum_f grad[m_k,f] * feat[i,f] with f in order, is edge_dot_kernel.
 // feat_grad[i,f] = sum_k grad[m_k,f] * w[i,k]: one warp per hit, lanes over the features, k in order.
+// Lanes fetch 32 slots with their weights, then the rows of 8 neighbours are requested together.
 __global__ void __launch_bounds__(256)
 push_grad_features_kernel(const float *__restrict__ grad, const float *__restrict__ weights,
-                          const int *__restrict__ nidx, float *__restrict__ feat_grad, int n_vert, int K, int F)
+                          const int *__restrict__ nidx, float *__restrict__ feat_grad, int n_vert, int K, int F,
+                          const int *__restrict__ order)
 {
+    constexpr int U = 8;
     const int lane = threadIdx.x & 31;
-    const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (i >= n_vert) return;
-    for (int f = lane; f < F; f += 32) {
+    const int slot = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (slot >= n_vert) return;
+    const int i = order ? order[slot] : slot;  // processing order only
+    for (int f0 = 0; f0 < F; f0 += 32) {
+        const bool in = f0 + lane < F;
         float acc = 0.f;
-        for (int k = 0; k < K; k++) {
-            const int m = nidx[(size_t)i * K + k];
-            if (m < 0 || m >= n_vert) continue;
-            acc = __fadd_rn(acc, __fmul_rn(grad[(size_t)m * F + f], weights[(size_t)i * K + k]));
+        for (int k0 = 0; k0 < K; k0 += 32) {
+            int my_m = -1;
+            float my_w = 0.f;
+            if (k0 + lane < K) {
+                my_m = nidx[(size_t)i * K + k0 + lane];
+                my_w = weights[(size_t)i * K + k0 + lane];
+                if (my_m >= n_vert) my_m = -1;
+            }
+            const int n_here = min(32, K - k0);
+            for (int q0 = 0; q0 < n_here; q0 += U) {
+                float g[U], w[U];
+                int m[U];
+#pragma unroll
+                for (int q = 0; q < U; q++) {
+                    m[q] = __shfl_sync(0xffffffffu, my_m, (q0 + q) & 31);
+                    w[q] = __shfl_sync(0xffffffffu, my_w, (q0 + q) & 31);
+                    g[q] = in && m[q] >= 0 ? __ldg(grad + (size_t)m[q] * F + f0 + lane) : 0.f;
+                }
+#pragma unroll
+                for (int q = 0; q < U; q++)
+                    if (q0 + q < n_here && m[q] >= 0) acc = __fadd_rn(acc, __fmul_rn(g[q], w[q]));
+            }
         }
-        feat_grad[(size_t)i * F + f] = acc;
+        if (in) feat_grad[(size_t)i * F + f0 + lane] = acc;
     }
-}
-
-// w_grad[i,k] = sum_f grad[m_k,f] * feat[i,f]: one thread per (hit, slot), f in order.
-__global__ void __launch_bounds__(256)
-push_grad_weights_kernel(const float *__restrict__ grad, const float *__restrict__ feat,
-                         const int *__restrict__ nidx, float *__restrict__ w_grad, long long n_edges,
-                         int n_vert, int K, int F)
-{
-    const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n_edges) return;
-    const int m = nidx[e];
-    float acc = 0.f;
-    if (m >= 0 && m < n_vert) {
-        const int i = (int)(e / K);
-        for (int f = 0; f < F; f++)
-            acc = __fadd_rn(acc, __fmul_rn(__ldg(grad + (size_t)m * F + f), feat[(size_t)i * F + f]));
-    }
-    w_grad[e] = acc;
 }
 
 }  // namespace
@@ -93,7 +77,15 @@ using namespace hgc;
 
 extern "C" int hgc_push_knn_grad(
         const float *d_grad, const float *d_weights, const float *d_feat, const int *d_idxs,
-        float *d_feat_grad, float *d_w_grad, int n_vert, int n_neigh, int n_feat, hgc_stream_t stream_)
+        float *d_feat_grad, float *d_w_grad, int n_vert, int n_neigh, int n_feat, hgc_stream_t stream)
+{
+    return hgc_push_knn_grad_ordered(d_grad, d_weights, d_feat, d_idxs, d_feat_grad, d_w_grad, n_vert, n_neigh, n_feat,
+                                     nullptr, stream);
+}
+
+extern "C" int hgc_push_knn_grad_ordered(
+        const float *d_grad, const float *d_weights, const float *d_feat, const int *d_idxs,
+        float *d_feat_grad, float *d_w_grad, int n_vert, int n_neigh, int n_feat, const int *d_order, hgc_stream_t stream_)
 {
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     if (n_vert < 0 || n_neigh < 0 || n_feat < 0) return HGC_ERR_INVALID_ARGUMENT;
@@ -103,12 +95,13 @@ extern "C" int hgc_push_knn_grad(
     if (ne > 0 && (!d_weights || !d_idxs || !d_w_grad)) return HGC_ERR_INVALID_ARGUMENT;
     if (n_feat > 0) {
         push_grad_features_kernel<<<div_up(n_vert, 8), 256, 0, stream>>>(d_grad, d_weights, d_idxs, d_feat_grad,
-                                                                        n_vert, n_neigh, n_feat);
+                                                                        n_vert, n_neigh, n_feat, d_order);
         HGC_LAUNCH_CHECK();
     }
     if (ne > 0) {
-        push_grad_weights_kernel<<<div_up(ne, 256), 256, 0, stream>>>(d_grad, d_feat, d_idxs, d_w_grad, ne, n_vert,
-                                                                     n_neigh, n_feat);
+        const bool vec4 = n_feat % 4 == 0 && (reinterpret_cast<uintptr_t>(d_feat) & 15u) == 0;
+        edge_dot_kernel<false, false><<<div_up(ne, 256), 256, 0, stream>>>(d_feat, n_feat, d_grad, nullptr, d_idxs, d_w_grad,
+                                                                          ne, n_vert, n_neigh, n_feat, vec4, d_order, nullptr);
         HGC_LAUNCH_CHECK();
     }
     return HGC_OK;
@@ -132,7 +125,15 @@ extern "C" int hgc_local_distance(
 
 extern "C" int hgc_push_knn(
         const float *d_weights, const float *d_feat, const int *d_idxs, float *d_out_feat,
-        int n_vert, int n_neigh, int n_feat, void *workspace, size_t workspace_bytes, hgc_stream_t stream_)
+        int n_vert, int n_neigh, int n_feat, void *workspace, size_t workspace_bytes, hgc_stream_t stream)
+{
+    return hgc_push_knn_ordered(d_weights, d_feat, d_idxs, d_out_feat, n_vert, n_neigh, n_feat, nullptr, workspace,
+                                workspace_bytes, stream);
+}
+
+extern "C" int hgc_push_knn_ordered(
+        const float *d_weights, const float *d_feat, const int *d_idxs, float *d_out_feat,
+        int n_vert, int n_neigh, int n_feat, const int *d_order, void *workspace, size_t workspace_bytes, hgc_stream_t stream_)
 {
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     if (n_vert < 0 || n_neigh < 0 || n_feat < 0) return HGC_ERR_INVALID_ARGUMENT;
@@ -146,11 +147,13 @@ extern "C" int hgc_push_knn(
     const size_t need = hgc_knn_grad_workspace_bytes(n_vert, n_neigh);
     if (int rc = check_workspace(workspace, workspace_bytes, need)) return rc;
     Carver ws(workspace);
-    HGC_CUDA_TRY(cudaMemsetAsync(ws.status(), 0, kAlign, stream));
+    // sums in (hit, slot) order (modules/compiled/push_knn_kernel.cc:35-71; the reference's GPU kernel scatters with
+    // atomicAdd, push_knn_kernel.cu.cc:61)
     const Incoming b = incoming_layout(ws, n_vert, n_neigh);
-    if (int rc = build_incoming(d_idxs, n_vert, n_neigh, b, stream)) return rc;
-    push_knn_kernel<<<div_up(n_vert, 8), 256, 0, stream>>>(d_weights, d_feat, b.bounds, b.sedges, d_out_feat,
-                                                          n_vert, n_neigh, n_feat);
-    HGC_LAUNCH_CHECK();
+    if (int rc = build_incoming(d_idxs, n_vert, n_neigh, b, ws.status(), stream)) return rc;
+    for (int f0 = 0; f0 < n_feat; f0 += 64)
+        if (int rc = launch_edge_sum_slab<kSumPlain>(d_feat, n_feat, d_weights, nullptr, nullptr, b.bounds, b.edges, d_out_feat,
+                                                     n_vert, n_neigh, n_feat, f0, d_order, stream))
+            return rc;
     return HGC_OK;
 }

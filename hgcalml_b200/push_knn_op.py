@@ -6,7 +6,7 @@ import torch
 from . import _capi as C
 
 
-def _push_knn(w, f, nidx):
+def _push_knn(w, f, nidx, order=None):
     """The registered op ``PushKnn`` (modules/compiled/push_knn_module.cc:7-11): every hit adds its
     features, weighted per neighbour slot, to its neighbours: ``out[nidx[i,k]] += f[i] * w[i,k]``.
     Contributions are summed in (i, k) order, so the result does not change from run to run."""
@@ -17,21 +17,23 @@ def _push_knn(w, f, nidx):
         raise C.HgcError("PushKnn expects weights and indices of equal shape and one feature row per vertex")
     out = torch.empty_like(f)
     ws = C.workspace(C.lib.hgc_knn_grad_workspace_bytes(n, k), f.device)
-    C.check(C.lib.hgc_push_knn(C.ptr(w), C.ptr(f), C.ptr(nidx), C.ptr(out), n, k, f.shape[1],
-                               C.ptr(ws), ws.numel(), C.stream_of(f)), "PushKnn")
+    C.check(C.lib.hgc_push_knn_ordered(C.ptr(w), C.ptr(f), C.ptr(nidx), C.ptr(out), n, k, f.shape[1], C.ptr(order),
+                                       C.ptr(ws), ws.numel(), C.stream_of(f)), "PushKnn")
     return out
 
 
-def PushKnnGrad(grad, weights, features, indices):
+def PushKnnGrad(grad, weights, features, indices, order=None):
     """The registered op ``PushKnnGrad`` (modules/compiled/push_knn_grad_module.cc:7-13).
-    Returns ``(weight_grad [N,K], feature_grad [N,F])``."""
+    Returns ``(weight_grad [N,K], feature_grad [N,F])``.  ``order`` (optional int32 permutation of the hits) only
+    sets the order in which hits are processed."""
     C.require_cuda(grad, weights, features, indices)
     g, w, f, idx = C.f32(grad), C.f32(weights), C.f32(features), C.i32(indices)
     n, k = idx.shape
     wg = torch.empty_like(w)
     fg = torch.empty_like(f)
-    C.check(C.lib.hgc_push_knn_grad(C.ptr(g), C.ptr(w), C.ptr(f), C.ptr(idx), C.ptr(fg), C.ptr(wg),
-                                    n, k, f.shape[1], C.stream_of(f)), "PushKnnGrad")
+    order = C.order_of(indices, n) if order is None else C.i32(order)
+    C.check(C.lib.hgc_push_knn_grad_ordered(C.ptr(g), C.ptr(w), C.ptr(f), C.ptr(idx), C.ptr(fg), C.ptr(wg),
+                                            n, k, f.shape[1], C.ptr(order), C.stream_of(f)), "PushKnnGrad")
     return wg, fg
 
 
@@ -39,12 +41,13 @@ class _PushKnnFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, w, f, nidx):
         ctx.save_for_backward(w, f, nidx)
-        return _push_knn(w, f, nidx)
+        ctx.order = C.order_of(nidx, nidx.shape[0])
+        return _push_knn(w, f, nidx, ctx.order)
 
     @staticmethod
     def backward(ctx, grad):
         w, f, nidx = ctx.saved_tensors
-        wg, fg = PushKnnGrad(grad.contiguous(), w, f, nidx)
+        wg, fg = PushKnnGrad(grad, w, f, nidx, order=ctx.order)
         return wg, fg, None
 
 

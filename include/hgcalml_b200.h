@@ -173,6 +173,12 @@ int hgc_accumulate_knn(
         float *d_out_feat, int *d_out_maxidxs,
         int n_vert, int n_neigh, int n_feat, int n_out_feat, int n_moments, int mean_and_max,
         hgc_stream_t stream);
+/* with a processing order: d_order (may be NULL) is a permutation of the hits, results do not depend on it */
+int hgc_accumulate_knn_ordered(
+        const float *d_weights, const float *d_feat, const int *d_idxs,
+        float *d_out_feat, int *d_out_maxidxs,
+        int n_vert, int n_neigh, int n_feat, int n_out_feat, int n_moments, int mean_and_max,
+        const int *d_order, hgc_stream_t stream);
 
 /* Same op with the weighting of the Python wrapper fused in (modules/accknn_op.py:52):
  * weight = exp(-(distance_scale * d_distances[v,k])), the product rounded to float32 first, so
@@ -292,7 +298,7 @@ int hgc_build_and_assign_condensates(
  * coordinates, d_grad_coord [n_vert, n_coords]; d_dist is accepted and not read, as in the
  * reference.  Deterministic for the same reason.
  *
- * Both take a workspace of hgc_knn_grad_workspace_bytes (about 24 bytes per (hit, slot) pair) and
+ * Both take a workspace of hgc_knn_grad_workspace_bytes (about 16 bytes per (hit, slot) pair) and
  * need n_vert * n_neigh < 2^31.
  * ------------------------------------------------------------------------------------- */
 size_t hgc_knn_grad_workspace_bytes(int n_vert, int n_neigh);
@@ -317,6 +323,11 @@ int hgc_select_knn_grad(
         const float *d_grad_dist, const int *d_indices, const float *d_dist, const float *d_coord,
         float *d_grad_coord, int n_vert, int n_neigh, int n_coords,
         void *workspace, size_t workspace_bytes, hgc_stream_t stream);
+/* with a processing order, as above */
+int hgc_select_knn_grad_ordered(
+        const float *d_grad_dist, const int *d_indices, const float *d_dist, const float *d_coord,
+        float *d_grad_coord, int n_vert, int n_neigh, int n_coords, const int *d_order,
+        void *workspace, size_t workspace_bytes, hgc_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------
  * Sibling ops on the same neighbour tables (used by the graph-condensation layers).
@@ -336,12 +347,19 @@ int hgc_local_distance(
 int hgc_push_knn(
         const float *d_weights, const float *d_feat, const int *d_idxs, float *d_out_feat,
         int n_vert, int n_neigh, int n_feat, void *workspace, size_t workspace_bytes, hgc_stream_t stream);
+/* with a processing order: d_order (may be NULL) is a permutation of the hits, results do not depend on it */
+int hgc_push_knn_ordered(
+        const float *d_weights, const float *d_feat, const int *d_idxs, float *d_out_feat,
+        int n_vert, int n_neigh, int n_feat, const int *d_order, void *workspace, size_t workspace_bytes, hgc_stream_t stream);
 /* PushKnnGrad -- replaces PushKnnGradOpFunctor (modules/compiled/push_knn_grad_kernel.h; argument order as
  * there): d_feat_grad[i,f] = sum_k d_grad[m_k,f] * d_weights[i,k], d_w_grad[i,k] = sum_f d_grad[m_k,f] *
  * d_feat[i,f], both summed in order.  No workspace. */
 int hgc_push_knn_grad(
         const float *d_grad, const float *d_weights, const float *d_feat, const int *d_idxs,
         float *d_feat_grad, float *d_w_grad, int n_vert, int n_neigh, int n_feat, hgc_stream_t stream);
+int hgc_push_knn_grad_ordered(
+        const float *d_grad, const float *d_weights, const float *d_feat, const int *d_idxs,
+        float *d_feat_grad, float *d_w_grad, int n_vert, int n_neigh, int n_feat, const int *d_order, hgc_stream_t stream);
 
 #ifdef __cplusplus
 }

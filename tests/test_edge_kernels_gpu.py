@@ -1,0 +1,77 @@
+"""Transposed neighbour lists and the kernels over them where they change shape: list lengths around the sizes
+sorted in registers, hubs with thousands of incoming edges, feature widths around the slabs, K that is no power of
+two, and a processing order.  Bit for bit against the CPU checker."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import bits
+from test_ops_gpu import T, N
+
+pytestmark = pytest.mark.gpu
+
+
+def _table(n, K, seed):
+    """Random neighbours; some hits get exactly 0, 1, 31 .. 129 and thousands of incoming edges."""
+    rng = np.random.default_rng(seed)
+    idx = rng.integers(40, n, (n, K)).astype(np.int32)
+    idx[rng.random((n, K)) < 0.1] = -1
+    flat = idx.reshape(-1)
+    at = rng.permutation(flat.size)
+    for m, count in enumerate([0, 1, 31, 32, 33, 63, 64, 65, 127, 128, 129, 300, min(5000, flat.size // 3)]):
+        flat[at[:count]] = m
+        at = at[count:]
+    idx[::7, 0] = np.arange(n)[::7]
+    idx[::7, K - 1] = np.arange(n)[::7]  # the hit itself a second time
+    return idx, rng
+
+
+@pytest.mark.parametrize("n,K,F,mm", [(2500, 16, 64, True), (2500, 12, 65, True), (1500, 9, 130, True), (1500, 8, 31, True),
+                                      (1500, 33, 33, False), (800, 1, 4, True)])
+def test_accumulate_knn_grad(cuda, oracle, n, K, F, mm):
+    from hgcalml_b200.accknn_op import AccumulateKnnGrad, AccumulateLinKnn
+    idx, rng = _table(n, max(K, 2), n + K)
+    idx = np.ascontiguousarray(idx[:, :K])
+    feat = rng.standard_normal((n, F), dtype=np.float32)
+    w = rng.random((n, K), dtype=np.float32)
+    out, maxidx = AccumulateLinKnn(T(w, cuda), T(feat, cuda), T(idx, cuda), mean_and_max=mm)
+    g = rng.standard_normal(tuple(out.shape), dtype=np.float32)
+    rw, rf = oracle.op_accumulate_knn_grad(g, w, feat, idx, N(maxidx))
+    order = T(rng.permutation(n).astype(np.int32), cuda)
+    for o in (None, order):
+        gw, gf = AccumulateKnnGrad(T(g, cuda), T(w, cuda), T(feat, cuda), T(idx, cuda), maxidx, order=o)
+        assert np.array_equal(bits(N(gw)), bits(rw)) and np.array_equal(bits(N(gf)), bits(rf))
+
+
+@pytest.mark.parametrize("n,K,F", [(2500, 16, 32), (1200, 7, 70), (600, 40, 3)])
+def test_push_knn_and_gradients(cuda, oracle, n, K, F):
+    from hgcalml_b200.push_knn_op import PushKnn, PushKnnGrad
+    from hgcalml_b200.binned_select_knn_op import SelectKnnGrad
+    idx, rng = _table(n, K, n)
+    w = rng.random((n, K), dtype=np.float32)
+    f, g = (rng.standard_normal((n, F), dtype=np.float32) for _ in range(2))
+    c = rng.standard_normal((n, 4), dtype=np.float32)
+    table = T(idx, cuda)
+    order = T(rng.permutation(n).astype(np.int32), cuda)
+    for o in (None, order):
+        if o is not None:
+            from hgcalml_b200 import _capi
+            _capi.set_order(table, o)
+        assert np.array_equal(bits(N(PushKnn(T(w, cuda), T(f, cuda), table))), bits(oracle.op_push_knn(w, f, idx)))
+        rw, rf = oracle.op_push_knn_grad(g, w, f, idx)
+        gw, gf = PushKnnGrad(T(g, cuda), T(w, cuda), T(f, cuda), table)
+        assert np.array_equal(bits(N(gw)), bits(rw)) and np.array_equal(bits(N(gf)), bits(rf))
+        ref = oracle.op_select_knn_grad(w, idx, c)
+        assert np.array_equal(bits(N(SelectKnnGrad(T(w, cuda), table, None, T(c, cuda)))), bits(ref))
+
+
+def test_search_notes_its_order(cuda):
+    from hgcalml_b200 import _capi
+    from hgcalml_b200.binned_select_knn_op import BinnedSelectKnn, BinnedSelectKnnDifferentiable
+    c = torch.rand((3000, 3), device=cuda)
+    rs = torch.tensor([0, 3000], dtype=torch.int32, device=cuda)
+    idx, _, sorting = BinnedSelectKnn(8, c, rs, return_sorting=True)
+    assert torch.equal(_capi.order_of(idx, 3000), sorting)
+    assert _capi.order_of(idx[:2000], 2000) is None and _capi.order_of(idx, 2999) is None
+    idx, _ = BinnedSelectKnnDifferentiable(8, c.requires_grad_(True), rs)
+    assert torch.equal(_capi.order_of(idx, 3000), sorting)
