@@ -77,37 +77,40 @@ __device__ __forceinline__ float set_eq(float a, float b)
     return r;
 }
 
-// EXACT: the row has exactly LPH * VPL float4 (then the row width is a compile-time constant and no
+// VW: floats per load (4, or 2 and 1 for widths and addresses that allow no more); a lane owns VPL vectors of them.
+// EXACT: the row has exactly LPH * VPL vectors (then the row width is a compile-time constant and no
 // lane is idle).
-template <int LPH, int VPL, int CH, int THREADS, int MINB, bool EXP, bool WITH_ARG, bool EXACT>
+template <int VW, int LPH, int VPL, int CH, int THREADS, int MINB, bool EXP, bool WITH_ARG, bool EXACT>
 __global__ void __launch_bounds__(THREADS, MINB)
-accumulate_vec_kernel(const float *__restrict__ weights, const float4 *__restrict__ feat,
+accumulate_vec_kernel(const float *__restrict__ weights, const float *__restrict__ feat,
                       const int *__restrict__ idxs, float *__restrict__ out, int *__restrict__ out_arg,
-                      int n_vert, int K, int ldk, int F4_arg, int n_out_feat, bool mean_and_max,
-                      const int *__restrict__ order, float scale, bool sub_self)
+                      int n_vert, int K, int ldk, int F_arg, int n_out_feat, bool mean_and_max,
+                      const int *__restrict__ order, float scale, bool sub_self, int tile_steps)
 {
-    const int F4 = EXACT ? LPH * VPL : F4_arg;
+    const int F = EXACT ? LPH * VPL * VW : F_arg;
+    const int n_vec = EXACT ? LPH * VPL : F_arg / VW;
     constexpr int G = THREADS / LPH;  // hits a block works on at a time
-    constexpr int NP = VPL * 2;       // packed pairs per lane per row
-    constexpr int NE = VPL * 4;       // floats per lane per row
+    constexpr int NE = VPL * VW;      // floats per lane per row
+    constexpr int NP = NE / 2;        // packed pairs per lane per row
+    static_assert(NE % 2 == 0, "floats are processed in pairs");
     static_assert(LPH % CH == 0 && CH % 2 == 0, "rows are requested CH at a time and processed in pairs");
     const int gl = threadIdx.x % LPH;  // lane inside the group
     const int grp = threadIdx.x / LPH;
     const float inv_count = (float)K;
-    // float4 column of this lane's u-th vector; lanes beyond the row read column 0 and store nothing
+    // vector column of this lane's u-th vector; lanes beyond the row read column 0 and store nothing
     int col[VPL];
 #pragma unroll
-    for (int u = 0; u < VPL; u++) col[u] = (EXACT || (gl + u * LPH) < F4) ? (gl + u * LPH) : 0;
+    for (int u = 0; u < VPL; u++) col[u] = (EXACT || (gl + u * LPH) < n_vec) ? (gl + u * LPH) : 0;
 
-    // A block walks tiles of kAccTileSteps * G consecutive hits (of the processing order), G at a
+    // A block walks tiles of tile_steps * G consecutive hits (of the processing order), G at a
     // time, and the grid moves over the batch tile by tile: with a spatially coherent order the
     // neighbour rows of one step are still in L1 for the next, and all blocks work inside one
     // window of the batch at any time.
     const long long total_steps = ((long long)n_vert + G - 1) / G;
-    const long long n_tiles = (total_steps + kAccTileSteps - 1) / kAccTileSteps;
+    const long long n_tiles = (total_steps + tile_steps - 1) / tile_steps;
     for (long long tile = blockIdx.x; tile < n_tiles; tile += gridDim.x)
-    for (int ts = 0; ts < kAccTileSteps; ts++) {
-        const long long step = tile * kAccTileSteps + ts;
+    for (int ts = 0; ts < tile_steps; ts++) {
+        const long long step = tile * tile_steps + ts;
         if (step >= total_steps) break;  // uniform over the block
         const long long g = step * G + grp;
         const bool live = g < n_vert;
@@ -162,9 +165,15 @@ accumulate_vec_kernel(const float *__restrict__ weights, const float4 *__restric
                         w[kk] = __shfl_sync(0xffffffffu, my_w, s0 + kk, LPH);
 #pragma unroll
                         for (int u = 0; u < VPL; u++) {
-                            const float4 *p = feat + (size_t)j * F4 + col[u];
-                            asm volatile("ld.global.nc.v2.b64 {%0,%1}, [%2];"
-                                         : "=l"(f[kk][2 * u]), "=l"(f[kk][2 * u + 1]) : "l"(p));
+                            const float *p = feat + (size_t)j * F + col[u] * VW;
+                            if constexpr (VW == 4) {
+                                asm volatile("ld.global.nc.v2.b64 {%0,%1}, [%2];"
+                                             : "=l"(f[kk][2 * u]), "=l"(f[kk][2 * u + 1]) : "l"(p));
+                            } else if constexpr (VW == 2) {
+                                asm volatile("ld.global.nc.b64 %0, [%1];" : "=l"(f[kk][u]) : "l"(p));
+                            } else if (u % 2 == 0) {
+                                f[kk][u / 2] = pack2(__ldg(p), __ldg(feat + (size_t)j * F + col[u + 1 < VPL ? u + 1 : u]));
+                            }
                         }
                     }
 #pragma unroll
@@ -208,59 +217,76 @@ accumulate_vec_kernel(const float *__restrict__ weights, const float4 *__restric
                 const bool first = (c0 + kk) == 0;
                 const float sf = (float)(c0 + kk);
 #pragma unroll
-                for (int u = 0; u < VPL; u++) {
-                    const float4 fv = __ldg(feat + (size_t)j * F4 + col[u]);
-                    const float fc[4] = {fv.x, fv.y, fv.z, fv.w};
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        float sx, sy, ax, ay;
-                        unpack2(sum[2 * u + h], sx, sy);
-                        unpack2(argslot[2 * u + h], ax, ay);
-                        const float tx = __fmul_rn(fc[2 * h], w), ty = __fmul_rn(fc[2 * h + 1], w);
-                        sx = __fadd_rn(sx, tx);
-                        sy = __fadd_rn(sy, ty);
-                        if (tx >= best[4 * u + 2 * h] || first) { best[4 * u + 2 * h] = tx; ax = sf; }
-                        if (ty >= best[4 * u + 2 * h + 1] || first) { best[4 * u + 2 * h + 1] = ty; ay = sf; }
-                        sum[2 * u + h] = pack2(sx, sy);
-                        argslot[2 * u + h] = pack2(ax, ay);
-                    }
+                for (int e = 0; e < NP; e++) {
+                    const float *row = feat + (size_t)j * F;
+                    const float fx = __ldg(row + col[2 * e / VW] * VW + (2 * e) % VW);
+                    const float fy = __ldg(row + col[(2 * e + 1) / VW] * VW + (2 * e + 1) % VW);
+                    float sx, sy, ax, ay;
+                    unpack2(sum[e], sx, sy);
+                    unpack2(argslot[e], ax, ay);
+                    const float tx = __fmul_rn(fx, w), ty = __fmul_rn(fy, w);
+                    sx = __fadd_rn(sx, tx);
+                    sy = __fadd_rn(sy, ty);
+                    if (tx >= best[2 * e] || first) { best[2 * e] = tx; ax = sf; }
+                    if (ty >= best[2 * e + 1] || first) { best[2 * e + 1] = ty; ay = sf; }
+                    sum[e] = pack2(sx, sy);
+                    argslot[e] = pack2(ax, ay);
                 }
             }
         }
 
         if (live) {
+            float *row = out + (size_t)v * n_out_feat;
+            const int *ir = idxs + (size_t)v * ldk;
+            // slot -> neighbour id; no slot ever took the maximum: 0, the CPU op's initial value
+            auto neighbour = [ir](float slot) { return slot < 0.f ? 0 : ir[(int)slot]; };
+            if constexpr (VW == 4) {
 #pragma unroll
-            for (int u = 0; u < VPL; u++) {
-                const int vec = gl + u * LPH;
-                if (!EXACT && vec >= F4) continue;
-                float sx, sy, sz, sw;
-                unpack2(sum[2 * u], sx, sy);
-                unpack2(sum[2 * u + 1], sz, sw);
-                float4 m = make_float4(__fdiv_rn(sx, inv_count), __fdiv_rn(sy, inv_count),
-                                       __fdiv_rn(sz, inv_count), __fdiv_rn(sw, inv_count));
-                float4 mx = make_float4(best[4 * u], best[4 * u + 1], best[4 * u + 2], best[4 * u + 3]);
-                if (sub_self) {
-                    // the hit's own row is taken off the mean and the max (one rounding each)
-                    const float4 own = __ldg(feat + (size_t)v * F4 + vec);
-                    m = make_float4(__fsub_rn(m.x, own.x), __fsub_rn(m.y, own.y), __fsub_rn(m.z, own.z), __fsub_rn(m.w, own.w));
-                    mx = make_float4(__fsub_rn(mx.x, own.x), __fsub_rn(mx.y, own.y), __fsub_rn(mx.z, own.z), __fsub_rn(mx.w, own.w));
+                for (int u = 0; u < VPL; u++) {
+                    const int vec = gl + u * LPH;
+                    if (!EXACT && vec >= n_vec) continue;
+                    float sx, sy, sz, sw;
+                    unpack2(sum[2 * u], sx, sy);
+                    unpack2(sum[2 * u + 1], sz, sw);
+                    float4 m = make_float4(__fdiv_rn(sx, inv_count), __fdiv_rn(sy, inv_count),
+                                           __fdiv_rn(sz, inv_count), __fdiv_rn(sw, inv_count));
+                    float4 mx = make_float4(best[4 * u], best[4 * u + 1], best[4 * u + 2], best[4 * u + 3]);
+                    if (sub_self) {
+                        // the hit's own row is taken off the mean and the max (one rounding each)
+                        const float4 own = __ldg(reinterpret_cast<const float4 *>(feat + (size_t)v * F) + vec);
+                        m = make_float4(__fsub_rn(m.x, own.x), __fsub_rn(m.y, own.y), __fsub_rn(m.z, own.z), __fsub_rn(m.w, own.w));
+                        mx = make_float4(__fsub_rn(mx.x, own.x), __fsub_rn(mx.y, own.y), __fsub_rn(mx.z, own.z), __fsub_rn(mx.w, own.w));
+                    }
+                    __stcs(reinterpret_cast<float4 *>(row) + vec, m);  // results are written once and not read again here
+                    if (mean_and_max) {
+                        __stcs(reinterpret_cast<float4 *>(row + F) + vec, mx);
+                        if (WITH_ARG) {
+                            float a0, a1, a2, a3;
+                            unpack2(argslot[2 * u], a0, a1);
+                            unpack2(argslot[2 * u + 1], a2, a3);
+                            __stcs(reinterpret_cast<int4 *>(out_arg + (size_t)v * F) + vec,
+                                   make_int4(neighbour(a0), neighbour(a1), neighbour(a2), neighbour(a3)));
+                        }
+                    }
                 }
-                float4 *row = reinterpret_cast<float4 *>(out + (size_t)v * n_out_feat);
-                __stcs(row + vec, m);  // results are written once and not read again by this kernel
-                if (mean_and_max) {
-                    __stcs(row + F4 + vec, mx);
-                    if (WITH_ARG) {
-                        // slot -> neighbour id; no slot ever took the maximum: 0, the CPU op's initial value
-                        float a0, a1, a2, a3;
-                        unpack2(argslot[2 * u], a0, a1);
-                        unpack2(argslot[2 * u + 1], a2, a3);
-                        const int *ir = idxs + (size_t)v * ldk;
-                        int4 a;
-                        a.x = a0 < 0.f ? 0 : ir[(int)a0];
-                        a.y = a1 < 0.f ? 0 : ir[(int)a1];
-                        a.z = a2 < 0.f ? 0 : ir[(int)a2];
-                        a.w = a3 < 0.f ? 0 : ir[(int)a3];
-                        __stcs(reinterpret_cast<int4 *>(out_arg + (size_t)v * F4 * 4) + vec, a);
+            } else {
+#pragma unroll
+                for (int q = 0; q < NE; q++) {
+                    const int vec = gl + (q / VW) * LPH, f = vec * VW + q % VW;
+                    if (!EXACT && vec >= n_vec) continue;
+                    float s0, s1, a0, a1;
+                    unpack2(sum[q / 2], s0, s1);
+                    unpack2(argslot[q / 2], a0, a1);
+                    float m = __fdiv_rn(q % 2 ? s1 : s0, inv_count), mx = best[q];
+                    if (sub_self) {
+                        const float own = __ldg(feat + (size_t)v * F + f);
+                        m = __fsub_rn(m, own);
+                        mx = __fsub_rn(mx, own);
+                    }
+                    __stcs(row + f, m);
+                    if (mean_and_max) {
+                        __stcs(row + F + f, mx);
+                        if (WITH_ARG) __stcs(out_arg + (size_t)v * F + f, neighbour(q % 2 ? a1 : a0));
                     }
                 }
             }
@@ -268,7 +294,7 @@ accumulate_vec_kernel(const float *__restrict__ weights, const float4 *__restric
     }
 }
 
-// Any feature count / alignment: one warp per hit, lanes stride over the features.
+// Wide rows of odd length or alignment: one warp per hit, lanes stride over the features.
 template <bool EXP>
 __global__ void __launch_bounds__(kAccThreads)
 accumulate_scalar_kernel(const float *__restrict__ weights, const float *__restrict__ feat,
@@ -308,22 +334,25 @@ accumulate_scalar_kernel(const float *__restrict__ weights, const float *__restr
     }
 }
 
-template <int LPH, int VPL, int CH, int THREADS, int MINB>
+template <int VW, int LPH, int VPL, int CH, int THREADS, int MINB>
 int launch_vec(bool exp_w, bool with_arg, const float *w, const float *feat, const int *idxs, float *out,
-               int *out_arg, int n_vert, int K, int ldk, int F4, int n_out, bool mm, const int *order,
+               int *out_arg, int n_vert, int K, int ldk, int F, int n_out, bool mm, const int *order,
                float scale, bool sub_self, cudaStream_t stream)
 {
     constexpr int G = THREADS / LPH;
-    const long long n_tiles = div_up(div_up(n_vert, G), kAccTileSteps);
+    const int n_steps = div_up(n_vert, G);
+    // tiles of fewer steps where there would be less than two blocks per SM: 700 hits at F = 32 16 -> 3.5 us
+    int tile_steps = kAccTileSteps;
+    while (tile_steps > 1 && div_up(n_steps, tile_steps) < 2 * sm_count()) tile_steps >>= 1;
+    const long long n_tiles = div_up(n_steps, tile_steps);
     // one block per tile up to 32 blocks per SM (blocks beyond that walk several tiles): measured faster on
     // the 64-event batch than a grid of resident blocks only, which keeps the SMs less evenly loaded
     long long blocks = (long long)sm_count() * 32;
     if (blocks > n_tiles) blocks = n_tiles;
-    const float4 *f4 = reinterpret_cast<const float4 *>(feat);
 #define HGC_GO(E, A, X)                                                                                    \
-    accumulate_vec_kernel<LPH, VPL, CH, THREADS, MINB, E, A, X><<<(int)blocks, THREADS, 0, stream>>>(      \
-            w, f4, idxs, out, out_arg, n_vert, K, ldk, F4, n_out, mm, order, scale, sub_self)
-#define HGC_GO2(E, A) do { if (F4 == LPH * VPL) HGC_GO(E, A, true); else HGC_GO(E, A, false); } while (0)
+    accumulate_vec_kernel<VW, LPH, VPL, CH, THREADS, MINB, E, A, X><<<(int)blocks, THREADS, 0, stream>>>(  \
+            w, feat, idxs, out, out_arg, n_vert, K, ldk, F, n_out, mm, order, scale, sub_self, tile_steps)
+#define HGC_GO2(E, A) do { if (VW == 4 && F == LPH * VPL * VW) HGC_GO(E, A, (VW == 4)); else HGC_GO(E, A, false); } while (0)
     if (exp_w) { if (with_arg) HGC_GO2(true, true); else HGC_GO2(true, false); }
     else       { if (with_arg) HGC_GO2(false, true); else HGC_GO2(false, false); }
 #undef HGC_GO2
@@ -345,9 +374,11 @@ int accumulate_dispatch(bool exp_w, const float *w, const float *feat, const int
     const bool mm = mean_and_max != 0;
     const bool with_arg = mm && out_arg != nullptr;
     auto aligned16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+    auto aligned8 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 7u) == 0; };
     const bool vec_ok = (F % 4 == 0) && (ld_out % 4 == 0) && F <= 512 && aligned16(feat) && aligned16(out) &&
                         (!with_arg || aligned16(out_arg));
-    if (!vec_ok) {
+    const bool pair_ok = !vec_ok && F % 2 == 0 && F <= 256 && aligned8(feat);
+    if (!vec_ok && !pair_ok && F > 128) {
         long long blocks = div_up(n_vert, kAccThreads / kWarp);
         const long long cap = (long long)sm_count() * 32;
         if (blocks > cap) blocks = cap;
@@ -360,17 +391,32 @@ int accumulate_dispatch(bool exp_w, const float *w, const float *feat, const int
         HGC_LAUNCH_CHECK();
         return HGC_OK;
     }
+#define HGC_VEC(W, L, V, C, T, M) return launch_vec<W, L, V, C, T, M>(exp_w, with_arg, w, feat, idxs, out, out_arg, n_vert, K, ldk, F, n_out, mm, order, scale, sub_self, stream)
+    // floats per load, lanes per hit, vectors per lane, rows in flight, block size, blocks per SM
+    if (!vec_ok) {
+        // widths that are no multiple of four (or unaligned rows): the same kernel with 8- or 4-byte loads.  F = 22,
+        // K = 41, 114k hits: 195 -> 96 us against a warp per hit that read every index and weight in all lanes
+        if (pair_ok) {
+            if (F <= 16) HGC_VEC(2, 8, 1, 4, 256, 4);
+            if (F <= 32) HGC_VEC(2, 16, 1, 4, 256, 4);
+            if (F <= 64) HGC_VEC(2, 32, 1, 4, 256, 4);
+            if (F <= 128) HGC_VEC(2, 32, 2, 4, 256, 4);
+            HGC_VEC(2, 32, 4, 4, 256, 2);
+        }
+        if (F <= 16) HGC_VEC(1, 8, 2, 4, 256, 4);
+        if (F <= 32) HGC_VEC(1, 16, 2, 4, 256, 4);
+        if (F <= 64) HGC_VEC(1, 32, 2, 4, 256, 4);
+        HGC_VEC(1, 32, 4, 4, 256, 4);
+    }
     const int F4 = F / 4;
-#define HGC_VEC(L, V, C, T, M) return launch_vec<L, V, C, T, M>(exp_w, with_arg, w, feat, idxs, out, out_arg, n_vert, K, ldk, F4, n_out, mm, order, scale, sub_self, stream)
-    // lanes per hit x float4 per lane, rows in flight, block size, blocks per SM
-    if (F4 <= 4) HGC_VEC(4, 1, 4, 1024, 1);  // measured at F = 16: 2.55 ms against 3.12 ms with 4 blocks of 256 (6.4 M hits)
-    if (F4 <= 8) HGC_VEC(8, 1, 4, 256, 4);
+    if (F4 <= 4) HGC_VEC(4, 4, 1, 4, 1024, 1);  // measured at F = 16: 2.55 ms against 3.12 ms with 4 blocks of 256 (6.4 M hits)
+    if (F4 <= 8) HGC_VEC(4, 8, 1, 4, 256, 4);
     // F = 64: one block of 768 threads per SM works on 96 consecutive hits at a time (measured best on the
     // 64-event batch: the rows those hits share are found in L1)
-    if (F4 <= 16) HGC_VEC(8, 2, 4, 768, 1);
-    if (F4 <= 32) HGC_VEC(16, 2, 4, 768, 1);
-    if (F4 <= 64) HGC_VEC(32, 2, 4, 768, 1);
-    HGC_VEC(32, 4, 2, 512, 1);
+    if (F4 <= 16) HGC_VEC(4, 8, 2, 4, 768, 1);
+    if (F4 <= 32) HGC_VEC(4, 16, 2, 4, 768, 1);
+    if (F4 <= 64) HGC_VEC(4, 32, 2, 4, 768, 1);
+    HGC_VEC(4, 32, 4, 2, 512, 1);
 #undef HGC_VEC
 }
 
