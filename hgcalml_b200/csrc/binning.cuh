@@ -21,6 +21,7 @@ struct GridParams {
     // next bit from the coordinate whose cells are currently the largest.
     float all_min[kMaxBinDims]; // batch minimum of every coordinate
     float all_ext[kMaxBinDims]; // cell extent the code starts from: bin width or batch range
+    float range[kMaxBinDims];   // batch extent of every coordinate
     float curve_scale;          // 1 / largest extent of the batch over all ordered coordinates (0: no extent)
     int sub_seq[kSubBits];      // coordinate that supplies bit k of the code (most significant first)
     int sub_bit[kSubBits];      // and the bit of its 16-bit position

@@ -2,6 +2,7 @@
 #pragma once
 #include "common.cuh"
 #include "binning.cuh"
+#include "knn_device.cuh"
 
 namespace hgc {
 
@@ -27,11 +28,7 @@ __device__ __forceinline__ void range_of_block(const float *__restrict__ coords,
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int c = 0; c < kMaxBinDims; c++) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            mn[c] = fminf(mn[c], __shfl_xor_sync(0xffffffffu, mn[c], o));
-            mx[c] = fmaxf(mx[c], __shfl_xor_sync(0xffffffffu, mx[c], o));
-        }
+        if (c < n_dims) { mn[c] = warp_min_f32(mn[c]); mx[c] = warp_max_f32(mx[c]); }
         if (lane == 0) { s_mn[warp][c] = mn[c]; s_mx[warp][c] = mx[c]; }
     }
     __syncthreads();
@@ -51,9 +48,10 @@ __device__ __forceinline__ void grid_from_partials(const float *partial, int n_p
                   int pre_normalized, GridParams *__restrict__ g)
 {
     // min / max over the per-block partial results: thread t looks at coordinate t % 8 of every
-    // (kGridSetupThreads / 8)-th partial, a shared-memory pass combines the threads of a coordinate
-    static_assert(kMaxBinDims == 8 && kGridSetupThreads % 8 == 0, "layout of the reduction");
-    __shared__ float s_mn[kGridSetupThreads], s_mx[kGridSetupThreads];
+    // (kGridSetupThreads / 8)-th partial; shuffles combine the lanes of a coordinate, shared memory the warps
+    static_assert(kMaxBinDims == 8 && kGridSetupThreads % 32 == 0, "layout of the reduction");
+    constexpr int kGridWarps = kGridSetupThreads / 32;
+    __shared__ float s_mn[kGridWarps][8], s_mx[kGridWarps][8];
     {
         const int cc = threadIdx.x & 7;
         float a = INFINITY, b = -INFINITY;
@@ -61,8 +59,12 @@ __device__ __forceinline__ void grid_from_partials(const float *partial, int n_p
             a = fminf(a, __ldcg(partial + ((size_t)p * 2 + 0) * kMaxBinDims + cc));  // perhaps written in this launch
             b = fmaxf(b, __ldcg(partial + ((size_t)p * 2 + 1) * kMaxBinDims + cc));
         }
-        s_mn[threadIdx.x] = a;
-        s_mx[threadIdx.x] = b;
+#pragma unroll
+        for (int o = 8; o < 32; o <<= 1) {
+            a = fminf(a, __shfl_xor_sync(0xffffffffu, a, o));
+            b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, o));
+        }
+        if ((threadIdx.x & 31) < 8) { s_mn[threadIdx.x >> 5][cc] = a; s_mx[threadIdx.x >> 5][cc] = b; }
     }
     __syncthreads();
     if (threadIdx.x >= 32) return;  // the rest is one warp's work
@@ -70,9 +72,10 @@ __device__ __forceinline__ void grid_from_partials(const float *partial, int n_p
     float mn = 0.f, mx = 0.f;
     if (c < n_all) {
         mn = INFINITY; mx = -INFINITY;
-        for (int t = c; t < kGridSetupThreads; t += 8) {
-            mn = fminf(mn, s_mn[t]);
-            mx = fmaxf(mx, s_mx[t]);
+#pragma unroll
+        for (int w = 0; w < kGridWarps; w++) {
+            mn = fminf(mn, s_mn[w][c]);
+            mx = fmaxf(mx, s_mx[w][c]);
         }
     }
     // The wrapper shifts by the minimum first; x -> x - mn is monotone, so the shifted extremes
@@ -112,28 +115,21 @@ __device__ __forceinline__ void grid_from_partials(const float *partial, int n_p
     if (c < kMaxBinDims) { g->all_min[c] = mn; g->all_ext[c] = ext; }
     float span = c < n_all ? mx - mn : 0.f;
     if (!isfinite(span)) span = 0.f;
+    const float own_span = span;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) span = fmaxf(span, __shfl_xor_sync(0xffffffffu, span, o));
+    if (c < kMaxBinDims) g->range[c] = own_span;
     if (c == 0) g->curve_scale = span > 0.f ? 1.f / span : 0.f;
-    float cell[kMaxBinDims];
-#pragma unroll
-    for (int k = 0; k < kMaxBinDims; k++) cell[k] = __shfl_sync(0xffffffffu, ext, k);
-    if (c == 0) {
-        int used[kMaxBinDims];
-#pragma unroll
-        for (int q = 0; q < kMaxBinDims; q++) used[q] = 0;
-        for (int k = 0; k < kSubBits; k++) {
-            int best = 0;
-#pragma unroll
-            for (int q = 1; q < kMaxBinDims; q++)
-                if (cell[q] > cell[best]) best = q;
-            g->sub_seq[k] = best;
-#pragma unroll
-            for (int q = 0; q < kMaxBinDims; q++)
-                if (q == best) {
-                    cell[q] *= 0.5f;
-                    g->sub_bit[k] = 15 - used[q]++;
-                }
+    // lane q holds the cell of coordinate q; the largest one (the first among equals) supplies the next bit
+    float cell = c < kMaxBinDims ? fmaxf(ext, 0.f) : -1.f;
+    int used = 0;
+    for (int k = 0; k < kSubBits; k++) {
+        const float top = warp_max_f32(cell);
+        const int first = __ffs(__ballot_sync(0xffffffffu, cell == top)) - 1;
+        if (c == first) {
+            g->sub_seq[k] = c;
+            g->sub_bit[k] = 15 - used++;
+            cell *= 0.5f;
         }
     }
 }

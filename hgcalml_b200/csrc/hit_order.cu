@@ -16,74 +16,14 @@
 #include "common.cuh"
 #include "binning_device.cuh"
 #include "hit_order.cuh"
+#include "hit_order_device.cuh"
 
 namespace hgc {
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = kOrderThreads;
 constexpr int kWarps = kThreads / kWarp;
 constexpr int kRounds = kOrderTile / kThreads;
-
-template <typename Op>
-__device__ __forceinline__ int block_scan_inclusive(int v, Op op, int identity, int *s_warp)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v = op(v, t);
-    }
-    __syncthreads();  // s_warp may still be read by the previous scan
-    if (lane == 31) s_warp[warp] = v;
-    __syncthreads();
-    int before = identity;
-    for (int w = 0; w < warp; w++) before = op(before, s_warp[w]);
-    return op(before, v);
-}
-
-// First position, tile, chunk and super-chunk of every event, and of the run of hits that lie beyond the last
-// event.  Row splits are clamped to an ascending sequence inside [0, n_vert], so the layout stays
-// inside its arrays whatever they hold.  One block of kThreads.
-__device__ void event_layout(const int *__restrict__ row_splits, int n_events, int n_vert, const HitOrder &o)
-{
-    __shared__ int s_warp[kWarps];
-    __shared__ int s_last[4];
-    auto add = [](int a, int b) { return a + b; };
-    auto mx = [](int a, int b) { return a > b ? a : b; };
-    int pos = 0, tile = 0, chunk = 0, super = 0;  // carried over from the events before
-    for (int base = 0; base <= n_events; base += kThreads) {
-        const int e = base + threadIdx.x;
-        // end of event e; the last entry (the hits beyond the last event) ends with the batch
-        int end = e < n_events ? min(max(row_splits[e + 1], 0), n_vert) : n_vert;
-        end = mx(pos, block_scan_inclusive(end, mx, 0, s_warp));
-        int begin = __shfl_up_sync(0xffffffffu, end, 1);
-        __syncthreads();
-        if ((threadIdx.x & 31) == 31) s_warp[threadIdx.x >> 5] = end;
-        __syncthreads();
-        if ((threadIdx.x & 31) == 0) begin = threadIdx.x == 0 ? pos : s_warp[(threadIdx.x >> 5) - 1];
-        const int n = e <= n_events ? end - begin : 0;
-        const int nt = (n + kOrderTile - 1) / kOrderTile, nc = (n + 31) / 32, ns = (nc + 31) / 32;
-        const int ti = tile + block_scan_inclusive(nt, add, 0, s_warp);
-        const int ci = chunk + block_scan_inclusive(nc, add, 0, s_warp);
-        const int si = super + block_scan_inclusive(ns, add, 0, s_warp);
-        if (e <= n_events) {
-            o.event_pos[e] = begin;
-            o.event_tile[e] = ti - nt;
-            o.event_chunk[e] = ci - nc;
-            o.event_super[e] = si - ns;
-            if (e == n_events) {
-                o.event_pos[e + 1] = end;
-                o.event_tile[e + 1] = ti;
-                o.event_chunk[e + 1] = ci;
-                o.event_super[e + 1] = si;
-            }
-        }
-        __syncthreads();
-        if (threadIdx.x == kThreads - 1) { s_last[0] = end; s_last[1] = ti; s_last[2] = ci; s_last[3] = si; }
-        __syncthreads();
-        pos = s_last[0]; tile = s_last[1]; chunk = s_last[2]; super = s_last[3];
-    }
-}
 
 // Range of the coordinates over the batch; the first block also lays out the events, the last one to
 // finish derives the grid.
@@ -106,27 +46,6 @@ range_and_layout_kernel(const float *__restrict__ coords, int C, int n_dims, int
     grid_from_partials(o.partial, gridDim.x, n_dims, n_all, row_splits, n_rs, n_bins, n_neigh, 0, o.grid);
 }
 
-__device__ __forceinline__ int event_of_tile(const int *__restrict__ event_tile, int n_events, int tile)
-{
-    int lo = 0, hi = n_events;  // last event whose first tile is <= tile (events without hits share one)
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (event_tile[mid] <= tile) lo = mid; else hi = mid - 1;
-    }
-    return lo;
-}
-
-struct Tile { int event, first, n; };  // positions [first, first + n)
-
-__device__ __forceinline__ bool find_tile(const HitOrder &o, int n_events, int tile, Tile *t)
-{
-    if (tile >= o.event_tile[n_events + 1]) return false;
-    t->event = event_of_tile(o.event_tile, n_events, tile);
-    t->first = o.event_pos[t->event] + (tile - o.event_tile[t->event]) * kOrderTile;
-    t->n = min(o.event_pos[t->event + 1] - t->first, kOrderTile);
-    return true;
-}
-
 // Keys of both orders, digit counts of the tile (first pass) and of the event (all passes).
 //   order 0: bin number inside the event (as modules/compiled/bin_by_coordinates_kernel.cc:64-113: truncating float
 //            division, last dimension fastest, out-of-range bins forced to 0), then the 16-bit locality code
@@ -138,7 +57,7 @@ order_keys_kernel(const float *__restrict__ coords, int C, int n_dims, HitOrder 
 {
     __shared__ int s_hist[2][kOrderPasses][256];
     __shared__ unsigned short s_frac[kMaxBinDims][kThreads];
-    Tile t;
+    HitTile t;
     if (!find_tile(o, n_events, blockIdx.x, &t)) return;
     for (int i = threadIdx.x; i < 2 * kOrderPasses * 256; i += kThreads) (&s_hist[0][0][0])[i] = 0;
     __syncthreads();
@@ -212,7 +131,7 @@ order_pass_kernel(HitOrder o, int n_events, int tiles_cap, int pass, int *__rest
     __shared__ int s_count[kWarps][256];
     __shared__ int s_warp[kWarps];
     const int order = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d = threadIdx.x;
-    Tile t;
+    HitTile t;
     if (!find_tile(o, n_events, blockIdx.x, &t)) return;
     const unsigned *__restrict__ key_in = o.key[order][pass & 1];
     const int *__restrict__ val_in = o.val[order][pass & 1];
@@ -297,6 +216,16 @@ order_pass_kernel(HitOrder o, int n_events, int tiles_cap, int pass, int *__rest
 
 }  // namespace
 
+int range_and_layout(const float *coords, int n_coords, int n_bin_dims, const int *row_splits, int n_rs, int n_bins,
+                     int n_neigh, int n_vert, const HitOrder &o, unsigned *status, cudaStream_t stream)
+{
+    range_and_layout_kernel<<<range_partial_blocks(n_vert), kThreads, 0, stream>>>(
+            coords, n_coords, n_bin_dims, n_coords < kMaxBinDims ? n_coords : kMaxBinDims, n_vert, row_splits, n_rs, n_bins,
+            n_neigh, o, status + 8);
+    HGC_LAUNCH_CHECK();
+    return HGC_OK;
+}
+
 int order_hits(const float *coords, int n_coords, int n_bin_dims, const int *row_splits, int n_rs, int n_bins, int n_neigh,
                int n_vert, int bin_bits, const HitOrder &o, int *bin_perm, int *rank, int *curve_perm,
                unsigned *status, cudaStream_t stream)
@@ -305,9 +234,8 @@ int order_hits(const float *coords, int n_coords, int n_bin_dims, const int *row
     if (bin_bits + kSubBits > 32) return HGC_ERR_UNSUPPORTED;
     const int n_events = n_rs - 1;
     const int n_all = n_coords < kMaxBinDims ? n_coords : kMaxBinDims;
-    range_and_layout_kernel<<<range_partial_blocks(n_vert), kThreads, 0, stream>>>(
-            coords, n_coords, n_bin_dims, n_all, n_vert, row_splits, n_rs, n_bins, n_neigh, o, status + 8);
-    HGC_LAUNCH_CHECK();
+    if (int rc = range_and_layout(coords, n_coords, n_bin_dims, row_splits, n_rs, n_bins, n_neigh, n_vert, o, status, stream))
+        return rc;
     const int tiles = (int)order_tiles_cap(n_vert, n_events);
 #define HGC_KEYS(D, B)                                                                                            \
     case D: order_keys_kernel<D, B><<<tiles, kThreads, 0, stream>>>(coords, n_coords, n_bin_dims, o, n_events, tiles, status); break

@@ -52,6 +52,11 @@ inline size_t hit_order_zeroed_bytes(int n_vert, int n_events)
     return s.used;
 }
 
+// Coordinate range and grid of the batch (o.grid, through o.partial) and the event layout (o.event_*).  status[8] counts
+// the blocks that are done and must be zero.
+int range_and_layout(const float *coords, int n_coords, int n_bin_dims, const int *row_splits, int n_rs, int n_bins,
+                     int n_neigh, int n_vert, const HitOrder &o, unsigned *status, cudaStream_t stream);
+
 // Grid of the batch, event layout, and both orders:
 //   bin_perm[p]: hit at position p of the order by (event, bin, locality code, hit number); rank[hit] is its inverse
 //   curve_perm[p]: hit at position p of the order by (event, position on a Hilbert curve, hit number)
