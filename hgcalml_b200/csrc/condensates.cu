@@ -20,6 +20,7 @@
 // bin inputs are accepted for interface compatibility and not read.
 #include <cooperative_groups.h>
 #include "common.cuh"
+#include "condensates.cuh"
 
 namespace hgc {
 namespace {
@@ -29,38 +30,17 @@ constexpr int kClaimThreads = 1024;
 constexpr int kAssignThreads = 256;
 constexpr int kCondTile = 256;
 
-struct CondList {        // per event e, entries [row_splits_h[e], row_splits_h[e] + count[e])
-    float *centre;       // [n_h][dims]
-    float *radius_sq;    // [n_h]
-    int *subset_pos;     // [n_h]  position in the *_h arrays
-    int *lonely;         // [n_h]  1: masked hit that only claims itself
-    int *count;          // [num_rows]
-};
-
-__device__ __forceinline__ unsigned ordered_bits(float f)
-{
-    const unsigned b = __float_as_uint(f);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-
 // Sort key of a high-beta hit: 0 for hits the reference's pick loop takes in position order (it
 // tests no_condensation_mask_h at index 0 or 1 only, binned_assign_to_condensates_kernel.cc:193),
 // else 1 + descending beta.
 __global__ void priority_keys_kernel(const float *__restrict__ beta_h, const int *__restrict__ mask_h,
-                                     const int *__restrict__ row_splits_h, int num_rows, int n_h_max,
-                                     const int *__restrict__ n_h_dev,
+                                     const int *__restrict__ row_splits_h, int num_rows, int n_h,
                                      int *__restrict__ beta_keys, int *__restrict__ event_keys)
 {
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n_h = n_h_dev ? min(n_h_max, *n_h_dev) : n_h_max;
     if (a >= n_h) return;
     const bool flagged = mask_h[a > 0 ? 1 : 0] != 0;  // n_h >= 2 whenever a > 0
-    unsigned key = 0u;
-    if (!flagged) {
-        const unsigned desc = ~ordered_bits(beta_h[a]);
-        key = desc == 0xffffffffu ? desc : desc + 1u;
-    }
-    beta_keys[a] = (int)key;
+    beta_keys[a] = (int)priority_key(beta_h[a], flagged);
     int lo = 1, hi = num_rows + 1;
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
@@ -70,10 +50,9 @@ __global__ void priority_keys_kernel(const float *__restrict__ beta_h, const int
 }
 
 __global__ void gather_int_kernel(const int *__restrict__ src, const int *__restrict__ idx,
-                                  int *__restrict__ dst, int n_max, const int *__restrict__ n_dev)
+                                  int *__restrict__ dst, int n)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int n = n_dev ? min(n_max, *n_dev) : n_max;
     if (i < n) dst[i] = src[idx[i]];
 }
 
@@ -100,45 +79,10 @@ __global__ void init_outputs_kernel(int *__restrict__ status_h, int *__restrict_
 // All blocks take the same decisions from the same data, so only the condensate lists that later
 // kernels read are published (by block 0).  The barriers are the hardware cluster barrier; every
 // block of a cluster runs the same number of windows and batches, so none can be left waiting.
-//
-// A condensate is held as NR float4: its coordinates and, in the last slot, its squared radius (-1
-// for a masked condensate, which covers nothing but itself): NR = 1 up to 3 dimensions, 2 up to 7,
-// 3 for 8.
 constexpr int kClusterBlocks = 8;
 constexpr int kWindow = kClusterBlocks * kClaimThreads;
 constexpr int kBatch = 32;
 constexpr int kStageInts = 8 + kBatch * (3 * 4 + 2);  // block counts, batch records, positions, flags
-
-template <int NR> struct Rec { float v[NR * 4]; };
-template <int NR> __host__ __device__ constexpr int rec_dims() { return NR == 3 ? 8 : NR * 4 - 1; }
-template <int NR> __host__ __device__ constexpr int rec_r2_slot() { return NR == 3 ? 8 : NR * 4 - 1; }
-
-template <int NR>
-__device__ __forceinline__ Rec<NR> load_rec_shared(const float4 *p)
-{
-    Rec<NR> r;
-#pragma unroll
-    for (int u = 0; u < NR; u++) {
-        const float4 q = p[u];
-        r.v[4 * u] = q.x; r.v[4 * u + 1] = q.y; r.v[4 * u + 2] = q.z; r.v[4 * u + 3] = q.w;
-    }
-    return r;
-}
-
-// Squared distance over the first `dims` slots: subtract, multiply, add, each rounded on its own, in
-// coordinate order (the reference's loop, binned_assign_to_condensates_kernel.cc:88-91,103-106).
-template <int NR>
-__device__ __forceinline__ float rec_distsq(const Rec<NR> &c, const Rec<NR> &x, int dims)
-{
-    float s = 0.f;
-#pragma unroll
-    for (int d = 0; d < rec_dims<NR>(); d++)
-        if (d < dims) {
-            const float t = __fsub_rn(c.v[d], x.v[d]);
-            s = __fadd_rn(s, __fmul_rn(t, t));
-        }
-    return s;
-}
 
 template <int NR>
 __global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(kClaimThreads)
@@ -146,8 +90,9 @@ claim_kernel(int dims, const float *__restrict__ ccoords_h, const float *__restr
              const int *__restrict__ mask_h, const int *__restrict__ original_indices_h,
              const int *__restrict__ row_splits_h, const int *__restrict__ order,
              int *__restrict__ status_h, int *__restrict__ alpha_indices, int *__restrict__ stage_all,
-             CondList cl)
+             CondList cl, const int *__restrict__ use_grid)
 {
+    if (use_grid && *use_grid) return;
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     __shared__ float4 s_rec[kCondTile][NR];
@@ -204,7 +149,7 @@ claim_kernel(int dims, const float *__restrict__ ccoords_h, const float *__restr
             __syncthreads();
             if (open && my_mask == 0) {
                 for (int c = 0; c < nt; c++) {
-                    const Rec<NR> r = load_rec_shared<NR>(s_rec[c]);
+                    const Rec<NR> r = load_rec<NR>(s_rec[c]);
                     if (rec_distsq<NR>(r, x, dims) <= r.v[rec_r2_slot<NR>()]) { open = false; break; }
                 }
             }
@@ -261,8 +206,8 @@ claim_kernel(int dims, const float *__restrict__ ccoords_h, const float *__restr
             if (warp < m) {
                 bool cov = false;
                 if (lane < m && lane > warp && !(s_b_flags[warp] & 1) && !(s_b_flags[lane] & 2)) {
-                    const Rec<NR> ci = load_rec_shared<NR>(s_b[warp]);
-                    const Rec<NR> cj = load_rec_shared<NR>(s_b[lane]);
+                    const Rec<NR> ci = load_rec<NR>(s_b[warp]);
+                    const Rec<NR> cj = load_rec<NR>(s_b[lane]);
                     cov = rec_distsq<NR>(ci, cj, dims) <= ci.v[rec_r2_slot<NR>()];
                 }
                 const unsigned cm = __ballot_sync(0xffffffffu, cov);
@@ -278,7 +223,7 @@ claim_kernel(int dims, const float *__restrict__ ccoords_h, const float *__restr
             if (rank == 0 && warp == 0 && ((cond >> lane) & 1u)) {  // publish the new condensates, in order
                 const int slot = off + n_cond + __popc(cond & ((1u << lane) - 1u));
                 const int pos = s_b_pos[lane];
-                const Rec<NR> c = load_rec_shared<NR>(s_b[lane]);
+                const Rec<NR> c = load_rec<NR>(s_b[lane]);
 #pragma unroll
                 for (int d = 0; d < rec_dims<NR>(); d++)
                     if (d < dims) cl.centre[(size_t)slot * dims + d] = c.v[d];
@@ -295,7 +240,7 @@ claim_kernel(int dims, const float *__restrict__ ccoords_h, const float *__restr
                     for (unsigned cm = cond; cm; cm &= cm - 1u) {
                         const int i = __ffs(cm) - 1;
                         if (s_b_flags[i] & 1) continue;  // a masked condensate covers nothing but itself
-                        const Rec<NR> c = load_rec_shared<NR>(s_b[i]);
+                        const Rec<NR> c = load_rec<NR>(s_b[i]);
                         if (rec_distsq<NR>(c, x, dims) <= c.v[rec_r2_slot<NR>()]) { open = false; break; }
                     }
                 }
@@ -396,7 +341,7 @@ assign_kernel(int dims, const float *__restrict__ ccoords, const int *__restrict
                         done = true;
                         break;
                     }
-                    const Rec<NR> r = load_rec_shared<NR>(s_rec[c]);
+                    const Rec<NR> r = load_rec<NR>(s_rec[c]);
                     const float dsq = rec_distsq<NR>(r, x, dims);
                     if (__fmul_rn(min_distance, cl.radius_sq[off + c0 + c]) >= dsq) {
                         best = c0 + c; best_off = off;
@@ -406,7 +351,7 @@ assign_kernel(int dims, const float *__restrict__ ccoords, const int *__restrict
                 continue;
             }
             for (int c = 0; c < nt; c++) {
-                const Rec<NR> r = load_rec_shared<NR>(s_rec[c]);
+                const Rec<NR> r = load_rec<NR>(s_rec[c]);
                 const float dsq = rec_distsq<NR>(r, x, dims);
                 const float r2 = r.v[rec_r2_slot<NR>()];
                 if (!(dsq <= r2)) continue;
@@ -430,7 +375,25 @@ assign_kernel(int dims, const float *__restrict__ ccoords, const int *__restrict
 
 }  // namespace
 
-// defined in radix_sort.cu
+size_t claim_stage_ints(int num_rows) { return (size_t)(num_rows > 0 ? num_rows : 0) * kStageInts; }
+
+int launch_claim_windows(int dims, const float *ccoords_h, const float *dist_h, const int *mask_h,
+                         const int *original_indices_h, const int *row_splits_h, const int *order, int *status_h,
+                         int *alpha_indices, int *stage, const CondList &cl, int num_rows, const int *use_grid,
+                         cudaStream_t stream)
+{
+#define HGC_CLAIM(NR)                                                                                        \
+    claim_kernel<NR><<<num_rows * kClusterBlocks, kClaimThreads, 0, stream>>>(                                 \
+            dims, ccoords_h, dist_h, mask_h, original_indices_h, row_splits_h, order, status_h, alpha_indices, \
+            stage, cl, use_grid)
+    if (rec_size(dims) == 1) HGC_CLAIM(1);
+    else if (rec_size(dims) == 2) HGC_CLAIM(2);
+    else HGC_CLAIM(3);
+#undef HGC_CLAIM
+    HGC_LAUNCH_CHECK();
+    return HGC_OK;
+}
+
 }  // namespace hgc
 
 using namespace hgc;
@@ -456,7 +419,7 @@ void cond_layout(W &ws, int n_h, int num_rows, int dims, CondBuffers *out)
     b.cl.subset_pos = ws.template take<int>(n);
     b.cl.lonely = ws.template take<int>(n);
     b.cl.count = ws.template take<int>(num_rows > 0 ? num_rows : 0);
-    b.stage = ws.template take<int>((size_t)(num_rows > 0 ? num_rows : 0) * kStageInts);
+    b.stage = ws.template take<int>(claim_stage_ints(num_rows));
     if (out) *out = b;
 }
 struct CondSizer {
@@ -474,10 +437,7 @@ extern "C" size_t hgc_binned_assign_to_condensates_workspace_bytes(int n_vert, i
     return w.s.used;
 }
 
-namespace hgc {
-// The op with the number of high-beta hits either exact on the host (d_n_vert_h == nullptr) or in
-// device memory (then n_vert_h is an upper bound that sizes workspace and launches).
-int assign_to_condensates(
+extern "C" int hgc_binned_assign_to_condensates(
         int dimensions, int dimensions_binning,
         const float *d_ccoords_h, const float *d_dist_h, const float *d_beta_h,
         const int *d_no_condensation_mask_h,
@@ -487,8 +447,8 @@ int assign_to_condensates(
         const int *d_indices_to_filtered,
         int *d_assignment, int *d_association, int *d_n_condensates, int *d_alpha_indices,
         const int *d_bin_splits, const int *d_n_bins, const float *d_bin_widths,
-        const int *d_row_splits, int num_rows, int n_vert, int n_vert_h, const int *d_n_vert_h,
-        int assign_by_max_beta, void *workspace, size_t workspace_bytes, hgc_stream_t stream_)
+        const int *d_row_splits, int num_rows, int n_vert, int n_vert_h, int assign_by_max_beta,
+        void *workspace, size_t workspace_bytes, hgc_stream_t stream_)
 {
     (void)dimensions_binning; (void)d_dist; (void)d_bin_splits; (void)d_n_bins; (void)d_bin_widths;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
@@ -518,22 +478,17 @@ int assign_to_condensates(
     if (n_vert_h > 0 && num_rows > 0) {
         priority_keys_kernel<<<div_up(n_vert_h, 256), 256, 0, stream>>>(d_beta_h, d_no_condensation_mask_h,
                                                                         d_row_splits_h, num_rows, n_vert_h,
-                                                                        d_n_vert_h, b.beta_keys, b.event_keys);
+                                                                        b.beta_keys, b.event_keys);
         HGC_LAUNCH_CHECK();
         // stable sort by priority, then stable sort by event: per event, priority order
-        if (int rc = sort_pairs(b.beta_keys, nullptr, b.k1, b.v1, b.tk, b.tv, b.hist, n_vert_h, 32, stream, d_n_vert_h)) return rc;
-        gather_int_kernel<<<div_up(n_vert_h, 256), 256, 0, stream>>>(b.event_keys, b.v1, b.k1, n_vert_h, d_n_vert_h);
+        if (int rc = sort_pairs(b.beta_keys, nullptr, b.k1, b.v1, b.tk, b.tv, b.hist, n_vert_h, 32, stream)) return rc;
+        gather_int_kernel<<<div_up(n_vert_h, 256), 256, 0, stream>>>(b.event_keys, b.v1, b.k1, n_vert_h);
         HGC_LAUNCH_CHECK();
-        if (int rc = sort_pairs(b.k1, b.v1, b.k2, b.v2, b.tk, b.tv, b.hist, n_vert_h, bits_for(num_rows), stream, d_n_vert_h)) return rc;
-#define HGC_CLAIM(NR)                                                                                       \
-    claim_kernel<NR><<<num_rows * kClusterBlocks, kClaimThreads, 0, stream>>>(                                \
-            dimensions, d_ccoords_h, d_dist_h, d_no_condensation_mask_h, d_original_indices_h, d_row_splits_h, \
-            b.v2, d_high_assigned_status_h, d_alpha_indices, b.stage, b.cl)
-        if (dimensions <= 3) HGC_CLAIM(1);
-        else if (dimensions <= 7) HGC_CLAIM(2);
-        else HGC_CLAIM(3);
-#undef HGC_CLAIM
-        HGC_LAUNCH_CHECK();
+        if (int rc = sort_pairs(b.k1, b.v1, b.k2, b.v2, b.tk, b.tv, b.hist, n_vert_h, bits_for(num_rows), stream)) return rc;
+        if (int rc = launch_claim_windows(dimensions, d_ccoords_h, d_dist_h, d_no_condensation_mask_h, d_original_indices_h,
+                                          d_row_splits_h, b.v2, d_high_assigned_status_h, d_alpha_indices, b.stage, b.cl,
+                                          num_rows, nullptr, stream))
+            return rc;
     }
     condensate_totals_kernel<<<1, 32, 0, stream>>>(b.cl.count, num_rows, d_n_condensates);
     HGC_LAUNCH_CHECK();
@@ -550,26 +505,4 @@ int assign_to_condensates(
         HGC_LAUNCH_CHECK();
     }
     return HGC_OK;
-}
-}  // namespace hgc
-
-extern "C" int hgc_binned_assign_to_condensates(
-        int dimensions, int dimensions_binning,
-        const float *d_ccoords_h, const float *d_dist_h, const float *d_beta_h,
-        const int *d_no_condensation_mask_h,
-        int *d_high_assigned_status_h,
-        const int *d_original_indices_h, const int *d_row_splits_h,
-        const float *d_ccoords, const float *d_dist, const int *d_no_condensation_mask,
-        const int *d_indices_to_filtered,
-        int *d_assignment, int *d_association, int *d_n_condensates, int *d_alpha_indices,
-        const int *d_bin_splits, const int *d_n_bins, const float *d_bin_widths,
-        const int *d_row_splits, int num_rows, int n_vert, int n_vert_h, int assign_by_max_beta,
-        void *workspace, size_t workspace_bytes, hgc_stream_t stream)
-{
-    return hgc::assign_to_condensates(
-            dimensions, dimensions_binning, d_ccoords_h, d_dist_h, d_beta_h, d_no_condensation_mask_h,
-            d_high_assigned_status_h, d_original_indices_h, d_row_splits_h, d_ccoords, d_dist,
-            d_no_condensation_mask, d_indices_to_filtered, d_assignment, d_association, d_n_condensates,
-            d_alpha_indices, d_bin_splits, d_n_bins, d_bin_widths, d_row_splits, num_rows, n_vert, n_vert_h,
-            nullptr, assign_by_max_beta, workspace, workspace_bytes, stream);
 }

@@ -1,125 +1,771 @@
-// Wrapper-level BuildAndAssignCondensatesBinned: the tensor glue of modules/assign_condensate_op.py:245-310
-// around the op (threshold scaling, shift by the batch minimum, BinByCoordinates, sort by bin, gathers,
-// the high-beta filter with its index maps, the op, the mapping back and the condensate flags) as one
-// call on the device.  The one value the host needs in between is the number of high-beta hits (it
-// sizes the op's filtered inputs, as the boolean masks do in the reference); it is read back once.
+// Wrapper-level BuildAndAssignCondensatesBinned: the Python function of modules/assign_condensate_op.py:245-310
+// (threshold scaling, shift by the batch minimum, binning, sort by bin, high-beta filter, the op, mapping back,
+// condensate flags) on the hits in the caller's order.
+//
+// The reference's loop takes the free high-beta hit with the largest beta, makes it a condensate and lets it claim
+// what is inside its radius.  Only two things of the wrapper's preparation can be seen in the result: the shift of
+// the coordinates (it rounds them), and the order by bin, which decides between hits of equal beta.  So no
+// hit is moved: the high-beta hits alone are listed and sorted, by bin and then by beta, and every hit is tested
+// where it is.
+//
+//   count_high, order_high   high-beta hits of every event, packed, with their sort keys
+//   order_pass               stable sort by (event, beta descending, bin, hit), a launch per 8-bit digit
+//   claim_grid               which of them are condensates, see there
+//   list_condensates         their lists, in priority order and by grid cell
+//   assign_hits              every hit against the condensates of the 27 cells around it
+//
+// The sort of all hits by bin, the gathers and the test of every hit against every condensate of its event
+// are gone, and the claim pass settles some forty condensates per round instead of up to 32 per batch of a window.
+#include <cooperative_groups.h>
 #include "common.cuh"
-#include "binning.cuh"
+#include "binning_device.cuh"
+#include "condensates.cuh"
+#include "hit_order.cuh"
+#include "hit_order_device.cuh"
 #include "../../include/hgcalml_b200.h"
 
 namespace hgc {
 namespace {
 
 constexpr int kMaxCondDims = 8;
+constexpr int kThreads = kOrderThreads;
+constexpr int kWarps = kThreads / kWarp;
+constexpr int kRounds = kOrderTile / kThreads;
+constexpr int kClusterBlocks = 8;
+constexpr int kClaimThreads = 1024;
+constexpr int kClaimStep = kClusterBlocks * kClaimThreads;  // hits of an event looked at together
+constexpr int kMaxCells = 13824;   // 24 per coordinate; a block keeps two words per cell in shared memory
+constexpr int kMinCells = 64;      // fewer cells than this settle too few condensates per round: windows instead
 
-// Sorted position i takes hit perm[i]: coordinates shifted by the batch minimum of every dimension
-// (ccoords -= reduce_min(ccoords, axis=0)), distance over the threshold, mask, and the high-beta flag
-// (betas > beta_threshold or mask > 0).
-__global__ void gather_sorted_kernel(const float *__restrict__ ccoords, const float *__restrict__ betas,
-                                     const float *__restrict__ dist, const int *__restrict__ mask,
-                                     const int *__restrict__ perm, const GridParams *__restrict__ grid,
-                                     int dims, float distance_threshold, float beta_threshold,
-                                     float *__restrict__ s_ccoords, float *__restrict__ s_betas,
-                                     float *__restrict__ s_dist, int *__restrict__ s_mask,
-                                     int *__restrict__ high, int n)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int src = perm[i];
-    for (int c = 0; c < dims; c++)
-        s_ccoords[(size_t)i * dims + c] = __fsub_rn(ccoords[(size_t)src * dims + c], grid->all_min[c]);
-    const float b = betas[src];
-    const int m = mask ? mask[src] : 0;
-    s_betas[i] = b;
-    s_dist[i] = __fdiv_rn(dist[src], distance_threshold);
-    s_mask[i] = m;
-    high[i] = (b > beta_threshold || m > 0) ? 1 : 0;
-}
+typedef unsigned long long u64;
 
-// high_excl = exclusive prefix sum of the flags.  Writes indices_to_filtered, the filtered copies,
-// and the filtered row splits; total[0] = number of high-beta hits.
-__global__ void compact_high_kernel(const int *__restrict__ high_excl, const float *__restrict__ s_ccoords,
-                                    const float *__restrict__ s_betas, const float *__restrict__ s_dist,
-                                    const int *__restrict__ s_mask, const int *__restrict__ perm, int dims,
-                                    float beta_threshold, int *__restrict__ itf, float *__restrict__ h_ccoords,
-                                    float *__restrict__ h_betas, float *__restrict__ h_dist,
-                                    int *__restrict__ h_mask, int *__restrict__ h_orig, int n)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const bool is_high = s_betas[i] > beta_threshold || s_mask[i] > 0;
-    const int pos = high_excl[i];
-    itf[i] = is_high ? pos : -1;
-    if (!is_high) return;
-    for (int c = 0; c < dims; c++) h_ccoords[(size_t)pos * dims + c] = s_ccoords[(size_t)i * dims + c];
-    h_betas[pos] = s_betas[i];
-    h_dist[pos] = s_dist[i];
-    h_mask[pos] = s_mask[i];
-    h_orig[pos] = perm[i];
-}
-
-__global__ void filtered_row_splits_kernel(const int *__restrict__ high_excl, const float *__restrict__ s_betas,
-                                           const int *__restrict__ s_mask, float beta_threshold,
-                                           const int *__restrict__ row_splits, int n_rs, int n,
-                                           int *__restrict__ row_splits_h, int *__restrict__ total)
-{
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e > n_rs) return;
-    int all = 0;
-    if (n > 0) all = high_excl[n - 1] + ((s_betas[n - 1] > beta_threshold || s_mask[n - 1] > 0) ? 1 : 0);
-    if (e == n_rs) { total[0] = all; return; }
-    const int r = row_splits[e];
-    row_splits_h[e] = r >= n ? all : (r <= 0 ? 0 : high_excl[r]);
-}
-
-// Back to the caller's order: out[perm[i]] = sorted[i].
-__global__ void scatter_back_kernel(const int *__restrict__ s_assignment, const int *__restrict__ s_asso,
-                                    const int *__restrict__ perm, int *__restrict__ assignment,
-                                    int *__restrict__ asso, unsigned char *__restrict__ is_cond, int n)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int dst = perm[i];
-    assignment[dst] = s_assignment[i];
-    asso[dst] = s_asso[i];
-    is_cond[i] = 0;
-}
-
-// alpha_indices[alpha_indices != -1], and the flags of those hits.  Within an event's filtered range
-// the op lists the condensates first and pads with -1, so entry a of event e moves to
-// n_condensates[e] + (a - row_splits_h[e]).
-__global__ void compact_alpha_kernel(const int *__restrict__ alpha_h, const int *__restrict__ row_splits_h,
-                                     const int *__restrict__ n_condensates, int num_rows, int n_h_max,
-                                     const int *__restrict__ n_h_dev,
-                                     int *__restrict__ alpha_out, unsigned char *__restrict__ is_cond)
-{
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= min(n_h_max, *n_h_dev)) return;
-    const int id = alpha_h[a];
-    if (id < 0) return;
-    int lo = 1, hi = num_rows + 1;  // event = number of row_splits_h[1..num_rows] that are <= a
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (row_splits_h[mid] <= a) lo = mid + 1; else hi = mid;
-    }
-    const int e = lo - 1;
-    alpha_out[n_condensates[e] + (a - row_splits_h[e])] = id;
-    is_cond[id] = 1;
-}
-
-__global__ void fill_minus_one_kernel(int *__restrict__ p, int n)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = -1;
-}
-
-struct Plan {
-    int cb;
-    long long max_bins;
-    int n_bins_sc;
+// Grid over the condensates: cells at least as wide as the largest radius, over up to three coordinates.
+struct CondGrid {
+    int dims;        // gridded coordinates, 1 .. 3
+    int n[3];        // cells per coordinate (1 beyond dims)
+    float inv[3];    // cells per unit
 };
 
-// n_bins_sc of the wrapper (assign_condensate_op.py:265-266) and an upper bound on the grid's size.
+struct Plan {
+    int cb;             // binned dimensions
+    int bin_passes;     // 8-bit digits of a bin number inside an event
+    int n_bins_sc;
+    int cells;          // upper bound on the grid cells per event
+    int cells_per_dim;
+    int max_settled;    // upper bound on cells of which no two touch
+};
+
+struct Buffers {
+    // zeroed together with the status word
+    int *tile_hist;       // [pass][tile][256]
+    int *event_hist;      // [pass][event][256]
+    int *count;           // [num_rows] condensates
+    int *cell_count;      // [num_rows][cells + 1]
+    unsigned *max_radius; // [1] bits of the largest radius
+    // not zeroed
+    HitOrder layout;      // only grid, partial and the event layout
+    int *use_grid;        // [1]
+    u64 *first_two;       // [2] smallest (bin, hit) keys of the high-beta hits
+    int *tile_count, *row_splits_h;
+    u64 *key[2];
+    int *val[2];
+    int *order;
+    float *h_ccoords, *h_dist;
+    int *h_mask, *h_orig, *status_h;
+    float4 *p_rec;        // high-beta hits in priority order
+    int *p_flag;          // their masks' signs (1: condensate that covers nothing, -1: cannot be covered), then their cells
+    unsigned *open, *bitmap;
+    CondList cl;
+    int *alpha_h, *stage;
+    float4 *c_rec;        // condensates by cell
+    int *c_rank;
+};
+
+__device__ __forceinline__ CondGrid make_cond_grid(const GridParams *__restrict__ g, const unsigned *__restrict__ max_radius,
+                                                   int dims, int cells_per_dim)
+{
+    // cells a little wider than the largest radius, so that what a condensate covers is at most one cell away whatever
+    // the rounding
+    const float width = __uint_as_float(*max_radius) * 1.001f;
+    CondGrid c;
+    c.dims = dims < 3 ? dims : 3;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        c.n[d] = 1;
+        c.inv[d] = 0.f;
+        if (d < c.dims) {
+            const float ext = g->range[d];
+            const float w = fmaxf(width, ext / (float)cells_per_dim);
+            if (ext > 0.f && w < ext) {
+                c.inv[d] = 1.f / w;
+                c.n[d] = min((int)(ext * c.inv[d]) + 1, cells_per_dim);
+            }
+        }
+    }
+    return c;
+}
+
+template <int NR>
+__device__ __forceinline__ void cell_of(const CondGrid &c, const Rec<NR> &x, int (&at)[3])
+{
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+        at[d] = d < rec_dims<NR>() ? min(max((int)(x.v[d] * c.inv[d]), 0), c.n[d] - 1) : 0;
+}
+
+// A hit is high if its beta is above the threshold or its mask is positive.
+__device__ __forceinline__ bool is_high(const float *__restrict__ betas, const int *__restrict__ mask, int v, float threshold)
+{
+    return betas[v] > threshold || (mask && mask[v] > 0);
+}
+
+__device__ __forceinline__ unsigned bin_of(const float *__restrict__ ccoords, int dims, int cb, const GridParams *__restrict__ g,
+                                           int v, unsigned *status)
+{
+    // as modules/compiled/bin_by_coordinates_kernel.cc:64-113
+    unsigned flat = 0u;
+    int stride = 1;
+    for (int c = cb - 1; c >= 0; c--) {
+        int ci = __float2int_rz(__fdiv_rn(__fsub_rn(ccoords[(size_t)v * dims + c], g->shift[c]), g->bin_width));
+        const int nb = g->n_bins[c];
+        if (ci < 0 || ci >= nb) {
+            ci = 0;
+            flag_status(status, HGC_STATUS_BIN_OUT_OF_RANGE);
+        }
+        flat += (unsigned)(ci * stride);
+        stride *= nb;
+    }
+    return flat;
+}
+
+// High-beta hits of every tile; initial values of the outputs that later kernels fill in places.
+__global__ void __launch_bounds__(kThreads)
+count_high_kernel(const float *__restrict__ betas, const int *__restrict__ mask, float beta_threshold, HitOrder o,
+                  int n_events, int *__restrict__ tile_count, int *__restrict__ alpha_out, unsigned char *__restrict__ is_cond,
+                  u64 *__restrict__ first_two)
+{
+    HitTile t;
+    if (!find_tile(o, n_events, blockIdx.x, &t)) return;
+    if (blockIdx.x == 0 && threadIdx.x < 2) first_two[threadIdx.x] = ~0ull;
+    __shared__ int s_warp[kWarps];
+    int n = 0;
+    for (int i = threadIdx.x; i < t.n; i += kThreads) {
+        const int v = t.first + i;
+        n += t.event < n_events && is_high(betas, mask, v, beta_threshold) ? 1 : 0;
+        alpha_out[v] = -1;
+        is_cond[v] = 0;
+    }
+    n = __reduce_add_sync(0xffffffffu, n);
+    if ((threadIdx.x & 31) == 0) s_warp[threadIdx.x >> 5] = n;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kWarps; w++) n += s_warp[w];
+        tile_count[blockIdx.x] = n;
+    }
+}
+
+// The first (SECOND: the second) high-beta hit of the batch in the order by bin.  Only run when there is a mask: the
+// reference's pick loop tests no_condensation_mask_h at index 0 or 1 of that order instead of at the hit
+// (binned_assign_to_condensates_kernel.cc:193).
+template <bool SECOND>
+__global__ void __launch_bounds__(kThreads)
+first_high_kernel(const float *__restrict__ ccoords, const float *__restrict__ betas, const int *__restrict__ mask,
+                  float beta_threshold, int dims, int cb, HitOrder o, int n_events, u64 *__restrict__ first_two)
+{
+    HitTile t;
+    if (!find_tile(o, n_events, blockIdx.x, &t) || t.event >= n_events) return;
+    const u64 first = SECOND ? first_two[0] : 0ull;
+    for (int i = threadIdx.x; i < t.n; i += kThreads) {
+        const int v = t.first + i;
+        if (!is_high(betas, mask, v, beta_threshold)) continue;
+        const u64 flat = (u64)t.event * (unsigned)o.grid->bins_per_event + bin_of(ccoords, dims, cb, o.grid, v, nullptr);
+        const u64 key = flat << 31 | (unsigned)v;
+        if (!SECOND || key > first) atomicMin(first_two + (SECOND ? 1 : 0), key);
+    }
+}
+
+// Packs the high-beta hits of every event (in the caller's order) with what the claim pass needs and their sort keys:
+// beta in the high word, bin in the low one.
+__global__ void __launch_bounds__(kThreads)
+order_high_kernel(const float *__restrict__ ccoords, const float *__restrict__ betas, const float *__restrict__ dist,
+                  const int *__restrict__ mask, float beta_threshold, float distance_threshold, int dims, int cb,
+                  int bin_passes, int n_events, Buffers b, unsigned *status)
+{
+    extern __shared__ int s_hist[];  // [passes][256]
+    __shared__ int s_warp[kWarps];
+    __shared__ int s_base;
+    const HitOrder &o = b.layout;
+    const int n_tiles = o.event_tile[n_events + 1], passes = bin_passes + 4;
+    if (blockIdx.x == 0) {
+        // row splits of the packed hits
+        int carry = 0;
+        for (int base = 0; base < n_tiles; base += kThreads) {
+            const int q = base + threadIdx.x;
+            const int n = q < n_tiles ? b.tile_count[q] : 0;
+            const int incl = carry + block_scan_inclusive(n, [](int x, int y) { return x + y; }, 0, s_warp);
+            if (q < n_tiles) b.stage[q] = incl;
+            __syncthreads();
+            if (threadIdx.x == kThreads - 1) s_base = incl;
+            __syncthreads();
+            carry = s_base;
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e <= n_events; e += kThreads) {
+            const int q = o.event_tile[e];
+            b.row_splits_h[e] = q > 0 ? b.stage[q - 1] : 0;
+        }
+        __syncthreads();
+    }
+    HitTile t;
+    if (!find_tile(o, n_events, blockIdx.x, &t) || t.event >= n_events) return;
+    int before = 0, event_start = 0;
+    const int tile0 = o.event_tile[t.event];
+    for (int q = threadIdx.x; q < (int)blockIdx.x; q += kThreads) {
+        const int n = b.tile_count[q];
+        before += n;
+        event_start += q < tile0 ? n : 0;
+    }
+    __shared__ int s_sum[2];
+    if (threadIdx.x < 2) s_sum[threadIdx.x] = 0;
+    for (int i = threadIdx.x; i < passes * 256; i += kThreads) s_hist[i] = 0;
+    __syncthreads();
+    before = __reduce_add_sync(0xffffffffu, before);
+    event_start = __reduce_add_sync(0xffffffffu, event_start);
+    if ((threadIdx.x & 31) == 0) { atomicAdd(&s_sum[0], before); atomicAdd(&s_sum[1], event_start); }
+    __syncthreads();
+    int run = s_sum[0];
+    const int start = s_sum[1];
+    float radius_max = 0.f;
+    for (int r = 0; r < kRounds; r++) {
+        if (r * kThreads >= t.n) break;  // uniform
+        const int i = r * kThreads + threadIdx.x, v = t.first + i;
+        const bool high = i < t.n && is_high(betas, mask, v, beta_threshold);
+        const int incl = block_scan_inclusive(high ? 1 : 0, [](int x, int y) { return x + y; }, 0, s_warp);
+        if (high) {
+            const int a = run + incl - 1;
+            const int m = mask ? mask[v] : 0;
+            const float radius = __fdiv_rn(dist[v], distance_threshold);
+            for (int c = 0; c < dims; c++)
+                b.h_ccoords[(size_t)a * dims + c] = __fsub_rn(ccoords[(size_t)v * dims + c], o.grid->all_min[c]);
+            b.h_dist[a] = radius;
+            b.h_mask[a] = m;
+            b.h_orig[a] = v;
+            b.status_h[a] = 0;
+            if (m <= 0) radius_max = fmaxf(radius_max, fabsf(radius));
+            bool flagged = false;
+            if (mask) {
+                const int id0 = (int)(b.first_two[0] & 0x7fffffffull), id1 = (int)(b.first_two[1] & 0x7fffffffull);
+                flagged = mask[v == id0 ? id0 : id1] != 0;  // there is a second one when v is not the first
+            }
+            const u64 key = (u64)priority_key(betas[v], flagged) << 32 | bin_of(ccoords, dims, cb, o.grid, v, status);
+            b.key[0][a] = key;
+            for (int p = 0; p < passes; p++) {
+                const int shift = p < bin_passes ? 8 * p : 32 + 8 * (p - bin_passes);
+                atomicAdd(&s_hist[p * 256 + (int)((key >> shift) & 255u)], 1);
+            }
+            // the packed hits make tiles of their own
+            atomicAdd(&b.tile_hist[(size_t)(tile0 + (a - start) / kOrderTile) * 256 + (int)(key & 255u)], 1);
+        }
+        __syncthreads();
+        if (threadIdx.x == kThreads - 1) s_base = incl;
+        __syncthreads();
+        run += s_base;
+    }
+    radius_max = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(radius_max)));
+    if ((threadIdx.x & 31) == 0 && radius_max > 0.f) atomicMax(b.max_radius, __float_as_uint(radius_max));
+    __syncthreads();
+    for (int p = 0; p < passes; p++) {
+        const int c = s_hist[p * 256 + threadIdx.x];
+        if (c) atomicAdd(&b.event_hist[((size_t)p * (n_events + 1) + t.event) * 256 + threadIdx.x], c);
+    }
+}
+
+// One pass of the stable sort of the packed hits, event by event (see hit_order.cu).  The last pass (NR > 0) writes the
+// order, and the hits' records in that order.
+template <bool FIRST, int NR>
+__global__ void __launch_bounds__(kThreads)
+order_pass_kernel(Buffers b, int n_events, int tiles_cap, int pass, int shift, int next_shift, int dims)
+{
+    __shared__ int s_count[kWarps][256];
+    __shared__ int s_warp[kWarps];
+    const HitOrder &o = b.layout;
+    if ((int)blockIdx.x >= o.event_tile[n_events]) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d = threadIdx.x;
+    const int e = event_of_tile(o.event_tile, n_events, blockIdx.x);
+    const int off = b.row_splits_h[e], n_h = b.row_splits_h[e + 1] - off;
+    const int local = ((int)blockIdx.x - o.event_tile[e]) * kOrderTile;
+    const int n = min(n_h - local, kOrderTile);
+    if (n <= 0) return;
+    const u64 *__restrict__ key_in = b.key[pass & 1] + off + local;
+    const int *__restrict__ val_in = b.val[pass & 1] + off + local;
+    u64 key[kRounds];
+    int val[kRounds];
+    const int warp_base = warp * (kRounds * kWarp);
+#pragma unroll
+    for (int r = 0; r < kRounds; r++) {
+        const int i = warp_base + r * kWarp + lane;
+        key[r] = i < n ? key_in[i] : 0ull;
+        val[r] = FIRST ? off + local + i : i < n ? val_in[i] : 0;
+    }
+    int start = off;
+    {
+        const int mine = b.event_hist[((size_t)pass * (n_events + 1) + e) * 256 + d];
+        start += block_scan_inclusive(mine, [](int x, int y) { return x + y; }, 0, s_warp) - mine;
+        const int *__restrict__ h = b.tile_hist + (size_t)pass * tiles_cap * 256 + d;
+        int sum = 0;
+#pragma unroll 8
+        for (int q = o.event_tile[e]; q < (int)blockIdx.x; q++) sum += h[(size_t)q * 256];
+        start += sum;
+    }
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) s_count[w][d] = 0;
+    unsigned peers[kRounds];
+#pragma unroll
+    for (int r = 0; r < kRounds; r++) {
+        const unsigned dg = warp_base + r * kWarp + lane < n ? (unsigned)(key[r] >> shift) & 255u : 256u;
+        peers[r] = __match_any_sync(0xffffffffu, dg);
+    }
+    __syncthreads();
+    int place[kRounds];
+#pragma unroll
+    for (int r = 0; r < kRounds; r++) {
+        const bool ok = warp_base + r * kWarp + lane < n;
+        const unsigned dg = (unsigned)(key[r] >> shift) & 255u, before = peers[r] & ((1u << lane) - 1u);
+        const int seen = ok ? s_count[warp][dg] : 0;
+        place[r] = seen + __popc(before);
+        __syncwarp();
+        if (ok && before == 0u) s_count[warp][dg] = seen + __popc(peers[r]);
+        __syncwarp();
+    }
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kWarps; w++) {
+        const int c = s_count[w][d];
+        s_count[w][d] = start;
+        start += c;
+    }
+    __syncthreads();
+    int *__restrict__ next_hist = b.tile_hist + (size_t)(pass + 1) * tiles_cap * 256;
+    const int tile0 = o.event_tile[e];
+#pragma unroll
+    for (int r = 0; r < kRounds; r++) {
+        if (warp_base + r * kWarp + lane < n) {
+            const int dst = s_count[warp][(unsigned)(key[r] >> shift) & 255u] + place[r];
+            if constexpr (NR > 0) {
+                const int a = val[r], m = b.h_mask[a];
+                b.order[dst] = a;
+                Rec<NR> x;
+#pragma unroll
+                for (int c = 0; c < NR * 4; c++) x.v[c] = 0.f;
+#pragma unroll
+                for (int c = 0; c < rec_dims<NR>(); c++)
+                    if (c < dims) x.v[c] = b.h_ccoords[(size_t)a * dims + c];
+                x.v[rec_r2_slot<NR>()] = __fmul_rn(b.h_dist[a], b.h_dist[a]);
+                store_rec<NR>(b.p_rec + (size_t)dst * NR, x);
+                b.p_flag[dst] = (m > 0) - (m < 0);
+            } else {
+                b.key[(pass + 1) & 1][dst] = key[r];
+                b.val[(pass + 1) & 1][dst] = val[r];
+                const int q = tile0 + (dst - off) / kOrderTile;
+                atomicAdd(&next_hist[(size_t)q * 256 + ((unsigned)(key[r] >> next_shift) & 255u)], 1);
+            }
+        }
+    }
+}
+
+// Which of the high-beta hits are condensates: those that no condensate earlier in the priority order covers.  A cluster
+// of 8 blocks per event, in rounds.  A hit that comes first among the open hits of its own cell and of the cells around
+// it cannot be covered by an open one, so the first open hits of all cells that are first among their neighbours are
+// settled together; then every open hit that one of them covers is closed.  500 blobs on 2700 cells take about 13
+// rounds.  Masked hits (mask > 0) are condensates from the start: nothing covers them and they cover nothing; hits with a
+// negative mask cover others but are not covered.
+//
+// Everything a round looks up is in shared memory: every block keeps the first open hit of every cell among its own hits,
+// the blocks merge those tables (an eighth of the cells each) through distributed shared memory, and every block works
+// out for itself which are settled and copies their records.  A round is two cluster barriers.  With the tables and
+// records in L2 a round took 24 us, most of it in dependent loads, before (64k open hits per event).
+// A round costs that much however many hits it settles, so a grid of few cells (a radius that spans the event) is
+// left to the windows of claim_kernel.
+template <int NR>
+__global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(kClaimThreads)
+claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max_settled)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    extern __shared__ int s_dyn[];
+    __shared__ int s_left[2][kClusterBlocks];
+    __shared__ int s_count, s_sum;
+    int *s_best = s_dyn, *s_min = s_dyn + cells_cap;               // cells_cap is a multiple of 4
+    float4 *s_rec = reinterpret_cast<float4 *>(s_min + cells_cap);  // [max_settled][NR]
+    int *s_pos = reinterpret_cast<int *>(s_rec + (size_t)max_settled * NR);
+    const CondGrid grid = make_cond_grid(b.layout.grid, b.max_radius, dims, cells_per_dim);
+    const int n_cells = grid.n[0] * grid.n[1] * grid.n[2];
+    const bool use = n_cells >= kMinCells;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *b.use_grid = use ? 1 : 0;
+    if (!use) return;  // the same in every block
+    constexpr int U = NR == 1 ? 4 : NR == 2 ? 2 : 1;  // hits whose data is requested together
+    constexpr int kFree = 0x7fffffff;
+    const int e = blockIdx.x / kClusterBlocks, t = threadIdx.x, lane = t & 31;
+    const int rank = (int)cluster.block_rank();
+    const int g = rank * kClaimThreads + t;
+    const int off = b.row_splits_h[e], n_h = b.row_splits_h[e + 1] - off;
+    const int n_steps = (n_h + kClaimStep - 1) / kClaimStep;
+    const int word0 = off / 32 + e;
+    const float4 *__restrict__ recs = b.p_rec + (size_t)off * NR;
+    int *__restrict__ cells = b.p_flag + off;
+    unsigned *__restrict__ open_words = b.open + (size_t)word0 * 32 + g;  // word w of this thread: [w * kClaimStep], w > 0
+
+    for (int c = t; c < n_cells; c += kClaimThreads) s_best[c] = kFree;
+    if (t == 0) s_count = s_sum = 0;
+    // this thread's hits are p = k * kClaimStep + g; 32 of them share a word of open bits, kept in memory beyond the first
+    unsigned open0 = 0u;
+    int n_mine = 0;  // condensates among them
+    for (int k = 0; k < n_steps; k++) {
+        const int p = k * kClaimStep + g;
+        bool is_open = false, lonely = false;
+        if (p < n_h) {
+            const int flag = cells[p];
+            const Rec<NR> x = load_rec<NR>(recs + (size_t)p * NR);
+            int at[3];
+            cell_of<NR>(grid, x, at);
+            // cell coordinates in 8 bits each (7 for the first); the sign bit: cannot be covered
+            cells[p] = at[0] << 16 | at[1] << 8 | at[2] | (flag != 0 ? (int)0x80000000 : 0);
+            lonely = flag > 0;
+            is_open = !lonely;
+        }
+        if ((k & 31) == 0 && k > 0) open_words[(size_t)(k / 32) * kClaimStep] = 0u;
+        if (is_open) {
+            if (k < 32) open0 |= 1u << k;
+            else open_words[(size_t)(k / 32) * kClaimStep] |= 1u << (k & 31);
+        }
+        n_mine += lonely ? 1 : 0;
+        const unsigned bits = __ballot_sync(0xffffffffu, lonely);
+        if (lane == 0 && p < n_h) b.bitmap[word0 + p / 32] = bits;
+    }
+    __syncthreads();
+    auto flat = [&grid](int at) { return (((at >> 16) & 127) * grid.n[1] + ((at >> 8) & 255)) * grid.n[2] + (at & 255); };
+    const int slice = (n_cells + kClusterBlocks - 1) / kClusterBlocks;
+
+    for (int round = 0; round <= n_h; round++) {
+        // first open hit of every cell, among this block's
+        for (int w = 0; w * 32 < n_steps; w++) {
+            unsigned u = w == 0 ? open0 : open_words[(size_t)w * kClaimStep];
+            while (u) {
+                int p[U], at[U];
+#pragma unroll
+                for (int q = 0; q < U; q++) {
+                    p[q] = u ? (w * 32 + __ffs(u) - 1) * kClaimStep + g : -1;
+                    u &= u - 1u;
+                }
+#pragma unroll
+                for (int q = 0; q < U; q++) at[q] = p[q] >= 0 ? cells[p[q]] : 0;
+#pragma unroll
+                for (int q = 0; q < U; q++)
+                    if (p[q] >= 0) {
+                        const int c = flat(at[q]);
+                        if (s_best[c] > p[q]) atomicMin(s_best + c, p[q]);
+                    }
+            }
+        }
+        cluster.sync();
+        if (round > 0) {
+            int total = 0;
+#pragma unroll
+            for (int r = 0; r < kClusterBlocks; r++) total += s_left[(round - 1) & 1][r];
+            if (total == 0) break;  // the same in every block of the cluster; nobody looks at another block from here on
+        }
+        // merged, for all blocks
+        for (int c = rank * slice + t; c < min((rank + 1) * slice, n_cells); c += kClaimThreads) {
+            int v[kClusterBlocks], m = kFree;
+#pragma unroll
+            for (int r = 0; r < kClusterBlocks; r++) v[r] = *cluster.map_shared_rank(s_best + c, r);
+#pragma unroll
+            for (int r = 0; r < kClusterBlocks; r++) m = min(m, v[r]);
+#pragma unroll
+            for (int r = 0; r < kClusterBlocks; r++) *cluster.map_shared_rank(s_min + c, r) = m;
+        }
+        cluster.sync();
+        // which of them are first among the cells around
+        for (int c = t; c < n_cells; c += kClaimThreads) {
+            const int p = s_min[c];
+            int settled = -1;
+            if (p != kFree) {
+                const int z = c % grid.n[2], y = c / grid.n[2] % grid.n[1], x = c / (grid.n[2] * grid.n[1]);
+                bool first = true;
+                for (int i = max(x - 1, 0); i <= min(x + 1, grid.n[0] - 1); i++)
+                    for (int j = max(y - 1, 0); j <= min(y + 1, grid.n[1] - 1); j++)
+                        for (int l = max(z - 1, 0); l <= min(z + 1, grid.n[2] - 1); l++)
+                            first = first && s_min[(i * grid.n[1] + j) * grid.n[2] + l] >= p;
+                if (first) {
+                    settled = atomicAdd(&s_count, 1);  // in any order
+                    s_pos[settled] = p;
+                    store_rec<NR>(s_rec + (size_t)settled * NR, load_rec<NR>(recs + (size_t)p * NR));
+                }
+            }
+            s_best[c] = settled;
+        }
+        __syncthreads();
+        // and, for every cell, which of the 27 cells around it hold one (no two next to each other do)
+        for (int c = t; c < n_cells; c += kClaimThreads) {
+            const int z = c % grid.n[2], y = c / grid.n[2] % grid.n[1], x = c / (grid.n[2] * grid.n[1]);
+            int near_ = 0;
+#pragma unroll
+            for (int k = 0; k < 27; k++) {
+                const int i = x + k / 9 - 1, j = y + k / 3 % 3 - 1, l = z + k % 3 - 1;
+                if (i >= 0 && i < grid.n[0] && j >= 0 && j < grid.n[1] && l >= 0 && l < grid.n[2] &&
+                    s_best[(i * grid.n[1] + j) * grid.n[2] + l] >= 0)
+                    near_ |= 1 << k;
+            }
+            s_min[c] = near_;
+        }
+        __syncthreads();
+        // close them and what they cover
+        int left = 0;
+        for (int w = 0; w * 32 < n_steps; w++) {
+            unsigned word = w == 0 ? open0 : open_words[(size_t)w * kClaimStep], u = word;
+            while (u) {
+                int bit[U], at[U], near_[U];
+                Rec<NR> mine[U];
+#pragma unroll
+                for (int q = 0; q < U; q++) {
+                    bit[q] = u ? __ffs(u) - 1 : -1;
+                    u &= u - 1u;
+                }
+#pragma unroll
+                for (int q = 0; q < U; q++) at[q] = bit[q] >= 0 ? cells[(w * 32 + bit[q]) * kClaimStep + g] : 0;
+#pragma unroll
+                for (int q = 0; q < U; q++) {
+                    near_[q] = bit[q] >= 0 ? s_min[flat(at[q])] : 0;
+                    if (near_[q]) mine[q] = load_rec<NR>(recs + (size_t)((w * 32 + bit[q]) * kClaimStep + g) * NR);
+                }
+#pragma unroll
+                for (int q = 0; q < U; q++) {
+                    if (near_[q] == 0) continue;
+                    const int p = (w * 32 + bit[q]) * kClaimStep + g;
+                    const int x = (at[q] >> 16) & 127, y = (at[q] >> 8) & 255, z = at[q] & 255;
+                    bool stays = true;
+                    if ((near_[q] >> 13) & 1) {  // one in its own cell
+                        if (s_pos[s_best[flat(at[q])]] == p) {
+                            atomicOr(b.bitmap + word0 + p / 32, 1u << (p & 31));
+                            n_mine++;
+                            stays = false;
+                        }
+                    }
+                    if (at[q] >= 0)
+                        for (int m = near_[q]; m && stays; m &= m - 1) {
+                            const int k = __ffs(m) - 1;
+                            const int s = s_best[((x + k / 9 - 1) * grid.n[1] + y + k / 3 % 3 - 1) * grid.n[2] + z + k % 3 - 1];
+                            const Rec<NR> c = load_rec<NR>(s_rec + (size_t)s * NR);
+                            if (rec_distsq<NR>(c, mine[q], dims) <= c.v[rec_r2_slot<NR>()]) stays = false;
+                        }
+                    if (!stays) word &= ~(1u << bit[q]);
+                }
+            }
+            if (w == 0) open0 = word;
+            else open_words[(size_t)w * kClaimStep] = word;
+            left += __popc(word);
+        }
+        left = __reduce_add_sync(0xffffffffu, left);
+        if (lane == 0 && left) atomicAdd(&s_sum, left);
+        __syncthreads();
+        if (t < kClusterBlocks) *cluster.map_shared_rank(&s_left[round & 1][rank], t) = s_sum;
+        for (int c = t; c < n_cells; c += kClaimThreads) s_best[c] = kFree;
+        if (t == 0) s_count = 0;
+        __syncthreads();
+        if (t == 0) s_sum = 0;  // added to again only after the next cluster barriers
+    }
+    n_mine = __reduce_add_sync(0xffffffffu, n_mine);
+    if (lane == 0 && n_mine) atomicAdd(b.count + e, n_mine);
+}
+
+// Lists of an event's condensates: in priority order (alpha_idx, flags, the rank of masked ones) and by grid cell.
+template <int NR>
+__global__ void __launch_bounds__(1024)
+list_condensates_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int *__restrict__ n_condensates,
+                        int *__restrict__ alpha_out, unsigned char *__restrict__ is_cond, int *__restrict__ assignment)
+{
+    __shared__ int s_warp[32];
+    __shared__ int s_base, s_before;
+    const int e = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const CondGrid grid = make_cond_grid(b.layout.grid, b.max_radius, dims, cells_per_dim);
+    const int n_cells = grid.n[0] * grid.n[1] * grid.n[2];
+    const bool by_grid = *b.use_grid != 0;
+    const int off = b.row_splits_h[e], n_h = b.row_splits_h[e + 1] - off;
+    const int word0 = off / 32 + e;
+    int *__restrict__ cell_start = b.cell_count + (size_t)e * (cells_cap + 1);
+    auto block_scan = [&](int v) {  // inclusive, over 1024 threads
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += x;
+        }
+        __syncthreads();
+        if (lane == 31) s_warp[warp] = v;
+        __syncthreads();
+        int w = s_warp[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += x;
+        }
+        const int before = __shfl_sync(0xffffffffu, w, warp > 0 ? warp - 1 : 0);
+        return v + (warp > 0 ? before : 0);
+    };
+    // condensates of the events before
+    int before = 0;
+    for (int q = t; q < e; q += 1024) before += b.count[q];
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (t == 0) s_before = 0;
+    __syncthreads();
+    if (lane == 0) atomicAdd(&s_before, before);
+    __syncthreads();
+    before = s_before;
+
+    auto cell_at = [&](int a, Rec<NR> *x) {  // -1: covers nothing
+#pragma unroll
+        for (int d = 0; d < NR * 4; d++) x->v[d] = 0.f;
+#pragma unroll
+        for (int d = 0; d < rec_dims<NR>(); d++)
+            if (d < dims) x->v[d] = b.h_ccoords[(size_t)a * dims + d];
+        x->v[rec_r2_slot<NR>()] = __fmul_rn(b.h_dist[a], b.h_dist[a]);
+        int at[3];
+        cell_of<NR>(grid, *x, at);
+        return b.h_mask[a] > 0 ? -1 : (at[0] * grid.n[1] + at[1]) * grid.n[2] + at[2];
+    };
+    int carry = 0;
+    const int n_words = (n_h + 31) / 32;
+    for (int base = 0; base < n_words; base += 1024) {
+        const int w = base + t;
+        unsigned bits = 0u;
+        if (w < n_words) {
+            if (by_grid) {
+                bits = b.bitmap[word0 + w];
+            } else {
+                for (int i = 0; i < 32; i++)
+                    if (w * 32 + i < n_h && b.status_h[b.order[off + w * 32 + i]]) bits |= 1u << i;
+            }
+        }
+        const int incl = block_scan(__popc(bits));
+        int r = carry + incl - __popc(bits);
+        for (; bits; bits &= bits - 1u, r++) b.cl.subset_pos[off + r] = b.order[off + w * 32 + __ffs(bits) - 1];
+        __syncthreads();
+        if (t == 1023) s_base = carry + incl;
+        __syncthreads();
+        carry = s_base;
+    }
+    const int n_cond = carry;
+    if (t == 0) {
+        if (e == 0) n_condensates[0] = 0;
+        n_condensates[e + 1] = before + n_cond;
+    }
+    for (int r = t; r < n_cond; r += 1024) {
+        const int a = b.cl.subset_pos[off + r], id = b.h_orig[a];
+        alpha_out[before + r] = id;
+        is_cond[id] = 1;
+        Rec<NR> x;
+        const int cell = cell_at(a, &x);
+        if (cell >= 0) atomicAdd(cell_start + cell, 1);
+        else assignment[id] = r;  // a masked hit is assigned to itself: picked up by assign_hits_kernel
+    }
+    __syncthreads();
+    carry = 0;
+    for (int base = 0; base <= n_cells; base += 1024) {
+        const int c = base + t;
+        const int n = c < n_cells ? __ldcg(cell_start + c) : 0;
+        const int incl = block_scan(n);
+        if (c <= n_cells) cell_start[c] = carry + incl;  // end of the cell: filling counts down to its start
+        __syncthreads();
+        if (t == 1023) s_base = carry + incl;
+        __syncthreads();
+        carry = s_base;
+    }
+    for (int r = t; r < n_cond; r += 1024) {
+        Rec<NR> x;
+        const int cell = cell_at(b.cl.subset_pos[off + r], &x);
+        if (cell < 0) continue;
+        const int at = atomicSub(cell_start + cell, 1) - 1;
+        store_rec<NR>(b.c_rec + (size_t)(off + at) * NR, x);
+        b.c_rank[off + at] = r;
+    }
+}
+
+// Every hit against the condensates of the cells around it.  Of those that cover it the first in priority order wins
+// (by_max_beta), or the reference's distance fold is applied to them in priority order
+// (binned_assign_to_condensates_kernel.cc:80-125).  A masked hit is only ever assigned to itself.
+template <int NR>
+__global__ void __launch_bounds__(kThreads)
+assign_hits_kernel(Buffers b, const float *__restrict__ ccoords, const int *__restrict__ mask, int dims, int n_events,
+                   int cells_cap, int cells_per_dim, bool by_max_beta, int *assignment, int *__restrict__ association,
+                   const unsigned char *__restrict__ is_cond, const int *__restrict__ n_condensates,
+                   const int *__restrict__ alpha)
+{
+    HitTile t;
+    if (!find_tile(b.layout, n_events, blockIdx.x / kRounds, &t)) return;
+    const int i = (blockIdx.x % kRounds) * kThreads + threadIdx.x;
+    if (i >= t.n) return;
+    const CondGrid grid = make_cond_grid(b.layout.grid, b.max_radius, dims, cells_per_dim);
+    const bool real = t.event < n_events;
+    const int off = real ? b.row_splits_h[t.event] : 0, first_alpha = real ? n_condensates[t.event] : 0;
+    const int n_cond = real ? n_condensates[t.event + 1] - first_alpha : 0;
+    const int *__restrict__ cell_start = b.cell_count + (size_t)(real ? t.event : 0) * (cells_cap + 1);
+    const int v = t.first + i;
+    int found = -1;
+    if (n_cond > 0) {
+        const int m = mask ? mask[v] : 0;
+        if (m != 0) {
+            if (m > 0 && is_cond[v]) found = assignment[v];  // its own rank
+        } else {
+            Rec<NR> x;
+#pragma unroll
+            for (int d = 0; d < NR * 4; d++) x.v[d] = 0.f;
+#pragma unroll
+            for (int d = 0; d < rec_dims<NR>(); d++)
+                if (d < dims) x.v[d] = __fsub_rn(ccoords[(size_t)v * dims + d], b.layout.grid->all_min[d]);
+            int at[3];
+            cell_of<NR>(grid, x, at);
+            const int lo2 = max(at[2] - 1, 0), hi2 = min(at[2] + 1, grid.n[2] - 1);
+            // cells along the last coordinate follow each other: nine ranges of the list, requested together
+            int begin[9], end[9];
+#pragma unroll
+            for (int k = 0; k < 9; k++) {
+                const int p = at[0] + k / 3 - 1, q = at[1] + k % 3 - 1;
+                begin[k] = end[k] = 0;
+                if (p >= 0 && p < grid.n[0] && q >= 0 && q < grid.n[1]) {
+                    const int *row = cell_start + (p * grid.n[1] + q) * grid.n[2];
+                    begin[k] = __ldg(row + lo2);
+                    end[k] = __ldg(row + hi2 + 1);
+                }
+            }
+            float min_distance = 10e20f;
+            int last = -1;
+            for (;;) {
+                // first condensate after `last` that covers the hit, and whether there are more
+                int next = 0x7fffffff, n_after = 0;
+                float next_dsq = 0.f, next_r2 = 0.f;
+#pragma unroll
+                for (int w = 0; w < 9; w++)
+                    for (int k = begin[w]; k < end[w]; k++) {
+                        const Rec<NR> c = load_rec<NR>(b.c_rec + (size_t)(off + k) * NR);
+                        const float dsq = rec_distsq<NR>(c, x, dims), r2 = c.v[rec_r2_slot<NR>()];
+                        if (!(dsq <= r2)) continue;
+                        const int rank = __ldg(b.c_rank + off + k);
+                        if (rank <= last) continue;
+                        n_after++;
+                        if (rank < next) { next = rank; next_dsq = dsq; next_r2 = r2; }
+                    }
+                if (n_after == 0) break;
+                if (by_max_beta) { found = next; break; }
+                if (__fmul_rn(min_distance, next_r2) >= next_dsq) { found = next; min_distance = next_dsq; }
+                if (n_after == 1) break;
+                last = next;
+            }
+        }
+    }
+    assignment[v] = found;
+    association[v] = found >= 0 ? alpha[first_alpha + found] : -1;
+}
+
+// n_bins_sc of the wrapper (assign_condensate_op.py:265-266), sort passes and grid size.
 bool make_plan(int n_vert, int dims, int nbin_dims, int n_rs, Plan *p)
 {
     p->cb = dims < nbin_dims ? dims : nbin_dims;
@@ -128,83 +774,117 @@ bool make_plan(int n_vert, int dims, int nbin_dims, int n_rs, Plan *p)
     nb = nb > 25 ? 25 : nb;
     nb = nb < 4 ? 4 : nb;
     p->n_bins_sc = nb;
-    long long b = n_rs > 1 ? n_rs - 1 : 1;
-    for (int d = 0; d < p->cb; d++) {
-        b *= nb + 1;
-        if (b > (1LL << 30)) return false;
-    }
-    p->max_bins = b;
+    long long b = 1;
+    for (int d = 0; d < p->cb; d++) b *= nb + 1;
+    if (b * (n_rs > 1 ? n_rs - 1 : 1) > (1LL << 30)) return false;
+    p->bin_passes = (bits_for(b - 1) + 7) / 8;
+    // as many cells as an average event has hits, within limits
+    long long cells = n_rs > 1 ? n_vert / (n_rs - 1) : n_vert;
+    cells = cells < 4 * kMinCells ? 4 * kMinCells : cells > kMaxCells ? kMaxCells : cells;
+    const int gd = dims < 3 ? dims : 3;
+    auto power = [gd](long long x) { return gd == 1 ? x : gd == 2 ? x * x : x * x * x; };
+    int per = 1;
+    while (per < 120 && power(per + 1) <= cells) per++;  // cell numbers along a coordinate are kept in 7 or 8 bits
+    p->cells_per_dim = per;
+    p->cells = ((int)power(per) + 3) / 4 * 4;
+    p->max_settled = (int)power((per + 1) / 2);
     return true;
 }
 
-struct Buffers {
-    GridParams *grid;
-    float *partial;
-    int *keys, *skeys, *perm, *tk, *tv, *hist, *high, *scan_tmp, *itf, *s_mask, *h_mask, *h_orig;
-    int *row_splits_h, *total, *s_assignment, *s_asso, *alpha_h, *status_h;
-    float *s_ccoords, *s_betas, *s_dist, *h_ccoords, *h_betas, *h_dist;
-    void *op_ws;
-    size_t op_ws_bytes;
-};
-
 template <typename W>
-void layout(W &ws, int n_vert, int dims, int num_rows, Buffers *out)
+void layout(W &ws, int n_vert, int dims, int num_rows, const Plan &p, Buffers *out, size_t *zeroed)
 {
-    const size_t n = n_vert > 0 ? n_vert : 0;
-    const size_t d = dims > 0 ? dims : 1;
+    const size_t n = n_vert > 0 ? n_vert : 0, rows = num_rows > 0 ? num_rows : 0;
+    const size_t d = dims > 0 ? dims : 1, nr = rec_size((int)d), e = rows + 2;
+    const size_t tiles = order_tiles_cap(n_vert, (int)rows), passes = p.bin_passes + 4;
+    const size_t words = n / 32 + rows + 1;
     Buffers b;
-    b.grid = ws.template take<GridParams>(1);
-    b.partial = ws.template take<float>((size_t)range_partial_blocks(n_vert) * 2 * kMaxBinDims);
-    b.keys = ws.template take<int>(n);
-    b.skeys = ws.template take<int>(n);
-    b.perm = ws.template take<int>(n);
-    b.tk = ws.template take<int>(n);
-    b.tv = ws.template take<int>(n);
-    b.hist = ws.template take<int>(sort_hist_ints(n_vert));
-    b.high = ws.template take<int>(n);
-    b.scan_tmp = ws.template take<int>(scan_scratch_ints(n_vert));
-    b.itf = ws.template take<int>(n);
-    b.s_mask = ws.template take<int>(n);
+    b.tile_hist = ws.template take<int>((passes + 1) * tiles * 256);
+    b.event_hist = ws.template take<int>(passes * (rows + 1) * 256);
+    b.count = ws.template take<int>(rows);
+    b.cell_count = ws.template take<int>(rows * (p.cells + 1));
+    b.max_radius = ws.template take<unsigned>(1);
+    if (zeroed) *zeroed = ws.used_bytes();
+    b.layout = HitOrder();
+    b.layout.grid = ws.template take<GridParams>(1);
+    b.layout.partial = ws.template take<float>((size_t)range_partial_blocks(n_vert) * 2 * kMaxBinDims);
+    b.layout.event_pos = ws.template take<int>(e);
+    b.layout.event_tile = ws.template take<int>(e);
+    b.layout.event_chunk = ws.template take<int>(e);
+    b.layout.event_super = ws.template take<int>(e);
+    b.use_grid = ws.template take<int>(1);
+    b.first_two = ws.template take<u64>(2);
+    b.tile_count = ws.template take<int>(tiles);
+    b.row_splits_h = ws.template take<int>(rows + 1);
+    for (int i = 0; i < 2; i++) {
+        b.key[i] = ws.template take<u64>(n);
+        b.val[i] = ws.template take<int>(n);
+    }
+    b.order = ws.template take<int>(n);
+    b.h_ccoords = ws.template take<float>(n * d);
+    b.h_dist = ws.template take<float>(n);
     b.h_mask = ws.template take<int>(n);
     b.h_orig = ws.template take<int>(n);
-    b.row_splits_h = ws.template take<int>((size_t)num_rows + 1);
-    b.total = ws.template take<int>(1);
-    b.s_assignment = ws.template take<int>(n);
-    b.s_asso = ws.template take<int>(n);
-    b.alpha_h = ws.template take<int>(n);
     b.status_h = ws.template take<int>(n);
-    b.s_ccoords = ws.template take<float>(n * d);
-    b.s_betas = ws.template take<float>(n);
-    b.s_dist = ws.template take<float>(n);
-    b.h_ccoords = ws.template take<float>(n * d);
-    b.h_betas = ws.template take<float>(n);
-    b.h_dist = ws.template take<float>(n);
-    b.op_ws_bytes = hgc_binned_assign_to_condensates_workspace_bytes(n_vert, n_vert, num_rows, dims);
-    b.op_ws = ws.template take<unsigned char>(b.op_ws_bytes);
+    b.p_rec = ws.template take<float4>(n * nr);
+    b.p_flag = ws.template take<int>(n);
+    b.open = ws.template take<unsigned>(words * 32 + kClaimStep);
+    b.bitmap = ws.template take<unsigned>(words);
+    b.cl.centre = ws.template take<float>(n * d);
+    b.cl.radius_sq = ws.template take<float>(n);
+    b.cl.subset_pos = ws.template take<int>(n);
+    b.cl.lonely = ws.template take<int>(n);
+    b.cl.count = b.count;
+    b.alpha_h = ws.template take<int>(n);
+    const size_t stage = claim_stage_ints(num_rows);
+    b.stage = ws.template take<int>(stage > tiles ? stage : tiles);
+    b.c_rec = ws.template take<float4>(n * nr);
+    b.c_rank = ws.template take<int>(n);
     if (out) *out = b;
 }
 
 struct SizerW {
     Sizer s;
     template <typename T> T *take(size_t n) { s.take<T>(n); return nullptr; }
+    size_t used_bytes() const { return s.used; }
 };
+struct CarverW {
+    Carver c;
+    template <typename T> T *take(size_t n) { return c.take<T>(n); }
+    size_t used_bytes() const { return c.used; }
+};
+
+// The last sort pass, the claims, the lists and the assignment, for records of NR float4.
+template <int NR>
+int run_claims(const Buffers &b, const Plan &p, int dims, int num_rows, int tiles, const float *ccoords, const int *mask,
+               bool by_max_beta, int *assignment, int *association, int *alpha_idx, unsigned char *is_cond,
+               int *n_condensates, cudaStream_t stream)
+{
+    const int last = p.bin_passes + 3;
+    order_pass_kernel<false, NR><<<tiles, kThreads, 0, stream>>>(b, num_rows, tiles, last, 32 + 24, 0, dims);
+    HGC_LAUNCH_CHECK();
+    const size_t smem = 2 * sizeof(int) * (size_t)p.cells + (size_t)p.max_settled * (NR * sizeof(float4) + sizeof(int));
+    // (set on every call: the setting belongs to the current device)
+    HGC_CUDA_TRY(cudaFuncSetAttribute(claim_grid_kernel<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    claim_grid_kernel<NR><<<num_rows * kClusterBlocks, kClaimThreads, smem, stream>>>(b, dims, p.cells, p.cells_per_dim,
+                                                                                      p.max_settled);
+    HGC_LAUNCH_CHECK();
+    if (int rc = launch_claim_windows(dims, b.h_ccoords, b.h_dist, b.h_mask, b.h_orig, b.row_splits_h, b.order, b.status_h,
+                                      b.alpha_h, b.stage, b.cl, num_rows, b.use_grid, stream))
+        return rc;
+    list_condensates_kernel<NR><<<num_rows, 1024, 0, stream>>>(b, dims, p.cells, p.cells_per_dim, n_condensates, alpha_idx,
+                                                               is_cond, assignment);
+    HGC_LAUNCH_CHECK();
+    assign_hits_kernel<NR><<<tiles * kRounds, kThreads, 0, stream>>>(b, ccoords, mask, dims, num_rows, p.cells,
+                                                                     p.cells_per_dim, by_max_beta, assignment, association,
+                                                                     is_cond, n_condensates, alpha_idx);
+    HGC_LAUNCH_CHECK();
+    return HGC_OK;
+}
 
 }  // namespace
 }  // namespace hgc
 
-namespace hgc {
-int assign_to_condensates(
-        int dimensions, int dimensions_binning,
-        const float *d_ccoords_h, const float *d_dist_h, const float *d_beta_h,
-        const int *d_no_condensation_mask_h, int *d_high_assigned_status_h,
-        const int *d_original_indices_h, const int *d_row_splits_h,
-        const float *d_ccoords, const float *d_dist, const int *d_no_condensation_mask,
-        const int *d_indices_to_filtered,
-        int *d_assignment, int *d_association, int *d_n_condensates, int *d_alpha_indices,
-        const int *d_bin_splits, const int *d_n_bins, const float *d_bin_widths,
-        const int *d_row_splits, int num_rows, int n_vert, int n_vert_h, const int *d_n_vert_h,
-        int assign_by_max_beta, void *workspace, size_t workspace_bytes, hgc_stream_t stream);
-}
 using namespace hgc;
 
 extern "C" size_t hgc_build_and_assign_condensates_workspace_bytes(int n_vert, int dimensions, int n_rs,
@@ -214,7 +894,7 @@ extern "C" size_t hgc_build_and_assign_condensates_workspace_bytes(int n_vert, i
     if (dimensions < 1 || dimensions > kMaxCondDims || n_rs < 1 || !make_plan(n_vert, dimensions, nbin_dims, n_rs, &p))
         return 0;
     SizerW w;
-    layout(w, n_vert, dimensions, n_rs - 1, nullptr);
+    layout(w, n_vert, dimensions, n_rs - 1, p, nullptr, nullptr);
     return w.s.used;
 }
 
@@ -240,57 +920,64 @@ extern "C" int hgc_build_and_assign_condensates(
         return HGC_ERR_INVALID_ARGUMENT;
     const size_t need = hgc_build_and_assign_condensates_workspace_bytes(n_vert, dimensions, n_rs, nbin_dims);
     if (int rc = check_workspace(workspace, workspace_bytes, need)) return rc;
-    Carver ws(workspace);
-    Buffers b;
-    layout(ws, n_vert, dimensions, num_rows, &b);
-    HGC_CUDA_TRY(cudaMemsetAsync(ws.status(), 0, kAlign, stream));
     if (h_n_alpha) *h_n_alpha = 0;
-    if (n_vert == 0) {
+    if (n_vert == 0 || num_rows == 0) {
+        HGC_CUDA_TRY(cudaMemsetAsync(workspace, 0, kAlign, stream));
         HGC_CUDA_TRY(cudaMemsetAsync(d_n_condensates, 0, sizeof(int) * (size_t)n_rs, stream));
+        if (n_vert > 0) {
+            const size_t bytes = sizeof(int) * (size_t)n_vert;
+            HGC_CUDA_TRY(cudaMemsetAsync(d_assignment, 0xff, bytes, stream));
+            HGC_CUDA_TRY(cudaMemsetAsync(d_association, 0xff, bytes, stream));
+            HGC_CUDA_TRY(cudaMemsetAsync(d_alpha_idx, 0xff, bytes, stream));
+            HGC_CUDA_TRY(cudaMemsetAsync(d_is_cond, 0, (size_t)n_vert, stream));
+        }
         return HGC_OK;
     }
+    CarverW ws{Carver(workspace)};
+    unsigned *status = ws.c.status();
+    Buffers b;
+    size_t zeroed = 0;
+    layout(ws, n_vert, dimensions, num_rows, p, &b, &zeroed);
+    HGC_CUDA_TRY(cudaMemsetAsync(workspace, 0, zeroed, stream));
 
-    // grid of BinByCoordinates(ccoords[:, :nbin_dims] - min, n_bins=n_bins_sc, pre_normalized=True), keys, order
-    if (int rc = compute_grid(d_ccoords, dimensions, p.cb, dimensions, n_vert, d_row_splits, n_rs, p.n_bins_sc,
-                              32, /*pre_normalized=*/0, b.partial, b.grid, stream))
+    // grid of BinByCoordinates(ccoords[:, :nbin_dims] - min, n_bins=n_bins_sc, pre_normalized=True)
+    if (int rc = range_and_layout(d_ccoords, dimensions, p.cb, d_row_splits, n_rs, p.n_bins_sc, 32, n_vert, b.layout, status,
+                                  stream))
         return rc;
-    if (int rc = launch_bin_keys(d_ccoords, dimensions, p.cb, b.grid->shift, d_row_splits, n_rs,
-                                 &b.grid->bin_width, b.grid->n_bins, nullptr, nullptr, b.keys, n_vert, 0,
-                                 &b.grid->n_total_bins, ws.status(), stream))
-        return rc;
-    if (int rc = sort_pairs(b.keys, nullptr, b.skeys, b.perm, b.tk, b.tv, b.hist, n_vert, bits_for(p.max_bins), stream))
-        return rc;
-    const int blocks = div_up(n_vert, 256);
-    gather_sorted_kernel<<<blocks, 256, 0, stream>>>(d_ccoords, d_betas, d_dist, d_no_condensation_mask, b.perm,
-                                                     b.grid, dimensions, distance_threshold, beta_threshold,
-                                                     b.s_ccoords, b.s_betas, b.s_dist, b.s_mask, b.high, n_vert);
+    const int tiles = (int)order_tiles_cap(n_vert, num_rows);
+    count_high_kernel<<<tiles, kThreads, 0, stream>>>(d_betas, d_no_condensation_mask, beta_threshold, b.layout, num_rows,
+                                                      b.tile_count, d_alpha_idx, d_is_cond, b.first_two);
     HGC_LAUNCH_CHECK();
-    if (int rc = exclusive_scan_ints(b.high, n_vert, b.scan_tmp, stream)) return rc;
-    compact_high_kernel<<<blocks, 256, 0, stream>>>(b.high, b.s_ccoords, b.s_betas, b.s_dist, b.s_mask, b.perm,
-                                                    dimensions, beta_threshold, b.itf, b.h_ccoords, b.h_betas,
-                                                    b.h_dist, b.h_mask, b.h_orig, n_vert);
+    if (d_no_condensation_mask) {
+        first_high_kernel<false><<<tiles, kThreads, 0, stream>>>(d_ccoords, d_betas, d_no_condensation_mask, beta_threshold,
+                                                                 dimensions, p.cb, b.layout, num_rows, b.first_two);
+        HGC_LAUNCH_CHECK();
+        first_high_kernel<true><<<tiles, kThreads, 0, stream>>>(d_ccoords, d_betas, d_no_condensation_mask, beta_threshold,
+                                                                dimensions, p.cb, b.layout, num_rows, b.first_two);
+        HGC_LAUNCH_CHECK();
+    }
+    const int passes = p.bin_passes + 4;
+    order_high_kernel<<<tiles, kThreads, sizeof(int) * 256 * passes, stream>>>(
+            d_ccoords, d_betas, d_dist, d_no_condensation_mask, beta_threshold, distance_threshold, dimensions, p.cb,
+            p.bin_passes, num_rows, b, status);
     HGC_LAUNCH_CHECK();
-    filtered_row_splits_kernel<<<div_up(n_rs + 1, 256), 256, 0, stream>>>(b.high, b.s_betas, b.s_mask, beta_threshold,
-                                                                          d_row_splits, n_rs, n_vert,
-                                                                          b.row_splits_h, b.total);
-    HGC_LAUNCH_CHECK();
-    // The number of high-beta hits stays on the device: the op is launched for up to n_vert of them
-    // and reads the count itself, so nothing waits for the host here.
-    if (int rc = assign_to_condensates(
-                dimensions, p.cb, b.h_ccoords, b.h_dist, b.h_betas, b.h_mask, b.status_h, b.h_orig, b.row_splits_h,
-                b.s_ccoords, b.s_dist, b.s_mask, b.itf, b.s_assignment, b.s_asso, d_n_condensates, b.alpha_h,
-                nullptr, b.grid->n_bins, &b.grid->bin_width, d_row_splits, num_rows, n_vert, n_vert, b.total,
-                assign_by_max_beta, b.op_ws, b.op_ws_bytes, stream_))
-        return rc;
-
-    scatter_back_kernel<<<blocks, 256, 0, stream>>>(b.s_assignment, b.s_asso, b.perm, d_assignment, d_association,
-                                                    d_is_cond, n_vert);
-    HGC_LAUNCH_CHECK();
-    fill_minus_one_kernel<<<blocks, 256, 0, stream>>>(d_alpha_idx, n_vert);
-    HGC_LAUNCH_CHECK();
-    compact_alpha_kernel<<<blocks, 256, 0, stream>>>(b.alpha_h, b.row_splits_h, d_n_condensates, num_rows, n_vert,
-                                                     b.total, d_alpha_idx, d_is_cond);
-    HGC_LAUNCH_CHECK();
+    auto shift_of = [&p](int pass) { return pass < p.bin_passes ? 8 * pass : 32 + 8 * (pass - p.bin_passes); };
+    for (int i = 0; i + 1 < passes; i++) {  // the last one belongs to run_claims
+        if (i == 0)
+            order_pass_kernel<true, 0><<<tiles, kThreads, 0, stream>>>(b, num_rows, tiles, i, shift_of(i), shift_of(i + 1), dimensions);
+        else
+            order_pass_kernel<false, 0><<<tiles, kThreads, 0, stream>>>(b, num_rows, tiles, i, shift_of(i), shift_of(i + 1), dimensions);
+        HGC_LAUNCH_CHECK();
+    }
+    int rc = HGC_ERR_UNSUPPORTED;
+#define HGC_RUN(NR)                                                                                                  \
+    rc = run_claims<NR>(b, p, dimensions, num_rows, tiles, d_ccoords, d_no_condensation_mask, assign_by_max_beta != 0, \
+                        d_assignment, d_association, d_alpha_idx, d_is_cond, d_n_condensates, stream)
+    if (rec_size(dimensions) == 1) HGC_RUN(1);
+    else if (rec_size(dimensions) == 2) HGC_RUN(2);
+    else HGC_RUN(3);
+#undef HGC_RUN
+    if (rc) return rc;
     if (h_n_alpha) {
         HGC_CUDA_TRY(cudaMemcpyAsync(h_n_alpha, d_n_condensates + num_rows, sizeof(int), cudaMemcpyDeviceToHost, stream));
         HGC_CUDA_TRY(cudaStreamSynchronize(stream));
