@@ -394,10 +394,10 @@ claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ int s_dyn[];
     __shared__ int s_left[2][kClusterBlocks];
-    __shared__ int s_count, s_sum;
+    __shared__ int s_count, s_sum, s_listed;
     int *s_best = s_dyn, *s_min = s_dyn + cells_cap;               // cells_cap is a multiple of 4
     float4 *s_rec = reinterpret_cast<float4 *>(s_min + cells_cap);  // [max_settled][NR]
-    int *s_pos = reinterpret_cast<int *>(s_rec + (size_t)max_settled * NR);
+    int *s_pos = reinterpret_cast<int *>(s_rec + (size_t)max_settled * NR), *s_at = s_pos + max_settled;
     const CondGrid grid = make_cond_grid(b.layout.grid, b.max_radius, dims, cells_per_dim);
     const int n_cells = grid.n[0] * grid.n[1] * grid.n[2];
     const bool use = n_cells >= kMinCells;
@@ -416,7 +416,7 @@ claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max
     unsigned *__restrict__ open_words = b.open + (size_t)word0 * 32 + g;  // word w of this thread: [w * kClaimStep], w > 0
 
     for (int c = t; c < n_cells; c += kClaimThreads) s_best[c] = kFree;
-    if (t == 0) s_count = s_sum = 0;
+    if (t == 0) s_count = s_sum = s_listed = 0;
     // this thread's hits are p = k * kClaimStep + g; 32 of them share a word of open bits, kept in memory beyond the first
     unsigned open0 = 0u;
     int n_mine = 0;  // condensates among them
@@ -485,38 +485,46 @@ claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max
             for (int r = 0; r < kClusterBlocks; r++) *cluster.map_shared_rank(s_min + c, r) = m;
         }
         cluster.sync();
-        // which of them are first among the cells around
-        for (int c = t; c < n_cells; c += kClaimThreads) {
-            const int p = s_min[c];
-            int settled = -1;
-            if (p != kFree) {
-                const int z = c % grid.n[2], y = c / grid.n[2] % grid.n[1], x = c / (grid.n[2] * grid.n[1]);
-                bool first = true;
-                for (int i = max(x - 1, 0); i <= min(x + 1, grid.n[0] - 1); i++)
-                    for (int j = max(y - 1, 0); j <= min(y + 1, grid.n[1] - 1); j++)
-                        for (int l = max(z - 1, 0); l <= min(z + 1, grid.n[2] - 1); l++)
-                            first = first && s_min[(i * grid.n[1] + j) * grid.n[2] + l] >= p;
-                if (first) {
-                    settled = atomicAdd(&s_count, 1);  // in any order
-                    s_pos[settled] = p;
-                    store_rec<NR>(s_rec + (size_t)settled * NR, load_rec<NR>(recs + (size_t)p * NR));
-                }
-            }
-            s_best[c] = settled;
+        // which of them are first among the cells around: occupied cells are listed first, since later rounds have few
+        for (int c0 = t - lane; c0 < n_cells; c0 += kClaimThreads) {
+            const int c = c0 + lane;
+            const bool occupied = c < n_cells && s_min[c] != kFree;
+            const unsigned m = __ballot_sync(0xffffffffu, occupied);
+            int base = 0;
+            if (lane == 0 && m) base = atomicAdd(&s_listed, __popc(m));
+            base = __shfl_sync(0xffffffffu, base, 0);
+            if (occupied) s_best[base + __popc(m & ((1u << lane) - 1u))] = c;  // the merged table has its place
         }
         __syncthreads();
-        // and, for every cell, which of the 27 cells around it hold one (no two next to each other do)
-        for (int c = t; c < n_cells; c += kClaimThreads) {
+        const int n_listed = s_listed;
+        for (int i0 = t; i0 < n_listed; i0 += kClaimThreads) {
+            const int c = s_best[i0], p = s_min[c];
             const int z = c % grid.n[2], y = c / grid.n[2] % grid.n[1], x = c / (grid.n[2] * grid.n[1]);
-            int near_ = 0;
-#pragma unroll
-            for (int k = 0; k < 27; k++) {
-                const int i = x + k / 9 - 1, j = y + k / 3 % 3 - 1, l = z + k % 3 - 1;
-                if (i >= 0 && i < grid.n[0] && j >= 0 && j < grid.n[1] && l >= 0 && l < grid.n[2] &&
-                    s_best[(i * grid.n[1] + j) * grid.n[2] + l] >= 0)
-                    near_ |= 1 << k;
+            bool first = true;
+            for (int i = max(x - 1, 0); first && i <= min(x + 1, grid.n[0] - 1); i++)
+                for (int j = max(y - 1, 0); first && j <= min(y + 1, grid.n[1] - 1); j++) {
+                    const int *row = s_min + (i * grid.n[1] + j) * grid.n[2];
+                    first = row[max(z - 1, 0)] >= p && row[z] >= p && row[min(z + 1, grid.n[2] - 1)] >= p;
+                }
+            if (first) {
+                const int s = atomicAdd(&s_count, 1);  // in any order
+                s_pos[s] = p;
+                s_at[s] = x << 16 | y << 8 | z;
+                store_rec<NR>(s_rec + (size_t)s * NR, load_rec<NR>(recs + (size_t)p * NR));
             }
-            s_min[c] = near_;
+        }
+        __syncthreads();
+        // and, for every cell, which of the 27 cells around it hold one (no two next to each other do): s_min takes
+        // those bits, s_best of a cell that holds one its number
+        for (int c = t; c < n_cells; c += kClaimThreads) s_min[c] = 0;
+        __syncthreads();
+        for (int i = t; i < s_count * 27; i += kClaimThreads) {
+            const int s = i / 27, k = i % 27, at = s_at[s];
+            const int x = (at >> 16) + k / 9 - 1, y = ((at >> 8) & 255) + k / 3 % 3 - 1, z = (at & 255) + k % 3 - 1;
+            if (x < 0 || x >= grid.n[0] || y < 0 || y >= grid.n[1] || z < 0 || z >= grid.n[2]) continue;
+            const int c = (x * grid.n[1] + y) * grid.n[2] + z;
+            atomicOr(s_min + c, 1 << (26 - k));  // seen from there, the cell is on the opposite side
+            if (k == 13) s_best[c] = s;
         }
         __syncthreads();
         // close them and what they cover
@@ -570,7 +578,7 @@ claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max
         __syncthreads();
         if (t < kClusterBlocks) *cluster.map_shared_rank(&s_left[round & 1][rank], t) = s_sum;
         for (int c = t; c < n_cells; c += kClaimThreads) s_best[c] = kFree;
-        if (t == 0) s_count = 0;
+        if (t == 0) s_count = s_listed = 0;
         __syncthreads();
         if (t == 0) s_sum = 0;  // added to again only after the next cluster barriers
     }
@@ -863,7 +871,7 @@ int run_claims(const Buffers &b, const Plan &p, int dims, int num_rows, int tile
     const int last = p.bin_passes + 3;
     order_pass_kernel<false, NR><<<tiles, kThreads, 0, stream>>>(b, num_rows, tiles, last, 32 + 24, 0, dims);
     HGC_LAUNCH_CHECK();
-    const size_t smem = 2 * sizeof(int) * (size_t)p.cells + (size_t)p.max_settled * (NR * sizeof(float4) + sizeof(int));
+    const size_t smem = 2 * sizeof(int) * (size_t)p.cells + (size_t)p.max_settled * (NR * sizeof(float4) + 2 * sizeof(int));
     // (set on every call: the setting belongs to the current device)
     HGC_CUDA_TRY(cudaFuncSetAttribute(claim_grid_kernel<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     claim_grid_kernel<NR><<<num_rows * kClusterBlocks, kClaimThreads, smem, stream>>>(b, dims, p.cells, p.cells_per_dim,
