@@ -51,6 +51,8 @@ def _load():
         "hgc_binned_select_knn_ragged": (I, [P] * 6 + [I] * 8 + [P, S, P]),
         "hgc_build_and_assign_condensates_workspace_bytes": (S, [I] * 4),
         "hgc_build_and_assign_condensates": (I, [P] * 11 + [I] * 3 + [ctypes.c_float] * 2 + [I] * 2 + [P, S, P]),
+        "hgc_merge_noise_workspace_bytes": (S, [I, I]),
+        "hgc_merge_noise": (I, [P] * 12 + [I, I] + [P, S, P]),
         "hgc_local_distance": (I, [P, P, P, I, I, I, I, P]),
         "hgc_push_knn": (I, [P, P, P, P, I, I, I, P, S, P]),
         "hgc_push_knn_ordered": (I, [P, P, P, P, I, I, I, P, P, S, P]),

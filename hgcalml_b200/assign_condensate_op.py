@@ -1,7 +1,6 @@
 """Host-side mirror of HGCalML's ``modules/assign_condensate_op.py`` on torch CUDA tensors."""
 from __future__ import annotations
 
-import ctypes
 import math
 
 import torch
@@ -50,34 +49,32 @@ def merge_noise_as_indiv_cp(assignment, asso_idx, alpha_idx, is_cond, n_condensa
     point of its own.  Per event the noise hits take the shower numbers 0..n_noise-1 in hit order and
     the real showers are shifted up by n_noise; ``alpha_idx`` lists, per event, the noise hits first
     and then the condensates; noise hits are associated to themselves and flagged as condensates."""
-    dev = assignment.device
-    rs = row_splits.to(torch.int64)
-    n = assignment.shape[0]
-    num_rows = rs.shape[0] - 1
-    a = assignment[:, 0].to(torch.int64)
-    seg = torch.repeat_interleave(torch.arange(num_rows, device=dev), rs[1:] - rs[:-1])
-    noise = a < 0
-    csum = torch.cumsum(noise.to(torch.int64), 0)
-    before_event = torch.cat([torch.zeros(1, dtype=torch.int64, device=dev), csum])[rs[:-1]]
-    x = torch.where(noise, csum - before_event[seg], torch.zeros_like(csum))  # 1-based rank among the event's noise
-    n_noise = torch.zeros(num_rows, dtype=torch.int64, device=dev).scatter_reduce(0, seg, x, "amax", include_self=True)
-    new_assignment = torch.where(noise, x - 1, a + n_noise[seg]).to(torch.int32)
+    C.require_cuda(assignment, asso_idx, alpha_idx, is_cond)
+    return _merge_noise(C.i32(assignment).reshape(-1), C.i32(asso_idx), C.i32(alpha_idx),
+                        is_cond.to(torch.bool).contiguous().reshape(-1), C.i32(n_condensates),
+                        C.i32(row_splits, assignment.device))
 
-    allrange = torch.arange(n, device=dev)
-    nc = n_condensates.to(torch.int64)
-    cond_event = torch.repeat_interleave(torch.arange(num_rows, device=dev), nc[1:] - nc[:-1])
-    noise_idx = allrange[noise]
-    # per event: noise hits, then condensates -- a stable sort by (event, kind)
-    keys = torch.cat([seg[noise] * 2, cond_event * 2 + 1])
-    vals = torch.cat([noise_idx, alpha_idx.to(torch.int64)])
-    new_alpha = vals[torch.sort(keys, stable=True).indices].to(torch.int32)
 
-    cond = is_cond[:, 0].clone()
-    cond[asso_idx < 0] = True
-    new_asso = torch.where(asso_idx < 0, allrange.to(asso_idx.dtype), asso_idx)
-    per_event = torch.zeros(num_rows, dtype=torch.int64, device=dev).scatter_add(0, seg, cond.to(torch.int64))
-    new_ncond = torch.cat([n_condensates[0:1].to(torch.int64), torch.cumsum(per_event, 0)]).to(torch.int32)
-    return new_assignment[:, None], new_asso, new_alpha, cond[:, None], new_ncond
+def _host_int():
+    # page-locked, so that the copy that fills it needs no staging
+    return torch.empty((1,), dtype=torch.int32, pin_memory=True)
+
+
+def _merge_noise(assignment, asso, alpha, is_cond, n_condensates, row_splits):
+    # alpha may be longer than the list of condensates: its length is n_condensates[-1]
+    dev, n, n_rs = assignment.device, assignment.shape[0], row_splits.shape[0]
+    new = torch.empty((4, n), dtype=torch.int32, device=dev)  # assignment, association, alpha (up to 2 n)
+    cond = torch.empty((n,), dtype=torch.bool, device=dev)
+    n_cond = torch.empty((n_rs,), dtype=torch.int32, device=dev)
+    ws = C.workspace(C.lib.hgc_merge_noise_workspace_bytes(n, n_rs), dev)
+    n_alpha = _host_int()
+    if alpha.shape[0] == 0:
+        alpha = new  # nothing is read from it
+    C.check(C.lib.hgc_merge_noise(
+        C.ptr(assignment), C.ptr(asso), C.ptr(alpha), C.ptr(is_cond), C.ptr(n_condensates), C.ptr(row_splits),
+        new[0].data_ptr(), new[1].data_ptr(), new[2].data_ptr(), C.ptr(cond), C.ptr(n_cond), n_alpha.data_ptr(),
+        n, n_rs, C.ptr(ws), ws.numel(), C.stream_of(assignment)), "merge_noise_as_indiv_cp")
+    return new[0][:, None], new[1], new[2:].reshape(-1)[:n_alpha.item()], cond[:, None], n_cond
 
 
 def _segment_ids_to_row_splits(ids, num_segments):
@@ -93,7 +90,7 @@ def BuildAndAssignCondensatesBinned(ccoords, betas, dist, row_splits, beta_thres
     Returns ``assignment [N,1], association [N], alpha_idx, is_cond [N,1], n_condensates`` with the
     reference's meaning.  Everything up to ``keep_noise`` is one library call
     (``hgc_build_and_assign_condensates``: threshold scaling, shift, binning, stable sort by bin,
-    high-beta filter, the op, mapping back); the ``keep_noise`` renumbering runs as tensor ops."""
+    high-beta filter, the op, mapping back); the ``keep_noise`` renumbering is a second one."""
     assert 1 <= nbin_dims <= 6
     assert 0. <= beta_threshold <= 1.
     assert distance_threshold > 0.
@@ -113,20 +110,19 @@ def BuildAndAssignCondensatesBinned(ccoords, betas, dist, row_splits, beta_thres
     assignment = torch.empty((n,), dtype=torch.int32, device=dev)
     asso = torch.empty((n,), dtype=torch.int32, device=dev)
     alpha = torch.empty((n,), dtype=torch.int32, device=dev)
-    is_cond = torch.empty((n,), dtype=torch.uint8, device=dev)
+    is_cond = torch.empty((n,), dtype=torch.bool, device=dev)
     n_condensates = torch.empty((n_rs,), dtype=torch.int32, device=dev)
     ws = C.workspace(C.lib.hgc_build_and_assign_condensates_workspace_bytes(n, dims, n_rs, nbin_dims), dev)
-    n_alpha = ctypes.c_int(0)
+    n_alpha = None if keep_noise else _host_int()  # the number of condensates is not needed in between
     C.check(C.lib.hgc_build_and_assign_condensates(
         C.ptr(ccoords), C.ptr(betas), C.ptr(dist), C.ptr(mask), C.ptr(row_splits),
         C.ptr(assignment), C.ptr(asso), C.ptr(alpha), C.ptr(is_cond), C.ptr(n_condensates),
-        ctypes.addressof(n_alpha), n, dims, n_rs, float(beta_threshold), float(distance_threshold),
+        C.ptr(n_alpha), n, dims, n_rs, float(beta_threshold), float(distance_threshold),
         int(bool(assign_by_max_beta)), nbin_dims, C.ptr(ws), ws.numel(), C.stream_of(ccoords)),
         "BuildAndAssignCondensatesBinned")
-    out = (assignment[:, None], asso, alpha[:n_alpha.value], is_cond.to(torch.bool)[:, None], n_condensates)
     if keep_noise:
-        out = merge_noise_as_indiv_cp(*out, row_splits)
-    return out
+        return _merge_noise(assignment, asso, alpha, is_cond, n_condensates, row_splits)
+    return assignment[:, None], asso, alpha[:n_alpha.item()], is_cond[:, None], n_condensates
 
 
 def BuildAndAssignCondensatesBinnedStepwise(ccoords, betas, dist, row_splits, beta_threshold,

@@ -12,7 +12,7 @@
  *    caller passes it.  The device that owns `stream` and the d_ pointers must be the calling
  *    thread's current device (cudaSetDevice) when an entry is called.  The entries that wait
  *    for their own stream say so: hgc_workspace_status, hgc_binned_select_knn_static_status and
- *    hgc_build_and_assign_condensates when it is asked for the condensate count on the host.
+ *    hgc_build_and_assign_condensates and hgc_merge_noise when asked for a count on the host.
  *  - Return value: HGC_OK or a negative HGC_ERR_* code.  Nothing throws, nothing prints.
  *    Problems that only the device can see (an index outside its table, a bin outside the
  *    grid, an iteration cap reached) set a status word in the workspace, which
@@ -267,8 +267,8 @@ int hgc_binned_assign_to_condensates(
  *          d_n_condensates [n_rs] cumulative count
  *   h_n_alpha (host, may be NULL): receives the number of condensates; the call then returns after
  *          the stream has finished.
- * The number of high-beta hits never leaves the device (the op's kernels and sorts are launched for
- * up to n_vert of them and read the count themselves), so with h_n_alpha == NULL the call is a plain
+ * The number of high-beta hits never leaves the device (kernels are launched for up to n_vert of them
+ * and read the count themselves), so with h_n_alpha == NULL the call is a plain
  * enqueue like every other entry. */
 size_t hgc_build_and_assign_condensates_workspace_bytes(int n_vert, int dimensions, int n_rs, int nbin_dims);
 int hgc_build_and_assign_condensates(
@@ -278,6 +278,23 @@ int hgc_build_and_assign_condensates(
         int *d_n_condensates, int *h_n_alpha,
         int n_vert, int dimensions, int n_rs, float beta_threshold, float distance_threshold,
         int assign_by_max_beta, int nbin_dims,
+        void *workspace, size_t workspace_bytes, hgc_stream_t stream);
+
+/* merge_noise_as_indiv_cp (modules/assign_condensate_op.py:16-44, the wrapper's keep_noise): every noise
+ * hit (d_assignment < 0) becomes a condensation point of its own.  Per event the noise hits take the
+ * shower numbers 0 .. n_noise-1 in hit order and the others move up by n_noise; d_new_alpha_idx lists
+ * per event the noise hits, then the condensates; noise hits are associated to themselves and flagged.
+ *   d_assignment, d_association, d_is_cond [n_vert], d_alpha_idx, d_n_condensates [n_rs]: as written by
+ *          hgc_build_and_assign_condensates (only the first d_n_condensates[n_rs-1] entries of d_alpha_idx are read)
+ *   outputs [n_vert] (d_new_alpha_idx [2 n_vert]) and d_new_n_condensates [n_rs]; they must not overlap inputs
+ *   h_n_alpha (host, may be NULL): receives the number of entries of d_new_alpha_idx; the call then
+ *          returns after the stream has finished. */
+size_t hgc_merge_noise_workspace_bytes(int n_vert, int n_rs);
+int hgc_merge_noise(
+        const int *d_assignment, const int *d_association, const int *d_alpha_idx, const unsigned char *d_is_cond,
+        const int *d_n_condensates, const int *d_row_splits,
+        int *d_new_assignment, int *d_new_association, int *d_new_alpha_idx, unsigned char *d_new_is_cond,
+        int *d_new_n_condensates, int *h_n_alpha, int n_vert, int n_rs,
         void *workspace, size_t workspace_bytes, hgc_stream_t stream);
 
 /* ---------------------------------------------------------------------------------------
