@@ -30,7 +30,6 @@ namespace {
 constexpr int kMaxCondDims = 8;
 constexpr int kThreads = kOrderThreads;
 constexpr int kWarps = kThreads / kWarp;
-constexpr int kRounds = kOrderTile / kThreads;
 constexpr int kClusterBlocks = 8;
 constexpr int kClaimThreads = 1024;
 constexpr int kClaimStep = kClusterBlocks * kClaimThreads;  // hits of an event looked at together
@@ -236,9 +235,8 @@ order_high_kernel(const float *__restrict__ ccoords, const float *__restrict__ b
     int run = s_sum[0];
     const int start = s_sum[1];
     float radius_max = 0.f;
-    for (int r = 0; r < kRounds; r++) {
-        if (r * kThreads >= t.n) break;  // uniform
-        const int i = r * kThreads + threadIdx.x, v = t.first + i;
+    for (int i0 = 0; i0 < t.n; i0 += kThreads) {
+        const int i = i0 + threadIdx.x, v = t.first + i;
         const bool high = i < t.n && is_high(betas, mask, v, beta_threshold);
         const int incl = block_scan_inclusive(high ? 1 : 0, [](int x, int y) { return x + y; }, 0, s_warp);
         if (high) {
@@ -264,7 +262,7 @@ order_high_kernel(const float *__restrict__ ccoords, const float *__restrict__ b
                 atomicAdd(&s_hist[p * 256 + (int)((key >> shift) & 255u)], 1);
             }
             // the packed hits make tiles of their own
-            atomicAdd(&b.tile_hist[(size_t)(tile0 + (a - start) / kOrderTile) * 256 + (int)(key & 255u)], 1);
+            atomicAdd(&b.tile_hist[(size_t)(tile0 + (a - start) / o.tile) * 256 + (int)(key & 255u)], 1);
         }
         __syncthreads();
         if (threadIdx.x == kThreads - 1) s_base = incl;
@@ -282,10 +280,11 @@ order_high_kernel(const float *__restrict__ ccoords, const float *__restrict__ b
 
 // One pass of the stable sort of the packed hits, event by event (see hit_order.cu).  The last pass (NR > 0) writes the
 // order, and the hits' records in that order.
-template <bool FIRST, int NR>
+template <int kRounds, bool FIRST, int NR>
 __global__ void __launch_bounds__(kThreads)
 order_pass_kernel(Buffers b, int n_events, int tiles_cap, int pass, int shift, int next_shift, int dims)
 {
+    constexpr int kTile = kRounds * kThreads;
     __shared__ int s_count[kWarps][256];
     __shared__ int s_warp[kWarps];
     const HitOrder &o = b.layout;
@@ -293,8 +292,8 @@ order_pass_kernel(Buffers b, int n_events, int tiles_cap, int pass, int shift, i
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d = threadIdx.x;
     const int e = event_of_tile(o.event_tile, n_events, blockIdx.x);
     const int off = b.row_splits_h[e], n_h = b.row_splits_h[e + 1] - off;
-    const int local = ((int)blockIdx.x - o.event_tile[e]) * kOrderTile;
-    const int n = min(n_h - local, kOrderTile);
+    const int local = ((int)blockIdx.x - o.event_tile[e]) * kTile;
+    const int n = min(n_h - local, kTile);
     if (n <= 0) return;
     const u64 *__restrict__ key_in = b.key[pass & 1] + off + local;
     const int *__restrict__ val_in = b.val[pass & 1] + off + local;
@@ -313,7 +312,7 @@ order_pass_kernel(Buffers b, int n_events, int tiles_cap, int pass, int shift, i
         start += block_scan_inclusive(mine, [](int x, int y) { return x + y; }, 0, s_warp) - mine;
         const int *__restrict__ h = b.tile_hist + (size_t)pass * tiles_cap * 256 + d;
         int sum = 0;
-#pragma unroll 8
+#pragma unroll 16
         for (int q = o.event_tile[e]; q < (int)blockIdx.x; q++) sum += h[(size_t)q * 256];
         start += sum;
     }
@@ -366,7 +365,7 @@ order_pass_kernel(Buffers b, int n_events, int tiles_cap, int pass, int shift, i
             } else {
                 b.key[(pass + 1) & 1][dst] = key[r];
                 b.val[(pass + 1) & 1][dst] = val[r];
-                const int q = tile0 + (dst - off) / kOrderTile;
+                const int q = tile0 + (dst - off) / kTile;
                 atomicAdd(&next_hist[(size_t)q * 256 + ((unsigned)(key[r] >> next_shift) & 255u)], 1);
             }
         }
@@ -708,8 +707,8 @@ assign_hits_kernel(Buffers b, const float *__restrict__ ccoords, const int *__re
                    const int *__restrict__ alpha)
 {
     HitTile t;
-    if (!find_tile(b.layout, n_events, blockIdx.x / kRounds, &t)) return;
-    const int i = (blockIdx.x % kRounds) * kThreads + threadIdx.x;
+    if (!find_tile(b.layout, n_events, blockIdx.x / (b.layout.tile / kThreads), &t)) return;
+    const int i = (blockIdx.x % (b.layout.tile / kThreads)) * kThreads + threadIdx.x;
     if (i >= t.n) return;
     const CondGrid grid = make_cond_grid(b.layout.grid, b.max_radius, dims, cells_per_dim);
     const bool real = t.event < n_events;
@@ -814,6 +813,7 @@ void layout(W &ws, int n_vert, int dims, int num_rows, const Plan &p, Buffers *o
     b.max_radius = ws.template take<unsigned>(1);
     if (zeroed) *zeroed = ws.used_bytes();
     b.layout = HitOrder();
+    b.layout.tile = order_tile(n_vert);
     b.layout.grid = ws.template take<GridParams>(1);
     b.layout.partial = ws.template take<float>((size_t)range_partial_blocks(n_vert) * 2 * kMaxBinDims);
     b.layout.event_pos = ws.template take<int>(e);
@@ -862,6 +862,18 @@ struct CarverW {
     size_t used_bytes() const { return c.used; }
 };
 
+template <bool FIRST, int NR>
+int launch_pass(const Buffers &b, int num_rows, int tiles, int pass, int shift, int next_shift, int dims, cudaStream_t stream)
+{
+    switch (b.layout.tile) {
+        case 512: order_pass_kernel<2, FIRST, NR><<<tiles, kThreads, 0, stream>>>(b, num_rows, tiles, pass, shift, next_shift, dims); break;
+        case 1024: order_pass_kernel<4, FIRST, NR><<<tiles, kThreads, 0, stream>>>(b, num_rows, tiles, pass, shift, next_shift, dims); break;
+        default: order_pass_kernel<8, FIRST, NR><<<tiles, kThreads, 0, stream>>>(b, num_rows, tiles, pass, shift, next_shift, dims);
+    }
+    HGC_LAUNCH_CHECK();
+    return HGC_OK;
+}
+
 // The last sort pass, the claims, the lists and the assignment, for records of NR float4.
 template <int NR>
 int run_claims(const Buffers &b, const Plan &p, int dims, int num_rows, int tiles, const float *ccoords, const int *mask,
@@ -869,8 +881,7 @@ int run_claims(const Buffers &b, const Plan &p, int dims, int num_rows, int tile
                int *n_condensates, cudaStream_t stream)
 {
     const int last = p.bin_passes + 3;
-    order_pass_kernel<false, NR><<<tiles, kThreads, 0, stream>>>(b, num_rows, tiles, last, 32 + 24, 0, dims);
-    HGC_LAUNCH_CHECK();
+    if (int rc = launch_pass<false, NR>(b, num_rows, tiles, last, 32 + 24, 0, dims, stream)) return rc;
     const size_t smem = 2 * sizeof(int) * (size_t)p.cells + (size_t)p.max_settled * (NR * sizeof(float4) + 2 * sizeof(int));
     // (set on every call: the setting belongs to the current device)
     HGC_CUDA_TRY(cudaFuncSetAttribute(claim_grid_kernel<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -883,7 +894,7 @@ int run_claims(const Buffers &b, const Plan &p, int dims, int num_rows, int tile
     list_condensates_kernel<NR><<<num_rows, 1024, 0, stream>>>(b, dims, p.cells, p.cells_per_dim, n_condensates, alpha_idx,
                                                                is_cond, assignment);
     HGC_LAUNCH_CHECK();
-    assign_hits_kernel<NR><<<tiles * kRounds, kThreads, 0, stream>>>(b, ccoords, mask, dims, num_rows, p.cells,
+    assign_hits_kernel<NR><<<tiles * (b.layout.tile / kThreads), kThreads, 0, stream>>>(b, ccoords, mask, dims, num_rows, p.cells,
                                                                      p.cells_per_dim, by_max_beta, assignment, association,
                                                                      is_cond, n_condensates, alpha_idx);
     HGC_LAUNCH_CHECK();
@@ -971,11 +982,9 @@ extern "C" int hgc_build_and_assign_condensates(
     HGC_LAUNCH_CHECK();
     auto shift_of = [&p](int pass) { return pass < p.bin_passes ? 8 * pass : 32 + 8 * (pass - p.bin_passes); };
     for (int i = 0; i + 1 < passes; i++) {  // the last one belongs to run_claims
-        if (i == 0)
-            order_pass_kernel<true, 0><<<tiles, kThreads, 0, stream>>>(b, num_rows, tiles, i, shift_of(i), shift_of(i + 1), dimensions);
-        else
-            order_pass_kernel<false, 0><<<tiles, kThreads, 0, stream>>>(b, num_rows, tiles, i, shift_of(i), shift_of(i + 1), dimensions);
-        HGC_LAUNCH_CHECK();
+        if (int rc = i == 0 ? launch_pass<true, 0>(b, num_rows, tiles, i, shift_of(i), shift_of(i + 1), dimensions, stream)
+                            : launch_pass<false, 0>(b, num_rows, tiles, i, shift_of(i), shift_of(i + 1), dimensions, stream))
+            return rc;
     }
     int rc = HGC_ERR_UNSUPPORTED;
 #define HGC_RUN(NR)                                                                                                  \

@@ -23,7 +23,6 @@ namespace {
 
 constexpr int kThreads = kOrderThreads;
 constexpr int kWarps = kThreads / kWarp;
-constexpr int kRounds = kOrderTile / kThreads;
 
 // Range of the coordinates over the batch; the first block also lays out the events, the last one to
 // finish derives the grid.
@@ -64,9 +63,7 @@ order_keys_kernel(const float *__restrict__ coords, int C, int n_dims, HitOrder 
     if (t.event == n_events && threadIdx.x == 0) flag_status(status, HGC_STATUS_FLAT_BIN_OVERFLOW);
     const GridParams *__restrict__ g = o.grid;
     const float bw = g->bin_width, scale = g->curve_scale * (float)(1u << B);
-    for (int r = 0; r < kRounds; r++) {
-        const int i = r * kThreads + threadIdx.x;
-        if (i >= t.n) break;
+    for (int i = threadIdx.x; i < t.n; i += kThreads) {
         const int v = t.first + i;
         float x[D];
 #pragma unroll
@@ -123,7 +120,7 @@ order_keys_kernel(const float *__restrict__ coords, int C, int n_dims, HitOrder 
 }
 
 // One pass of both sorts.  LAST: the permutation (and, for order 0, its inverse) is written instead of keys and values.
-template <bool FIRST, bool LAST>
+template <int kRounds, bool FIRST, bool LAST>
 __global__ void __launch_bounds__(kThreads)
 order_pass_kernel(HitOrder o, int n_events, int tiles_cap, int pass, int *__restrict__ bin_perm,
                   int *__restrict__ rank, int *__restrict__ curve_perm)
@@ -158,7 +155,7 @@ order_pass_kernel(HitOrder o, int n_events, int tiles_cap, int pass, int *__rest
         start += block_scan_inclusive(mine, [](int a, int b) { return a + b; }, 0, s_warp) - mine;
         const int *__restrict__ h = o.tile_hist + (size_t)(order * kOrderPasses + pass) * tiles_cap * 256 + d;
         int sum = 0;
-#pragma unroll 8
+#pragma unroll 16
         for (int q = o.event_tile[t.event]; q < (int)blockIdx.x; q++) sum += h[(size_t)q * 256];
         start += sum;
     }
@@ -207,7 +204,7 @@ order_pass_kernel(HitOrder o, int n_events, int tiles_cap, int pass, int *__rest
             } else {
                 o.key[order][(pass + 1) & 1][dst] = key[r];
                 o.val[order][(pass + 1) & 1][dst] = val[r];
-                const int q = tile0 + (dst - pos0) / kOrderTile;
+                const int q = tile0 + (dst - pos0) / (kRounds * kThreads);
                 atomicAdd(&next_hist[(size_t)q * 256 + ((key[r] >> (shift + 8)) & 255u)], 1);
             }
         }
@@ -253,12 +250,21 @@ int order_hits(const float *coords, int n_coords, int n_bin_dims, const int *row
     HGC_LAUNCH_CHECK();
     const dim3 grid(tiles, 2);
     for (int p = 0; p < kOrderPasses; p++) {
-        if (p == 0)
-            order_pass_kernel<true, false><<<grid, kThreads, 0, stream>>>(o, n_events, tiles, p, bin_perm, rank, curve_perm);
-        else if (p + 1 < kOrderPasses)
-            order_pass_kernel<false, false><<<grid, kThreads, 0, stream>>>(o, n_events, tiles, p, bin_perm, rank, curve_perm);
-        else
-            order_pass_kernel<false, true><<<grid, kThreads, 0, stream>>>(o, n_events, tiles, p, bin_perm, rank, curve_perm);
+#define HGC_PASS(R)                                                                                                  \
+    case R * kThreads:                                                                                               \
+        if (p == 0)                                                                                                  \
+            order_pass_kernel<R, true, false><<<grid, kThreads, 0, stream>>>(o, n_events, tiles, p, bin_perm, rank, curve_perm); \
+        else if (p + 1 < kOrderPasses)                                                                               \
+            order_pass_kernel<R, false, false><<<grid, kThreads, 0, stream>>>(o, n_events, tiles, p, bin_perm, rank, curve_perm); \
+        else                                                                                                         \
+            order_pass_kernel<R, false, true><<<grid, kThreads, 0, stream>>>(o, n_events, tiles, p, bin_perm, rank, curve_perm); \
+        break
+        switch (o.tile) {
+            HGC_PASS(2);
+            HGC_PASS(4);
+            HGC_PASS(8);
+        }
+#undef HGC_PASS
         HGC_LAUNCH_CHECK();
     }
     return HGC_OK;

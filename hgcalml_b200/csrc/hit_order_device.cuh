@@ -41,7 +41,7 @@ __device__ __forceinline__ void event_layout(const int *__restrict__ row_splits,
         int begin = __shfl_up_sync(0xffffffffu, end, 1);
         if (e == 0) begin = 0;
         const int n = e <= n_events ? end - begin : 0;
-        const int nt = (n + kOrderTile - 1) / kOrderTile, nc = (n + 31) / 32, ns = (nc + 31) / 32;
+        const int nt = (n + o.tile - 1) / o.tile, nc = (n + 31) / 32, ns = (nc + 31) / 32;
         int ti = nt, ci = nc, si = ns;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -79,7 +79,7 @@ __device__ __forceinline__ void event_layout(const int *__restrict__ row_splits,
         __syncthreads();
         if ((threadIdx.x & 31) == 0) begin = threadIdx.x == 0 ? pos : s_warp[(threadIdx.x >> 5) - 1];
         const int n = e <= n_events ? end - begin : 0;
-        const int nt = (n + kOrderTile - 1) / kOrderTile, nc = (n + 31) / 32, ns = (nc + 31) / 32;
+        const int nt = (n + o.tile - 1) / o.tile, nc = (n + 31) / 32, ns = (nc + 31) / 32;
         const int ti = tile + block_scan_inclusive(nt, add, 0, s_warp);
         const int ci = chunk + block_scan_inclusive(nc, add, 0, s_warp);
         const int si = super + block_scan_inclusive(ns, add, 0, s_warp);
@@ -118,8 +118,8 @@ __device__ __forceinline__ bool find_tile(const HitOrder &o, int n_events, int t
 {
     if (tile >= o.event_tile[n_events + 1]) return false;
     t->event = event_of_tile(o.event_tile, n_events, tile);
-    t->first = o.event_pos[t->event] + (tile - o.event_tile[t->event]) * kOrderTile;
-    t->n = min(o.event_pos[t->event + 1] - t->first, kOrderTile);
+    t->first = o.event_pos[t->event] + (tile - o.event_tile[t->event]) * o.tile;
+    t->n = min(o.event_pos[t->event + 1] - t->first, o.tile);
     return true;
 }
 

@@ -10,7 +10,6 @@ namespace hgc {
 namespace {
 
 constexpr int kThreads = kOrderThreads;
-constexpr int kRounds = kOrderTile / kThreads;
 
 __global__ void __launch_bounds__(kThreads)
 layout_kernel(const int *__restrict__ row_splits, int n_events, int n_vert, HitOrder o)
@@ -105,9 +104,8 @@ merge_noise_kernel(const int *__restrict__ assignment, const int *__restrict__ a
     const int before_event = s_sum[0], n_noise = s_sum[2] - s_sum[0];
     const int cond0 = n_cond[t.event] - n_cond[0], cond1 = n_cond[t.event + 1] - n_cond[0];
     int run = s_sum[1] - s_sum[0];  // noise hits of the event before this tile
-    for (int r = 0; r < kRounds; r++) {
-        if (r * kThreads >= t.n) break;  // uniform
-        const int i = r * kThreads + threadIdx.x, v = t.first + i;
+    for (int i0 = 0; i0 < t.n; i0 += kThreads) {
+        const int i = i0 + threadIdx.x, v = t.first + i;
         const bool in = i < t.n;
         const int as = in ? assignment[v] : 0;
         const bool noise = in && as < 0;
@@ -140,6 +138,7 @@ void layout(W &ws, int n_vert, int n_rs, HitOrder *o, int2 **counts, int **n_alp
     const int n_events = n_rs > 1 ? n_rs - 1 : 0;
     const size_t e = (size_t)n_events + 2;
     *o = HitOrder();
+    o->tile = order_tile(n_vert);
     o->event_pos = ws.template take<int>(e);
     o->event_tile = ws.template take<int>(e);
     o->event_chunk = ws.template take<int>(e);
