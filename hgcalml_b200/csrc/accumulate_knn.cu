@@ -87,6 +87,7 @@ accumulate_vec_kernel(const float *__restrict__ weights, const float *__restrict
                       int n_vert, int K, int ldk, int F_arg, int n_out_feat, bool mean_and_max,
                       const int *__restrict__ order, float scale, bool sub_self, int tile_steps)
 {
+    pdl_begin();
     const int F = EXACT ? LPH * VPL * VW : F_arg;
     const int n_vec = EXACT ? LPH * VPL : F_arg / VW;
     constexpr int G = THREADS / LPH;  // hits a block works on at a time
@@ -302,6 +303,7 @@ accumulate_scalar_kernel(const float *__restrict__ weights, const float *__restr
                          int n_vert, int K, int ldk, int F, int n_out_feat, bool mean_and_max,
                          const int *__restrict__ order, float scale, bool sub_self)
 {
+    pdl_begin();
     const int lane = threadIdx.x & 31;
     const int warps_per_block = kAccThreads / kWarp;
     for (long long g = (long long)blockIdx.x * warps_per_block + (threadIdx.x >> 5); g < n_vert;
@@ -350,8 +352,8 @@ int launch_vec(bool exp_w, bool with_arg, const float *w, const float *feat, con
     long long blocks = (long long)sm_count() * 32;
     if (blocks > n_tiles) blocks = n_tiles;
 #define HGC_GO(E, A, X)                                                                                    \
-    accumulate_vec_kernel<VW, LPH, VPL, CH, THREADS, MINB, E, A, X><<<(int)blocks, THREADS, 0, stream>>>(  \
-            w, feat, idxs, out, out_arg, n_vert, K, ldk, F, n_out, mm, order, scale, sub_self, tile_steps)
+    HGC_CUDA_TRY(launch_overlapped(n_vert, accumulate_vec_kernel<VW, LPH, VPL, CH, THREADS, MINB, E, A, X>, (int)blocks, THREADS, 0, stream, \
+            w, feat, idxs, out, out_arg, n_vert, K, ldk, F, n_out, mm, order, scale, sub_self, tile_steps))
 #define HGC_GO2(E, A) do { if (VW == 4 && F == LPH * VPL * VW) HGC_GO(E, A, (VW == 4)); else HGC_GO(E, A, false); } while (0)
     if (exp_w) { if (with_arg) HGC_GO2(true, true); else HGC_GO2(true, false); }
     else       { if (with_arg) HGC_GO2(false, true); else HGC_GO2(false, false); }
@@ -383,11 +385,9 @@ int accumulate_dispatch(bool exp_w, const float *w, const float *feat, const int
         const long long cap = (long long)sm_count() * 32;
         if (blocks > cap) blocks = cap;
         if (exp_w)
-            accumulate_scalar_kernel<true><<<(int)blocks, kAccThreads, 0, stream>>>(
-                    w, feat, idxs, out, with_arg ? out_arg : nullptr, n_vert, K, ldk, F, n_out, mm, order, scale, sub_self);
+            HGC_CUDA_TRY(launch_overlapped(n_vert, accumulate_scalar_kernel<true>, (int)blocks, kAccThreads, 0, stream, w, feat, idxs, out, with_arg ? out_arg : nullptr, n_vert, K, ldk, F, n_out, mm, order, scale, sub_self));
         else
-            accumulate_scalar_kernel<false><<<(int)blocks, kAccThreads, 0, stream>>>(
-                    w, feat, idxs, out, with_arg ? out_arg : nullptr, n_vert, K, ldk, F, n_out, mm, order, scale, sub_self);
+            HGC_CUDA_TRY(launch_overlapped(n_vert, accumulate_scalar_kernel<false>, (int)blocks, kAccThreads, 0, stream, w, feat, idxs, out, with_arg ? out_arg : nullptr, n_vert, K, ldk, F, n_out, mm, order, scale, sub_self));
         HGC_LAUNCH_CHECK();
         return HGC_OK;
     }

@@ -20,6 +20,7 @@ __global__ void bin_keys_kernel(const float *__restrict__ coords, int coord_stri
                                 const int *__restrict__ n_total_bins_dev, unsigned *status,
                                 const GridParams *__restrict__ grid, int n_all, int *__restrict__ sub_keys)
 {
+    pdl_begin();
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= n_vert) return;
     unsigned frac[kMaxBinDims];  // position inside the cell as a 16-bit fraction (ordering code only)
@@ -87,6 +88,7 @@ __global__ void bin_keys_kernel(const float *__restrict__ coords, int coord_stri
 
 __global__ void adjacent_difference_kernel(const int *__restrict__ bounds, int *__restrict__ out, int n)
 {
+    pdl_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = bounds[i + 1] - bounds[i];
 }
@@ -97,6 +99,7 @@ __global__ void __launch_bounds__(256)
 range_partial_kernel(const float *__restrict__ coords, int coord_stride, int n_dims, int n_vert,
                      float *__restrict__ partial /* [gridDim.x][2][kMaxBinDims] */)
 {
+    pdl_begin();
     range_of_block(coords, coord_stride, n_dims, n_vert, partial);
 }
 
@@ -106,6 +109,7 @@ grid_setup_kernel(const float *__restrict__ partial, int n_partials, int n_dims,
                   const int *__restrict__ row_splits, int n_rs, int n_bins_arg, int n_neigh,
                   int pre_normalized, GridParams *__restrict__ g)
 {
+    pdl_begin();
     grid_from_partials(partial, n_partials, n_dims, n_all, row_splits, n_rs, n_bins_arg, n_neigh, pre_normalized, g);
 }
 
@@ -116,10 +120,10 @@ int compute_grid(const float *coords, int coord_stride, int n_dims, int n_all, i
     if (n_all < n_dims) n_all = n_dims;
     if (n_all > kMaxBinDims) n_all = kMaxBinDims;
     const int blocks = range_partial_blocks(n_vert);
-    range_partial_kernel<<<blocks, 256, 0, stream>>>(coords, coord_stride, n_all, n_vert, partial);
+    HGC_CUDA_TRY(launch_pdl(range_partial_kernel, blocks, 256, 0, stream, coords, coord_stride, n_all, n_vert, partial));
     HGC_LAUNCH_CHECK();
-    grid_setup_kernel<<<1, kGridSetupThreads, 0, stream>>>(partial, blocks, n_dims, n_all, row_splits, n_rs, n_bins_arg,
-                                           n_neigh, pre_normalized, grid);
+    HGC_CUDA_TRY(launch_pdl(grid_setup_kernel, 1, kGridSetupThreads, 0, stream, partial, blocks, n_dims, n_all, row_splits, n_rs, n_bins_arg,
+                                           n_neigh, pre_normalized, grid));
     HGC_LAUNCH_CHECK();
     return HGC_OK;
 }
@@ -140,9 +144,8 @@ int launch_bin_keys(const float *coords, int coord_stride, int n_dims, const flo
 {
     if (n_vert <= 0) return HGC_OK;
     if (n_all > kMaxBinDims) n_all = kMaxBinDims;
-    bin_keys_kernel<<<div_up(n_vert, 256), 256, 0, stream>>>(
-            coords, coord_stride, n_dims, shift, row_splits, n_rs, bin_width, n_bins, assigned, flat_out,
-            sort_keys, n_vert, n_total_bins, n_total_bins_dev, status, grid, n_all, grid ? sub_keys : nullptr);
+    HGC_CUDA_TRY(launch_pdl(bin_keys_kernel, div_up(n_vert, 256), 256, 0, stream, coords, coord_stride, n_dims, shift, row_splits, n_rs, bin_width, n_bins, assigned, flat_out,
+            sort_keys, n_vert, n_total_bins, n_total_bins_dev, status, grid, n_all, grid ? sub_keys : nullptr));
     HGC_LAUNCH_CHECK();
     return HGC_OK;
 }
@@ -202,7 +205,7 @@ extern "C" int hgc_bin_by_coordinates(
                             bits_for(n_total_bins), stream))
         return rc;
     if (int rc = boundaries_from_sorted_keys(skeys, n_vert, bounds, n_total_bins, stream)) return rc;
-    adjacent_difference_kernel<<<div_up(n_total_bins, 256), 256, 0, stream>>>(bounds, d_n_per_bin, n_total_bins);
+    HGC_CUDA_TRY(launch_pdl(adjacent_difference_kernel, div_up(n_total_bins, 256), 256, 0, stream, bounds, d_n_per_bin, n_total_bins));
     HGC_LAUNCH_CHECK();
     return HGC_OK;
 }

@@ -37,6 +37,7 @@ __global__ void priority_keys_kernel(const float *__restrict__ beta_h, const int
                                      const int *__restrict__ row_splits_h, int num_rows, int n_h,
                                      int *__restrict__ beta_keys, int *__restrict__ event_keys)
 {
+    pdl_begin();
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     if (a >= n_h) return;
     const bool flagged = mask_h[a > 0 ? 1 : 0] != 0;  // n_h >= 2 whenever a > 0
@@ -52,6 +53,7 @@ __global__ void priority_keys_kernel(const float *__restrict__ beta_h, const int
 __global__ void gather_int_kernel(const int *__restrict__ src, const int *__restrict__ idx,
                                   int *__restrict__ dst, int n)
 {
+    pdl_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) dst[i] = src[idx[i]];
 }
@@ -59,6 +61,7 @@ __global__ void gather_int_kernel(const int *__restrict__ src, const int *__rest
 __global__ void init_outputs_kernel(int *__restrict__ status_h, int *__restrict__ alpha, int n_h,
                                     int *__restrict__ assignment, int *__restrict__ association, int n)
 {
+    pdl_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n_h) { status_h[i] = 0; alpha[i] = -1; }
     if (i < n) { assignment[i] = -1; association[i] = -1; }
@@ -92,6 +95,7 @@ claim_kernel(int dims, const float *__restrict__ ccoords_h, const float *__restr
              int *__restrict__ status_h, int *__restrict__ alpha_indices, int *__restrict__ stage_all,
              CondList cl, const int *__restrict__ use_grid)
 {
+    pdl_begin();
     if (use_grid && *use_grid) return;
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
@@ -256,6 +260,7 @@ claim_kernel(int dims, const float *__restrict__ ccoords_h, const float *__restr
 __global__ void condensate_totals_kernel(const int *__restrict__ count, int num_rows,
                                          int *__restrict__ n_condensates)
 {
+    pdl_begin();
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         int run = 0;
         n_condensates[0] = 0;
@@ -275,6 +280,7 @@ assign_kernel(int dims, const float *__restrict__ ccoords, const int *__restrict
               int n_vert, bool by_max_beta, CondList cl, int *__restrict__ assignment,
               int *__restrict__ association)
 {
+    pdl_begin();
     __shared__ float4 s_rec[kCondTile][NR];
     __shared__ int s_pos[kCondTile];
     __shared__ int s_lonely[kCondTile];
@@ -383,9 +389,9 @@ int launch_claim_windows(int dims, const float *ccoords_h, const float *dist_h, 
                          cudaStream_t stream)
 {
 #define HGC_CLAIM(NR)                                                                                        \
-    claim_kernel<NR><<<num_rows * kClusterBlocks, kClaimThreads, 0, stream>>>(                                 \
+    HGC_CUDA_TRY(launch_pdl(claim_kernel<NR>, num_rows * kClusterBlocks, kClaimThreads, 0, stream, \
             dims, ccoords_h, dist_h, mask_h, original_indices_h, row_splits_h, order, status_h, alpha_indices, \
-            stage, cl, use_grid)
+            stage, cl, use_grid))
     if (rec_size(dims) == 1) HGC_CLAIM(1);
     else if (rec_size(dims) == 2) HGC_CLAIM(2);
     else HGC_CLAIM(3);
@@ -470,19 +476,19 @@ extern "C" int hgc_binned_assign_to_condensates(
 
     const int n_init = n_vert > n_vert_h ? n_vert : n_vert_h;
     if (n_init > 0) {
-        init_outputs_kernel<<<div_up(n_init, 256), 256, 0, stream>>>(d_high_assigned_status_h, d_alpha_indices,
-                                                                     n_vert_h, d_assignment, d_association, n_vert);
+        HGC_CUDA_TRY(launch_pdl(init_outputs_kernel, div_up(n_init, 256), 256, 0, stream, d_high_assigned_status_h, d_alpha_indices,
+                                                                     n_vert_h, d_assignment, d_association, n_vert));
         HGC_LAUNCH_CHECK();
     }
     if (num_rows > 0) HGC_CUDA_TRY(cudaMemsetAsync(b.cl.count, 0, sizeof(int) * (size_t)num_rows, stream));
     if (n_vert_h > 0 && num_rows > 0) {
-        priority_keys_kernel<<<div_up(n_vert_h, 256), 256, 0, stream>>>(d_beta_h, d_no_condensation_mask_h,
+        HGC_CUDA_TRY(launch_pdl(priority_keys_kernel, div_up(n_vert_h, 256), 256, 0, stream, d_beta_h, d_no_condensation_mask_h,
                                                                         d_row_splits_h, num_rows, n_vert_h,
-                                                                        b.beta_keys, b.event_keys);
+                                                                        b.beta_keys, b.event_keys));
         HGC_LAUNCH_CHECK();
         // stable sort by priority, then stable sort by event: per event, priority order
         if (int rc = sort_pairs(b.beta_keys, nullptr, b.k1, b.v1, b.tk, b.tv, b.hist, n_vert_h, 32, stream)) return rc;
-        gather_int_kernel<<<div_up(n_vert_h, 256), 256, 0, stream>>>(b.event_keys, b.v1, b.k1, n_vert_h);
+        HGC_CUDA_TRY(launch_pdl(gather_int_kernel, div_up(n_vert_h, 256), 256, 0, stream, b.event_keys, b.v1, b.k1, n_vert_h));
         HGC_LAUNCH_CHECK();
         if (int rc = sort_pairs(b.k1, b.v1, b.k2, b.v2, b.tk, b.tv, b.hist, n_vert_h, bits_for(num_rows), stream)) return rc;
         if (int rc = launch_claim_windows(dimensions, d_ccoords_h, d_dist_h, d_no_condensation_mask_h, d_original_indices_h,
@@ -490,14 +496,14 @@ extern "C" int hgc_binned_assign_to_condensates(
                                           num_rows, nullptr, stream))
             return rc;
     }
-    condensate_totals_kernel<<<1, 32, 0, stream>>>(b.cl.count, num_rows, d_n_condensates);
+    HGC_CUDA_TRY(launch_pdl(condensate_totals_kernel, 1, 32, 0, stream, b.cl.count, num_rows, d_n_condensates));
     HGC_LAUNCH_CHECK();
     if (n_vert > 0 && n_vert_h > 0 && num_rows > 0) {
 #define HGC_ASSIGN(NR)                                                                                         \
-    assign_kernel<NR><<<div_up(n_vert, kAssignThreads), kAssignThreads, 0, stream>>>(                            \
+    HGC_CUDA_TRY(launch_pdl(assign_kernel<NR>, div_up(n_vert, kAssignThreads), kAssignThreads, 0, stream, \
             dimensions, d_ccoords, d_no_condensation_mask, d_indices_to_filtered, d_original_indices_h,          \
             d_row_splits, d_row_splits_h, num_rows, n_vert, assign_by_max_beta != 0, b.cl, d_assignment,         \
-            d_association)
+            d_association))
         if (dimensions <= 3) HGC_ASSIGN(1);
         else if (dimensions <= 7) HGC_ASSIGN(2);
         else HGC_ASSIGN(3);

@@ -143,6 +143,7 @@ count_high_kernel(const float *__restrict__ betas, const int *__restrict__ mask,
                   int n_events, int *__restrict__ tile_count, int *__restrict__ alpha_out, unsigned char *__restrict__ is_cond,
                   u64 *__restrict__ first_two)
 {
+    pdl_begin();
     HitTile t;
     if (!find_tile(o, n_events, blockIdx.x, &t)) return;
     if (blockIdx.x == 0 && threadIdx.x < 2) first_two[threadIdx.x] = ~0ull;
@@ -171,6 +172,7 @@ __global__ void __launch_bounds__(kThreads)
 first_high_kernel(const float *__restrict__ ccoords, const float *__restrict__ betas, const int *__restrict__ mask,
                   float beta_threshold, int dims, int cb, HitOrder o, int n_events, u64 *__restrict__ first_two)
 {
+    pdl_begin();
     HitTile t;
     if (!find_tile(o, n_events, blockIdx.x, &t) || t.event >= n_events) return;
     const u64 first = SECOND ? first_two[0] : 0ull;
@@ -190,6 +192,7 @@ order_high_kernel(const float *__restrict__ ccoords, const float *__restrict__ b
                   const int *__restrict__ mask, float beta_threshold, float distance_threshold, int dims, int cb,
                   int bin_passes, int n_events, Buffers b, unsigned *status)
 {
+    pdl_begin();
     extern __shared__ int s_hist[];  // [passes][256]
     __shared__ int s_warp[kWarps];
     __shared__ int s_base;
@@ -284,6 +287,7 @@ template <int kRounds, bool FIRST, int NR>
 __global__ void __launch_bounds__(kThreads)
 order_pass_kernel(Buffers b, int n_events, int tiles_cap, int pass, int shift, int next_shift, int dims)
 {
+    pdl_begin();
     constexpr int kTile = kRounds * kThreads;
     __shared__ int s_count[kWarps][256];
     __shared__ int s_warp[kWarps];
@@ -389,6 +393,7 @@ template <int NR>
 __global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(kClaimThreads)
 claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max_settled)
 {
+    pdl_begin();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ int s_dyn[];
@@ -591,6 +596,7 @@ __global__ void __launch_bounds__(1024)
 list_condensates_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int *__restrict__ n_condensates,
                         int *__restrict__ alpha_out, unsigned char *__restrict__ is_cond, int *__restrict__ assignment)
 {
+    pdl_begin();
     __shared__ int s_warp[32];
     __shared__ int s_base, s_before;
     const int e = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -706,6 +712,7 @@ assign_hits_kernel(Buffers b, const float *__restrict__ ccoords, const int *__re
                    const unsigned char *__restrict__ is_cond, const int *__restrict__ n_condensates,
                    const int *__restrict__ alpha)
 {
+    pdl_begin();
     HitTile t;
     if (!find_tile(b.layout, n_events, blockIdx.x / (b.layout.tile / kThreads), &t)) return;
     const int i = (blockIdx.x % (b.layout.tile / kThreads)) * kThreads + threadIdx.x;
@@ -866,9 +873,9 @@ template <bool FIRST, int NR>
 int launch_pass(const Buffers &b, int num_rows, int tiles, int pass, int shift, int next_shift, int dims, cudaStream_t stream)
 {
     switch (b.layout.tile) {
-        case 512: order_pass_kernel<2, FIRST, NR><<<tiles, kThreads, 0, stream>>>(b, num_rows, tiles, pass, shift, next_shift, dims); break;
-        case 1024: order_pass_kernel<4, FIRST, NR><<<tiles, kThreads, 0, stream>>>(b, num_rows, tiles, pass, shift, next_shift, dims); break;
-        default: order_pass_kernel<8, FIRST, NR><<<tiles, kThreads, 0, stream>>>(b, num_rows, tiles, pass, shift, next_shift, dims);
+        case 512: HGC_CUDA_TRY(launch_pdl(order_pass_kernel<2, FIRST, NR>, tiles, kThreads, 0, stream, b, num_rows, tiles, pass, shift, next_shift, dims)); break;
+        case 1024: HGC_CUDA_TRY(launch_pdl(order_pass_kernel<4, FIRST, NR>, tiles, kThreads, 0, stream, b, num_rows, tiles, pass, shift, next_shift, dims)); break;
+        default: HGC_CUDA_TRY(launch_pdl(order_pass_kernel<8, FIRST, NR>, tiles, kThreads, 0, stream, b, num_rows, tiles, pass, shift, next_shift, dims));
     }
     HGC_LAUNCH_CHECK();
     return HGC_OK;
@@ -885,18 +892,18 @@ int run_claims(const Buffers &b, const Plan &p, int dims, int num_rows, int tile
     const size_t smem = 2 * sizeof(int) * (size_t)p.cells + (size_t)p.max_settled * (NR * sizeof(float4) + 2 * sizeof(int));
     // (set on every call: the setting belongs to the current device)
     HGC_CUDA_TRY(cudaFuncSetAttribute(claim_grid_kernel<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    claim_grid_kernel<NR><<<num_rows * kClusterBlocks, kClaimThreads, smem, stream>>>(b, dims, p.cells, p.cells_per_dim,
-                                                                                      p.max_settled);
+    HGC_CUDA_TRY(launch_pdl(claim_grid_kernel<NR>, num_rows * kClusterBlocks, kClaimThreads, smem, stream, b, dims, p.cells, p.cells_per_dim,
+                                                                                      p.max_settled));
     HGC_LAUNCH_CHECK();
     if (int rc = launch_claim_windows(dims, b.h_ccoords, b.h_dist, b.h_mask, b.h_orig, b.row_splits_h, b.order, b.status_h,
                                       b.alpha_h, b.stage, b.cl, num_rows, b.use_grid, stream))
         return rc;
-    list_condensates_kernel<NR><<<num_rows, 1024, 0, stream>>>(b, dims, p.cells, p.cells_per_dim, n_condensates, alpha_idx,
-                                                               is_cond, assignment);
+    HGC_CUDA_TRY(launch_pdl(list_condensates_kernel<NR>, num_rows, 1024, 0, stream, b, dims, p.cells, p.cells_per_dim, n_condensates, alpha_idx,
+                                                               is_cond, assignment));
     HGC_LAUNCH_CHECK();
-    assign_hits_kernel<NR><<<tiles * (b.layout.tile / kThreads), kThreads, 0, stream>>>(b, ccoords, mask, dims, num_rows, p.cells,
+    HGC_CUDA_TRY(launch_pdl(assign_hits_kernel<NR>, tiles * (b.layout.tile / kThreads), kThreads, 0, stream, b, ccoords, mask, dims, num_rows, p.cells,
                                                                      p.cells_per_dim, by_max_beta, assignment, association,
-                                                                     is_cond, n_condensates, alpha_idx);
+                                                                     is_cond, n_condensates, alpha_idx));
     HGC_LAUNCH_CHECK();
     return HGC_OK;
 }
@@ -964,21 +971,20 @@ extern "C" int hgc_build_and_assign_condensates(
                                   stream))
         return rc;
     const int tiles = (int)order_tiles_cap(n_vert, num_rows);
-    count_high_kernel<<<tiles, kThreads, 0, stream>>>(d_betas, d_no_condensation_mask, beta_threshold, b.layout, num_rows,
-                                                      b.tile_count, d_alpha_idx, d_is_cond, b.first_two);
+    HGC_CUDA_TRY(launch_pdl(count_high_kernel, tiles, kThreads, 0, stream, d_betas, d_no_condensation_mask, beta_threshold, b.layout, num_rows,
+                                                      b.tile_count, d_alpha_idx, d_is_cond, b.first_two));
     HGC_LAUNCH_CHECK();
     if (d_no_condensation_mask) {
-        first_high_kernel<false><<<tiles, kThreads, 0, stream>>>(d_ccoords, d_betas, d_no_condensation_mask, beta_threshold,
-                                                                 dimensions, p.cb, b.layout, num_rows, b.first_two);
+        HGC_CUDA_TRY(launch_pdl(first_high_kernel<false>, tiles, kThreads, 0, stream, d_ccoords, d_betas, d_no_condensation_mask, beta_threshold,
+                                                                 dimensions, p.cb, b.layout, num_rows, b.first_two));
         HGC_LAUNCH_CHECK();
-        first_high_kernel<true><<<tiles, kThreads, 0, stream>>>(d_ccoords, d_betas, d_no_condensation_mask, beta_threshold,
-                                                                dimensions, p.cb, b.layout, num_rows, b.first_two);
+        HGC_CUDA_TRY(launch_pdl(first_high_kernel<true>, tiles, kThreads, 0, stream, d_ccoords, d_betas, d_no_condensation_mask, beta_threshold,
+                                                                dimensions, p.cb, b.layout, num_rows, b.first_two));
         HGC_LAUNCH_CHECK();
     }
     const int passes = p.bin_passes + 4;
-    order_high_kernel<<<tiles, kThreads, sizeof(int) * 256 * passes, stream>>>(
-            d_ccoords, d_betas, d_dist, d_no_condensation_mask, beta_threshold, distance_threshold, dimensions, p.cb,
-            p.bin_passes, num_rows, b, status);
+    HGC_CUDA_TRY(launch_pdl(order_high_kernel, tiles, kThreads, sizeof(int) * 256 * passes, stream, d_ccoords, d_betas, d_dist, d_no_condensation_mask, beta_threshold, distance_threshold, dimensions, p.cb,
+            p.bin_passes, num_rows, b, status));
     HGC_LAUNCH_CHECK();
     auto shift_of = [&p](int pass) { return pass < p.bin_passes ? 8 * pass : 32 + 8 * (pass - p.bin_passes); };
     for (int i = 0; i + 1 < passes; i++) {  // the last one belongs to run_claims

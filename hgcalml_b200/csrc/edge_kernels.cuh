@@ -24,6 +24,7 @@ edge_sum_kernel(const float *__restrict__ x, int ldx, const float *__restrict__ 
                 const int *__restrict__ edges, float *__restrict__ out, int n_vert, int K, int F, int f0,
                 const int *__restrict__ order)
 {
+    pdl_begin();
     constexpr int U = 8;
     const int lane = threadIdx.x & 31;
     const int slot = blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -104,6 +105,7 @@ static __global__ void __launch_bounds__(256)
 arg_flags_kernel(const int *__restrict__ arg, const int *__restrict__ nidx, unsigned *__restrict__ flags, int n_vert,
                  int K, int F, int f0)
 {
+    pdl_begin();
     const int lane = threadIdx.x & 31;
     const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
     if (i >= n_vert) return;
@@ -137,6 +139,7 @@ edge_dot_kernel(const float *__restrict__ own, int ld_own, const float *__restri
                 const int *__restrict__ nidx, float *__restrict__ out, long long n_edges, int n_vert, int K, int F,
                 bool vec4, const int *__restrict__ order, unsigned *__restrict__ flags)
 {
+    pdl_begin();
     constexpr int kRow = 36;
     __shared__ __align__(16) float s_x[8][32 * kRow];
     const int lane = threadIdx.x & 31;
@@ -225,7 +228,7 @@ int launch_edge_sum_slab(const float *x, int ldx, const float *weights, const un
                          const int *order, cudaStream_t stream)
 {
     const int blocks = div_up(n_vert, 8);
-#define HGC_SUM(FPL, P) edge_sum_kernel<FPL, MODE, P><<<blocks, 256, 0, stream>>>(x, ldx, weights, flags, nidx, bounds, edges, out, n_vert, K, F, f0, order)
+#define HGC_SUM(FPL, P) HGC_CUDA_TRY(launch_overlapped(n_vert, edge_sum_kernel<FPL, MODE, P>, blocks, 256, 0, stream, x, ldx, weights, flags, nidx, bounds, edges, out, n_vert, K, F, f0, order))
     const bool pow2 = MODE == kSumPlain || (K & (K - 1)) == 0;
     if (F - f0 <= 32) { if (pow2) HGC_SUM(1, true); else HGC_SUM(1, false); }
     else              { if (pow2) HGC_SUM(2, true); else HGC_SUM(2, false); }

@@ -31,6 +31,7 @@ range_and_layout_kernel(const float *__restrict__ coords, int C, int n_dims, int
                         const int *__restrict__ row_splits, int n_rs, int n_bins, int n_neigh, HitOrder o,
                         unsigned *arrived)
 {
+    pdl_begin();
     __shared__ bool s_last;
     range_of_block(coords, C, n_all, n_vert, o.partial);
     __syncthreads();
@@ -54,6 +55,7 @@ __global__ void __launch_bounds__(kThreads)
 order_keys_kernel(const float *__restrict__ coords, int C, int n_dims, HitOrder o, int n_events, int tiles_cap,
                   unsigned *status)
 {
+    pdl_begin();
     __shared__ int s_hist[2][kOrderPasses][256];
     __shared__ unsigned short s_frac[kMaxBinDims][kThreads];
     HitTile t;
@@ -125,6 +127,7 @@ __global__ void __launch_bounds__(kThreads)
 order_pass_kernel(HitOrder o, int n_events, int tiles_cap, int pass, int *__restrict__ bin_perm,
                   int *__restrict__ rank, int *__restrict__ curve_perm)
 {
+    pdl_begin();
     __shared__ int s_count[kWarps][256];
     __shared__ int s_warp[kWarps];
     const int order = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d = threadIdx.x;
@@ -216,9 +219,8 @@ order_pass_kernel(HitOrder o, int n_events, int tiles_cap, int pass, int *__rest
 int range_and_layout(const float *coords, int n_coords, int n_bin_dims, const int *row_splits, int n_rs, int n_bins,
                      int n_neigh, int n_vert, const HitOrder &o, unsigned *status, cudaStream_t stream)
 {
-    range_and_layout_kernel<<<range_partial_blocks(n_vert), kThreads, 0, stream>>>(
-            coords, n_coords, n_bin_dims, n_coords < kMaxBinDims ? n_coords : kMaxBinDims, n_vert, row_splits, n_rs, n_bins,
-            n_neigh, o, status + 8);
+    HGC_CUDA_TRY(launch_pdl(range_and_layout_kernel, range_partial_blocks(n_vert), kThreads, 0, stream, coords, n_coords, n_bin_dims, n_coords < kMaxBinDims ? n_coords : kMaxBinDims, n_vert, row_splits, n_rs, n_bins,
+            n_neigh, o, status + 8));
     HGC_LAUNCH_CHECK();
     return HGC_OK;
 }
@@ -235,7 +237,7 @@ int order_hits(const float *coords, int n_coords, int n_bin_dims, const int *row
         return rc;
     const int tiles = (int)order_tiles_cap(n_vert, n_events);
 #define HGC_KEYS(D, B)                                                                                            \
-    case D: order_keys_kernel<D, B><<<tiles, kThreads, 0, stream>>>(coords, n_coords, n_bin_dims, o, n_events, tiles, status); break
+    case D: HGC_CUDA_TRY(launch_pdl(order_keys_kernel<D, B>, tiles, kThreads, 0, stream, coords, n_coords, n_bin_dims, o, n_events, tiles, status)); break
     switch (n_all) {
         HGC_KEYS(2, 16);
         HGC_KEYS(3, 10);
@@ -253,11 +255,11 @@ int order_hits(const float *coords, int n_coords, int n_bin_dims, const int *row
 #define HGC_PASS(R)                                                                                                  \
     case R * kThreads:                                                                                               \
         if (p == 0)                                                                                                  \
-            order_pass_kernel<R, true, false><<<grid, kThreads, 0, stream>>>(o, n_events, tiles, p, bin_perm, rank, curve_perm); \
+            HGC_CUDA_TRY(launch_pdl(order_pass_kernel<R, true, false>, grid, kThreads, 0, stream, o, n_events, tiles, p, bin_perm, rank, curve_perm)); \
         else if (p + 1 < kOrderPasses)                                                                               \
-            order_pass_kernel<R, false, false><<<grid, kThreads, 0, stream>>>(o, n_events, tiles, p, bin_perm, rank, curve_perm); \
+            HGC_CUDA_TRY(launch_pdl(order_pass_kernel<R, false, false>, grid, kThreads, 0, stream, o, n_events, tiles, p, bin_perm, rank, curve_perm)); \
         else                                                                                                         \
-            order_pass_kernel<R, false, true><<<grid, kThreads, 0, stream>>>(o, n_events, tiles, p, bin_perm, rank, curve_perm); \
+            HGC_CUDA_TRY(launch_pdl(order_pass_kernel<R, false, true>, grid, kThreads, 0, stream, o, n_events, tiles, p, bin_perm, rank, curve_perm)); \
         break
         switch (o.tile) {
             HGC_PASS(2);

@@ -19,6 +19,7 @@ __global__ void __launch_bounds__(256)
 count_targets_kernel(const int *__restrict__ nidx, long long n_edges, int n_vert, int *__restrict__ count,
                      int *__restrict__ place)
 {
+    pdl_begin();
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n_edges) return;
     const int m = nidx[e];
@@ -29,6 +30,7 @@ __global__ void __launch_bounds__(256)
 place_edges_kernel(const int *__restrict__ nidx, const int *__restrict__ place, long long n_edges, int n_vert,
                    const int *__restrict__ bounds, int *__restrict__ edges)
 {
+    pdl_begin();
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n_edges) return;
     const int m = nidx[e];
@@ -72,6 +74,7 @@ __device__ __forceinline__ void sort_list(int *list, int n, int lane)
 __global__ void __launch_bounds__(256)
 sort_lists_kernel(const int *__restrict__ bounds, int *__restrict__ edges, int n_vert, int *__restrict__ long_lists)
 {
+    pdl_begin();
     const int m = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (m >= n_vert) return;
     const int begin = bounds[m], n = bounds[m + 1] - begin;
@@ -87,6 +90,7 @@ __global__ void __launch_bounds__(256)
 sort_long_lists_kernel(const int *__restrict__ bounds, int *edges, int *tmp, const int *__restrict__ long_lists,
                        int n_passes)
 {
+    pdl_begin();
     __shared__ int s_run[256], s_count[8][256], s_warp[8];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int n_long = long_lists[0];
@@ -146,18 +150,18 @@ int build_incoming(const int *nidx, int n_vert, int n_neigh, const Incoming &b, 
     const long long ne = (long long)n_vert * n_neigh;
     // the status word, the counts (bounds) and the number of long lists lie one after another
     HGC_CUDA_TRY(cudaMemsetAsync(status, 0, (size_t)(reinterpret_cast<char *>(b.long_lists + 1) - reinterpret_cast<char *>(status)), stream));
-    count_targets_kernel<<<div_up(ne, 256), 256, 0, stream>>>(nidx, ne, n_vert, b.bounds, b.place);
+    HGC_CUDA_TRY(launch_overlapped(n_vert, count_targets_kernel, div_up(ne, 256), 256, 0, stream, nidx, ne, n_vert, b.bounds, b.place));
     HGC_LAUNCH_CHECK();
     if (int rc = exclusive_scan_ints(b.bounds, n_vert + 1, b.scan, stream)) return rc;
-    place_edges_kernel<<<div_up(ne, 256), 256, 0, stream>>>(nidx, b.place, ne, n_vert, b.bounds, b.edges);
+    HGC_CUDA_TRY(launch_overlapped(n_vert, place_edges_kernel, div_up(ne, 256), 256, 0, stream, nidx, b.place, ne, n_vert, b.bounds, b.edges));
     HGC_LAUNCH_CHECK();
-    sort_lists_kernel<<<div_up(n_vert, 8), 256, 0, stream>>>(b.bounds, b.edges, n_vert, b.long_lists);
+    HGC_CUDA_TRY(launch_overlapped(n_vert, sort_lists_kernel, div_up(n_vert, 8), 256, 0, stream, b.bounds, b.edges, n_vert, b.long_lists));
     HGC_LAUNCH_CHECK();
     if (ne > 128) {
         int blocks = sm_count();
         if (blocks > ne / 129) blocks = (int)(ne / 129);
         if (blocks < 1) blocks = 1;
-        sort_long_lists_kernel<<<blocks, 256, 0, stream>>>(b.bounds, b.edges, b.place, b.long_lists, (bits_for(ne) + 7) / 8);
+        HGC_CUDA_TRY(launch_pdl(sort_long_lists_kernel, blocks, 256, 0, stream, b.bounds, b.edges, b.place, b.long_lists, (bits_for(ne) + 7) / 8));
         HGC_LAUNCH_CHECK();
     }
     return HGC_OK;

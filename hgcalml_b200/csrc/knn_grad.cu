@@ -25,6 +25,7 @@ select_grad_kernel(const float *__restrict__ grad_dist, const int *__restrict__ 
                    const int *__restrict__ edges, float *__restrict__ grad_coord, int n_vert, int K, int C, bool vec4,
                    const int *__restrict__ order)
 {
+    pdl_begin();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (long long)n_vert * C) return;
     const int row = (int)(t / C), c = (int)(t - (long long)row * C);
@@ -145,18 +146,16 @@ extern "C" int hgc_accumulate_knn_grad_ordered(
     auto aligned16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     const bool vec4 = n_feat % 4 == 0 && aligned16(d_grad_from_out_features) && (!mm || aligned16(d_max_feat_indices));
     if (mm)
-        edge_dot_kernel<true, true><<<div_up(ne, 256), 256, 0, stream>>>(
-                d_grad_from_out_features, n_grad_from_out_feat, d_feat, d_max_feat_indices, d_neigh_indices,
-                d_out_grad_distances, ne, n_vert, n_neigh, n_feat, vec4, d_order, b.flags);
+        HGC_CUDA_TRY(launch_overlapped(n_vert, edge_dot_kernel<true, true>, div_up(ne, 256), 256, 0, stream, d_grad_from_out_features, n_grad_from_out_feat, d_feat, d_max_feat_indices, d_neigh_indices,
+                d_out_grad_distances, ne, n_vert, n_neigh, n_feat, vec4, d_order, b.flags));
     else
-        edge_dot_kernel<true, false><<<div_up(ne, 256), 256, 0, stream>>>(
-                d_grad_from_out_features, n_grad_from_out_feat, d_feat, nullptr, d_neigh_indices, d_out_grad_distances, ne,
-                n_vert, n_neigh, n_feat, vec4, d_order, nullptr);
+        HGC_CUDA_TRY(launch_overlapped(n_vert, edge_dot_kernel<true, false>, div_up(ne, 256), 256, 0, stream, d_grad_from_out_features, n_grad_from_out_feat, d_feat, nullptr, d_neigh_indices, d_out_grad_distances, ne,
+                n_vert, n_neigh, n_feat, vec4, d_order, nullptr));
     HGC_LAUNCH_CHECK();
     for (int f0 = 0; f0 < n_feat; f0 += 64) {
         if (mm && f0 > 0) {  // the bits of the first slab are a by-product of the weights' gradient
-            arg_flags_kernel<<<div_up(n_vert, 8), 256, 0, stream>>>(d_max_feat_indices, d_neigh_indices, b.flags, n_vert,
-                                                                    n_neigh, n_feat, f0);
+            HGC_CUDA_TRY(launch_overlapped(n_vert, arg_flags_kernel, div_up(n_vert, 8), 256, 0, stream, d_max_feat_indices, d_neigh_indices, b.flags, n_vert,
+                                                                    n_neigh, n_feat, f0));
             HGC_LAUNCH_CHECK();
         }
         const int rc = mm ? launch_edge_sum_slab<kSumMeanMax>(d_grad_from_out_features, n_grad_from_out_feat, d_distances,
@@ -201,9 +200,9 @@ extern "C" int hgc_select_knn_grad_ordered(
     }
     if (int rc = build_incoming(d_indices, n_vert, n_neigh, b, ws.status(), stream)) return rc;
     const long long total = (long long)n_vert * n_coords;
-    select_grad_kernel<<<div_up(total, 256), 256, 0, stream>>>(d_grad_dist, d_indices, d_coord, b.bounds, b.edges,
+    HGC_CUDA_TRY(launch_overlapped(n_vert, select_grad_kernel, div_up(total, 256), 256, 0, stream, d_grad_dist, d_indices, d_coord, b.bounds, b.edges,
                                                               d_grad_coord, n_vert, n_neigh, n_coords,
-                                                              n_neigh % 4 == 0 && ((reinterpret_cast<uintptr_t>(d_grad_dist) | reinterpret_cast<uintptr_t>(d_indices)) & 15u) == 0, d_order);
+                                                              n_neigh % 4 == 0 && ((reinterpret_cast<uintptr_t>(d_grad_dist) | reinterpret_cast<uintptr_t>(d_indices)) & 15u) == 0, d_order));
     HGC_LAUNCH_CHECK();
     return HGC_OK;
 }

@@ -13,12 +13,14 @@ namespace {
 
 __global__ void gather_kernel(const int *__restrict__ src, const int *__restrict__ perm, int *__restrict__ dst, int n)
 {
+    pdl_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) dst[i] = src[perm[i]];
 }
 
 __global__ void invert_perm_kernel(const int *__restrict__ perm, int *__restrict__ inv, int n)
 {
+    pdl_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) inv[perm[i]] = i;
 }
@@ -145,11 +147,11 @@ extern "C" int hgc_binned_select_knn_ragged(
             return rc;
         if (int rc = sort_pairs(b.subkeys, nullptr, b.k1, b.v1, b.tkeys, b.tvals, b.hist, n_vert, kSubBits, stream))
             return rc;
-        gather_kernel<<<div_up(n_vert, 256), 256, 0, stream>>>(b.keys, b.v1, b.k1, n_vert);
+        HGC_CUDA_TRY(launch_pdl(gather_kernel, div_up(n_vert, 256), 256, 0, stream, b.keys, b.v1, b.k1, n_vert));
         HGC_LAUNCH_CHECK();
         if (int rc = sort_pairs(b.k1, b.v1, b.keys, perm, b.tkeys, b.tvals, b.hist, n_vert, bits_for(p.max_bins), stream))
             return rc;
-        invert_perm_kernel<<<div_up(n_vert, 256), 256, 0, stream>>>(perm, b.rank, n_vert);
+        HGC_CUDA_TRY(launch_pdl(invert_perm_kernel, div_up(n_vert, 256), 256, 0, stream, perm, b.rank, n_vert));
         HGC_LAUNCH_CHECK();
     }
     const int *direction = use_direction ? d_direction : nullptr;

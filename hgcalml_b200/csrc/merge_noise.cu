@@ -14,6 +14,7 @@ constexpr int kThreads = kOrderThreads;
 __global__ void __launch_bounds__(kThreads)
 layout_kernel(const int *__restrict__ row_splits, int n_events, int n_vert, HitOrder o)
 {
+    pdl_begin();
     event_layout(row_splits, n_events, n_vert, o);
 }
 
@@ -21,6 +22,7 @@ __global__ void __launch_bounds__(kThreads)
 count_noise_kernel(const int *__restrict__ assignment, const int *__restrict__ association,
                    const unsigned char *__restrict__ is_cond, HitOrder o, int n_events, int2 *__restrict__ counts)
 {
+    pdl_begin();
     HitTile t;
     if (!find_tile(o, n_events, blockIdx.x, &t)) return;
     __shared__ int s_noise, s_points;
@@ -47,6 +49,7 @@ merge_noise_kernel(const int *__restrict__ assignment, const int *__restrict__ a
                    int *__restrict__ new_alpha, unsigned char *__restrict__ new_is_cond, int *__restrict__ new_n_cond,
                    int *__restrict__ n_alpha)
 {
+    pdl_begin();
     __shared__ int s_warp[kThreads / kWarp];
     __shared__ int s_sum[3];  // noise hits before the event, before the tile, up to the end of the event
     __shared__ int s_base;
@@ -182,14 +185,14 @@ extern "C" int hgc_merge_noise(
     layout(ws, n_vert, n_rs, &o, &counts, &n_alpha);
     const int n_events = n_rs - 1, tiles = (int)order_tiles_cap(n_vert, n_events);
     HGC_CUDA_TRY(cudaMemsetAsync(ws.status(), 0, kAlign, stream));
-    layout_kernel<<<1, kThreads, 0, stream>>>(d_row_splits, n_events, n_vert, o);
+    HGC_CUDA_TRY(launch_pdl(layout_kernel, 1, kThreads, 0, stream, d_row_splits, n_events, n_vert, o));
     HGC_LAUNCH_CHECK();
-    count_noise_kernel<<<tiles, kThreads, 0, stream>>>(d_assignment, d_association, d_is_cond, o, n_events, counts);
+    HGC_CUDA_TRY(launch_pdl(count_noise_kernel, tiles, kThreads, 0, stream, d_assignment, d_association, d_is_cond, o, n_events, counts));
     HGC_LAUNCH_CHECK();
-    merge_noise_kernel<<<tiles + 1, kThreads, 0, stream>>>(d_assignment, d_association, d_alpha_idx, d_is_cond,
+    HGC_CUDA_TRY(launch_pdl(merge_noise_kernel, tiles + 1, kThreads, 0, stream, d_assignment, d_association, d_alpha_idx, d_is_cond,
                                                            d_n_condensates, o, n_events, counts, d_new_assignment,
                                                            d_new_association, d_new_alpha_idx, d_new_is_cond,
-                                                           d_new_n_condensates, n_alpha);
+                                                           d_new_n_condensates, n_alpha));
     HGC_LAUNCH_CHECK();
     if (h_n_alpha) {
         HGC_CUDA_TRY(cudaMemcpyAsync(h_n_alpha, n_alpha, sizeof(int), cudaMemcpyDeviceToHost, stream));

@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(kSortThreads)
 digit_count_kernel(const int *__restrict__ keys, int n, int shift,
                    int *__restrict__ block_hist, int n_blocks)
 {
+    pdl_begin();
     __shared__ int counts[kSortWarps][kDigits];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int d = threadIdx.x; d < kSortWarps * kDigits; d += kSortThreads) (&counts[0][0])[d] = 0;
@@ -60,6 +61,7 @@ constexpr int kScanTile = 4096;
 
 __global__ void __launch_bounds__(1024) scan_tiles_kernel(int *__restrict__ data, int len, int *__restrict__ tile_sums)
 {
+    pdl_begin();
     __shared__ int warp_sums[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int base = blockIdx.x * kScanTile + threadIdx.x * 4;
@@ -99,6 +101,7 @@ __global__ void __launch_bounds__(1024) scan_tiles_kernel(int *__restrict__ data
 __global__ void __launch_bounds__(1024) add_tile_offsets_kernel(int *__restrict__ data, int len,
                                                                 const int *__restrict__ tile_sums)
 {
+    pdl_begin();
     __shared__ int warp_sums[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int sum = 0;
@@ -117,6 +120,7 @@ __global__ void __launch_bounds__(kSortThreads)
 digit_scatter_kernel(const int *__restrict__ keys_in, const int *__restrict__ vals_in,
                      int *__restrict__ keys_out, int *__restrict__ vals_out, int n, int shift, const int *__restrict__ block_offsets, int n_blocks)
 {
+    pdl_begin();
     __shared__ int counts[kSortWarps][kDigits];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int d = threadIdx.x; d < kSortWarps * kDigits; d += kSortThreads) (&counts[0][0])[d] = 0;
@@ -174,6 +178,7 @@ digit_scatter_kernel(const int *__restrict__ keys_in, const int *__restrict__ va
 __global__ void boundaries_kernel(const int *__restrict__ keys, int n, int *__restrict__ bounds,
                                   int n_bins)
 {
+    pdl_begin();
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b > n_bins) return;
     int lo = 0, hi = n;
@@ -186,6 +191,7 @@ __global__ void boundaries_kernel(const int *__restrict__ keys, int n, int *__re
 
 __global__ void fill_int_kernel(int *__restrict__ p, int n, int v)
 {
+    pdl_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) p[i] = v;
 }
@@ -204,10 +210,10 @@ int exclusive_scan_ints(int *data, int len, int *tile_sums, cudaStream_t stream)
 {
     if (len <= 0) return HGC_OK;
     const int n_tiles = div_up(len, kScanTile);
-    scan_tiles_kernel<<<n_tiles, 1024, 0, stream>>>(data, len, tile_sums);
+    HGC_CUDA_TRY(launch_pdl(scan_tiles_kernel, n_tiles, 1024, 0, stream, data, len, tile_sums));
     HGC_LAUNCH_CHECK();
     if (n_tiles > 1) {
-        add_tile_offsets_kernel<<<n_tiles, 1024, 0, stream>>>(data, len, tile_sums);
+        HGC_CUDA_TRY(launch_pdl(add_tile_offsets_kernel, n_tiles, 1024, 0, stream, data, len, tile_sums));
         HGC_LAUNCH_CHECK();
     }
     return HGC_OK;
@@ -228,12 +234,12 @@ int sort_pairs(const int *keys_in, const int *vals_in, int *keys_out, int *vals_
     const int *src_v = vals_in;
     for (int p = 0; p < passes; p++) {
         const int shift = 8 * p;
-        digit_count_kernel<<<n_blocks, kSortThreads, 0, stream>>>(src_k, n, shift, block_hist, n_blocks);
+        HGC_CUDA_TRY(launch_pdl(digit_count_kernel, n_blocks, kSortThreads, 0, stream, src_k, n, shift, block_hist, n_blocks));
         HGC_LAUNCH_CHECK();
         const int table = kDigits * n_blocks;
         if (int rc = exclusive_scan_ints(block_hist, table, block_hist + table, stream)) return rc;
-        digit_scatter_kernel<<<n_blocks, kSortThreads, 0, stream>>>(src_k, src_v, kbuf[dst], vbuf[dst], n, shift,
-                                                                    block_hist, n_blocks);
+        HGC_CUDA_TRY(launch_pdl(digit_scatter_kernel, n_blocks, kSortThreads, 0, stream, src_k, src_v, kbuf[dst], vbuf[dst], n, shift,
+                                                                    block_hist, n_blocks));
         HGC_LAUNCH_CHECK();
         src_k = kbuf[dst];
         src_v = vbuf[dst];
@@ -246,9 +252,9 @@ int boundaries_from_sorted_keys(const int *sorted_keys, int n, int *bin_boundari
                                 cudaStream_t stream)
 {
     if (n <= 0) {
-        fill_int_kernel<<<div_up(n_bins + 1, 256), 256, 0, stream>>>(bin_boundaries, n_bins + 1, 0);
+        HGC_CUDA_TRY(launch_pdl(fill_int_kernel, div_up(n_bins + 1, 256), 256, 0, stream, bin_boundaries, n_bins + 1, 0));
     } else {
-        boundaries_kernel<<<div_up(n_bins + 1, 256), 256, 0, stream>>>(sorted_keys, n, bin_boundaries, n_bins);
+        HGC_CUDA_TRY(launch_pdl(boundaries_kernel, div_up(n_bins + 1, 256), 256, 0, stream, sorted_keys, n, bin_boundaries, n_bins));
     }
     HGC_LAUNCH_CHECK();
     return HGC_OK;

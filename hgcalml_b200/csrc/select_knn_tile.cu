@@ -30,6 +30,7 @@ pack_tiles_kernel(const float *__restrict__ coords, int C, const int *__restrict
                   const int *__restrict__ rank_of,
                   const int *__restrict__ direction, int n_events, HitOrder o, TileScratch s, int nv4, int nobody)
 {
+    pdl_begin();
     extern __shared__ float s_c[];  // [min(C, kSplitDims)][1024] coordinates in curve order
     __shared__ float s_lo[32][16], s_hi[32][16];
     __shared__ unsigned s_x[kPackThreads];
@@ -154,9 +155,8 @@ int build_tiles(const float *coords, int n_coords, const int *curve_perm, const 
 {
     if (n_vert <= 0) return HGC_OK;
     const size_t smem = sizeof(float) * kPackThreads * (n_coords < kSplitDims ? n_coords : kSplitDims);
-    pack_tiles_kernel<<<(int)tile_supers_cap(n_vert, n_events), kPackThreads, smem, stream>>>(
-            coords, n_coords, curve_perm, rank_of, direction, n_events, o, s, (n_coords + 3) / 4,
-            (int)(tile_chunks_cap(n_vert, n_events) * 32));
+    HGC_CUDA_TRY(launch_pdl(pack_tiles_kernel, (int)tile_supers_cap(n_vert, n_events), kPackThreads, smem, stream, coords, n_coords, curve_perm, rank_of, direction, n_events, o, s, (n_coords + 3) / 4,
+            (int)(tile_chunks_cap(n_vert, n_events) * 32)));
     HGC_LAUNCH_CHECK();
     return HGC_OK;
 }

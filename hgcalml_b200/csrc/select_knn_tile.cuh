@@ -312,6 +312,7 @@ template <int NV4, int L>
 __global__ void __launch_bounds__(kTileThreads, L <= 2 && NV4 == 1 ? HGC_TILE_MIN_BLOCKS : (L <= 4 ? 6 : 3))
 select_knn_tile_kernel(const TileKnnArgs a)
 {
+    pdl_begin();
     using S = TileShape<L>;
     __shared__ knn_key s_buf[kTileWarps][S::kCap];
     __shared__ unsigned s_list[kTileListCap];  // chunk id << 5 | distance class
@@ -630,7 +631,7 @@ select_knn_tile_kernel(const TileKnnArgs a)
 template <int NV4, int L>
 int launch_tile_l(const TileKnnArgs &a, int n_tiles, cudaStream_t stream)
 {
-    select_knn_tile_kernel<NV4, L><<<n_tiles, kTileThreads, 0, stream>>>(a);
+    HGC_CUDA_TRY(launch_overlapped(a.nobody, select_knn_tile_kernel<NV4, L>, n_tiles, kTileThreads, 0, stream, a));
     HGC_LAUNCH_CHECK();
     return HGC_OK;
 }

@@ -12,6 +12,7 @@ namespace {
 __global__ void local_distance_kernel(const int *__restrict__ nidx, const float *__restrict__ coords,
                                       float *__restrict__ dist, int C, int n_in, long long n_edges, int K)
 {
+    pdl_begin();
     const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n_edges) return;
     const int i = (int)(e / K);
@@ -35,6 +36,7 @@ push_grad_features_kernel(const float *__restrict__ grad, const float *__restric
                           const int *__restrict__ nidx, float *__restrict__ feat_grad, int n_vert, int K, int F,
                           const int *__restrict__ order)
 {
+    pdl_begin();
     constexpr int U = 8;
     const int lane = threadIdx.x & 31;
     const int slot = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -94,14 +96,14 @@ extern "C" int hgc_push_knn_grad_ordered(
     if (n_feat > 0 && (!d_grad || !d_feat || !d_feat_grad)) return HGC_ERR_INVALID_ARGUMENT;
     if (ne > 0 && (!d_weights || !d_idxs || !d_w_grad)) return HGC_ERR_INVALID_ARGUMENT;
     if (n_feat > 0) {
-        push_grad_features_kernel<<<div_up(n_vert, 8), 256, 0, stream>>>(d_grad, d_weights, d_idxs, d_feat_grad,
-                                                                        n_vert, n_neigh, n_feat, d_order);
+        HGC_CUDA_TRY(launch_overlapped(n_vert, push_grad_features_kernel, div_up(n_vert, 8), 256, 0, stream, d_grad, d_weights, d_idxs, d_feat_grad,
+                                                                        n_vert, n_neigh, n_feat, d_order));
         HGC_LAUNCH_CHECK();
     }
     if (ne > 0) {
         const bool vec4 = n_feat % 4 == 0 && (reinterpret_cast<uintptr_t>(d_feat) & 15u) == 0;
-        edge_dot_kernel<false, false><<<div_up(ne, 256), 256, 0, stream>>>(d_feat, n_feat, d_grad, nullptr, d_idxs, d_w_grad,
-                                                                          ne, n_vert, n_neigh, n_feat, vec4, d_order, nullptr);
+        HGC_CUDA_TRY(launch_overlapped(n_vert, edge_dot_kernel<false, false>, div_up(ne, 256), 256, 0, stream, d_feat, n_feat, d_grad, nullptr, d_idxs, d_w_grad,
+                                                                          ne, n_vert, n_neigh, n_feat, vec4, d_order, nullptr));
         HGC_LAUNCH_CHECK();
     }
     return HGC_OK;
@@ -117,8 +119,8 @@ extern "C" int hgc_local_distance(
     const long long ne = (long long)n_out_vert * n_neigh;
     if (ne == 0) return HGC_OK;
     if (!d_neigh_idxs || !d_distances || (n_coords > 0 && !d_coords)) return HGC_ERR_INVALID_ARGUMENT;
-    local_distance_kernel<<<div_up(ne, 256), 256, 0, stream>>>(d_neigh_idxs, d_coords, d_distances, n_coords,
-                                                              n_in_vert, ne, n_neigh);
+    HGC_CUDA_TRY(launch_pdl(local_distance_kernel, div_up(ne, 256), 256, 0, stream, d_neigh_idxs, d_coords, d_distances, n_coords,
+                                                              n_in_vert, ne, n_neigh));
     HGC_LAUNCH_CHECK();
     return HGC_OK;
 }
