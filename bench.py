@@ -37,7 +37,7 @@ UNIT = "hits/s"
 NCU = {
     "accumulate_knn": {"dram_bytes_per_hit": 1782, "algorithmic_bytes_per_hit": 1536},
     "accumulate_knn_no_argmax": {"dram_bytes_per_hit": 1314, "algorithmic_bytes_per_hit": 1280},
-    "select_knn": {"dram_bytes_per_hit": 437, "issue_active_pct": 73.6, "warp_instructions_per_query": 2368},
+    "select_knn": {"dram_bytes_per_hit": 433, "issue_active_pct": 90.4, "warp_instructions_per_query": 5715},
 }
 
 
