@@ -75,6 +75,15 @@ def collect_neighbours(features, neighbour_indices, distancesq, *, first_slot: i
     return view, maxidx
 
 
+def _copy_columns(x, out, column: int):
+    """``out[:, column:column + x.shape[1]] = x`` for a row-major buffer."""
+    if x.requires_grad:
+        out[:, column:] = x
+        return
+    C.check(C.lib.hgc_copy_columns(C.ptr(x), out.data_ptr() + 4 * column, out.stride(0), x.shape[0], x.shape[1],
+                                   C.stream_of(x)), "copy_columns")
+
+
 class _Dense(torch.nn.Module):
     """``tf.keras.layers.Dense``: ``activation(x @ kernel + bias)`` with the kernel stored [in, out]."""
 
@@ -84,10 +93,17 @@ class _Dense(torch.nn.Module):
         torch.nn.init.xavier_uniform_(self.kernel)  # Keras' default glorot_uniform
         self.bias = torch.nn.Parameter(torch.zeros(n_out)) if use_bias else None
         self.activation = _activation(activation)
+        # bias and activation in one pass where no gradient is recorded
+        self.fused_relu = {None: 0, "linear": 0, "relu": 1}.get(activation) if not callable(activation) else None
 
     def forward(self, x):
         y = x @ self.kernel
         if self.bias is not None:
+            if self.fused_relu is not None and y.is_cuda and not y.requires_grad and y.dtype == torch.float32 and \
+                    y.dim() == 2 and y.is_contiguous() and self.bias.dtype == torch.float32:
+                C.check(C.lib.hgc_bias_act(C.ptr(y), C.ptr(self.bias), y.shape[0], y.shape[1], self.fused_relu,
+                                           C.stream_of(y)), "dense layer")
+                return y
             y = y + self.bias
         return self.activation(y)
 
@@ -133,7 +149,7 @@ class RaggedGravNet(torch.nn.Module):
         cat = torch.empty((n, 2 * p + f_in), dtype=torch.float32, device=x.device)
         collect_neighbours(features, idx, dist, first_slot=1, n_neighbours=self.n_neighbours,
                            subtract_self=True, out=cat, out_column=0, order=sorting)
-        cat[:, 2 * p:] = x
+        _copy_columns(x, cat, 2 * p)
         outfeats = self.output_feature_transform(cat)
         if self.return_self:
             return outfeats, coordinates, idx, dist
@@ -168,5 +184,5 @@ class DistanceWeightedMessagePassing(torch.nn.Module):
             features, _ = collect_neighbours(prev_feat, neighbor_indices, distancesq, subtract_self=True,
                                              out=cat, out_column=col, order=order)
             col += 2 * f
-        cat[:, total:] = x
+        _copy_columns(x, cat, total)
         return cat

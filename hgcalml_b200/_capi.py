@@ -47,6 +47,8 @@ def _load():
         "hgc_accumulate_knn_ordered": (I, [P] * 5 + [I] * 6 + [P, P]),
         "hgc_accumulate_knn_exp": (I, [P] * 5 + [I] * 5 + [ctypes.c_float, P, P]),
         "hgc_gravnet_collect": (I, [P, P, I, I, I, P, P, I, P, I, I, ctypes.c_float, I, P, P]),
+        "hgc_bias_act": (I, [P, P, I, I, I, P]),
+        "hgc_copy_columns": (I, [P, P, I, I, I, P]),
         "hgc_binned_select_knn_ragged_workspace_bytes": (S, [I] * 6),
         "hgc_binned_select_knn_ragged": (I, [P] * 6 + [I] * 8 + [P, S, P]),
         "hgc_build_and_assign_condensates_workspace_bytes": (S, [I] * 4),

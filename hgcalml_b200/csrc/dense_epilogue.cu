@@ -1,0 +1,84 @@
+// What follows the library GEMM of a dense layer, and the concatenation buffer of the GravNet layers.
+#include "common.cuh"
+
+namespace hgc {
+namespace {
+
+// y = max(y + bias, 0) (RELU) or y + bias in place, V floats per thread: one pass over the rows instead of one for the bias
+// and one for the activation (200k x 64: 45 -> 16 us).
+template <int V, bool RELU>
+__global__ void __launch_bounds__(256)
+bias_act_kernel(float *__restrict__ y, const float *__restrict__ bias, long long n_vec, int f_vec)
+{
+    pdl_begin();
+    const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (t >= n_vec) return;
+    const int c = (int)(t % f_vec) * V;
+    float v[V];
+    if constexpr (V == 4) {
+        const float4 q = reinterpret_cast<const float4 *>(y)[t];
+        v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+    } else {
+        v[0] = y[t];
+    }
+#pragma unroll
+    for (int k = 0; k < V; k++) {
+        v[k] = __fadd_rn(v[k], __ldg(bias + c + k));
+        if (RELU) v[k] = v[k] < 0.f ? 0.f : v[k];  // NaN stays NaN
+    }
+    if constexpr (V == 4) reinterpret_cast<float4 *>(y)[t] = make_float4(v[0], v[1], v[2], v[3]);
+    else y[t] = v[0];
+}
+
+// Copies [n, f] rows into columns of a wider row-major buffer (200k x 64 floats: 37 -> 16 us against an elementwise copy).
+template <int V>
+__global__ void __launch_bounds__(256)
+copy_columns_kernel(const float *__restrict__ src, float *__restrict__ dst, int ld_dst, long long n_vec, int f_vec)
+{
+    pdl_begin();
+    const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (t >= n_vec) return;
+    const long long row = t / f_vec;
+    const int c = (int)(t - row * f_vec) * V;
+    if constexpr (V == 4) *reinterpret_cast<float4 *>(dst + row * ld_dst + c) = __ldg(reinterpret_cast<const float4 *>(src) + t);
+    else dst[row * ld_dst + c] = __ldg(src + t);
+}
+
+inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+}  // namespace
+}  // namespace hgc
+
+using namespace hgc;
+
+extern "C" int hgc_bias_act(float *d_y, const float *d_bias, int n, int n_feat, int relu, hgc_stream_t stream_)
+{
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    if (n < 0 || n_feat < 0) return HGC_ERR_INVALID_ARGUMENT;
+    if (n == 0 || n_feat == 0) return HGC_OK;
+    if (!d_y || !d_bias) return HGC_ERR_INVALID_ARGUMENT;
+    const bool vec = n_feat % 4 == 0 && aligned16(d_y);
+    const long long total = (long long)n * n_feat / (vec ? 4 : 1);
+    const int f_vec = n_feat / (vec ? 4 : 1), blocks = div_up(total, 256);
+    if (vec && relu) HGC_CUDA_TRY(launch_pdl(bias_act_kernel<4, true>, blocks, 256, 0, stream, d_y, d_bias, total, f_vec));
+    else if (vec) HGC_CUDA_TRY(launch_pdl(bias_act_kernel<4, false>, blocks, 256, 0, stream, d_y, d_bias, total, f_vec));
+    else if (relu) HGC_CUDA_TRY(launch_pdl(bias_act_kernel<1, true>, blocks, 256, 0, stream, d_y, d_bias, total, f_vec));
+    else HGC_CUDA_TRY(launch_pdl(bias_act_kernel<1, false>, blocks, 256, 0, stream, d_y, d_bias, total, f_vec));
+    HGC_LAUNCH_CHECK();
+    return HGC_OK;
+}
+
+extern "C" int hgc_copy_columns(const float *d_src, float *d_dst, int ld_dst, int n, int n_feat, hgc_stream_t stream_)
+{
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    if (n < 0 || n_feat < 0 || ld_dst < n_feat) return HGC_ERR_INVALID_ARGUMENT;
+    if (n == 0 || n_feat == 0) return HGC_OK;
+    if (!d_src || !d_dst) return HGC_ERR_INVALID_ARGUMENT;
+    const bool vec = n_feat % 4 == 0 && ld_dst % 4 == 0 && aligned16(d_src) && aligned16(d_dst);
+    const long long total = (long long)n * n_feat / (vec ? 4 : 1);
+    const int f_vec = n_feat / (vec ? 4 : 1), blocks = div_up(total, 256);
+    if (vec) HGC_CUDA_TRY(launch_pdl(copy_columns_kernel<4>, blocks, 256, 0, stream, d_src, d_dst, ld_dst, total, f_vec));
+    else HGC_CUDA_TRY(launch_pdl(copy_columns_kernel<1>, blocks, 256, 0, stream, d_src, d_dst, ld_dst, total, f_vec));
+    HGC_LAUNCH_CHECK();
+    return HGC_OK;
+}

@@ -212,6 +212,12 @@ int hgc_gravnet_collect(
         int n_vert, int n_feat, float distance_scale, int subtract_self, const int *d_order,
         hgc_stream_t stream);
 
+/* Around the dense layers of the GravNet layers: y[n, n_feat] += bias in place, then max(y, 0) when relu is set;
+ * and d_src[n, n_feat] copied into columns of a row-major buffer with row stride ld_dst floats (d_dst points at the
+ * first of them). */
+int hgc_bias_act(float *d_y, const float *d_bias, int n, int n_feat, int relu, hgc_stream_t stream);
+int hgc_copy_columns(const float *d_src, float *d_dst, int ld_dst, int n, int n_feat, hgc_stream_t stream);
+
 /* ---------------------------------------------------------------------------------------
  * BinnedSelectKnn, wrapper level -- replaces the whole Python function BinnedSelectKnn
  * (modules/binned_select_knn_op.py:32-95: BinByCoordinates + argsort + gathers + the op +

@@ -130,3 +130,19 @@ def test_distance_weighted_message_passing_vs_checker(cuda, oracle):
     assert (np.abs(got[:, :32] - ref[:, :32]) <= tol0).all()
     scale = np.abs(ref[:, 32:80]).mean()
     assert np.abs(got[:, 32:80] - ref[:, 32:80]).max() <= 1e-4 * max(scale, 1.)
+
+
+@pytest.mark.parametrize("n,f,shift", [(1, 1, 0), (300, 64, 0), (257, 7, 0), (1000, 64, 1)])
+def test_dense_epilogue_and_column_copy(cuda, n, f, shift):
+    from hgcalml_b200 import _capi as C
+    from hgcalml_b200.GravNetLayersRagged import _copy_columns
+    y, b = torch.randn((n, f), device=cuda), torch.randn((f,), device=cuda)
+    y[0, 0] = float("nan")
+    for relu in (0, 1):
+        got = y.clone()
+        C.check(C.lib.hgc_bias_act(C.ptr(got), C.ptr(b), n, f, relu, C.stream_of(got)), "bias_act")
+        want = torch.relu(y + b) if relu else y + b
+        assert torch.equal(got.nan_to_num(9.), want.nan_to_num(9.))
+    buf = torch.full((n, 2 * f + 4 + shift), 3., device=cuda)
+    _copy_columns(y, buf, f + 4 + shift)
+    assert torch.equal(buf[:, f + 4 + shift:].nan_to_num(9.), y.nan_to_num(9.)) and (buf[:, :f + 4 + shift] == 3.).all()
