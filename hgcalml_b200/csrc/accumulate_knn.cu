@@ -343,9 +343,9 @@ int launch_vec(bool exp_w, bool with_arg, const float *w, const float *feat, con
 {
     constexpr int G = THREADS / LPH;
     const int n_steps = div_up(n_vert, G);
-    // tiles of fewer steps where there would be less than two blocks per SM: 700 hits at F = 32 16 -> 3.5 us
+    // tiles of fewer steps where blocks would not fill the SMs once: 700 hits at F = 32 16 -> 3.5 us
     int tile_steps = kAccTileSteps;
-    while (tile_steps > 1 && div_up(n_steps, tile_steps) < 2 * sm_count()) tile_steps >>= 1;
+    while (tile_steps > 1 && div_up(n_steps, tile_steps) < MINB * sm_count()) tile_steps >>= 1;
     const long long n_tiles = div_up(n_steps, tile_steps);
     // one block per tile up to 32 blocks per SM (blocks beyond that walk several tiles): measured faster on
     // the 64-event batch than a grid of resident blocks only, which keeps the SMs less evenly loaded

@@ -51,9 +51,9 @@ int sm_count();
 // and wait in pdl_begin(), which takes about a microsecond off every step from one kernel to the next.  Every kernel
 // launched this way begins with pdl_begin(), in all of its blocks, so that "the kernel before has completed" holds
 // through any chain of them.  700 hits: 75 -> 56 us a call, 20k 131 -> 105 us.
-// launch_overlapped is for the kernels that live on L1 (search, gathers): above kOverlapHits they are launched in the
-// ordinary way, because blocks that become resident beside those of another kernel inherit its split between L1 and shared
-// memory (+2 to 3 % on calls of 100k hits and more).
+// launch_overlapped does so up to kOverlapHits hits: blocks that become resident early take room from the kernel that is
+// still running and inherit its split between L1 and shared memory, which costs more than it gains where kernels are
+// long (400k hits: sort passes overlapped 1824 us a call, not overlapped 1788 us).
 template <typename... Params, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args &&...args)
 {

@@ -219,7 +219,7 @@ order_pass_kernel(HitOrder o, int n_events, int tiles_cap, int pass, int *__rest
 int range_and_layout(const float *coords, int n_coords, int n_bin_dims, const int *row_splits, int n_rs, int n_bins,
                      int n_neigh, int n_vert, const HitOrder &o, unsigned *status, cudaStream_t stream)
 {
-    HGC_CUDA_TRY(launch_pdl(range_and_layout_kernel, range_partial_blocks(n_vert), kThreads, 0, stream, coords, n_coords, n_bin_dims, n_coords < kMaxBinDims ? n_coords : kMaxBinDims, n_vert, row_splits, n_rs, n_bins,
+    HGC_CUDA_TRY(launch_overlapped(n_vert, range_and_layout_kernel, range_partial_blocks(n_vert), kThreads, 0, stream, coords, n_coords, n_bin_dims, n_coords < kMaxBinDims ? n_coords : kMaxBinDims, n_vert, row_splits, n_rs, n_bins,
             n_neigh, o, status + 8));
     HGC_LAUNCH_CHECK();
     return HGC_OK;
@@ -237,7 +237,7 @@ int order_hits(const float *coords, int n_coords, int n_bin_dims, const int *row
         return rc;
     const int tiles = (int)order_tiles_cap(n_vert, n_events);
 #define HGC_KEYS(D, B)                                                                                            \
-    case D: HGC_CUDA_TRY(launch_pdl(order_keys_kernel<D, B>, tiles, kThreads, 0, stream, coords, n_coords, n_bin_dims, o, n_events, tiles, status)); break
+    case D: HGC_CUDA_TRY(launch_overlapped(n_vert, order_keys_kernel<D, B>, tiles, kThreads, 0, stream, coords, n_coords, n_bin_dims, o, n_events, tiles, status)); break
     switch (n_all) {
         HGC_KEYS(2, 16);
         HGC_KEYS(3, 10);
@@ -255,11 +255,11 @@ int order_hits(const float *coords, int n_coords, int n_bin_dims, const int *row
 #define HGC_PASS(R)                                                                                                  \
     case R * kThreads:                                                                                               \
         if (p == 0)                                                                                                  \
-            HGC_CUDA_TRY(launch_pdl(order_pass_kernel<R, true, false>, grid, kThreads, 0, stream, o, n_events, tiles, p, bin_perm, rank, curve_perm)); \
+            HGC_CUDA_TRY(launch_overlapped(n_vert, order_pass_kernel<R, true, false>, grid, kThreads, 0, stream, o, n_events, tiles, p, bin_perm, rank, curve_perm)); \
         else if (p + 1 < kOrderPasses)                                                                               \
-            HGC_CUDA_TRY(launch_pdl(order_pass_kernel<R, false, false>, grid, kThreads, 0, stream, o, n_events, tiles, p, bin_perm, rank, curve_perm)); \
+            HGC_CUDA_TRY(launch_overlapped(n_vert, order_pass_kernel<R, false, false>, grid, kThreads, 0, stream, o, n_events, tiles, p, bin_perm, rank, curve_perm)); \
         else                                                                                                         \
-            HGC_CUDA_TRY(launch_pdl(order_pass_kernel<R, false, true>, grid, kThreads, 0, stream, o, n_events, tiles, p, bin_perm, rank, curve_perm)); \
+            HGC_CUDA_TRY(launch_overlapped(n_vert, order_pass_kernel<R, false, true>, grid, kThreads, 0, stream, o, n_events, tiles, p, bin_perm, rank, curve_perm)); \
         break
         switch (o.tile) {
             HGC_PASS(2);

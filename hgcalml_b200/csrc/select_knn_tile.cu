@@ -155,7 +155,7 @@ int build_tiles(const float *coords, int n_coords, const int *curve_perm, const 
 {
     if (n_vert <= 0) return HGC_OK;
     const size_t smem = sizeof(float) * kPackThreads * (n_coords < kSplitDims ? n_coords : kSplitDims);
-    HGC_CUDA_TRY(launch_pdl(pack_tiles_kernel, (int)tile_supers_cap(n_vert, n_events), kPackThreads, smem, stream, coords, n_coords, curve_perm, rank_of, direction, n_events, o, s, (n_coords + 3) / 4,
+    HGC_CUDA_TRY(launch_overlapped(n_vert, pack_tiles_kernel, (int)tile_supers_cap(n_vert, n_events), kPackThreads, smem, stream, coords, n_coords, curve_perm, rank_of, direction, n_events, o, s, (n_coords + 3) / 4,
             (int)(tile_chunks_cap(n_vert, n_events) * 32)));
     HGC_LAUNCH_CHECK();
     return HGC_OK;
