@@ -65,6 +65,7 @@ def _load():
         "hgc_accumulate_knn_grad_ordered": (I, [P] * 7 + [I] * 6 + [P, P, S, P]),
         "hgc_select_knn_grad": (I, [P] * 5 + [I] * 3 + [P, S, P]),
         "hgc_select_knn_grad_ordered": (I, [P] * 5 + [I] * 3 + [P, P, S, P]),
+        "hgc_select_knn_grad_after": (I, [P] * 5 + [I] * 3 + [P, P, S, P]),
         "hgc_binned_assign_to_condensates_workspace_bytes": (S, [I] * 4),
         "hgc_binned_assign_to_condensates": (I, [I, I] + [P] * 4 + [P] + [P] * 2 + [P] * 4 + [P] * 4 + [P] * 3
                                              + [P, I, I, I, I] + [P, S, P]),
@@ -151,6 +152,34 @@ def order_of(idx, n: int):
     if order is None or order.shape[0] != n or idx.shape[0] != n or order.device != idx.device:
         return None
     return order
+
+
+class BackwardLists:
+    """Hands the transposed neighbour table from one backward op to a later one of the same backward pass.
+    One such object belongs to one differentiable search call; the autograd engine empties it when the pass ends."""
+    __slots__ = ("ws", "key")
+
+    def __init__(self):
+        self.ws = self.key = None
+
+    def clear(self):
+        self.ws = self.key = None
+
+    @staticmethod
+    def _key(idx):
+        return idx.data_ptr(), idx._version, idx.shape, stream_of(idx)
+
+    def put(self, idx, ws):
+        try:
+            torch.autograd.Variable._execution_engine.queue_callback(self.clear)
+        except RuntimeError:
+            return  # not inside a backward pass
+        self.ws, self.key = ws, self._key(idx)
+
+    def take(self, idx):
+        ws = self.ws if self.key == self._key(idx) else None
+        self.clear()
+        return ws
 
 
 def require_cuda(*tensors):

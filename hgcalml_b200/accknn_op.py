@@ -68,7 +68,8 @@ def AccumulateKnn(distances, features, indices, mean_and_max=True, force_tf=Fals
     return out, maxidx
 
 
-def AccumulateKnnGrad(grad_from_out_features, distances, features, neigh_indices, max_feat_indices, order=None):
+def AccumulateKnnGrad(grad_from_out_features, distances, features, neigh_indices, max_feat_indices, order=None,
+                      _lists=None):
     """The registered op ``AccumulateKnnGrad`` (modules/compiled/accumulate_knn_grad_module.cc:7-15), the
     gradient the reference attaches to the op ``AccumulateKnn`` (modules/accknn_op.py:71-90).
     ``distances`` are the forward op's weights.  ``order`` (optional int32 permutation of the hits, e.g.
@@ -95,6 +96,8 @@ def AccumulateKnnGrad(grad_from_out_features, distances, features, neigh_indices
                                                   C.ptr(gw), C.ptr(gf), n, k, f, g.shape[1], 0, int(mean_and_max),
                                                   C.ptr(order), C.ptr(ws), ws.numel(), C.stream_of(feat)),
             "AccumulateKnnGrad")
+    if _lists is not None and n > 0 and k > 0:
+        _lists.put(idx, ws)
     return gw, gf
 
 
@@ -107,6 +110,7 @@ class _AccumulateLinKnnFunction(torch.autograd.Function):
         out, maxidx = AccumulateLinKnn(weights, features, indices, mean_and_max=mean_and_max, order=order)
         ctx.save_for_backward(weights, features, indices, maxidx)
         ctx.order = order
+        ctx.lists = getattr(indices, "_hgc_lists", None)
         ctx.mark_non_differentiable(maxidx)
         ctx.set_materialize_grads(False)  # no zeros for the arg-max output
         return out, maxidx
@@ -116,7 +120,8 @@ class _AccumulateLinKnnFunction(torch.autograd.Function):
         if grad_out is None:
             return None, None, None, None, None
         weights, features, indices, maxidx = ctx.saved_tensors
-        gw, gf = AccumulateKnnGrad(grad_out, weights, features, indices, maxidx, order=ctx.order)
+        gw, gf = AccumulateKnnGrad(grad_out, weights, features, indices, maxidx, order=ctx.order,
+                                   _lists=ctx.lists)
         return gw, gf, None, None, None
 
 

@@ -84,7 +84,7 @@ def BinnedSelectKnn(K: int, coords, row_splits, direction=None, n_bins=None, max
     return idx, dist
 
 
-def SelectKnnGrad(grad_distances, indices, distances, coordinates, order=None):
+def SelectKnnGrad(grad_distances, indices, distances, coordinates, order=None, _lists=None):
     """The registered op ``SelectKnnGrad`` (modules/compiled/select_knn_grad_module.cc), which the
     reference attaches as the gradient of ``BinnedSelectKnn`` (modules/binned_select_knn_op.py:107-118):
     gradient of the squared neighbour distances with respect to the coordinates, ``[N, C]``.
@@ -94,11 +94,13 @@ def SelectKnnGrad(grad_distances, indices, distances, coordinates, order=None):
     d = None if distances is None else C.f32(distances)
     n, k = idx.shape
     out = torch.empty_like(coords)
-    ws = C.workspace(C.lib.hgc_knn_grad_workspace_bytes(n, k), coords.device)
+    ws = _lists.take(idx) if _lists is not None else None
+    run = C.lib.hgc_select_knn_grad_ordered if ws is None else C.lib.hgc_select_knn_grad_after
+    if ws is None:
+        ws = C.workspace(C.lib.hgc_knn_grad_workspace_bytes(n, k), coords.device)
     order = C.order_of(indices, n) if order is None else C.i32(order)
-    C.check(C.lib.hgc_select_knn_grad_ordered(C.ptr(g), C.ptr(idx), C.ptr(d), C.ptr(coords), C.ptr(out),
-                                              n, k, coords.shape[1], C.ptr(order), C.ptr(ws), ws.numel(),
-                                              C.stream_of(coords)), "SelectKnnGrad")
+    C.check(run(C.ptr(g), C.ptr(idx), C.ptr(d), C.ptr(coords), C.ptr(out), n, k, coords.shape[1], C.ptr(order),
+                C.ptr(ws), ws.numel(), C.stream_of(coords)), "SelectKnnGrad")
     return out
 
 
@@ -109,6 +111,7 @@ class _BinnedSelectKnnFunction(torch.autograd.Function):
                                     tf_compatible=tf_compatible)
         ctx.save_for_backward(coords, idx, dist)
         ctx.order = C.order_of(idx, idx.shape[0])
+        ctx.lists = idx._hgc_lists = C.BackwardLists()
         ctx.mark_non_differentiable(idx)
         ctx.set_materialize_grads(False)  # no zeros for the index output
         return idx, dist
@@ -118,7 +121,8 @@ class _BinnedSelectKnnFunction(torch.autograd.Function):
         if grad_dist is None:
             return None, None, None, None, None, None
         coords, idx, dist = ctx.saved_tensors
-        return SelectKnnGrad(grad_dist, idx, dist, coords, order=ctx.order), None, None, None, None, None
+        return SelectKnnGrad(grad_dist, idx, dist, coords, order=ctx.order,
+                             _lists=ctx.lists), None, None, None, None, None
 
 
 def BinnedSelectKnnDifferentiable(K, coords, row_splits, n_bins=None, max_bin_dims=3, tf_compatible=False):

@@ -178,12 +178,11 @@ extern "C" int hgc_select_knn_grad(
                                        nullptr, workspace, workspace_bytes, stream);
 }
 
-extern "C" int hgc_select_knn_grad_ordered(
-        const float *d_grad_dist, const int *d_indices, const float *d_dist, const float *d_coord,
-        float *d_grad_coord, int n_vert, int n_neigh, int n_coords, const int *d_order,
-        void *workspace, size_t workspace_bytes, hgc_stream_t stream_)
+// lists_ready: the workspace holds the transposed lists of this neighbour table already.
+static int select_knn_grad(const float *d_grad_dist, const int *d_indices, const float *d_coord, float *d_grad_coord,
+                           int n_vert, int n_neigh, int n_coords, const int *d_order, void *workspace,
+                           size_t workspace_bytes, bool lists_ready, hgc_stream_t stream_)
 {
-    (void)d_dist;  // an input of the op that its kernels never read
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     if (int rc = check_edge_count(n_vert, n_neigh)) return rc;
     if (n_coords < 0) return HGC_ERR_INVALID_ARGUMENT;
@@ -198,11 +197,32 @@ extern "C" int hgc_select_knn_grad_ordered(
         HGC_CUDA_TRY(cudaMemsetAsync(d_grad_coord, 0, sizeof(float) * (size_t)n_vert * n_coords, stream));
         return HGC_OK;
     }
-    if (int rc = build_incoming(d_indices, n_vert, n_neigh, b, ws.status(), stream)) return rc;
+    if (!lists_ready)
+        if (int rc = build_incoming(d_indices, n_vert, n_neigh, b, ws.status(), stream)) return rc;
     const long long total = (long long)n_vert * n_coords;
     HGC_CUDA_TRY(launch_overlapped(n_vert, select_grad_kernel, div_up(total, 256), 256, 0, stream, d_grad_dist, d_indices, d_coord, b.bounds, b.edges,
                                                               d_grad_coord, n_vert, n_neigh, n_coords,
                                                               n_neigh % 4 == 0 && ((reinterpret_cast<uintptr_t>(d_grad_dist) | reinterpret_cast<uintptr_t>(d_indices)) & 15u) == 0, d_order));
     HGC_LAUNCH_CHECK();
     return HGC_OK;
+}
+
+extern "C" int hgc_select_knn_grad_ordered(
+        const float *d_grad_dist, const int *d_indices, const float *d_dist, const float *d_coord,
+        float *d_grad_coord, int n_vert, int n_neigh, int n_coords, const int *d_order,
+        void *workspace, size_t workspace_bytes, hgc_stream_t stream)
+{
+    (void)d_dist;  // an input of the op that its kernels never read
+    return select_knn_grad(d_grad_dist, d_indices, d_coord, d_grad_coord, n_vert, n_neigh, n_coords, d_order, workspace,
+                           workspace_bytes, false, stream);
+}
+
+extern "C" int hgc_select_knn_grad_after(
+        const float *d_grad_dist, const int *d_indices, const float *d_dist, const float *d_coord,
+        float *d_grad_coord, int n_vert, int n_neigh, int n_coords, const int *d_order,
+        void *workspace, size_t workspace_bytes, hgc_stream_t stream)
+{
+    (void)d_dist;
+    return select_knn_grad(d_grad_dist, d_indices, d_coord, d_grad_coord, n_vert, n_neigh, n_coords, d_order, workspace,
+                           workspace_bytes, true, stream);
 }

@@ -352,6 +352,14 @@ int hgc_select_knn_grad_ordered(
         float *d_grad_coord, int n_vert, int n_neigh, int n_coords, const int *d_order,
         void *workspace, size_t workspace_bytes, hgc_stream_t stream);
 
+/* The same, later in a backward pass: `workspace` is the one that an hgc_accumulate_knn_grad(_ordered) call with the
+ * same d_indices, n_vert and n_neigh has left behind, unchanged since; the neighbour table, which both ops
+ * transpose, is not transposed a second time. */
+int hgc_select_knn_grad_after(
+        const float *d_grad_dist, const int *d_indices, const float *d_dist, const float *d_coord,
+        float *d_grad_coord, int n_vert, int n_neigh, int n_coords, const int *d_order,
+        void *workspace, size_t workspace_bytes, hgc_stream_t stream);
+
 /* ---------------------------------------------------------------------------------------
  * Sibling ops on the same neighbour tables (used by the graph-condensation layers).
  *

@@ -75,3 +75,26 @@ def test_search_notes_its_order(cuda):
     assert _capi.order_of(idx[:2000], 2000) is None and _capi.order_of(idx, 2999) is None
     idx, _ = BinnedSelectKnnDifferentiable(8, c.requires_grad_(True), rs)
     assert torch.equal(_capi.order_of(idx, 3000), sorting)
+
+
+def test_backward_ops_share_lists_within_a_pass_only(cuda):
+    """Gradients through both ops equal those of the ops called alone, pass after pass, also when the table changes
+    hands between passes; nothing is kept after a pass."""
+    from hgcalml_b200.accknn_op import AccumulateKnnDifferentiable, AccumulateKnnGrad
+    from hgcalml_b200.binned_select_knn_op import BinnedSelectKnnDifferentiable, SelectKnnGrad
+    g = torch.Generator(device=cuda).manual_seed(3)
+    c = torch.rand((3000, 3), generator=g, device=cuda).requires_grad_(True)
+    f = torch.randn((3000, 12), generator=g, device=cuda).requires_grad_(True)
+    rs = torch.tensor([0, 1800, 3000], dtype=torch.int32, device=cuda)
+    go = torch.randn((3000, 24), generator=g, device=cuda)
+    idx, d2 = BinnedSelectKnnDifferentiable(14, c, rs)
+    out, arg = AccumulateKnnDifferentiable(10. * d2, f, idx)
+    w = torch.exp(-(10. * d2)).detach()
+    gw, gf = AccumulateKnnGrad(go, w, f.detach(), idx, arg)
+    gc = SelectKnnGrad(gw * -w * 10., idx, d2.detach(), c.detach())
+    for _ in range(2):
+        rc, rf = torch.autograd.grad(out, (c, f), go, retain_graph=True)
+        assert torch.equal(rf, gf) and torch.allclose(rc, gc, rtol=1e-5, atol=1e-6)
+        assert idx._hgc_lists.ws is None
+    (rf,) = torch.autograd.grad(out, (f,), go, retain_graph=True)  # the search's gradient does not run
+    assert torch.equal(rf, gf) and idx._hgc_lists.ws is None
