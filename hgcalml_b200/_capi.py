@@ -78,6 +78,13 @@ def _load():
 
 
 lib = _load()
+
+try:
+    from . import _native as native  # noqa: F401  (host binding of the most frequent ops, links against `lib`)
+except ImportError as e:
+    raise ImportError(f"{os.path.join(_HERE, '_native.so')} cannot be loaded ({e}): build it with "
+                      f"`make -C {os.path.join(_HERE, 'csrc')}` (or __graft_entry__.build())") from e
+
 EXPORTED = [n for n in dir(lib) if n.startswith("hgc_")]
 
 
@@ -98,15 +105,19 @@ _raw_stream = torch._C._cuda_getCurrentRawStream if hasattr(torch._C, "_cuda_get
     lambda index: torch.cuda.current_stream(index).cuda_stream
 
 
-def stream_of(t: torch.Tensor):
-    """The current stream of the tensor's device.  The library launches on the calling thread's
-    current device, so that device must be the tensor's."""
+def check_device(t: torch.Tensor) -> int:
+    """The library launches on the calling thread's current device, so that device must be the tensor's."""
     index = t.get_device()
     if index != torch.cuda.current_device():
         raise HgcError(f"tensors live on {t.device} but the current CUDA device is "
                        f"cuda:{torch.cuda.current_device()}: call torch.cuda.set_device (or use "
                        "torch.cuda.device) before calling hgcalml_b200 ops")
-    return _raw_stream(index)
+    return index
+
+
+def stream_of(t: torch.Tensor):
+    """The current stream of the tensor's device."""
+    return _raw_stream(check_device(t))
 
 
 def workspace(nbytes: int, device) -> torch.Tensor:

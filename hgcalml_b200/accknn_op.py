@@ -6,7 +6,7 @@ import torch
 from . import _capi as C
 
 
-def _prepare(weights, features, indices, mean_and_max, with_max_idxs):
+def _prepare(weights, features, indices):
     C.require_cuda(weights, features, indices)
     weights, features, indices = C.f32(weights), C.f32(features), C.i32(indices)
     n, k = indices.shape
@@ -16,14 +16,8 @@ def _prepare(weights, features, indices, mean_and_max, with_max_idxs):
     if weights.shape[1] != k:
         raise C.HgcError("AccumulateKnnOp expects second dimension of distance and neighbour index "
                          "tensor to match")
-    n_out = 2 * f if mean_and_max else f
-    out = torch.empty((n, n_out), dtype=torch.float32, device=features.device)
-    maxidx = None
-    if with_max_idxs:
-        maxidx = torch.empty((n, f), dtype=torch.int32, device=features.device)
-        if not mean_and_max:
-            maxidx.zero_()
-    return weights, features, indices, out, maxidx, n, k, f, n_out
+    C.check_device(features)
+    return weights, features, indices
 
 
 def _order(order, indices, n):
@@ -39,12 +33,10 @@ def AccumulateLinKnn(weights, features, indices, mean_and_max=True, force_tf=Fal
     as is (modules/accknn_op.py:17-36, modules/compiled/accumulate_knn_module.cc:7-14).
     Returns ``(out_features [N, 2F or F], out_max_idxs [N, F])``."""
     del force_tf
-    w, feat, idx, out, maxidx, n, k, f, n_out = _prepare(weights, features, indices, mean_and_max,
-                                                        with_max_idxs)
-    C.check(C.lib.hgc_accumulate_knn_ordered(C.ptr(w), C.ptr(feat), C.ptr(idx), C.ptr(out), C.ptr(maxidx),
-                                             n, k, f, n_out, 0, int(bool(mean_and_max)),
-                                             C.ptr(_order(order, indices, n)), C.stream_of(feat)),
-            "AccumulateKnn")
+    w, feat, idx = _prepare(weights, features, indices)
+    out, maxidx, rc = C.native.accumulate(w, feat, idx, _order(order, indices, idx.shape[0]), bool(mean_and_max),
+                                          bool(with_max_idxs), False, 1.)
+    C.check(rc, "AccumulateKnn")
     return out, maxidx
 
 
@@ -58,13 +50,10 @@ def AccumulateKnn(distances, features, indices, mean_and_max=True, force_tf=Fals
     multiplied into the distances inside the kernel (``AccumulateKnn(10.*distsq, ..)`` of GravNet is
     ``distance_scale=10`` on the raw squared distances, without the extra elementwise pass)."""
     del force_tf
-    d, feat, idx, out, maxidx, n, k, f, n_out = _prepare(distances, features, indices, mean_and_max,
-                                                        with_max_idxs)
-    order = _order(order, indices, n)
-    C.check(C.lib.hgc_accumulate_knn_exp(C.ptr(d), C.ptr(feat), C.ptr(idx), C.ptr(out), C.ptr(maxidx),
-                                         n, k, f, n_out, int(bool(mean_and_max)), float(distance_scale),
-                                         C.ptr(order),
-                                         C.stream_of(feat)), "AccumulateKnn")
+    d, feat, idx = _prepare(distances, features, indices)
+    out, maxidx, rc = C.native.accumulate(d, feat, idx, _order(order, indices, idx.shape[0]), bool(mean_and_max),
+                                          bool(with_max_idxs), True, float(distance_scale))
+    C.check(rc, "AccumulateKnn")
     return out, maxidx
 
 
@@ -87,15 +76,9 @@ def AccumulateKnnGrad(grad_from_out_features, distances, features, neigh_indices
         maxidx = C.i32(max_feat_indices)
     else:
         maxidx = None
-    dev = feat.device
-    gw = torch.empty((n, k), dtype=torch.float32, device=dev)
-    gf = torch.empty((n, f), dtype=torch.float32, device=dev)
-    ws = C.workspace(C.lib.hgc_knn_grad_workspace_bytes(n, k), dev)
-    order = _order(order, neigh_indices, n)
-    C.check(C.lib.hgc_accumulate_knn_grad_ordered(C.ptr(g), C.ptr(w), C.ptr(feat), C.ptr(maxidx), C.ptr(idx),
-                                                  C.ptr(gw), C.ptr(gf), n, k, f, g.shape[1], 0, int(mean_and_max),
-                                                  C.ptr(order), C.ptr(ws), ws.numel(), C.stream_of(feat)),
-            "AccumulateKnnGrad")
+    C.check_device(feat)
+    gw, gf, ws, rc = C.native.accumulate_grad(g, w, feat, idx, maxidx, _order(order, neigh_indices, n))
+    C.check(rc, "AccumulateKnnGrad")
     if _lists is not None and n > 0 and k > 0:
         _lists.put(idx, ws)
     return gw, gf

@@ -60,24 +60,12 @@ def BinnedSelectKnn(K: int, coords, row_splits, direction=None, n_bins=None, max
     del max_radius, name
     C.require_cuda(coords, row_splits, direction)
     coords, row_splits = C.f32(coords), C.i32(row_splits)
-    use_direction = direction is not None
-    if use_direction:
+    if direction is not None:
         direction = C.i32(direction)
-    n, c = coords.shape
-    n_rs = row_splits.shape[0]
-    nb = -1 if n_bins is None else int(n_bins)
-    dev = coords.device
-    idx = torch.empty((n, K), dtype=torch.int32, device=dev)
-    dist = torch.empty((n, K), dtype=torch.float32, device=dev)
-    sorting = torch.empty((n,), dtype=torch.int32, device=dev)
-    nbytes = C.lib.hgc_binned_select_knn_ragged_workspace_bytes(n, K, c, n_rs, nb, max_bin_dims)
-    if nbytes == 0:
-        raise C.HgcError("BinnedSelectKnn: unsupported combination of sizes")
-    ws = C.workspace(nbytes, dev)
-    C.check(C.lib.hgc_binned_select_knn_ragged(
-        C.ptr(coords), C.ptr(row_splits), C.ptr(direction), C.ptr(idx), C.ptr(dist), C.ptr(sorting),
-        n, K, c, n_rs, nb, int(max_bin_dims), int(bool(tf_compatible)), int(use_direction),
-        C.ptr(ws), ws.numel(), C.stream_of(coords)), "BinnedSelectKnn")
+    C.check_device(coords)
+    idx, dist, sorting, rc = C.native.select_knn(coords, row_splits, direction, K, -1 if n_bins is None else int(n_bins),
+                                                 int(max_bin_dims), bool(tf_compatible))
+    C.check(rc, "BinnedSelectKnn")
     C.set_order(idx, sorting)
     if return_sorting:
         return idx, dist, sorting
@@ -91,16 +79,11 @@ def SelectKnnGrad(grad_distances, indices, distances, coordinates, order=None, _
     ``order`` (optional int32 permutation of the hits) only sets the order in which hits are processed."""
     C.require_cuda(grad_distances, indices, coordinates)
     g, idx, coords = C.f32(grad_distances), C.i32(indices), C.f32(coordinates)
-    d = None if distances is None else C.f32(distances)
-    n, k = idx.shape
-    out = torch.empty_like(coords)
-    ws = _lists.take(idx) if _lists is not None else None
-    run = C.lib.hgc_select_knn_grad_ordered if ws is None else C.lib.hgc_select_knn_grad_after
-    if ws is None:
-        ws = C.workspace(C.lib.hgc_knn_grad_workspace_bytes(n, k), coords.device)
-    order = C.order_of(indices, n) if order is None else C.i32(order)
-    C.check(run(C.ptr(g), C.ptr(idx), C.ptr(d), C.ptr(coords), C.ptr(out), n, k, coords.shape[1], C.ptr(order),
-                C.ptr(ws), ws.numel(), C.stream_of(coords)), "SelectKnnGrad")
+    del distances  # an input of the op that is never read
+    C.check_device(coords)
+    order = C.order_of(indices, idx.shape[0]) if order is None else C.i32(order)
+    out, rc = C.native.select_knn_grad(g, idx, coords, order, None if _lists is None else _lists.take(idx))
+    C.check(rc, "SelectKnnGrad")
     return out
 
 
