@@ -46,7 +46,9 @@ namespace hgc {
 
 constexpr int kTileWarps = 4;
 constexpr int kTileThreads = kTileWarps * kWarp;
-constexpr int kTileListCap = 1024;  // chunks in a tile's list; tiles that need more walk the boxes per query
+// Chunks in a tile's list; tiles that need more walk the boxes per query.  What the list takes of shared memory, L1 lacks:
+// 200k hits N(0,1)-like in four dimensions, four searches: 512 4.34, 1024 3.61, 1280 3.53, 2048 3.72 ms.
+constexpr int kTileListCap = 1280;
 constexpr int kTileBuckets = 32;      // classes of distance from the tile's centre
 constexpr int kTileClassBits = 5;
 
@@ -57,7 +59,7 @@ template <int L> struct TileShape {
     static constexpr int kWindow = L <= 2 ? 8 : 4 * L;                             // slack a prune may leave above K - 1
     static constexpr int kRep = 2 * L + 3;                                        // chunks a representative looks at
 };
-constexpr int kTileNear = 100;  // chunks within reach that a warp collects before it looks at their hits
+constexpr int kTileNear = 68;   // chunks within reach that a warp collects before it looks at their hits
 
 __device__ __forceinline__ unsigned redux_max_u32(unsigned v) { return __reduce_max_sync(0xffffffffu, v); }
 __device__ __forceinline__ int redux_add_i32(int v) { return __reduce_add_sync(0xffffffffu, v); }
@@ -247,7 +249,8 @@ struct TileQuery {
         n_near += __popc(m);
     }
 
-    // Looks at the hits of the noted chunks; the loads of four chunks are in flight together.
+    // Looks at the hits of the noted chunks; the loads of four chunks are in flight together (two for the last one or
+    // two: filling them up to four cost 5 %).
     __device__ __forceinline__ void look()
     {
         const float4 *__restrict__ pts = a->pts;
@@ -266,9 +269,14 @@ struct TileQuery {
                 j[0] = c.x + lane; j[1] = c.y + lane;
             }
 #pragma unroll
-            for (int u = 0; u < U; u++) { p[u] = load_point<NV4>(pts, (size_t)j[u]); j[u] = __ldg(ranks + j[u]); }
+            for (int u = 0; u < U; u++) {
+                if (u >= 2 && i + 2 >= n_near) break;  // uniform
+                p[u] = load_point<NV4>(pts, (size_t)j[u]);
+                j[u] = __ldg(ranks + j[u]);
+            }
 #pragma unroll
             for (int u = 0; u < U; u += 2) {
+                if (u >= 2 && i + 2 >= n_near) break;
                 append(distsq<NV4>(q, p[u]), j[u], true);
                 append(distsq<NV4>(q, p[u + 1]), j[u + 1], true);
                 if (cnt > S::kPruneAt) {
