@@ -400,7 +400,9 @@ def measure_kernels(torch, dev, coords, feats, rs, K, F, reps=3):
     idx, d2, sorting = BinnedSelectKnn(K, coords, rs, return_sorting=True)
     acc_ms = timed(lambda: AccumulateKnn(d2, feats, idx, order=sorting, distance_scale=10.))
     acc_na_ms = timed(lambda: AccumulateKnn(d2, feats, idx, order=sorting, distance_scale=10., with_max_idxs=False))
-    acc_unordered_ms = timed(lambda: AccumulateKnn(d2, feats, idx, distance_scale=10.))
+    unordered = idx.clone()  # the search notes its order with the table it returns, not with a copy
+    acc_unordered_ms = timed(lambda: AccumulateKnn(d2, feats, unordered, distance_scale=10.))
+    del unordered
     wrapper_ms = timed(lambda: BinnedSelectKnn(K, coords, rs))
     # op-level search on bin-sorted inputs
     n_first = int(rs[1].item())

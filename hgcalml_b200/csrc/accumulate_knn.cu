@@ -395,17 +395,18 @@ int accumulate_dispatch(bool exp_w, const float *w, const float *feat, const int
     // floats per load, lanes per hit, vectors per lane, rows in flight, block size, blocks per SM
     if (!vec_ok) {
         // widths that are no multiple of four (or unaligned rows): the same kernel with 8- or 4-byte loads.  F = 22,
-        // K = 41, 114k hits: 195 -> 96 us against a warp per hit that read every index and weight in all lanes
+        // K = 41, 114k hits: 195 -> 83 us against a warp per hit that read every index and weight in all lanes.  Fewer lanes with more
+        // vectors each: F = 22 83 us against 95, F = 50 169 against 190, F = 45 190 against 224
         if (pair_ok) {
             if (F <= 16) HGC_VEC(2, 8, 1, 4, 256, 4);
-            if (F <= 32) HGC_VEC(2, 16, 1, 4, 256, 4);
-            if (F <= 64) HGC_VEC(2, 32, 1, 4, 256, 4);
+            if (F <= 32) HGC_VEC(2, 8, 2, 4, 256, 4);
+            if (F <= 64) HGC_VEC(2, 16, 2, 4, 256, 4);
             if (F <= 128) HGC_VEC(2, 32, 2, 4, 256, 4);
             HGC_VEC(2, 32, 4, 4, 256, 2);
         }
         if (F <= 16) HGC_VEC(1, 8, 2, 4, 256, 4);
-        if (F <= 32) HGC_VEC(1, 16, 2, 4, 256, 4);
-        if (F <= 64) HGC_VEC(1, 32, 2, 4, 256, 4);
+        if (F <= 32) HGC_VEC(1, 8, 4, 4, 256, 4);
+        if (F <= 64) HGC_VEC(1, 16, 4, 4, 256, 4);
         HGC_VEC(1, 32, 4, 4, 256, 4);
     }
     const int F4 = F / 4;
