@@ -62,11 +62,7 @@ def collect_neighbours(features, neighbour_indices, distancesq, *, first_slot: i
             out_column < 0 or out_column + 2 * f > out.shape[1]:
         raise C.HgcError("collect_neighbours: out must be a row-major float32 [N, >= out_column + 2F] buffer")
     maxidx = torch.empty((n, f), dtype=torch.int32, device=feat.device) if with_max_idxs else None
-    if order is None:
-        order = C.order_of(neighbour_indices, n)
-    else:
-        C.require_cuda(order)
-        order = C.i32(order)
+    order = C.row_order(order, neighbour_indices, n)
     view = out[:, out_column:out_column + 2 * f]
     C.check(C.lib.hgc_gravnet_collect(C.ptr(dist), C.ptr(idx), ld, first_slot, k, C.ptr(feat),
                                       view.data_ptr() if n else None, out.stride(0), C.ptr(maxidx), n, f,

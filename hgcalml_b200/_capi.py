@@ -165,6 +165,17 @@ def order_of(idx, n: int):
     return order
 
 
+def row_order(order, idx, n: int):
+    """The processing order the caller names, else the one noted with the neighbour table, if any."""
+    if order is None:
+        return order_of(idx, n)
+    require_cuda(order)
+    if order.numel() != n or order.device != idx.device:
+        raise HgcError(f"order must be a permutation of the {n} hits on {idx.device}, not {order.numel()} entries on "
+                       f"{order.device}")
+    return i32(order)
+
+
 class BackwardLists:
     """Hands the transposed neighbour table from one backward op to a later one of the same backward pass.
     One such object belongs to one differentiable search call; the autograd engine empties it when the pass ends."""

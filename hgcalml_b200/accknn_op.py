@@ -20,21 +20,13 @@ def _prepare(weights, features, indices):
     return weights, features, indices
 
 
-def _order(order, indices, n):
-    """The processing order the caller names, else the one noted with the neighbour table, if any."""
-    if order is None:
-        return C.order_of(indices, n)
-    C.require_cuda(order)
-    return C.i32(order)
-
-
 def AccumulateLinKnn(weights, features, indices, mean_and_max=True, force_tf=False, with_max_idxs=True, order=None):
     """Accumulates neighbour features with linear weights: the registered op ``AccumulateKnn``
     as is (modules/accknn_op.py:17-36, modules/compiled/accumulate_knn_module.cc:7-14).
     Returns ``(out_features [N, 2F or F], out_max_idxs [N, F])``."""
     del force_tf
     w, feat, idx = _prepare(weights, features, indices)
-    out, maxidx, rc = C.native.accumulate(w, feat, idx, _order(order, indices, idx.shape[0]), bool(mean_and_max),
+    out, maxidx, rc = C.native.accumulate(w, feat, idx, C.row_order(order, indices, idx.shape[0]), bool(mean_and_max),
                                           bool(with_max_idxs), False, 1.)
     C.check(rc, "AccumulateKnn")
     return out, maxidx
@@ -51,7 +43,7 @@ def AccumulateKnn(distances, features, indices, mean_and_max=True, force_tf=Fals
     ``distance_scale=10`` on the raw squared distances, without the extra elementwise pass)."""
     del force_tf
     d, feat, idx = _prepare(distances, features, indices)
-    out, maxidx, rc = C.native.accumulate(d, feat, idx, _order(order, indices, idx.shape[0]), bool(mean_and_max),
+    out, maxidx, rc = C.native.accumulate(d, feat, idx, C.row_order(order, indices, idx.shape[0]), bool(mean_and_max),
                                           bool(with_max_idxs), True, float(distance_scale))
     C.check(rc, "AccumulateKnn")
     return out, maxidx
@@ -77,7 +69,7 @@ def AccumulateKnnGrad(grad_from_out_features, distances, features, neigh_indices
     else:
         maxidx = None
     C.check_device(feat)
-    gw, gf, ws, rc = C.native.accumulate_grad(g, w, feat, idx, maxidx, _order(order, neigh_indices, n))
+    gw, gf, ws, rc = C.native.accumulate_grad(g, w, feat, idx, maxidx, C.row_order(order, neigh_indices, n))
     C.check(rc, "AccumulateKnnGrad")
     if _lists is not None and n > 0 and k > 0:
         _lists.put(idx, ws)
@@ -89,7 +81,7 @@ class _AccumulateLinKnnFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, weights, features, indices, mean_and_max, order):
-        order = _order(order, indices, indices.shape[0])
+        order = C.row_order(order, indices, indices.shape[0])
         out, maxidx = AccumulateLinKnn(weights, features, indices, mean_and_max=mean_and_max, order=order)
         ctx.save_for_backward(weights, features, indices, maxidx)
         ctx.order = order

@@ -81,7 +81,7 @@ def SelectKnnGrad(grad_distances, indices, distances, coordinates, order=None, _
     g, idx, coords = C.f32(grad_distances), C.i32(indices), C.f32(coordinates)
     del distances  # an input of the op that is never read
     C.check_device(coords)
-    order = C.order_of(indices, idx.shape[0]) if order is None else C.i32(order)
+    order = C.row_order(order, indices, idx.shape[0])
     out, rc = C.native.select_knn_grad(g, idx, coords, order, None if _lists is None else _lists.take(idx))
     C.check(rc, "SelectKnnGrad")
     return out

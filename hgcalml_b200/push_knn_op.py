@@ -31,7 +31,7 @@ def PushKnnGrad(grad, weights, features, indices, order=None):
     n, k = idx.shape
     wg = torch.empty_like(w)
     fg = torch.empty_like(f)
-    order = C.order_of(indices, n) if order is None else C.i32(order)
+    order = C.row_order(order, indices, n)
     C.check(C.lib.hgc_push_knn_grad_ordered(C.ptr(g), C.ptr(w), C.ptr(f), C.ptr(idx), C.ptr(fg), C.ptr(wg),
                                             n, k, f.shape[1], C.ptr(order), C.stream_of(f)), "PushKnnGrad")
     return wg, fg

@@ -1,0 +1,29 @@
+"""What the Python layer must refuse or leave alone before it hands raw pointers to the library."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("wrong", ["host", "short", "long"])
+def test_an_order_that_does_not_fit_the_table_is_refused(cuda, wrong):
+    from hgcalml_b200 import _capi as C
+    from hgcalml_b200.accknn_op import AccumulateKnn, AccumulateKnnDifferentiable, AccumulateKnnGrad, AccumulateLinKnn
+    from hgcalml_b200.binned_select_knn_op import SelectKnnGrad
+    from hgcalml_b200.GravNetLayersRagged import collect_neighbours
+    from hgcalml_b200.push_knn_op import PushKnnGrad
+    n, k, f = 100, 4, 8
+    idx = torch.randint(0, n, (n, k), dtype=torch.int32, device=cuda)
+    w, x, c = torch.rand((n, k), device=cuda), torch.randn((n, f), device=cuda), torch.randn((n, 3), device=cuda)
+    good = torch.randperm(n, device=cuda).to(torch.int32)
+    order = {"host": good.cpu(), "short": good[:n - 1], "long": torch.cat([good, good[:1]])}[wrong]
+    _, arg = AccumulateLinKnn(w, x, idx)
+    calls = [lambda o: AccumulateKnn(w, x, idx, order=o), lambda o: AccumulateLinKnn(w, x, idx, order=o),
+             lambda o: AccumulateKnnDifferentiable(w, x, idx, order=o),
+             lambda o: AccumulateKnnGrad(torch.cat([x, x], 1), w, x, idx, arg, order=o),
+             lambda o: SelectKnnGrad(w, idx, None, c, order=o), lambda o: PushKnnGrad(x, w, x, idx, order=o),
+             lambda o: collect_neighbours(x, idx, w, order=o)]
+    for call in calls:
+        with pytest.raises(C.HgcError):
+            call(order)
+        call(good[:, None])  # any shape that holds the n entries is taken
