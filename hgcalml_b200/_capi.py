@@ -151,18 +151,41 @@ def i32(t, device=None):
     return _as(t, torch.int32, device)
 
 
+def version_of(t: torch.Tensor):
+    """Counts the changes made to a tensor in place; None where they are not counted (inference tensors)."""
+    return None if t.is_inference() else t._version
+
+
+class RowOrder:
+    """An order noted with a neighbour table."""
+    __slots__ = ("order", "version")
+
+    def __init__(self, order: torch.Tensor):
+        self.order, self.version = order, version_of(order)
+
+    def get(self, idx, n: int):
+        """The order, unless it belongs to other rows or has been written to since it was noted."""
+        order = self.order
+        if order.shape[0] != n or idx.shape[0] != n or order.device != idx.device or version_of(order) != self.version:
+            return None
+        return order
+
+
 def set_order(idx: torch.Tensor, order: torch.Tensor):
     """Notes with a neighbour table the order in which its rows are best processed (the search's sorting of the
     hits).  Ops that gather or scatter along the table look it up when the caller names no order; results do
     not depend on it, and a table without one (a slice, a copy) is processed row by row."""
-    idx._hgc_order = order
+    idx._hgc_order = RowOrder(order)
 
 
-def order_of(idx, n: int):
-    order = getattr(idx, "_hgc_order", None)
-    if order is None or order.shape[0] != n or idx.shape[0] != n or order.device != idx.device:
-        return None
-    return order
+def noted_order(idx):
+    """What set_order noted, for a later order_of with another view of the same table."""
+    return getattr(idx, "_hgc_order", None)
+
+
+def order_of(idx, n: int, note=None):
+    note = noted_order(idx) if note is None else note
+    return None if note is None else note.get(idx, n)
 
 
 def row_order(order, idx, n: int):

@@ -81,10 +81,11 @@ class _AccumulateLinKnnFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, weights, features, indices, mean_and_max, order):
-        order = C.row_order(order, indices, indices.shape[0])
+        if order is not None:
+            order = C.row_order(order, indices, indices.shape[0])
         out, maxidx = AccumulateLinKnn(weights, features, indices, mean_and_max=mean_and_max, order=order)
         ctx.save_for_backward(weights, features, indices, maxidx)
-        ctx.order = order
+        ctx.order, ctx.noted = order, C.noted_order(indices)
         ctx.lists = getattr(indices, "_hgc_lists", None)
         ctx.mark_non_differentiable(maxidx)
         ctx.set_materialize_grads(False)  # no zeros for the arg-max output
@@ -95,8 +96,8 @@ class _AccumulateLinKnnFunction(torch.autograd.Function):
         if grad_out is None:
             return None, None, None, None, None
         weights, features, indices, maxidx = ctx.saved_tensors
-        gw, gf = AccumulateKnnGrad(grad_out, weights, features, indices, maxidx, order=ctx.order,
-                                   _lists=ctx.lists)
+        order = C.order_of(indices, indices.shape[0], ctx.noted) if ctx.order is None else ctx.order
+        gw, gf = AccumulateKnnGrad(grad_out, weights, features, indices, maxidx, order=order, _lists=ctx.lists)
         return gw, gf, None, None, None
 
 

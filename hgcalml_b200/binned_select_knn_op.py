@@ -66,7 +66,8 @@ def BinnedSelectKnn(K: int, coords, row_splits, direction=None, n_bins=None, max
     idx, dist, sorting, rc = C.native.select_knn(coords, row_splits, direction, K, -1 if n_bins is None else int(n_bins),
                                                  int(max_bin_dims), bool(tf_compatible))
     C.check(rc, "BinnedSelectKnn")
-    C.set_order(idx, sorting)
+    if not (return_sorting and sorting.is_inference()):  # the caller could change it unnoticed
+        C.set_order(idx, sorting)
     if return_sorting:
         return idx, dist, sorting
     return idx, dist
@@ -93,7 +94,7 @@ class _BinnedSelectKnnFunction(torch.autograd.Function):
         idx, dist = BinnedSelectKnn(K, coords, row_splits, n_bins=n_bins, max_bin_dims=max_bin_dims,
                                     tf_compatible=tf_compatible)
         ctx.save_for_backward(coords, idx, dist)
-        ctx.order = C.order_of(idx, idx.shape[0])
+        ctx.order = C.noted_order(idx)
         ctx.lists = idx._hgc_lists = C.BackwardLists()
         ctx.mark_non_differentiable(idx)
         ctx.set_materialize_grads(False)  # no zeros for the index output
@@ -104,7 +105,7 @@ class _BinnedSelectKnnFunction(torch.autograd.Function):
         if grad_dist is None:
             return None, None, None, None, None, None
         coords, idx, dist = ctx.saved_tensors
-        return SelectKnnGrad(grad_dist, idx, dist, coords, order=ctx.order,
+        return SelectKnnGrad(grad_dist, idx, dist, coords, order=C.order_of(idx, idx.shape[0], ctx.order),
                              _lists=ctx.lists), None, None, None, None, None
 
 

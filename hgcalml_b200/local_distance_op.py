@@ -20,14 +20,14 @@ class _LocalDistanceFunction(torch.autograd.Function):
     def forward(ctx, coordinates, neighbour_idxs):
         dist = _local_distance(neighbour_idxs, coordinates)
         ctx.save_for_backward(coordinates, neighbour_idxs, dist)
-        ctx.order = C.order_of(neighbour_idxs, coordinates.shape[0])
+        ctx.order = C.noted_order(neighbour_idxs)
         return dist
 
     @staticmethod
     def backward(ctx, grad_dist):
         coords, idx, dist = ctx.saved_tensors
         # the reference registers SelectKnnGrad as the gradient (modules/local_distance_op.py:27-40)
-        return SelectKnnGrad(grad_dist, idx, dist, coords, order=ctx.order), None
+        return SelectKnnGrad(grad_dist, idx, dist, coords, order=C.order_of(idx, idx.shape[0], ctx.order)), None
 
 
 def LocalDistance(coords, neighbour_idxs):

@@ -41,13 +41,13 @@ class _PushKnnFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, w, f, nidx):
         ctx.save_for_backward(w, f, nidx)
-        ctx.order = C.order_of(nidx, nidx.shape[0])
-        return _push_knn(w, f, nidx, ctx.order)
+        ctx.order = C.noted_order(nidx)
+        return _push_knn(w, f, nidx, C.order_of(nidx, nidx.shape[0]))
 
     @staticmethod
     def backward(ctx, grad):
         w, f, nidx = ctx.saved_tensors
-        wg, fg = PushKnnGrad(grad, w, f, nidx, order=ctx.order)
+        wg, fg = PushKnnGrad(grad, w, f, nidx, order=C.order_of(nidx, nidx.shape[0], ctx.order))
         return wg, fg, None
 
 

@@ -27,3 +27,18 @@ def test_an_order_that_does_not_fit_the_table_is_refused(cuda, wrong):
         with pytest.raises(C.HgcError):
             call(order)
         call(good[:, None])  # any shape that holds the n entries is taken
+
+
+def test_a_sorting_whose_changes_are_not_counted_is_not_noted(cuda):
+    from hgcalml_b200 import _capi as C
+    from hgcalml_b200.binned_select_knn_op import BinnedSelectKnn
+    c, rs = torch.rand((300, 3), device=cuda), torch.tensor([0, 300], dtype=torch.int32, device=cuda)
+    with torch.inference_mode():
+        idx, _, sorting = BinnedSelectKnn(8, c, rs, return_sorting=True)
+        assert C.order_of(idx, 300) is None
+        idx, _ = BinnedSelectKnn(8, c, rs)  # no one else has it
+        assert torch.equal(C.order_of(idx, 300), sorting)
+    idx, _, sorting = BinnedSelectKnn(8, c, rs, return_sorting=True)
+    assert C.order_of(idx, 300) is not None
+    sorting += 300
+    assert C.order_of(idx, 300) is None
