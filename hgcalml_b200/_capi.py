@@ -158,16 +158,20 @@ def version_of(t: torch.Tensor):
 
 class RowOrder:
     """An order noted with a neighbour table."""
-    __slots__ = ("order", "version")
+    __slots__ = ("order", "version", "stream")
 
     def __init__(self, order: torch.Tensor):
         self.order, self.version = order, version_of(order)
+        self.stream = _raw_stream(order.get_device()) if order.is_cuda else None
 
     def get(self, idx, n: int):
-        """The order, unless it belongs to other rows or has been written to since it was noted."""
+        """The order, unless it belongs to other rows or has been written to since it was noted.  A caller that uses
+        the table on a second stream can see to the table's memory but not to the order's, so that is done here."""
         order = self.order
         if order.shape[0] != n or idx.shape[0] != n or order.device != idx.device or version_of(order) != self.version:
             return None
+        if self.stream is not None and _raw_stream(order.get_device()) != self.stream:
+            order.record_stream(torch.cuda.current_stream(order.device))
         return order
 
 

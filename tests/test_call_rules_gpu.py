@@ -42,3 +42,29 @@ def test_a_sorting_whose_changes_are_not_counted_is_not_noted(cuda):
     assert C.order_of(idx, 300) is not None
     sorting += 300
     assert C.order_of(idx, 300) is None
+
+
+def test_a_noted_order_lives_as_long_as_another_stream_needs_it(cuda):
+    """The table goes out of use on the host while a second stream has yet to read it: the memory of the order that was
+    noted with it must not be handed out on the first stream before that."""
+    from hgcalml_b200.accknn_op import AccumulateKnn
+    from hgcalml_b200.binned_select_knn_op import BinnedSelectKnn
+    n = 300001  # a size that nothing else here allocates
+    c, rs = torch.rand((n, 3), device=cuda), torch.tensor([0, n], dtype=torch.int32, device=cuda)
+    x = torch.randn((n, 8), device=cuda)
+    idx, d2, sorting = BinnedSelectKnn(8, c, rs, return_sorting=True)
+    want = AccumulateKnn(d2, x, idx)[0]
+    where = sorting.data_ptr()
+    del sorting
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(200_000_000)  # about 0.1 s
+        got, _ = AccumulateKnn(d2, x, idx)
+        for t in (idx, d2, x):
+            t.record_stream(side)
+    del idx, d2
+    new = [torch.empty((n,), dtype=torch.int32, device=cuda) for _ in range(8)]
+    assert not side.query() and where not in [t.data_ptr() for t in new]
+    side.synchronize()
+    assert torch.equal(got, want)
