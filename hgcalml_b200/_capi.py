@@ -5,6 +5,7 @@ error, and every entry point raises when the library reports a non-zero status.
 """
 from __future__ import annotations
 
+import collections
 import ctypes
 import os
 from ctypes import c_int, c_size_t, c_void_p
@@ -156,7 +157,21 @@ def version_of(t: torch.Tensor):
     return None if t.is_inference() else t._version
 
 
-class RowOrder:
+class _Note:
+    """Something kept in an attribute of a neighbour table.  Copies and files of a tensor take its attributes along; of
+    a note they get an empty dictionary, which every reader of tensor files accepts and the lookups below ignore."""
+    __slots__ = ()
+
+    def __reduce_ex__(self, protocol):
+        return collections.OrderedDict, ()
+
+
+def _noted(idx, name: str, kind):
+    note = getattr(idx, name, None)
+    return note if type(note) is kind else None
+
+
+class RowOrder(_Note):
     """An order noted with a neighbour table."""
     __slots__ = ("order", "version", "stream")
 
@@ -184,7 +199,7 @@ def set_order(idx: torch.Tensor, order: torch.Tensor):
 
 def noted_order(idx):
     """What set_order noted, for a later order_of with another view of the same table."""
-    return getattr(idx, "_hgc_order", None)
+    return _noted(idx, "_hgc_order", RowOrder)
 
 
 def order_of(idx, n: int, note=None):
@@ -203,7 +218,7 @@ def row_order(order, idx, n: int):
     return i32(order)
 
 
-class BackwardLists:
+class BackwardLists(_Note):
     """Hands the transposed neighbour table from one backward op to a later one of the same backward pass.
     One such object belongs to one differentiable search call; the autograd engine empties it when the pass ends."""
     __slots__ = ("ws", "key")
@@ -229,6 +244,10 @@ class BackwardLists:
         ws = self.ws if self.key == self._key(idx) else None
         self.clear()
         return ws
+
+
+def noted_lists(idx):
+    return _noted(idx, "_hgc_lists", BackwardLists)
 
 
 def require_cuda(*tensors):

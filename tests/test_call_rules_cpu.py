@@ -1,4 +1,7 @@
 """Rules of the Python layer that hold without a GPU."""
+import copy
+import io
+
 import torch
 
 
@@ -18,3 +21,14 @@ def test_a_noted_order_that_was_written_to_is_not_used():
     order += 1000
     assert C.order_of(idx, 50) is None
     assert C.order_of(idx, 50, note) is None  # as a backward pass asks
+
+
+def test_a_table_with_notes_can_be_saved_and_copied():
+    C, idx, order = _table()
+    idx._hgc_lists = C.BackwardLists()
+    file = io.BytesIO()
+    torch.save(idx, file)
+    file.seek(0)
+    for other in (torch.load(file, weights_only=True), copy.deepcopy(idx)):
+        assert torch.equal(other, idx)
+        assert C.noted_order(other) is None and C.order_of(other, 50) is None and C.noted_lists(other) is None
