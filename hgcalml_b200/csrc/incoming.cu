@@ -3,12 +3,14 @@
 // Targets are counted with integer atomics, which also hand every edge a place in its target's list; a prefix sum
 // gives the lists their room, the edges are written to their places, and every list is then sorted by edge id,
 // which takes out the order in which the atomics happened: the result is the same on every run.  Lists hold about
-// as many edges as a hit has neighbours, so a warp sorts one in registers; lists of more than 128 edges go to a
-// block of their own.
+// as many edges as a hit has neighbours, up to three times as many where hits lie densely, so a warp sorts one in
+// registers; longer lists than that (kWarpList) go to a block of their own.
 //
-// 12.8 M edges (200k hits, K = 64): 0.25 ms, against 0.75 ms with three passes of the stable radix sort over
-// (target, edge) pairs and a search for the list bounds, and 7 launches instead of 17.  Bound by the scattered
-// accesses to L2 (one atomic and one 4-byte write per edge).
+// Bound by the scattered accesses to L2 (one atomic and one 4-byte write per edge) while lists fit a warp.
+// 200k hits, lists built in: K = 16 0.095 ms, K = 64 0.32 ms, K = 128 0.68 ms, K = 256 1.6 ms.  The whole of
+// SelectKnnGrad: 0.52 ms at K = 64, 1.09 at 128, 2.7 at 256, against 1.05, 2.1 and 5.0 ms with three passes of the
+// stable radix sort over (target, edge) pairs and a search for the list bounds, which also took 17 launches instead
+// of 7.
 #include "incoming.cuh"
 #include "knn_device.cuh"
 
@@ -37,6 +39,34 @@ place_edges_kernel(const int *__restrict__ nidx, const int *__restrict__ place, 
     if (m >= 0 && m < n_vert) edges[bounds[m] + place[e]] = (int)e;
 }
 
+// Merges neighbouring ascending runs of M registers: compare with the mirrored run, then clean both bitonic halves.
+// A template parameter for the run, because the compiler stops unrolling a loop over it at 16 registers.
+template <int R, int M>
+__device__ __forceinline__ void merge_runs(unsigned (&v)[R], int lane)
+{
+#pragma unroll
+    for (int g = 0; g < R; g += 2 * M) {
+#pragma unroll
+        for (int i = 0; i < M; i++) {
+            const unsigned lo = v[g + i], hi = __shfl_xor_sync(0xffffffffu, v[g + 2 * M - 1 - i], 31);
+            v[g + i] = min(lo, hi);
+            v[g + 2 * M - 1 - i] = __shfl_xor_sync(0xffffffffu, max(lo, hi), 31);
+        }
+#pragma unroll
+        for (int h = M >> 1; h > 0; h >>= 1)
+#pragma unroll
+            for (int i = 0; i < 2 * M; i++)
+                if (!(i & h)) {
+                    const unsigned lo = v[g + i], hi = v[g + i + h];
+                    v[g + i] = min(lo, hi);
+                    v[g + i + h] = max(lo, hi);
+                }
+#pragma unroll
+        for (int i = 0; i < 2 * M; i++) v[g + i] = warp_bitonic_merge_u32(v[g + i], lane);
+    }
+    if constexpr (2 * M < R) merge_runs<R, 2 * M>(v, lane);
+}
+
 // Sorts 32 * R ids held by a warp (striped) and writes back the first n.
 template <int R>
 __device__ __forceinline__ void sort_list(int *list, int n, int lane)
@@ -45,33 +75,16 @@ __device__ __forceinline__ void sort_list(int *list, int n, int lane)
 #pragma unroll
     for (int r = 0; r < R; r++)
         v[r] = warp_sort_u32(r * 32 + lane < n ? (unsigned)list[r * 32 + lane] : 0xffffffffu, lane);
-    // merge runs of 1, then 2 registers: compare with the mirrored run, then clean both bitonic halves
-#pragma unroll
-    for (int m = 1; m < R; m <<= 1)
-#pragma unroll
-        for (int g = 0; g < R; g += 2 * m) {
-#pragma unroll
-            for (int i = 0; i < m; i++) {
-                const unsigned lo = v[g + i], hi = __shfl_xor_sync(0xffffffffu, v[g + 2 * m - 1 - i], 31);
-                v[g + i] = min(lo, hi);
-                v[g + 2 * m - 1 - i] = __shfl_xor_sync(0xffffffffu, max(lo, hi), 31);
-            }
-            if (m == 2)
-#pragma unroll
-                for (int h = 0; h < 4; h += 2) {
-                    const unsigned lo = v[g + h], hi = v[g + h + 1];
-                    v[g + h] = min(lo, hi);
-                    v[g + h + 1] = max(lo, hi);
-                }
-#pragma unroll
-            for (int i = 0; i < 2 * m; i++) v[g + i] = warp_bitonic_merge_u32(v[g + i], lane);
-        }
+    if constexpr (R > 1) merge_runs<R, 1>(v, lane);
 #pragma unroll
     for (int r = 0; r < R; r++)
         if (r * 32 + lane < n) list[r * 32 + lane] = (int)v[r];
 }
 
-__global__ void __launch_bounds__(256)
+// A warp per list.  32 registers, so that all 64 warps of an SM have a list: sixteen ids per lane then cost a few spills,
+// but with the 48 registers that they would take the short lists wait longer (K = 16, 200k hits: 95 -> 104 us).
+// Lists of 129 to 512 edges, a block each before: K = 96, 200k hits 4.4 -> 0.8 ms, K = 128 8.1 -> 1.1 ms for SelectKnnGrad.
+__global__ void __launch_bounds__(256, 8)
 sort_lists_kernel(const int *__restrict__ bounds, int *__restrict__ edges, int n_vert, int *__restrict__ long_lists)
 {
     pdl_begin();
@@ -82,10 +95,12 @@ sort_lists_kernel(const int *__restrict__ bounds, int *__restrict__ edges, int n
     if (n <= 32) sort_list<1>(edges + begin, n, lane);
     else if (n <= 64) sort_list<2>(edges + begin, n, lane);
     else if (n <= 128) sort_list<4>(edges + begin, n, lane);
+    else if (n <= 256) sort_list<8>(edges + begin, n, lane);
+    else if (n <= kWarpList) sort_list<16>(edges + begin, n, lane);
     else if (lane == 0) long_lists[1 + atomicAdd(long_lists, 1)] = m;
 }
 
-// Lists of more than 128 edges: a block per list, radix sort of 8-bit digits through global memory.
+// Lists of more than kWarpList edges: a block per list, radix sort of 8-bit digits through global memory.
 __global__ void __launch_bounds__(256)
 sort_long_lists_kernel(const int *__restrict__ bounds, int *edges, int *tmp, const int *__restrict__ long_lists,
                        int n_passes)
@@ -157,10 +172,12 @@ int build_incoming(const int *nidx, int n_vert, int n_neigh, const Incoming &b, 
     HGC_LAUNCH_CHECK();
     HGC_CUDA_TRY(launch_overlapped(n_vert, sort_lists_kernel, div_up(n_vert, 8), 256, 0, stream, b.bounds, b.edges, n_vert, b.long_lists));
     HGC_LAUNCH_CHECK();
-    if (ne > 128) {
-        int blocks = sm_count();
-        if (blocks > ne / 129) blocks = (int)(ne / 129);
-        if (blocks < 1) blocks = 1;
+    if (ne > kWarpList) {
+        // Eight blocks per SM where there are edges enough: 60k hits, K = 500, 44 % of the lists longer than this:
+        // 6.5 ms with one block per SM, 2.7 with four, 2.0 with eight.  Idle blocks cost 2 us per 1000, which a small
+        // table would notice (1 M edges: 38 -> 40 us), so no more than one for every four of the longest warp lists.
+        const long long want = ne / (4 * kWarpList), resident = 8 * sm_count();
+        const int blocks = (int)(want < 1 ? 1 : want < resident ? want : resident);
         HGC_CUDA_TRY(launch_pdl(sort_long_lists_kernel, blocks, 256, 0, stream, b.bounds, b.edges, b.place, b.long_lists, (bits_for(ne) + 7) / 8));
         HGC_LAUNCH_CHECK();
     }

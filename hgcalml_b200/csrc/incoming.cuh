@@ -6,9 +6,11 @@
 
 namespace hgc {
 
+constexpr int kWarpList = 512;  // longest list that a warp sorts in registers
+
 struct Incoming {
     int *bounds;          // [n_vert + 2] incoming edges of hit m are edges[bounds[m] .. bounds[m + 1])
-    int *long_lists;      // [1 + n_edges / 129 + 1] number of hits with more than 128 incoming edges, and the hits
+    int *long_lists;      // [1 + n_edges / (kWarpList + 1) + 1] number of hits with more than kWarpList incoming edges, and the hits
     int *scan;            // scratch of the prefix sum
     int *edges;           // [n_edges] edge ids e = hit * n_neigh + slot
     int *place;           // [n_edges] place of an edge in its target's list; scratch of the long sort afterwards
@@ -21,7 +23,7 @@ Incoming incoming_layout(W &ws, int n_vert, int n_neigh)
     const size_t n = n_vert > 0 ? n_vert : 0, ne = n * (size_t)(n_neigh > 0 ? n_neigh : 0);
     Incoming b;
     b.bounds = ws.template take<int>(n + 2);  // first, with long_lists: one memset clears both and the status word
-    b.long_lists = ws.template take<int>(ne / 129 + 2);
+    b.long_lists = ws.template take<int>(ne / (kWarpList + 1) + 2);
     b.scan = ws.template take<int>(scan_scratch_ints((int)n + 1));
     b.edges = ws.template take<int>(ne);
     b.place = ws.template take<int>(ne);

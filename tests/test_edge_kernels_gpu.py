@@ -98,3 +98,23 @@ def test_backward_ops_share_lists_within_a_pass_only(cuda):
         assert idx._hgc_lists.ws is None
     (rf,) = torch.autograd.grad(out, (f,), go, retain_graph=True)  # the search's gradient does not run
     assert torch.equal(rf, gf) and idx._hgc_lists.ws is None
+
+
+@pytest.mark.parametrize("K", [3, 64])
+def test_incoming_lists_around_the_longest_a_warp_sorts(cuda, oracle, K):
+    """Lists of up to 256 and 512 edges are sorted by a warp, longer ones by a block; the gradient adds in list order."""
+    from hgcalml_b200.binned_select_knn_op import SelectKnnGrad
+    rng = np.random.default_rng(K)
+    counts = [127, 128, 129, 255, 256, 257, 258, 511, 512, 513, 514, 1000, 2049]
+    n = 9000 // K + 40
+    flat = np.full(n * K, -1, np.int32)
+    at = rng.permutation(flat.size)
+    for m, count in enumerate(counts):
+        flat[at[:count]] = m
+        at = at[count:]
+    flat[at[::3]] = rng.integers(len(counts), n, at[::3].size)
+    idx = flat.reshape(n, K)
+    assert (np.bincount(idx[idx >= 0], minlength=n)[:len(counts)] == counts).all()
+    g, c = rng.standard_normal((n, K), dtype=np.float32), rng.standard_normal((n, 4), dtype=np.float32)
+    got = SelectKnnGrad(T(g, cuda), T(idx, cuda), None, T(c, cuda))
+    assert np.array_equal(bits(N(got)), bits(oracle.op_select_knn_grad(g, idx, c)))
