@@ -220,34 +220,35 @@ def row_order(order, idx, n: int):
 
 class BackwardLists(_Note):
     """Hands the transposed neighbour table from one backward op to a later one of the same backward pass.
-    One such object belongs to one differentiable search call; the autograd engine empties it when the pass ends."""
-    __slots__ = ("ws", "key")
+    One such object belongs to one differentiable search call and is noted with its table; an op whose forward pass got
+    that table, unchanged, joins it (autograd itself sees to it that the table stays as it was from then on).  The
+    lists are good on the stream they were built on; the autograd engine empties the object when the pass ends."""
+    __slots__ = ("version", "ws", "stream")
 
-    def __init__(self):
-        self.ws = self.key = None
+    def __init__(self, idx):
+        self.version = version_of(idx)
+        self.clear()
 
     def clear(self):
-        self.ws = self.key = None
+        self.ws = self.stream = None
 
-    @staticmethod
-    def _key(idx):
-        return idx.data_ptr(), idx._version, idx.shape, stream_of(idx)
-
-    def put(self, idx, ws):
+    def put(self, ws):
         try:
             torch.autograd.Variable._execution_engine.queue_callback(self.clear)
         except RuntimeError:
             return  # not inside a backward pass
-        self.ws, self.key = ws, self._key(idx)
+        self.ws, self.stream = ws, stream_of(ws)
 
-    def take(self, idx):
-        ws = self.ws if self.key == self._key(idx) else None
+    def take(self):
+        ws, stream = self.ws, self.stream
         self.clear()
-        return ws
+        return ws if ws is not None and stream == stream_of(ws) else None
 
 
 def noted_lists(idx):
-    return _noted(idx, "_hgc_lists", BackwardLists)
+    """The lists of the search that this table came from, unless it was written to since."""
+    lists = _noted(idx, "_hgc_lists", BackwardLists)
+    return lists if lists is not None and lists.version is not None and lists.version == version_of(idx) else None
 
 
 def require_cuda(*tensors):

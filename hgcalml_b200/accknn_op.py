@@ -72,7 +72,7 @@ def AccumulateKnnGrad(grad_from_out_features, distances, features, neigh_indices
     gw, gf, ws, rc = C.native.accumulate_grad(g, w, feat, idx, maxidx, C.row_order(order, neigh_indices, n))
     C.check(rc, "AccumulateKnnGrad")
     if _lists is not None and n > 0 and k > 0:
-        _lists.put(idx, ws)
+        _lists.put(ws)
     return gw, gf
 
 

@@ -83,7 +83,7 @@ def SelectKnnGrad(grad_distances, indices, distances, coordinates, order=None, _
     del distances  # an input of the op that is never read
     C.check_device(coords)
     order = C.row_order(order, indices, idx.shape[0])
-    out, rc = C.native.select_knn_grad(g, idx, coords, order, None if _lists is None else _lists.take(idx))
+    out, rc = C.native.select_knn_grad(g, idx, coords, order, None if _lists is None else _lists.take())
     C.check(rc, "SelectKnnGrad")
     return out
 
@@ -95,7 +95,7 @@ class _BinnedSelectKnnFunction(torch.autograd.Function):
                                     tf_compatible=tf_compatible)
         ctx.save_for_backward(coords, idx, dist)
         ctx.order = C.noted_order(idx)
-        ctx.lists = idx._hgc_lists = C.BackwardLists()
+        ctx.lists = idx._hgc_lists = C.BackwardLists(idx)
         ctx.mark_non_differentiable(idx)
         ctx.set_materialize_grads(False)  # no zeros for the index output
         return idx, dist

@@ -25,10 +25,18 @@ def test_a_noted_order_that_was_written_to_is_not_used():
 
 def test_a_table_with_notes_can_be_saved_and_copied():
     C, idx, order = _table()
-    idx._hgc_lists = C.BackwardLists()
+    idx._hgc_lists = C.BackwardLists(idx)
     file = io.BytesIO()
     torch.save(idx, file)
     file.seek(0)
     for other in (torch.load(file, weights_only=True), copy.deepcopy(idx)):
         assert torch.equal(other, idx)
         assert C.noted_order(other) is None and C.order_of(other, 50) is None and C.noted_lists(other) is None
+
+
+def test_backward_lists_belong_to_the_table_as_the_search_left_it():
+    C, idx, order = _table()
+    idx._hgc_lists = C.BackwardLists(idx)
+    assert C.noted_lists(idx) is idx._hgc_lists
+    idx[:, 2] = -1
+    assert C.noted_lists(idx) is None

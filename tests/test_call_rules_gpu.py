@@ -68,3 +68,23 @@ def test_a_noted_order_lives_as_long_as_another_stream_needs_it(cuda):
     assert not side.query() and where not in [t.data_ptr() for t in new]
     side.synchronize()
     assert torch.equal(got, want)
+
+
+def test_backward_lists_are_of_the_table_that_the_search_made(cuda):
+    """The accumulation runs on a table that was written to, and what both ops saved comes back as copies of that time:
+    the lists of the changed table are not those of the search."""
+    from hgcalml_b200.accknn_op import AccumulateKnnDifferentiable
+    from hgcalml_b200.binned_select_knn_op import BinnedSelectKnnDifferentiable, SelectKnnGrad
+    g = torch.Generator(device=cuda).manual_seed(5)
+    c = torch.rand((4000, 3), generator=g, device=cuda).requires_grad_(True)
+    f = torch.randn((4000, 8), generator=g, device=cuda)
+    rs = torch.tensor([0, 4000], dtype=torch.int32, device=cuda)
+    go = torch.randn((4000, 16), generator=g, device=cuda)
+    with torch.autograd.graph.save_on_cpu():
+        idx, d2 = BinnedSelectKnnDifferentiable(9, c, rs)
+        found = idx.clone()
+        idx[:, 4] = -1
+        out, _ = AccumulateKnnDifferentiable(10. * d2, f, idx)
+        d2.retain_grad()
+        out.backward(go)
+    assert torch.equal(c.grad, SelectKnnGrad(d2.grad, found, None, c.detach()))
