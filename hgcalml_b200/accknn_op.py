@@ -86,7 +86,7 @@ class _AccumulateLinKnnFunction(torch.autograd.Function):
         out, maxidx = AccumulateLinKnn(weights, features, indices, mean_and_max=mean_and_max, order=order)
         ctx.save_for_backward(weights, features, indices, maxidx)
         ctx.order, ctx.noted = order, C.noted_order(indices)
-        ctx.lists = C.noted_lists(indices)
+        ctx.lists = C.noted_lists(indices) if ctx.needs_input_grad[0] else None  # else no search comes after
         ctx.mark_non_differentiable(maxidx)
         ctx.set_materialize_grads(False)  # no zeros for the arg-max output
         return out, maxidx

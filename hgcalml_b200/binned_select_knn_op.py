@@ -95,7 +95,9 @@ class _BinnedSelectKnnFunction(torch.autograd.Function):
                                     tf_compatible=tf_compatible)
         ctx.save_for_backward(coords, idx, dist)
         ctx.order = C.noted_order(idx)
-        ctx.lists = idx._hgc_lists = C.BackwardLists(idx)
+        ctx.lists = None
+        if ctx.needs_input_grad[0]:
+            ctx.lists = idx._hgc_lists = C.BackwardLists(idx)
         ctx.mark_non_differentiable(idx)
         ctx.set_materialize_grads(False)  # no zeros for the index output
         return idx, dist

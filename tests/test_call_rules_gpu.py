@@ -88,3 +88,16 @@ def test_backward_lists_are_of_the_table_that_the_search_made(cuda):
         d2.retain_grad()
         out.backward(go)
     assert torch.equal(c.grad, SelectKnnGrad(d2.grad, found, None, c.detach()))
+
+
+def test_no_lists_are_kept_where_no_search_takes_them(cuda):
+    from hgcalml_b200 import _capi as C
+    from hgcalml_b200.accknn_op import AccumulateKnnDifferentiable
+    from hgcalml_b200.binned_select_knn_op import BinnedSelectKnnDifferentiable
+    c, rs = torch.rand((500, 3), device=cuda), torch.tensor([0, 500], dtype=torch.int32, device=cuda)
+    f = torch.randn((500, 8), device=cuda, requires_grad=True)
+    idx, d2 = BinnedSelectKnnDifferentiable(8, c, rs)
+    assert C.noted_lists(idx) is None
+    idx, d2 = BinnedSelectKnnDifferentiable(8, c.requires_grad_(True), rs)
+    out, _ = AccumulateKnnDifferentiable(d2.detach(), f, idx)
+    assert C.noted_lists(idx) is not None and out.grad_fn.lists is None
