@@ -92,11 +92,18 @@ class _Dense(torch.nn.Module):
         # bias and activation in one pass where no gradient is recorded
         self.fused_relu = {None: 0, "linear": 0, "relu": 1}.get(activation) if not callable(activation) else None
 
+    def _fuses(self, y):
+        """Bias and activation go over ``y`` in place, by raw pointers, where no one wants a gradient of either and the
+        bias is one dense row beside ``y``; every other form takes the tensor operations."""
+        b = self.bias
+        return (self.fused_relu is not None and y.is_cuda and y.dim() == 2 and y.dtype == torch.float32 and
+                y.is_contiguous() and not y.requires_grad and not (b.requires_grad and torch.is_grad_enabled()) and
+                b.device == y.device and b.dtype == torch.float32 and b.shape == y.shape[1:] and b.is_contiguous())
+
     def forward(self, x):
         y = x @ self.kernel
         if self.bias is not None:
-            if self.fused_relu is not None and y.is_cuda and not y.requires_grad and y.dtype == torch.float32 and \
-                    y.dim() == 2 and y.is_contiguous() and self.bias.dtype == torch.float32:
+            if self._fuses(y):
                 C.check(C.lib.hgc_bias_act(C.ptr(y), C.ptr(self.bias), y.shape[0], y.shape[1], self.fused_relu,
                                            C.stream_of(y)), "dense layer")
                 return y
