@@ -73,7 +73,7 @@ def collect_neighbours(features, neighbour_indices, distancesq, *, first_slot: i
 
 def _copy_columns(x, out, column: int):
     """``out[:, column:column + x.shape[1]] = x`` for a row-major buffer."""
-    if x.requires_grad:
+    if x.requires_grad or not C.values_only(x, out):
         out[:, column:] = x
         return
     C.check(C.lib.hgc_copy_columns(C.ptr(x), out.data_ptr() + 4 * column, out.stride(0), x.shape[0], x.shape[1],
@@ -93,12 +93,12 @@ class _Dense(torch.nn.Module):
         self.fused_relu = {None: 0, "linear": 0, "relu": 1}.get(activation) if not callable(activation) else None
 
     def _fuses(self, y):
-        """Bias and activation go over ``y`` in place, by raw pointers, where no one wants a gradient of either and the
-        bias is one dense row beside ``y``; every other form takes the tensor operations."""
+        """Bias and activation go over ``y`` in place, by raw pointers, where only the values count and the bias is one
+        dense row beside ``y``; every other form takes the tensor operations."""
         b = self.bias
-        return (self.fused_relu is not None and y.is_cuda and y.dim() == 2 and y.dtype == torch.float32 and
-                y.is_contiguous() and not y.requires_grad and not (b.requires_grad and torch.is_grad_enabled()) and
-                b.device == y.device and b.dtype == torch.float32 and b.shape == y.shape[1:] and b.is_contiguous())
+        return (self.fused_relu is not None and C.values_only(y, b) and y.is_cuda and y.dim() == 2 and
+                y.dtype == torch.float32 and y.is_contiguous() and b.device == y.device and
+                b.dtype == torch.float32 and b.shape == y.shape[1:] and b.is_contiguous())
 
     def forward(self, x):
         y = x @ self.kernel

@@ -11,6 +11,7 @@ import os
 from ctypes import c_int, c_size_t, c_void_p
 
 import torch
+import torch.autograd.forward_ad  # noqa: F401
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libhgcalml_b200.so")
@@ -249,6 +250,16 @@ def noted_lists(idx):
     """The lists of the search that this table came from, unless it was written to since."""
     lists = _noted(idx, "_hgc_lists", BackwardLists)
     return lists if lists is not None and lists.version is not None and lists.version == version_of(idx) else None
+
+
+def values_only(*tensors) -> bool:
+    """Whether a tensor operation may be replaced by a kernel on raw pointers: the tensors are plain ones, no gradient is
+    recorded for them, and no function transform, forward-mode level, dispatch mode or trace is to see the operation."""
+    return not (torch._C._are_functorch_transforms_active() or torch._C._len_torch_dispatch_stack() or
+                torch.autograd.forward_ad._current_level >= 0 or torch.jit.is_tracing() or
+                torch.compiler.is_compiling() or
+                any(type(t) not in (torch.Tensor, torch.nn.Parameter) for t in tensors) or
+                torch.is_grad_enabled() and any(t.requires_grad for t in tensors))
 
 
 def require_cuda(*tensors):

@@ -38,3 +38,26 @@ def test_a_bias_that_is_no_dense_row_beside_the_result(cuda):
         layer.bias = torch.nn.Parameter(whole.cpu())
         with pytest.raises(RuntimeError):
             layer(x)
+
+
+def test_forward_mode_vmap_and_modes_see_the_operations(cuda):
+    from torch.utils.flop_counter import FlopCounterMode
+    from hgcalml_b200.GravNetLayersRagged import _copy_columns
+    layer, x = _layer(cuda)
+    layer.requires_grad_(False)
+    t = torch.randn(x.shape, generator=torch.Generator(device=cuda).manual_seed(2), device=cuda)
+    z = x @ layer.kernel + layer.bias
+    y, dy = torch.func.jvp(layer, (x,), (t,))
+    assert torch.equal(y, torch.relu(z)) and torch.allclose(dy, (t @ layer.kernel) * (z > 0), rtol=1e-5, atol=1e-6)
+    with torch.autograd.forward_ad.dual_level():
+        out = torch.zeros((40, 9), device=cuda)
+        dual = torch.autograd.forward_ad.make_dual(x, t)
+        dy = torch.autograd.forward_ad.unpack_dual(layer(dual)).tangent
+        assert torch.allclose(dy, (t @ layer.kernel) * (z > 0), rtol=1e-5, atol=1e-6)
+        _copy_columns(dual, out, 3)
+        assert torch.equal(torch.autograd.forward_ad.unpack_dual(out).tangent[:, 3:], t)
+    assert torch.equal(torch.func.vmap(layer)(x.reshape(5, 8, 6)).reshape(40, 8), torch.relu(z))
+    assert torch.equal(torch.jit.trace(layer, x, check_trace=False)(2. * x), layer(2. * x))
+    with FlopCounterMode(display=False) as f:
+        assert torch.equal(layer(x), torch.relu(z))
+    assert f.get_total_flops() == 2 * 40 * 6 * 8
