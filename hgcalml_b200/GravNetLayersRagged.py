@@ -16,9 +16,14 @@ import torch
 from . import _capi as C
 from .binned_select_knn_op import BinnedSelectKnn
 
+
+def _linear(t):
+    return t
+
+
 _ACTIVATIONS = {
-    None: lambda t: t,
-    "linear": lambda t: t,
+    None: _linear,
+    "linear": _linear,
     "relu": torch.relu,
     "elu": torch.nn.functional.elu,
     "tanh": torch.tanh,
@@ -89,23 +94,21 @@ class _Dense(torch.nn.Module):
         torch.nn.init.xavier_uniform_(self.kernel)  # Keras' default glorot_uniform
         self.bias = torch.nn.Parameter(torch.zeros(n_out)) if use_bias else None
         self.activation = _activation(activation)
-        # bias and activation in one pass where no gradient is recorded
-        self.fused_relu = {None: 0, "linear": 0, "relu": 1}.get(activation) if not callable(activation) else None
 
     def _fuses(self, y):
         """Bias and activation go over ``y`` in place, by raw pointers, where only the values count and the bias is one
         dense row beside ``y``; every other form takes the tensor operations."""
         b = self.bias
-        return (self.fused_relu is not None and C.values_only(y, b) and y.is_cuda and y.dim() == 2 and
-                y.dtype == torch.float32 and y.is_contiguous() and b.device == y.device and
-                b.dtype == torch.float32 and b.shape == y.shape[1:] and b.is_contiguous())
+        return ((self.activation is torch.relu or self.activation is _linear) and C.values_only(y, b) and
+                y.is_cuda and y.dim() == 2 and y.dtype == torch.float32 and y.is_contiguous() and
+                b.device == y.device and b.dtype == torch.float32 and b.shape == y.shape[1:] and b.is_contiguous())
 
     def forward(self, x):
         y = x @ self.kernel
         if self.bias is not None:
             if self._fuses(y):
-                C.check(C.lib.hgc_bias_act(C.ptr(y), C.ptr(self.bias), y.shape[0], y.shape[1], self.fused_relu,
-                                           C.stream_of(y)), "dense layer")
+                C.check(C.lib.hgc_bias_act(C.ptr(y), C.ptr(self.bias), y.shape[0], y.shape[1],
+                                           int(self.activation is torch.relu), C.stream_of(y)), "dense layer")
                 return y
             y = y + self.bias
         return self.activation(y)

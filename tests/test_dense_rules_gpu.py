@@ -61,3 +61,12 @@ def test_forward_mode_vmap_and_modes_see_the_operations(cuda):
     with FlopCounterMode(display=False) as f:
         assert torch.equal(layer(x), torch.relu(z))
     assert f.get_total_flops() == 2 * 40 * 6 * 8
+
+
+def test_the_activation_that_the_layer_has_now_is_used(cuda):
+    layer, x = _layer(cuda)
+    with torch.no_grad():
+        z = x @ layer.kernel + layer.bias
+        assert torch.equal(layer(x), torch.relu(z))
+        layer.activation = torch.tanh
+        assert torch.equal(layer(x), torch.tanh(z))
