@@ -24,7 +24,7 @@ bias_act_kernel(float *__restrict__ y, const float *__restrict__ bias, long long
 #pragma unroll
     for (int k = 0; k < V; k++) {
         v[k] = __fadd_rn(v[k], __ldg(bias + c + k));
-        if (RELU) v[k] = v[k] < 0.f ? 0.f : v[k];  // NaN stays NaN
+        if (RELU) v[k] = v[k] <= 0.f ? 0.f : v[k];  // NaN stays NaN, -0 becomes 0
     }
     if constexpr (V == 4) reinterpret_cast<float4 *>(y)[t] = make_float4(v[0], v[1], v[2], v[3]);
     else y[t] = v[0];

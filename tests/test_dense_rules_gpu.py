@@ -70,3 +70,20 @@ def test_the_activation_that_the_layer_has_now_is_used(cuda):
         assert torch.equal(layer(x), torch.relu(z))
         layer.activation = torch.tanh
         assert torch.equal(layer(x), torch.tanh(z))
+
+
+def test_the_sign_of_zero_is_that_of_the_operations(cuda):
+    layer, _ = _layer(cuda, n_in=4, n_out=4)
+    with torch.no_grad():
+        layer.kernel.fill_(-0.)
+        layer.bias.copy_(torch.tensor([-0., 0., 1., -1.]))
+        x = torch.zeros((3, 4), device=cuda)
+        want = torch.relu(x @ layer.kernel + layer.bias)
+        got = layer(x)
+    assert torch.equal(got, want) and torch.equal(torch.signbit(got), torch.signbit(want))
+    from hgcalml_b200 import _capi as C
+    for relu in (0, 1):
+        y, b = torch.tensor([[-0., 0., -0., float("nan")]], device=cuda), torch.tensor([-0., -0., 0., 1.], device=cuda)
+        want = torch.relu(y + b) if relu else y + b
+        C.check(C.lib.hgc_bias_act(C.ptr(y), C.ptr(b), 1, 4, relu, C.stream_of(y)), "bias_act")
+        assert torch.equal(torch.signbit(y)[:, :3], torch.signbit(want)[:, :3]) and y[0, 3].isnan(), (relu, y, want)
