@@ -9,7 +9,7 @@ neighbour search does not depend on the grid.
 """
 from __future__ import annotations
 
-import threading
+import collections
 import weakref
 
 import numpy as np
@@ -22,21 +22,20 @@ from .binned_select_knn_op import BinnedSelectKnn
 # Stream triples of pipelines that no longer exist, per device: the caching allocator keeps memory per stream, so the
 # next pipeline finds the buffers of the last one instead of allocating (a first call on 8 x 100k hits spent 7 of 15 ms in
 # device allocations).  A triple belongs to one pipeline at a time; there are never more than pipelines lived at once.
+# Pipelines are also given up by the garbage collector, at any allocation of any thread, so nothing here waits: a deque
+# takes and hands out one triple at a time by itself, and the table of deques is only added to.
 _idle_streams = {}
-_idle_lock = threading.Lock()
 
 
 def _take_streams(device):
-    with _idle_lock:
-        idle = _idle_streams.setdefault(device, [])
-        if idle:
-            return idle.pop()
-    return tuple(torch.cuda.Stream(device) for _ in range(3))
+    try:
+        return _idle_streams[device].pop()
+    except (KeyError, IndexError):
+        return tuple(torch.cuda.Stream(device) for _ in range(3))
 
 
 def _give_streams(device, streams):
-    with _idle_lock:
-        _idle_streams[device].append(streams)
+    _idle_streams.setdefault(device, collections.deque()).append(streams)
 
 
 class KnnAccumulatePipeline:

@@ -1,6 +1,9 @@
 """Rules of the Python layer that hold without a GPU."""
 import copy
+import gc
 import io
+import threading
+import weakref
 
 import torch
 
@@ -40,3 +43,36 @@ def test_backward_lists_belong_to_the_table_as_the_search_left_it():
     assert C.noted_lists(idx) is idx._hgc_lists
     idx[:, 2] = -1
     assert C.noted_lists(idx) is None
+
+
+def test_pipelines_given_up_by_the_garbage_collector_wait_for_nothing(monkeypatch):
+    """A collection may start at any allocation, also at one that taking streams from the pool makes; the pipelines that
+    it finalises give their streams to the same pool from the same thread."""
+    from hgcalml_b200 import pipeline as P
+    monkeypatch.setattr(P, "_idle_streams", {})
+    monkeypatch.setattr(torch.cuda, "Stream", lambda device: object())
+
+    class Pipeline:
+        def __init__(self, key):
+            self.me = self  # only a collection finds it
+            weakref.finalize(self, P._give_streams, key, P._take_streams(key)).atexit = False
+
+    taken = []
+
+    def use():
+        threshold = gc.get_threshold()
+        gc.set_threshold(1)
+        try:
+            for key in ["a", "b", "c"] * 20:
+                Pipeline(key)
+                taken.append(P._take_streams(key + "x"))
+        finally:
+            gc.set_threshold(*threshold)
+
+    thread = threading.Thread(target=use, daemon=True)
+    thread.start()
+    thread.join(20.)
+    assert not thread.is_alive() and len(taken) == 60
+    gc.collect()
+    idle = [s for pool in P._idle_streams.values() for s in pool]
+    assert len(set(map(id, idle))) == len(idle)  # no triple is there twice
