@@ -49,10 +49,22 @@ def merge_noise_as_indiv_cp(assignment, asso_idx, alpha_idx, is_cond, n_condensa
     point of its own.  Per event the noise hits take the shower numbers 0..n_noise-1 in hit order and
     the real showers are shifted up by n_noise; ``alpha_idx`` lists, per event, the noise hits first
     and then the condensates; noise hits are associated to themselves and flagged as condensates."""
-    C.require_cuda(assignment, asso_idx, alpha_idx, is_cond)
-    return _merge_noise(C.i32(assignment).reshape(-1), C.i32(asso_idx), C.i32(alpha_idx),
-                        is_cond.to(torch.bool).contiguous().reshape(-1), C.i32(n_condensates),
-                        C.i32(row_splits, assignment.device))
+    C.require_cuda(assignment, asso_idx, alpha_idx, is_cond, n_condensates)
+    dev = assignment.device
+    assignment, asso_idx, alpha_idx = C.i32(assignment).reshape(-1), C.i32(asso_idx, dev), C.i32(alpha_idx, dev)
+    is_cond = is_cond.to(dev, torch.bool).contiguous().reshape(-1)
+    n_condensates, row_splits = C.i32(n_condensates, dev), C.i32(row_splits, dev)
+    n, n_rs = assignment.shape[0], row_splits.shape[0]
+    if asso_idx.numel() != n or is_cond.numel() != n:
+        raise C.HgcError("merge_noise_as_indiv_cp: assignment, asso_idx and is_cond must have one entry per hit")
+    if n_condensates.shape[0] != n_rs:
+        raise C.HgcError("merge_noise_as_indiv_cp: n_condensates must have an entry per row split")
+    counts, splits = torch.stack([n_condensates, row_splits]).cpu()  # the kernels go by them
+    if (counts[1:] < counts[:-1]).any() or counts[-1] - counts[0] > min(alpha_idx.numel(), n):
+        raise C.HgcError("merge_noise_as_indiv_cp: n_condensates must ascend, up to the length of alpha_idx")
+    if (splits[1:] < splits[:-1]).any() or splits[-1] - splits[0] != n:
+        raise C.HgcError("merge_noise_as_indiv_cp: the row splits must ascend and cover all hits")
+    return _merge_noise(assignment, asso_idx, alpha_idx, is_cond, n_condensates, row_splits)
 
 
 def _host_int():

@@ -101,3 +101,29 @@ def test_no_lists_are_kept_where_no_search_takes_them(cuda):
     idx, d2 = BinnedSelectKnnDifferentiable(8, c.requires_grad_(True), rs)
     out, _ = AccumulateKnnDifferentiable(d2.detach(), f, idx)
     assert C.noted_lists(idx) is not None and out.grad_fn.lists is None
+
+
+def test_merge_noise_refuses_what_its_kernels_could_not_read(cuda):
+    from hgcalml_b200 import _capi as C
+    from hgcalml_b200.assign_condensate_op import BuildAndAssignCondensatesBinned, merge_noise_as_indiv_cp
+    g = torch.Generator(device=cuda).manual_seed(7)
+    x, beta = torch.rand((900, 3), generator=g, device=cuda), torch.rand((900, 1), generator=g, device=cuda)
+    rs, dist = torch.tensor([0, 400, 900], dtype=torch.int32, device=cuda), torch.full((900, 1), .1, device=cuda)
+    call = lambda **kw: BuildAndAssignCondensatesBinned(x, beta, dist, rs, .9, assign_by_max_beta=True, **kw)
+    args = [*call(), rs]
+    got = merge_noise_as_indiv_cp(*args)
+    for a, b in zip(got, call(keep_noise=True)):
+        assert torch.equal(a, b)
+    assert len(args[2]) > 2
+
+    def refused(at, value):
+        with pytest.raises((C.HgcError, RuntimeError)):
+            merge_noise_as_indiv_cp(*[value if k == at else a for k, a in enumerate(args)])
+
+    refused(1, args[1][:-1])                                   # associations of fewer hits
+    refused(3, args[3][:-1])
+    refused(2, args[2][:-1])                                   # fewer condensates than are counted
+    refused(4, args[4][:-1])
+    refused(4, args[4].flip(0))                                # counts that descend
+    refused(5, rs - torch.tensor([0, 0, 1], dtype=torch.int32, device=cuda))  # a hit in no event
+    refused(4, args[4].cpu())
