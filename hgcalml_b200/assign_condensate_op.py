@@ -59,11 +59,9 @@ def merge_noise_as_indiv_cp(assignment, asso_idx, alpha_idx, is_cond, n_condensa
         raise C.HgcError("merge_noise_as_indiv_cp: assignment, asso_idx and is_cond must have one entry per hit")
     if n_condensates.shape[0] != n_rs:
         raise C.HgcError("merge_noise_as_indiv_cp: n_condensates must have an entry per row split")
-    counts, splits = torch.stack([n_condensates, row_splits]).cpu()  # the kernels go by them
+    counts = n_condensates.cpu()  # the kernels go by them
     if (counts[1:] < counts[:-1]).any() or counts[-1] - counts[0] > min(alpha_idx.numel(), n):
         raise C.HgcError("merge_noise_as_indiv_cp: n_condensates must ascend, up to the length of alpha_idx")
-    if (splits[1:] < splits[:-1]).any() or splits[-1] - splits[0] != n:
-        raise C.HgcError("merge_noise_as_indiv_cp: the row splits must ascend and cover all hits")
     return _merge_noise(assignment, asso_idx, alpha_idx, is_cond, n_condensates, row_splits)
 
 
@@ -86,6 +84,8 @@ def _merge_noise(assignment, asso, alpha, is_cond, n_condensates, row_splits):
         C.ptr(assignment), C.ptr(asso), C.ptr(alpha), C.ptr(is_cond), C.ptr(n_condensates), C.ptr(row_splits),
         new[0].data_ptr(), new[1].data_ptr(), new[2].data_ptr(), C.ptr(cond), C.ptr(n_cond), n_alpha.data_ptr(),
         n, n_rs, C.ptr(ws), ws.numel(), C.stream_of(assignment)), "merge_noise_as_indiv_cp")
+    if n_alpha.item() < 0:
+        raise C.HgcError("merge_noise_as_indiv_cp: the row splits must ascend and cover all hits")
     return new[0][:, None], new[1], new[2:].reshape(-1)[:n_alpha.item()], cond[:, None], n_cond
 
 

@@ -44,10 +44,10 @@ count_noise_kernel(const int *__restrict__ assignment, const int *__restrict__ a
 
 __global__ void __launch_bounds__(kThreads)
 merge_noise_kernel(const int *__restrict__ assignment, const int *__restrict__ association, const int *__restrict__ alpha,
-                   const unsigned char *__restrict__ is_cond, const int *__restrict__ n_cond, HitOrder o, int n_events,
-                   const int2 *__restrict__ counts, int *__restrict__ new_assignment, int *__restrict__ new_association,
-                   int *__restrict__ new_alpha, unsigned char *__restrict__ new_is_cond, int *__restrict__ new_n_cond,
-                   int *__restrict__ n_alpha)
+                   const unsigned char *__restrict__ is_cond, const int *__restrict__ n_cond,
+                   const int *__restrict__ row_splits, HitOrder o, int n_events, const int2 *__restrict__ counts,
+                   int *__restrict__ new_assignment, int *__restrict__ new_association, int *__restrict__ new_alpha,
+                   unsigned char *__restrict__ new_is_cond, int *__restrict__ new_n_cond, int *__restrict__ n_alpha)
 {
     pdl_begin();
     __shared__ int s_warp[kThreads / kWarp];
@@ -55,11 +55,13 @@ merge_noise_kernel(const int *__restrict__ assignment, const int *__restrict__ a
     __shared__ int s_base;
     auto add = [](int a, int b) { return a + b; };
     if (blockIdx.x == gridDim.x - 1) {
-        // the last block has no tile: the counts of all events, and the total
+        // the last block has no tile: the counts of all events, and the total; -1 where the events are not all hits
         int carry = n_cond[0];
+        bool bad = row_splits[0] != 0 || row_splits[n_events] != o.event_pos[n_events + 1];
         for (int e0 = 0; e0 < n_events; e0 += kThreads) {
             const int e = e0 + threadIdx.x;
             int points = 0;
+            bad = bad || (e < n_events && row_splits[e + 1] < row_splits[e]);
             if (e < n_events)
                 for (int q = o.event_tile[e]; q < o.event_tile[e + 1]; q++) points += counts[q].y;
             const int incl = carry + block_scan_inclusive(points, add, 0, s_warp);
@@ -72,9 +74,10 @@ merge_noise_kernel(const int *__restrict__ assignment, const int *__restrict__ a
         int noise = 0;
         for (int q = threadIdx.x; q < o.event_tile[n_events]; q += kThreads) noise += counts[q].x;
         const int all = block_scan_inclusive(noise, add, 0, s_warp);
+        bad = __syncthreads_or(bad ? 1 : 0) != 0;
         if (threadIdx.x == kThreads - 1) {
             new_n_cond[0] = n_cond[0];
-            *n_alpha = all + n_cond[n_events] - n_cond[0];
+            *n_alpha = bad ? -1 : all + n_cond[n_events] - n_cond[0];
         }
         return;
     }
@@ -190,7 +193,7 @@ extern "C" int hgc_merge_noise(
     HGC_CUDA_TRY(launch_pdl(count_noise_kernel, tiles, kThreads, 0, stream, d_assignment, d_association, d_is_cond, o, n_events, counts));
     HGC_LAUNCH_CHECK();
     HGC_CUDA_TRY(launch_pdl(merge_noise_kernel, tiles + 1, kThreads, 0, stream, d_assignment, d_association, d_alpha_idx, d_is_cond,
-                                                           d_n_condensates, o, n_events, counts, d_new_assignment,
+                                                           d_n_condensates, d_row_splits, o, n_events, counts, d_new_assignment,
                                                            d_new_association, d_new_alpha_idx, d_new_is_cond,
                                                            d_new_n_condensates, n_alpha));
     HGC_LAUNCH_CHECK();

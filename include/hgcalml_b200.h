@@ -293,8 +293,9 @@ int hgc_build_and_assign_condensates(
  *   d_assignment, d_association, d_is_cond [n_vert], d_alpha_idx, d_n_condensates [n_rs]: as written by
  *          hgc_build_and_assign_condensates (only the first d_n_condensates[n_rs-1] entries of d_alpha_idx are read)
  *   outputs [n_vert] (d_new_alpha_idx [2 n_vert]) and d_new_n_condensates [n_rs]; they must not overlap inputs
- *   h_n_alpha (host, may be NULL): receives the number of entries of d_new_alpha_idx; the call then
- *          returns after the stream has finished. */
+ *   h_n_alpha (host, may be NULL): receives the number of entries of d_new_alpha_idx, or -1 where the row
+ *          splits do not ascend from 0 to n_vert (the outputs are then of no use); the call returns after
+ *          the stream has finished. */
 size_t hgc_merge_noise_workspace_bytes(int n_vert, int n_rs);
 int hgc_merge_noise(
         const int *d_assignment, const int *d_association, const int *d_alpha_idx, const unsigned char *d_is_cond,

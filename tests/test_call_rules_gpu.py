@@ -127,3 +127,14 @@ def test_merge_noise_refuses_what_its_kernels_could_not_read(cuda):
     refused(4, args[4].flip(0))                                # counts that descend
     refused(5, rs - torch.tensor([0, 0, 1], dtype=torch.int32, device=cuda))  # a hit in no event
     refused(4, args[4].cpu())
+
+
+@pytest.mark.parametrize("splits", [[0, 400, 899], [1, 400, 900], [0, 901, 900], [0] * 400 + [500, 300, 900]])
+def test_kept_noise_needs_events_that_are_all_hits(cuda, splits):
+    """The renumbering is by event; hits in none were refused by the tensor operations, and are."""
+    from hgcalml_b200 import _capi as C
+    from hgcalml_b200.assign_condensate_op import BuildAndAssignCondensatesBinned
+    x, beta = torch.rand((900, 3), device=cuda), torch.rand((900, 1), device=cuda)
+    rs, dist = torch.tensor(splits, dtype=torch.int32, device=cuda), torch.full((900, 1), .1, device=cuda)
+    with pytest.raises(C.HgcError):
+        BuildAndAssignCondensatesBinned(x, beta, dist, rs, .9, assign_by_max_beta=True, keep_noise=True)
