@@ -121,16 +121,17 @@ order_keys_kernel(const float *__restrict__ coords, int C, int n_dims, HitOrder 
     }
 }
 
-// One pass of both sorts.  LAST: the permutation (and, for order 0, its inverse) is written instead of keys and values.
+// One pass of both sorts, or of that along the curve alone (first_order 1).  LAST: the permutation (and, for order 0,
+// its inverse) is written instead of keys and values.
 template <int kRounds, bool FIRST, bool LAST>
 __global__ void __launch_bounds__(kThreads)
-order_pass_kernel(HitOrder o, int n_events, int tiles_cap, int pass, int *__restrict__ bin_perm,
+order_pass_kernel(HitOrder o, int n_events, int tiles_cap, int pass, int first_order, int *__restrict__ bin_perm,
                   int *__restrict__ rank, int *__restrict__ curve_perm)
 {
     pdl_begin();
     __shared__ int s_count[kWarps][256];
     __shared__ int s_warp[kWarps];
-    const int order = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d = threadIdx.x;
+    const int order = first_order + blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, d = threadIdx.x;
     HitTile t;
     if (!find_tile(o, n_events, blockIdx.x, &t)) return;
     const unsigned *__restrict__ key_in = o.key[order][pass & 1];
@@ -250,16 +251,17 @@ int order_hits(const float *coords, int n_coords, int n_bin_dims, const int *row
     }
 #undef HGC_KEYS
     HGC_LAUNCH_CHECK();
-    const dim3 grid(tiles, 2);
+    const int first_order = bin_bits > 0 ? 0 : 1;
+    const dim3 grid(tiles, 2 - first_order);
     for (int p = 0; p < kOrderPasses; p++) {
 #define HGC_PASS(R)                                                                                                  \
     case R * kThreads:                                                                                               \
         if (p == 0)                                                                                                  \
-            HGC_CUDA_TRY(launch_overlapped(n_vert, order_pass_kernel<R, true, false>, grid, kThreads, 0, stream, o, n_events, tiles, p, bin_perm, rank, curve_perm)); \
+            HGC_CUDA_TRY(launch_overlapped(n_vert, order_pass_kernel<R, true, false>, grid, kThreads, 0, stream, o, n_events, tiles, p, first_order, bin_perm, rank, curve_perm)); \
         else if (p + 1 < kOrderPasses)                                                                               \
-            HGC_CUDA_TRY(launch_overlapped(n_vert, order_pass_kernel<R, false, false>, grid, kThreads, 0, stream, o, n_events, tiles, p, bin_perm, rank, curve_perm)); \
+            HGC_CUDA_TRY(launch_overlapped(n_vert, order_pass_kernel<R, false, false>, grid, kThreads, 0, stream, o, n_events, tiles, p, first_order, bin_perm, rank, curve_perm)); \
         else                                                                                                         \
-            HGC_CUDA_TRY(launch_overlapped(n_vert, order_pass_kernel<R, false, true>, grid, kThreads, 0, stream, o, n_events, tiles, p, bin_perm, rank, curve_perm)); \
+            HGC_CUDA_TRY(launch_overlapped(n_vert, order_pass_kernel<R, false, true>, grid, kThreads, 0, stream, o, n_events, tiles, p, first_order, bin_perm, rank, curve_perm)); \
         break
         switch (o.tile) {
             HGC_PASS(2);

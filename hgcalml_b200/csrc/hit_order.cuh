@@ -67,7 +67,8 @@ int range_and_layout(const float *coords, int n_coords, int n_bin_dims, const in
 //   bin_perm[p]: hit at position p of the order by (event, bin, locality code, hit number); rank[hit] is its inverse
 //   curve_perm[p]: hit at position p of the order by (event, position on a Hilbert curve, hit number)
 // The sort clears nothing: `o`'s histograms and `status` must be zero.  bin_bits: bits of a bin number inside
-// an event, at most 16.
+// an event, at most 16; 0 for grids that need more, whose order by bin is left to the caller (bin_perm and rank are
+// not written).
 int order_hits(const float *coords, int n_coords, int n_bin_dims, const int *row_splits, int n_rs, int n_bins, int n_neigh,
                int n_vert, int bin_bits, const HitOrder &o, int *bin_perm, int *rank, int *curve_perm,
                unsigned *status, cudaStream_t stream);

@@ -135,7 +135,7 @@ extern "C" int hgc_binned_select_knn_ragged(
     int *perm = d_sorting_out ? d_sorting_out : b.bin_perm;
     const bool wide = wide_bins(p, n_events);
     if (int rc = order_hits(d_coords, n_coords, p.cb, d_row_splits, n_rs, n_bins, n_neigh, n_vert,
-                            wide ? 16 : bits_for(p.max_bins / (n_events > 0 ? n_events : 1) - 1), b.order, perm, b.rank,
+                            wide ? 0 : bits_for(p.max_bins / (n_events > 0 ? n_events : 1) - 1), b.order, perm, b.rank,
                             b.curve_perm, ws.status(), stream))
         return rc;
     if (wide) {
