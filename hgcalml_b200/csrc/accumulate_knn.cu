@@ -17,11 +17,8 @@
 namespace hgc {
 namespace {
 
-#ifndef HGC_ACC_TILE_STEPS
-#define HGC_ACC_TILE_STEPS 8
-#endif
 // consecutive steps (of THREADS/LPH hits each) a block processes before it jumps to its next tile
-constexpr int kAccTileSteps = HGC_ACC_TILE_STEPS;
+constexpr int kAccTileSteps = 8;
 constexpr int kAccThreads = 256;  // block size of the scalar fallback
 
 typedef unsigned long long f32x2;  // two float32 in one 64-bit register

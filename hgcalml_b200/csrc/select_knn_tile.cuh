@@ -312,13 +312,9 @@ __device__ __forceinline__ float box_gap_distsq(const Point<NV4> &qlo, const Poi
     return s;
 }
 
-#ifndef HGC_TILE_MIN_BLOCKS
-#define HGC_TILE_MIN_BLOCKS 9
-#endif
-
 // (8 blocks per SM for 5 to 8 coordinates: 114k hits, K = 41 411 us, 6 blocks 427 us)
 template <int NV4, int L>
-__global__ void __launch_bounds__(kTileThreads, L <= 2 && NV4 == 1 ? HGC_TILE_MIN_BLOCKS : (L <= 2 && NV4 == 2 ? 8 : L <= 4 ? 6 : 3))
+__global__ void __launch_bounds__(kTileThreads, L <= 2 && NV4 == 1 ? 9 : (L <= 2 && NV4 == 2 ? 8 : L <= 4 ? 6 : 3))
 select_knn_tile_kernel(const TileKnnArgs a)
 {
     pdl_begin();

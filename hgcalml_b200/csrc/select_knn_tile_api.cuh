@@ -22,7 +22,6 @@ struct TileKnnArgs {
     int n_coords, K, tf_compat;
     int nobody;                // first point of a chunk that holds no hits
     int tile;                  // queries per tile: 4, 8, 16 or 32
-    int run;                   // tiles per block
     float guess;               // factor on a neighbouring query's squared K-th distance
     float expo;                // 2 / coordinates (growth of the squared distance with the count)
 };
