@@ -74,19 +74,29 @@ __device__ __forceinline__ float set_eq(float a, float b)
     return r;
 }
 
+template <int VW> struct Vec;
+template <> struct Vec<4> { typedef float4 type; };
+template <> struct Vec<2> { typedef float2 type; };
+template <> struct Vec<1> { typedef float type; };
+
 // VW: floats per load (4, or 2 and 1 for widths and addresses that allow no more); a lane owns VPL vectors of them.
+// Rows are addressed in vectors: in floats, the compiler keeps other addresses in registers, and at F = 128 the extra
+// spills cost a tenth of the time (200k hits, K = 64, arg-max written: 497 -> 541 us).
 // EXACT: the row has exactly LPH * VPL vectors (then the row width is a compile-time constant and no
 // lane is idle).
-template <int VW, int LPH, int VPL, int CH, int THREADS, int MINB, bool EXP, bool WITH_ARG, bool EXACT>
+// SMALL: tiles of as many steps as the launch says.  The tile length of the other batches is a compile-time constant:
+// read from the arguments it costs the kernel registers (200k hits, K = 200, F = 32 without arg-max 386 -> 422 us; K = 64,
+// F = 32 127 -> 142 us).
+template <int VW, int LPH, int VPL, int CH, int THREADS, int MINB, bool EXP, bool WITH_ARG, bool EXACT, bool SMALL>
 __global__ void __launch_bounds__(THREADS, MINB)
-accumulate_vec_kernel(const float *__restrict__ weights, const float *__restrict__ feat,
+accumulate_vec_kernel(const float *__restrict__ weights, const typename Vec<VW>::type *__restrict__ feat,
                       const int *__restrict__ idxs, float *__restrict__ out, int *__restrict__ out_arg,
-                      int n_vert, int K, int ldk, int F_arg, int n_out_feat, bool mean_and_max,
-                      const int *__restrict__ order, float scale, bool sub_self, int tile_steps)
+                      int n_vert, int K, int ldk, int n_vec_arg, int n_out_feat, bool mean_and_max,
+                      const int *__restrict__ order, float scale, bool sub_self, int small_steps)
 {
     pdl_begin();
-    const int F = EXACT ? LPH * VPL * VW : F_arg;
-    const int n_vec = EXACT ? LPH * VPL : F_arg / VW;
+    const int tile_steps = SMALL ? small_steps : kAccTileSteps;
+    const int n_vec = EXACT ? LPH * VPL : n_vec_arg;
     constexpr int G = THREADS / LPH;  // hits a block works on at a time
     constexpr int NE = VPL * VW;      // floats per lane per row
     constexpr int NP = NE / 2;        // packed pairs per lane per row
@@ -163,14 +173,14 @@ accumulate_vec_kernel(const float *__restrict__ weights, const float *__restrict
                         w[kk] = __shfl_sync(0xffffffffu, my_w, s0 + kk, LPH);
 #pragma unroll
                         for (int u = 0; u < VPL; u++) {
-                            const float *p = feat + (size_t)j * F + col[u] * VW;
+                            const typename Vec<VW>::type *p = feat + (size_t)j * n_vec + col[u];
                             if constexpr (VW == 4) {
                                 asm volatile("ld.global.nc.v2.b64 {%0,%1}, [%2];"
                                              : "=l"(f[kk][2 * u]), "=l"(f[kk][2 * u + 1]) : "l"(p));
                             } else if constexpr (VW == 2) {
                                 asm volatile("ld.global.nc.b64 %0, [%1];" : "=l"(f[kk][u]) : "l"(p));
                             } else if (u % 2 == 0) {
-                                f[kk][u / 2] = pack2(__ldg(p), __ldg(feat + (size_t)j * F + col[u + 1 < VPL ? u + 1 : u]));
+                                f[kk][u / 2] = pack2(__ldg(p), __ldg(feat + (size_t)j * n_vec + col[u + 1 < VPL ? u + 1 : u]));
                             }
                         }
                     }
@@ -214,30 +224,39 @@ accumulate_vec_kernel(const float *__restrict__ weights, const float *__restrict
                 if (j < 0) continue;
                 const bool first = (c0 + kk) == 0;
                 const float sf = (float)(c0 + kk);
+                constexpr int W = VW == 1 ? 2 : VW;  // floats looked at together
 #pragma unroll
-                for (int e = 0; e < NP; e++) {
-                    const float *row = feat + (size_t)j * F;
-                    const float fx = __ldg(row + col[2 * e / VW] * VW + (2 * e) % VW);
-                    const float fy = __ldg(row + col[(2 * e + 1) / VW] * VW + (2 * e + 1) % VW);
-                    float sx, sy, ax, ay;
-                    unpack2(sum[e], sx, sy);
-                    unpack2(argslot[e], ax, ay);
-                    const float tx = __fmul_rn(fx, w), ty = __fmul_rn(fy, w);
-                    sx = __fadd_rn(sx, tx);
-                    sy = __fadd_rn(sy, ty);
-                    if (tx >= best[2 * e] || first) { best[2 * e] = tx; ax = sf; }
-                    if (ty >= best[2 * e + 1] || first) { best[2 * e + 1] = ty; ay = sf; }
-                    sum[e] = pack2(sx, sy);
-                    argslot[e] = pack2(ax, ay);
+                for (int u = 0; u < NE / W; u++) {
+                    float fc[W];
+                    if constexpr (VW == 4) {
+                        const float4 fv = __ldg(feat + (size_t)j * n_vec + col[u]);
+                        fc[0] = fv.x; fc[1] = fv.y; fc[2] = fv.z; fc[3] = fv.w;
+                    } else if constexpr (VW == 2) {
+                        const float2 fv = __ldg(feat + (size_t)j * n_vec + col[u]);
+                        fc[0] = fv.x; fc[1] = fv.y;
+                    } else {
+                        fc[0] = __ldg(feat + (size_t)j * n_vec + col[2 * u]);
+                        fc[1] = __ldg(feat + (size_t)j * n_vec + col[2 * u + 1]);
+                    }
+#pragma unroll
+                    for (int h = 0; h < W / 2; h++) {
+                        const int e = u * (W / 2) + h;
+                        float sx, sy, ax, ay;
+                        unpack2(sum[e], sx, sy);
+                        unpack2(argslot[e], ax, ay);
+                        const float tx = __fmul_rn(fc[2 * h], w), ty = __fmul_rn(fc[2 * h + 1], w);
+                        sx = __fadd_rn(sx, tx);
+                        sy = __fadd_rn(sy, ty);
+                        if (tx >= best[2 * e] || first) { best[2 * e] = tx; ax = sf; }
+                        if (ty >= best[2 * e + 1] || first) { best[2 * e + 1] = ty; ay = sf; }
+                        sum[e] = pack2(sx, sy);
+                        argslot[e] = pack2(ax, ay);
+                    }
                 }
             }
         }
 
         if (live) {
-            float *row = out + (size_t)v * n_out_feat;
-            const int *ir = idxs + (size_t)v * ldk;
-            // slot -> neighbour id; no slot ever took the maximum: 0, the CPU op's initial value
-            auto neighbour = [ir](float slot) { return slot < 0.f ? 0 : ir[(int)slot]; };
             if constexpr (VW == 4) {
 #pragma unroll
                 for (int u = 0; u < VPL; u++) {
@@ -251,23 +270,33 @@ accumulate_vec_kernel(const float *__restrict__ weights, const float *__restrict
                     float4 mx = make_float4(best[4 * u], best[4 * u + 1], best[4 * u + 2], best[4 * u + 3]);
                     if (sub_self) {
                         // the hit's own row is taken off the mean and the max (one rounding each)
-                        const float4 own = __ldg(reinterpret_cast<const float4 *>(feat + (size_t)v * F) + vec);
+                        const float4 own = __ldg(feat + (size_t)v * n_vec + vec);
                         m = make_float4(__fsub_rn(m.x, own.x), __fsub_rn(m.y, own.y), __fsub_rn(m.z, own.z), __fsub_rn(m.w, own.w));
                         mx = make_float4(__fsub_rn(mx.x, own.x), __fsub_rn(mx.y, own.y), __fsub_rn(mx.z, own.z), __fsub_rn(mx.w, own.w));
                     }
-                    __stcs(reinterpret_cast<float4 *>(row) + vec, m);  // results are written once and not read again here
+                    float4 *row = reinterpret_cast<float4 *>(out + (size_t)v * n_out_feat);
+                    __stcs(row + vec, m);  // results are written once and not read again by this kernel
                     if (mean_and_max) {
-                        __stcs(reinterpret_cast<float4 *>(row + F) + vec, mx);
+                        __stcs(row + n_vec + vec, mx);
                         if (WITH_ARG) {
+                            // slot -> neighbour id; no slot ever took the maximum: 0, the CPU op's initial value
                             float a0, a1, a2, a3;
                             unpack2(argslot[2 * u], a0, a1);
                             unpack2(argslot[2 * u + 1], a2, a3);
-                            __stcs(reinterpret_cast<int4 *>(out_arg + (size_t)v * F) + vec,
-                                   make_int4(neighbour(a0), neighbour(a1), neighbour(a2), neighbour(a3)));
+                            const int *ir = idxs + (size_t)v * ldk;
+                            int4 a;
+                            a.x = a0 < 0.f ? 0 : ir[(int)a0];
+                            a.y = a1 < 0.f ? 0 : ir[(int)a1];
+                            a.z = a2 < 0.f ? 0 : ir[(int)a2];
+                            a.w = a3 < 0.f ? 0 : ir[(int)a3];
+                            __stcs(reinterpret_cast<int4 *>(out_arg + (size_t)v * n_vec * 4) + vec, a);
                         }
                     }
                 }
             } else {
+                const int F = n_vec * VW;
+                float *row = out + (size_t)v * n_out_feat;
+                const int *ir = idxs + (size_t)v * ldk;
 #pragma unroll
                 for (int q = 0; q < NE; q++) {
                     const int vec = gl + (q / VW) * LPH, f = vec * VW + q % VW;
@@ -277,14 +306,15 @@ accumulate_vec_kernel(const float *__restrict__ weights, const float *__restrict
                     unpack2(argslot[q / 2], a0, a1);
                     float m = __fdiv_rn(q % 2 ? s1 : s0, inv_count), mx = best[q];
                     if (sub_self) {
-                        const float own = __ldg(feat + (size_t)v * F + f);
+                        const float own = __ldg(reinterpret_cast<const float *>(feat) + (size_t)v * F + f);
                         m = __fsub_rn(m, own);
                         mx = __fsub_rn(mx, own);
                     }
                     __stcs(row + f, m);
                     if (mean_and_max) {
                         __stcs(row + F + f, mx);
-                        if (WITH_ARG) __stcs(out_arg + (size_t)v * F + f, neighbour(q % 2 ? a1 : a0));
+                        const float slot = q % 2 ? a1 : a0;
+                        if (WITH_ARG) __stcs(out_arg + (size_t)v * F + f, slot < 0.f ? 0 : ir[(int)slot]);
                     }
                 }
             }
@@ -340,22 +370,30 @@ int launch_vec(bool exp_w, bool with_arg, const float *w, const float *feat, con
 {
     constexpr int G = THREADS / LPH;
     const int n_steps = div_up(n_vert, G);
-    // tiles of fewer steps where blocks would not fill the SMs once: 700 hits at F = 32 16 -> 3.5 us
+    // Shorter tiles for batches that leave SMs without a block: halved while all of them still find room at once (700 hits,
+    // F = 32: 16 -> 3.5 us; 50k hits, F = 64, one block per SM: 131 -> 76 us), and with four blocks per SM and the arg-max
+    // once more (80k hits, F = 32: 51 -> 43 us, without the arg-max 39 either way).  Beyond that a second wave of half tiles
+    // takes as long as one of whole ones and finds fewer rows in L1 (300k hits, F = 16: 69 -> 73 us; 100k hits, F = 32 without
+    // the arg-max 40 -> 43 us).
     int tile_steps = kAccTileSteps;
-    while (tile_steps > 1 && div_up(n_steps, tile_steps) < MINB * sm_count()) tile_steps >>= 1;
+    const int slots = MINB * sm_count(), room = MINB > 1 && with_arg ? 2 * slots - 1 : slots;
+    while (tile_steps > 1 && 2 * div_up(n_steps, tile_steps) <= room) tile_steps >>= 1;
     const long long n_tiles = div_up(n_steps, tile_steps);
     // one block per tile up to 32 blocks per SM (blocks beyond that walk several tiles): measured faster on
     // the 64-event batch than a grid of resident blocks only, which keeps the SMs less evenly loaded
     long long blocks = (long long)sm_count() * 32;
     if (blocks > n_tiles) blocks = n_tiles;
-#define HGC_GO(E, A, X)                                                                                    \
-    HGC_CUDA_TRY(launch_overlapped(n_vert, accumulate_vec_kernel<VW, LPH, VPL, CH, THREADS, MINB, E, A, X>, (int)blocks, THREADS, 0, stream, \
-            w, feat, idxs, out, out_arg, n_vert, K, ldk, F, n_out, mm, order, scale, sub_self, tile_steps))
+#define HGC_GO1(E, A, X, S)                                                                                \
+    HGC_CUDA_TRY(launch_overlapped(n_vert, accumulate_vec_kernel<VW, LPH, VPL, CH, THREADS, MINB, E, A, X, S>, (int)blocks, THREADS, 0, stream, \
+            w, reinterpret_cast<const typename Vec<VW>::type *>(feat), idxs, out, out_arg, n_vert, K, ldk, F / VW, n_out, mm, order, \
+            scale, sub_self, tile_steps))
+#define HGC_GO(E, A, X) do { if (tile_steps == kAccTileSteps) HGC_GO1(E, A, X, false); else HGC_GO1(E, A, X, true); } while (0)
 #define HGC_GO2(E, A) do { if (VW == 4 && F == LPH * VPL * VW) HGC_GO(E, A, (VW == 4)); else HGC_GO(E, A, false); } while (0)
     if (exp_w) { if (with_arg) HGC_GO2(true, true); else HGC_GO2(true, false); }
     else       { if (with_arg) HGC_GO2(false, true); else HGC_GO2(false, false); }
 #undef HGC_GO2
 #undef HGC_GO
+#undef HGC_GO1
     HGC_LAUNCH_CHECK();
     return HGC_OK;
 }
