@@ -17,6 +17,9 @@ from . import _capi as C
 from .binned_select_knn_op import BinnedSelectKnn
 
 
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+
+
 def _linear(t):
     return t
 
@@ -78,11 +81,11 @@ def collect_neighbours(features, neighbour_indices, distancesq, *, first_slot: i
 
 def _copy_columns(x, out, column: int):
     """``out[:, column:column + x.shape[1]] = x`` for a row-major buffer."""
-    if x.requires_grad or not C.values_only(x, out):
+    rc = C.native.copy_columns(x, out, column) if type(x) in _PLAIN else C.NOT_TAKEN
+    if rc == C.NOT_TAKEN:
         out[:, column:] = x
-        return
-    C.check(C.lib.hgc_copy_columns(C.ptr(x), out.data_ptr() + 4 * column, out.stride(0), x.shape[0], x.shape[1],
-                                   C.stream_of(x)), "copy_columns")
+    else:
+        C.check(rc, "copy_columns")
 
 
 class _Dense(torch.nn.Module):
@@ -95,22 +98,19 @@ class _Dense(torch.nn.Module):
         self.bias = torch.nn.Parameter(torch.zeros(n_out)) if use_bias else None
         self.activation = _activation(activation)
 
-    def _fuses(self, y):
-        """Bias and activation go over ``y`` in place, by raw pointers, where only the values count and the bias is one
-        dense row beside ``y``; every other form takes the tensor operations."""
-        b = self.bias
-        return ((self.activation is torch.relu or self.activation is _linear) and C.values_only(y, b) and
-                y.is_cuda and y.dim() == 2 and y.dtype == torch.float32 and y.is_contiguous() and
-                b.device == y.device and b.dtype == torch.float32 and b.shape == y.shape[1:] and b.is_contiguous())
-
     def forward(self, x):
         y = x @ self.kernel
-        if self.bias is not None:
-            if self._fuses(y):
-                C.check(C.lib.hgc_bias_act(C.ptr(y), C.ptr(self.bias), y.shape[0], y.shape[1],
-                                           int(self.activation is torch.relu), C.stream_of(y)), "dense layer")
-                return y
-            y = y + self.bias
+        bias = self.bias
+        if bias is not None:
+            # bias and activation go over y in one pass, in place, where only the values count and the bias is one dense
+            # row beside y; every other form takes the tensor operations
+            relu = self.activation is torch.relu
+            if (relu or self.activation is _linear) and y.is_cuda and type(y) in _PLAIN and type(bias) in _PLAIN:
+                rc = C.native.bias_act(y, bias, relu)
+                if rc != C.NOT_TAKEN:
+                    C.check(rc, "dense layer")
+                    return y
+            y = y + bias
         return self.activation(y)
 
     def set_weights(self, weights: Sequence):

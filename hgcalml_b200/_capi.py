@@ -11,12 +11,12 @@ import os
 from ctypes import c_int, c_size_t, c_void_p
 
 import torch
-import torch.autograd.forward_ad  # noqa: F401
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libhgcalml_b200.so")
 
 HGC_OK = 0
+NOT_TAKEN = 1  # of the host binding: the arguments want the tensor operations
 STATUS_BITS = {1: "bin index out of range", 2: "flat bin index overflow",
                4: "gathered index out of range", 8: "iteration cap reached"}
 
@@ -174,20 +174,21 @@ def _noted(idx, name: str, kind):
 
 class RowOrder(_Note):
     """An order noted with a neighbour table."""
-    __slots__ = ("order", "version", "stream")
+    __slots__ = ("order", "n", "device", "version", "stream")
 
     def __init__(self, order: torch.Tensor):
-        self.order, self.version = order, version_of(order)
+        self.order, self.n, self.device, self.version = order, order.shape[0], order.device, version_of(order)
         self.stream = _raw_stream(order.get_device()) if order.is_cuda else None
 
     def get(self, idx, n: int):
         """The order, unless it belongs to other rows or has been written to since it was noted.  A caller that uses
         the table on a second stream can see to the table's memory but not to the order's, so that is done here."""
         order = self.order
-        if order.shape[0] != n or idx.shape[0] != n or order.device != idx.device or version_of(order) != self.version:
+        if self.n != n or idx.shape[0] != n or idx.device != self.device or \
+                self.version is not None and self.version != order._version:
             return None
-        if self.stream is not None and _raw_stream(order.get_device()) != self.stream:
-            order.record_stream(torch.cuda.current_stream(order.device))
+        if self.stream is not None and _raw_stream(self.device.index) != self.stream:
+            order.record_stream(torch.cuda.current_stream(self.device))
         return order
 
 
@@ -250,16 +251,6 @@ def noted_lists(idx):
     """The lists of the search that this table came from, unless it was written to since."""
     lists = _noted(idx, "_hgc_lists", BackwardLists)
     return lists if lists is not None and lists.version is not None and lists.version == version_of(idx) else None
-
-
-def values_only(*tensors) -> bool:
-    """Whether a tensor operation may be replaced by a kernel on raw pointers: the tensors are plain ones, no gradient is
-    recorded for them, and no function transform, forward-mode level, dispatch mode or trace is to see the operation."""
-    return not (torch._C._are_functorch_transforms_active() or torch._C._len_torch_dispatch_stack() or
-                torch.autograd.forward_ad._current_level >= 0 or torch.jit.is_tracing() or
-                torch.compiler.is_compiling() or
-                any(type(t) not in (torch.Tensor, torch.nn.Parameter) for t in tensors) or
-                torch.is_grad_enabled() and any(t.requires_grad for t in tensors))
 
 
 def require_cuda(*tensors):

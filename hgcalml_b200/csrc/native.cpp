@@ -5,6 +5,10 @@
 #include <torch/csrc/utils/pybind.h>
 #include <ATen/ATen.h>
 #include <ATen/ops/empty.h>
+#include <c10/core/GradMode.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
+#include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <optional>
 
@@ -90,6 +94,46 @@ std::tuple<Tensor, int> select_knn_grad(const Tensor &grad, const Tensor &indice
     return {out, rc};
 }
 
+// Whether a kernel on raw pointers may stand in for a tensor operation: no function transform, dispatch mode or trace is
+// to see the operation ..
+bool operations_are_seen()
+{
+    using c10::DispatchKey;
+    return c10::impl::dispatch_mode_enabled() ||
+           c10::impl::tls_is_dispatch_key_included(DispatchKey::FuncTorchDynamicLayerFrontMode) ||
+           c10::impl::tls_is_dispatch_key_included(DispatchKey::Functionalize) ||
+           c10::impl::tls_is_dispatch_key_included(DispatchKey::Tracer);
+}
+// .. and the tensor is a plain one on the current device, of which nothing but the values counts.
+bool values_only(const Tensor &t)
+{
+    return t.is_cuda() && t.get_device() == c10::cuda::current_device() && t.scalar_type() == at::kFloat && t.layout() == at::kStrided && !t.is_neg() &&
+           !t.unsafeGetTensorImpl()->is_python_dispatch() && !(t.requires_grad() && c10::GradMode::is_enabled()) &&
+           !t._fw_grad(0).defined();
+}
+
+constexpr int kNotTaken = 1;
+
+// y = act(y + bias) in place; kNotTaken where the tensor operations would do more than that
+int bias_act(const Tensor &y, const Tensor &bias, bool relu)
+{
+    if (operations_are_seen() || !values_only(y) || !values_only(bias) || y.dim() != 2 || !y.is_contiguous() ||
+        bias.dim() != 1 || bias.size(0) != y.size(1) || !bias.is_contiguous())
+        return kNotTaken;
+    return hgc_bias_act(data<float>(y), data<float>(bias), (int)y.size(0), (int)y.size(1), relu, stream_of(y));
+}
+
+// out[:, column:] = x, likewise
+int copy_columns(const Tensor &x, const Tensor &out, int column)
+{
+    if (operations_are_seen() || x.requires_grad() || !values_only(x) || !values_only(out) || x.dim() != 2 || out.dim() != 2 ||
+        !x.is_contiguous() || out.stride(1) != 1 || column < 0 || x.size(0) != out.size(0) ||
+        x.size(1) != out.size(1) - column)
+        return kNotTaken;
+    return hgc_copy_columns(data<float>(x), data<float>(out) + column, (int)out.stride(0), (int)x.size(0), (int)x.size(1),
+                            stream_of(x));
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_native, m)
@@ -100,4 +144,6 @@ PYBIND11_MODULE(_native, m)
     m.def("accumulate", &accumulate, unlocked);
     m.def("accumulate_grad", &accumulate_grad, unlocked);
     m.def("select_knn_grad", &select_knn_grad, unlocked);
+    m.def("bias_act", &bias_act, unlocked);
+    m.def("copy_columns", &copy_columns, unlocked);
 }
