@@ -28,47 +28,51 @@ __global__ void local_distance_kernel(const int *__restrict__ nidx, const float 
 }
 
 // PushKnnGrad (modules/compiled/push_knn_grad_kernel.cc:22-95): both parts are gathers.  The part w.r.t. the weights,
-// w_grad[i,k] = sum_f grad[m_k,f] * feat[i,f] with f in order, is edge_dot_kernel.
-// feat_grad[i,f] = sum_k grad[m_k,f] * w[i,k]: one warp per hit, lanes over the features, k in order.
-// Lanes fetch 32 slots with their weights, then the rows of 8 neighbours are requested together.
+// w_grad[i,k] = sum_f grad[m_k,f] * feat[i,f] with f in order, is edge_dot_kernel, and for narrow rows this one, a thread
+// per (hit, slot) that reads the neighbour's row itself: a row of a few floats is one sector, and edge_dot_kernel's loads
+// of 32 floats bring in nothing else (both parts, 200k hits, K = 64: F = 1 323 us against 493, F = 5 378 against 503, F = 13
+// 517 against 521; at F = 16 516 against 513).
+constexpr int kNarrow = 16;
+__global__ void __launch_bounds__(256)
+push_grad_weights_kernel(const float *__restrict__ grad, const float *__restrict__ feat, const int *__restrict__ nidx,
+                         float *__restrict__ w_grad, long long n_edges, int n_vert, int K, int F,
+                         const int *__restrict__ order)
+{
+    pdl_begin();
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n_edges) return;
+    const int row = (int)(t / K), i = order ? order[row] : row;  // processing order only
+    const long long e = (long long)i * K + (t - (long long)row * K);
+    const int m = nidx[e];
+    float acc = 0.f;
+    if (m >= 0 && m < n_vert)
+        for (int f = 0; f < F; f++)
+            acc = __fadd_rn(acc, __fmul_rn(__ldg(grad + (size_t)m * F + f), feat[(size_t)i * F + f]));
+    w_grad[e] = acc;
+}
+
+// feat_grad[i,f] = sum_k grad[m_k,f] * w[i,k]: one warp per hit, lanes over the features, k in order.  All lanes read slot
+// and weight, from one address.  (Handing them out by shuffles, with the rows of eight neighbours requested together, takes
+// longer at every width: 200k hits, K = 64, both gradients, F = 5 448 us against 378, 32 615 against 548, 64 1172 against 1029,
+// 200 4583 against 4242.)
 __global__ void __launch_bounds__(256)
 push_grad_features_kernel(const float *__restrict__ grad, const float *__restrict__ weights,
                           const int *__restrict__ nidx, float *__restrict__ feat_grad, int n_vert, int K, int F,
                           const int *__restrict__ order)
 {
     pdl_begin();
-    constexpr int U = 8;
     const int lane = threadIdx.x & 31;
     const int slot = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (slot >= n_vert) return;
     const int i = order ? order[slot] : slot;  // processing order only
-    for (int f0 = 0; f0 < F; f0 += 32) {
-        const bool in = f0 + lane < F;
+    for (int f = lane; f < F; f += 32) {
         float acc = 0.f;
-        for (int k0 = 0; k0 < K; k0 += 32) {
-            int my_m = -1;
-            float my_w = 0.f;
-            if (k0 + lane < K) {
-                my_m = nidx[(size_t)i * K + k0 + lane];
-                my_w = weights[(size_t)i * K + k0 + lane];
-                if (my_m >= n_vert) my_m = -1;
-            }
-            const int n_here = min(32, K - k0);
-            for (int q0 = 0; q0 < n_here; q0 += U) {
-                float g[U], w[U];
-                int m[U];
-#pragma unroll
-                for (int q = 0; q < U; q++) {
-                    m[q] = __shfl_sync(0xffffffffu, my_m, (q0 + q) & 31);
-                    w[q] = __shfl_sync(0xffffffffu, my_w, (q0 + q) & 31);
-                    g[q] = in && m[q] >= 0 ? __ldg(grad + (size_t)m[q] * F + f0 + lane) : 0.f;
-                }
-#pragma unroll
-                for (int q = 0; q < U; q++)
-                    if (q0 + q < n_here && m[q] >= 0) acc = __fadd_rn(acc, __fmul_rn(g[q], w[q]));
-            }
+        for (int k = 0; k < K; k++) {
+            const int m = nidx[(size_t)i * K + k];
+            if (m < 0 || m >= n_vert) continue;
+            acc = __fadd_rn(acc, __fmul_rn(grad[(size_t)m * F + f], weights[(size_t)i * K + k]));
         }
-        if (in) feat_grad[(size_t)i * F + f0 + lane] = acc;
+        feat_grad[(size_t)i * F + f] = acc;
     }
 }
 
@@ -102,7 +106,11 @@ extern "C" int hgc_push_knn_grad_ordered(
     }
     if (ne > 0) {
         const bool vec4 = n_feat % 4 == 0 && (reinterpret_cast<uintptr_t>(d_feat) & 15u) == 0;
-        HGC_CUDA_TRY(launch_overlapped(n_vert, edge_dot_kernel<false, false>, div_up(ne, 256), 256, 0, stream, d_feat, n_feat, d_grad, nullptr, d_idxs, d_w_grad,
+        if (n_feat < kNarrow)
+            HGC_CUDA_TRY(launch_overlapped(n_vert, push_grad_weights_kernel, div_up(ne, 256), 256, 0, stream, d_grad, d_feat, d_idxs, d_w_grad, ne,
+                                           n_vert, n_neigh, n_feat, d_order));
+        else
+            HGC_CUDA_TRY(launch_overlapped(n_vert, edge_dot_kernel<false, false>, div_up(ne, 256), 256, 0, stream, d_feat, n_feat, d_grad, nullptr, d_idxs, d_w_grad,
                                                                           ne, n_vert, n_neigh, n_feat, vec4, d_order, nullptr));
         HGC_LAUNCH_CHECK();
     }

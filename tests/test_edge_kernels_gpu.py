@@ -118,3 +118,16 @@ def test_incoming_lists_around_the_longest_a_warp_sorts(cuda, oracle, K):
     g, c = rng.standard_normal((n, K), dtype=np.float32), rng.standard_normal((n, 4), dtype=np.float32)
     got = SelectKnnGrad(T(g, cuda), T(idx, cuda), None, T(c, cuda))
     assert np.array_equal(bits(N(got)), bits(oracle.op_select_knn_grad(g, idx, c)))
+
+
+@pytest.mark.parametrize("F", [1, 15, 16, 17])
+def test_push_knn_grad_around_the_narrow_rows(cuda, oracle, F):
+    from hgcalml_b200.push_knn_op import PushKnnGrad
+    n, K = 900, 11
+    idx, rng = _table(n, K, F)
+    w = rng.random((n, K), dtype=np.float32)
+    f, g = (rng.standard_normal((n, F), dtype=np.float32) for _ in range(2))
+    rw, rf = oracle.op_push_knn_grad(g, w, f, idx)
+    for o in (None, T(rng.permutation(n).astype(np.int32), cuda)):
+        gw, gf = PushKnnGrad(T(g, cuda), T(w, cuda), T(f, cuda), T(idx, cuda), order=o)
+        assert np.array_equal(bits(N(gw)), bits(rw)) and np.array_equal(bits(N(gf)), bits(rf))
