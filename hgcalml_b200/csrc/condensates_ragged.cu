@@ -32,7 +32,7 @@ constexpr int kThreads = kOrderThreads;
 constexpr int kWarps = kThreads / kWarp;
 constexpr int kClusterBlocks = 8;
 constexpr int kClaimThreads = 1024;
-constexpr int kClaimStep = kClusterBlocks * kClaimThreads;  // hits of an event looked at together
+constexpr int kClaimStep = kClusterBlocks * kClaimThreads;
 constexpr int kMaxCells = 13824;   // 24 per coordinate; a block keeps two words per cell in shared memory
 constexpr int kMinCells = 64;      // fewer cells than this settle too few condensates per round: windows instead
 
@@ -377,11 +377,11 @@ order_pass_kernel(Buffers b, int n_events, int tiles_cap, int pass, int shift, i
 }
 
 // Which of the high-beta hits are condensates: those that no condensate earlier in the priority order covers.  A cluster
-// of 8 blocks per event, in rounds.  A hit that comes first among the open hits of its own cell and of the cells around
-// it cannot be covered by an open one, so the first open hits of all cells that are first among their neighbours are
-// settled together; then every open hit that one of them covers is closed.  500 blobs on 2700 cells take about 13
-// rounds.  Masked hits (mask > 0) are condensates from the start: nothing covers them and they cover nothing; hits with a
-// negative mask cover others but are not covered.
+// of 8 blocks per event (one block where there are many events), in rounds.  A hit that comes first among the open hits
+// of its own cell and of the cells around it cannot be covered by an open one, so the first open hits of all cells that
+// are first among their neighbours are settled together; then every open hit that one of them covers is closed.  500
+// blobs on 2700 cells take about 13 rounds.  Masked hits (mask > 0) are condensates from the start: nothing covers them
+// and they cover nothing; hits with a negative mask cover others but are not covered.
 //
 // Everything a round looks up is in shared memory: every block keeps the first open hit of every cell among its own hits,
 // the blocks merge those tables (an eighth of the cells each) through distributed shared memory, and every block works
@@ -389,15 +389,16 @@ order_pass_kernel(Buffers b, int n_events, int tiles_cap, int pass, int shift, i
 // records in L2 a round took 24 us, most of it in dependent loads, before (64k open hits per event).
 // A round costs that much however many hits it settles, so a grid of few cells (a radius that spans the event) is
 // left to the windows of claim_kernel.
-template <int NR>
-__global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(kClaimThreads)
+template <int NR, int CB>
+__global__ void __cluster_dims__(CB, 1, 1) __launch_bounds__(kClaimThreads)
 claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max_settled)
 {
     pdl_begin();
+    constexpr int kStep = CB * kClaimThreads;  // hits of an event looked at together
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ int s_dyn[];
-    __shared__ int s_left[2][kClusterBlocks];
+    __shared__ int s_left[2][CB];
     __shared__ int s_count, s_sum, s_listed;
     int *s_best = s_dyn, *s_min = s_dyn + cells_cap;               // cells_cap is a multiple of 4
     float4 *s_rec = reinterpret_cast<float4 *>(s_min + cells_cap);  // [max_settled][NR]
@@ -409,23 +410,23 @@ claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max
     if (!use) return;  // the same in every block
     constexpr int U = NR == 1 ? 4 : NR == 2 ? 2 : 1;  // hits whose data is requested together
     constexpr int kFree = 0x7fffffff;
-    const int e = blockIdx.x / kClusterBlocks, t = threadIdx.x, lane = t & 31;
+    const int e = blockIdx.x / CB, t = threadIdx.x, lane = t & 31;
     const int rank = (int)cluster.block_rank();
     const int g = rank * kClaimThreads + t;
     const int off = b.row_splits_h[e], n_h = b.row_splits_h[e + 1] - off;
-    const int n_steps = (n_h + kClaimStep - 1) / kClaimStep;
+    const int n_steps = (n_h + kStep - 1) / kStep;
     const int word0 = off / 32 + e;
     const float4 *__restrict__ recs = b.p_rec + (size_t)off * NR;
     int *__restrict__ cells = b.p_flag + off;
-    unsigned *__restrict__ open_words = b.open + (size_t)word0 * 32 + g;  // word w of this thread: [w * kClaimStep], w > 0
+    unsigned *__restrict__ open_words = b.open + (size_t)word0 * 32 + g;  // word w of this thread: [w * kStep], w > 0
 
     for (int c = t; c < n_cells; c += kClaimThreads) s_best[c] = kFree;
     if (t == 0) s_count = s_sum = s_listed = 0;
-    // this thread's hits are p = k * kClaimStep + g; 32 of them share a word of open bits, kept in memory beyond the first
+    // this thread's hits are p = k * kStep + g; 32 of them share a word of open bits, kept in memory beyond the first
     unsigned open0 = 0u;
     int n_mine = 0;  // condensates among them
     for (int k = 0; k < n_steps; k++) {
-        const int p = k * kClaimStep + g;
+        const int p = k * kStep + g;
         bool is_open = false, lonely = false;
         if (p < n_h) {
             const int flag = cells[p];
@@ -437,10 +438,10 @@ claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max
             lonely = flag > 0;
             is_open = !lonely;
         }
-        if ((k & 31) == 0 && k > 0) open_words[(size_t)(k / 32) * kClaimStep] = 0u;
+        if ((k & 31) == 0 && k > 0) open_words[(size_t)(k / 32) * kStep] = 0u;
         if (is_open) {
             if (k < 32) open0 |= 1u << k;
-            else open_words[(size_t)(k / 32) * kClaimStep] |= 1u << (k & 31);
+            else open_words[(size_t)(k / 32) * kStep] |= 1u << (k & 31);
         }
         n_mine += lonely ? 1 : 0;
         const unsigned bits = __ballot_sync(0xffffffffu, lonely);
@@ -448,17 +449,17 @@ claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max
     }
     __syncthreads();
     auto flat = [&grid](int at) { return (((at >> 16) & 127) * grid.n[1] + ((at >> 8) & 255)) * grid.n[2] + (at & 255); };
-    const int slice = (n_cells + kClusterBlocks - 1) / kClusterBlocks;
+    const int slice = (n_cells + CB - 1) / CB;
 
     for (int round = 0; round <= n_h; round++) {
         // first open hit of every cell, among this block's
         for (int w = 0; w * 32 < n_steps; w++) {
-            unsigned u = w == 0 ? open0 : open_words[(size_t)w * kClaimStep];
+            unsigned u = w == 0 ? open0 : open_words[(size_t)w * kStep];
             while (u) {
                 int p[U], at[U];
 #pragma unroll
                 for (int q = 0; q < U; q++) {
-                    p[q] = u ? (w * 32 + __ffs(u) - 1) * kClaimStep + g : -1;
+                    p[q] = u ? (w * 32 + __ffs(u) - 1) * kStep + g : -1;
                     u &= u - 1u;
                 }
 #pragma unroll
@@ -475,18 +476,18 @@ claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max
         if (round > 0) {
             int total = 0;
 #pragma unroll
-            for (int r = 0; r < kClusterBlocks; r++) total += s_left[(round - 1) & 1][r];
+            for (int r = 0; r < CB; r++) total += s_left[(round - 1) & 1][r];
             if (total == 0) break;  // the same in every block of the cluster; nobody looks at another block from here on
         }
         // merged, for all blocks
         for (int c = rank * slice + t; c < min((rank + 1) * slice, n_cells); c += kClaimThreads) {
-            int v[kClusterBlocks], m = kFree;
+            int v[CB], m = kFree;
 #pragma unroll
-            for (int r = 0; r < kClusterBlocks; r++) v[r] = *cluster.map_shared_rank(s_best + c, r);
+            for (int r = 0; r < CB; r++) v[r] = *cluster.map_shared_rank(s_best + c, r);
 #pragma unroll
-            for (int r = 0; r < kClusterBlocks; r++) m = min(m, v[r]);
+            for (int r = 0; r < CB; r++) m = min(m, v[r]);
 #pragma unroll
-            for (int r = 0; r < kClusterBlocks; r++) *cluster.map_shared_rank(s_min + c, r) = m;
+            for (int r = 0; r < CB; r++) *cluster.map_shared_rank(s_min + c, r) = m;
         }
         cluster.sync();
         // which of them are first among the cells around: occupied cells are listed first, since later rounds have few
@@ -534,7 +535,7 @@ claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max
         // close them and what they cover
         int left = 0;
         for (int w = 0; w * 32 < n_steps; w++) {
-            unsigned word = w == 0 ? open0 : open_words[(size_t)w * kClaimStep], u = word;
+            unsigned word = w == 0 ? open0 : open_words[(size_t)w * kStep], u = word;
             while (u) {
                 int bit[U], at[U], near_[U];
                 Rec<NR> mine[U];
@@ -544,16 +545,16 @@ claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max
                     u &= u - 1u;
                 }
 #pragma unroll
-                for (int q = 0; q < U; q++) at[q] = bit[q] >= 0 ? cells[(w * 32 + bit[q]) * kClaimStep + g] : 0;
+                for (int q = 0; q < U; q++) at[q] = bit[q] >= 0 ? cells[(w * 32 + bit[q]) * kStep + g] : 0;
 #pragma unroll
                 for (int q = 0; q < U; q++) {
                     near_[q] = bit[q] >= 0 ? s_min[flat(at[q])] : 0;
-                    if (near_[q]) mine[q] = load_rec<NR>(recs + (size_t)((w * 32 + bit[q]) * kClaimStep + g) * NR);
+                    if (near_[q]) mine[q] = load_rec<NR>(recs + (size_t)((w * 32 + bit[q]) * kStep + g) * NR);
                 }
 #pragma unroll
                 for (int q = 0; q < U; q++) {
                     if (near_[q] == 0) continue;
-                    const int p = (w * 32 + bit[q]) * kClaimStep + g;
+                    const int p = (w * 32 + bit[q]) * kStep + g;
                     const int x = (at[q] >> 16) & 127, y = (at[q] >> 8) & 255, z = at[q] & 255;
                     bool stays = true;
                     if ((near_[q] >> 13) & 1) {  // one in its own cell
@@ -574,13 +575,13 @@ claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max
                 }
             }
             if (w == 0) open0 = word;
-            else open_words[(size_t)w * kClaimStep] = word;
+            else open_words[(size_t)w * kStep] = word;
             left += __popc(word);
         }
         left = __reduce_add_sync(0xffffffffu, left);
         if (lane == 0 && left) atomicAdd(&s_sum, left);
         __syncthreads();
-        if (t < kClusterBlocks) *cluster.map_shared_rank(&s_left[round & 1][rank], t) = s_sum;
+        if (t < CB) *cluster.map_shared_rank(&s_left[round & 1][rank], t) = s_sum;
         for (int c = t; c < n_cells; c += kClaimThreads) s_best[c] = kFree;
         if (t == 0) s_count = s_listed = 0;
         __syncthreads();
@@ -895,10 +896,15 @@ int run_claims(const Buffers &b, const Plan &p, int dims, int num_rows, int tile
     const int last = p.bin_passes + 3;
     if (int rc = launch_pass<false, NR>(b, num_rows, tiles, last, 32 + 24, 0, dims, stream)) return rc;
     const size_t smem = 2 * sizeof(int) * (size_t)p.cells + (size_t)p.max_settled * (NR * sizeof(float4) + 2 * sizeof(int));
+    // An SM holds one block, so the chip 18 clusters of eight: more events than that wait for each other, and a block of its
+    // own for every event is faster whatever their size (without barriers across SMs, and without the registers that merging
+    // eight tables takes).  600 events of 100 hits 1.39 -> 0.29 ms, 40 of 5000 0.49 -> 0.26, 64 of 60k 1.71 -> 0.92.
+    const bool one_block = num_rows > sm_count() / kClusterBlocks;
+    const auto claim = one_block ? claim_grid_kernel<NR, 1> : claim_grid_kernel<NR, kClusterBlocks>;
     // (set on every call: the setting belongs to the current device)
-    HGC_CUDA_TRY(cudaFuncSetAttribute(claim_grid_kernel<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    HGC_CUDA_TRY(launch_pdl(claim_grid_kernel<NR>, num_rows * kClusterBlocks, kClaimThreads, smem, stream, b, dims, p.cells, p.cells_per_dim,
-                                                                                      p.max_settled));
+    HGC_CUDA_TRY(cudaFuncSetAttribute(claim, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    HGC_CUDA_TRY(launch_pdl(claim, num_rows * (one_block ? 1 : kClusterBlocks), kClaimThreads, smem, stream, b, dims, p.cells, p.cells_per_dim,
+                            p.max_settled));
     HGC_LAUNCH_CHECK();
     if (int rc = launch_claim_windows(dims, b.h_ccoords, b.h_dist, b.h_mask, b.h_orig, b.row_splits_h, b.order, b.status_h,
                                       b.alpha_h, b.stage, b.cl, num_rows, b.use_grid, stream))

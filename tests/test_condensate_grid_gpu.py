@@ -80,3 +80,15 @@ def test_noise_kept(cuda, oracle, sizes):
     _check(cuda, oracle, cc, beta, np.full_like(beta, 0.2), rs, thr=0.3, mask=mask, keep_noise=True)
     beta[:] = 0.  # nothing but noise
     _check(cuda, oracle, cc, beta, np.full_like(beta, 0.2), rs, thr=0.3, keep_noise=True)
+
+
+@pytest.mark.parametrize("dims", [3, 7])
+def test_a_block_per_event(cuda, oracle, dims):
+    """More events than clusters of eight blocks find room, one of them with more high hits than a thread's word holds."""
+    sizes = np.random.default_rng(29).integers(0, 700, 40)
+    sizes[7] = 36000
+    cc, beta, rs, rng = _batch(sizes, dims, 31)
+    cc *= 2.
+    beta[:] = rng.uniform(0.05, 1., beta.shape)  # nearly all are high
+    mask = rng.choice([0] * 30 + [1, -1], beta.shape).astype(np.int32)
+    _check(cuda, oracle, cc, beta, np.full_like(beta, 0.5), rs, mask=mask, modes=(True,))
