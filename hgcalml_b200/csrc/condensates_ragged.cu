@@ -34,7 +34,13 @@ constexpr int kClusterBlocks = 8;
 constexpr int kClaimThreads = 1024;
 constexpr int kClaimStep = kClusterBlocks * kClaimThreads;
 constexpr int kMaxCells = 13824;   // 24 per coordinate; a block keeps two words per cell in shared memory
-constexpr int kMinCells = 64;      // fewer cells than this settle too few condensates per round: windows instead
+constexpr int kMinCells = 64;      // the fewest that may be of use
+
+// Claims by grid, or over windows of the priority order.  The grid spans three coordinates: fewer cells than 64 settle too
+// few condensates per round, and with more coordinates than the grid has a cell holds hits that are far apart, of which
+// only the first is settled.  4 x 200k hits, radius 1.0 on a range of 6 (216 cells): 3 coordinates 0.47 ms by grid; 4
+// coordinates 1.74 ms and 1.56 over windows, 5 8.0 and 6.3, 8 69 and 48.  Radius 0.85 (512 cells): 4 2.0 by grid.
+__device__ __forceinline__ bool claims_by_grid(int n_cells, int dims) { return n_cells >= (dims <= 3 ? kMinCells : 512); }
 
 typedef unsigned long long u64;
 
@@ -387,8 +393,8 @@ order_pass_kernel(Buffers b, int n_events, int tiles_cap, int pass, int shift, i
 // the blocks merge those tables (an eighth of the cells each) through distributed shared memory, and every block works
 // out for itself which are settled and copies their records.  A round is two cluster barriers.  With the tables and
 // records in L2 a round took 24 us, most of it in dependent loads, before (64k open hits per event).
-// A round costs that much however many hits it settles, so a grid of few cells (a radius that spans the event) is
-// left to the windows of claim_kernel.
+// A round costs that much however many hits it settles, so grids that settle few are left to the windows of claim_kernel
+// (claims_by_grid).
 template <int NR, int CB>
 __global__ void __cluster_dims__(CB, 1, 1) __launch_bounds__(kClaimThreads)
 claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max_settled)
@@ -405,7 +411,7 @@ claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max
     int *s_pos = reinterpret_cast<int *>(s_rec + (size_t)max_settled * NR), *s_at = s_pos + max_settled;
     const CondGrid grid = make_cond_grid(b.layout.grid, b.max_radius, dims, cells_per_dim);
     const int n_cells = grid.n[0] * grid.n[1] * grid.n[2];
-    const bool use = n_cells >= kMinCells;
+    const bool use = claims_by_grid(n_cells, dims);
     if (blockIdx.x == 0 && threadIdx.x == 0) *b.use_grid = use ? 1 : 0;
     if (!use) return;  // the same in every block
     constexpr int U = NR == 1 ? 4 : NR == 2 ? 2 : 1;  // hits whose data is requested together

@@ -82,6 +82,16 @@ def test_noise_kept(cuda, oracle, sizes):
     _check(cuda, oracle, cc, beta, np.full_like(beta, 0.2), rs, thr=0.3, keep_noise=True)
 
 
+@pytest.mark.parametrize("dims,radius", [(3, 1.2), (3, 1.7), (4, 0.8), (4, 1.), (5, 1.2), (8, 0.7)])
+def test_few_cells_with_masks(cuda, oracle, dims, radius):
+    """Around the numbers of cells at which claims go from windows to the grid, and hits from all condensates to those
+    of the cells around them."""
+    cc, beta, rs, rng = _batch([2600, 0, 1500], dims, 23 + dims)
+    mask = rng.choice([0, 0, 0, 0, 1, -1], beta.shape).astype(np.int32)
+    radii = np.full_like(beta, radius) if dims == 4 else (radius * rng.uniform(0.7, 1., beta.shape)).astype(np.float32)
+    _check(cuda, oracle, cc, beta, radii, rs, mask=mask)
+
+
 @pytest.mark.parametrize("dims", [3, 7])
 def test_a_block_per_event(cuda, oracle, dims):
     """More events than clusters of eight blocks find room, one of them with more high hits than a thread's word holds."""
