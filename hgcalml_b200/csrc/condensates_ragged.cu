@@ -34,13 +34,21 @@ constexpr int kClusterBlocks = 8;
 constexpr int kClaimThreads = 1024;
 constexpr int kClaimStep = kClusterBlocks * kClaimThreads;
 constexpr int kMaxCells = 13824;   // 24 per coordinate; a block keeps two words per cell in shared memory
-constexpr int kMinCells = 64;      // the fewest that may be of use
+constexpr int kMinCells = 64;      // the fewest that may be of use, see the two rules
 
 // Claims by grid, or over windows of the priority order.  The grid spans three coordinates: fewer cells than 64 settle too
 // few condensates per round, and with more coordinates than the grid has a cell holds hits that are far apart, of which
 // only the first is settled.  4 x 200k hits, radius 1.0 on a range of 6 (216 cells): 3 coordinates 0.47 ms by grid; 4
 // coordinates 1.74 ms and 1.56 over windows, 5 8.0 and 6.3, 8 69 and 48.  Radius 0.85 (512 cells): 4 2.0 by grid.
 __device__ __forceinline__ bool claims_by_grid(int n_cells, int dims) { return n_cells >= (dims <= 3 ? kMinCells : 512); }
+// Hits against the condensates of the 27 cells around them, or against all in priority order.  The distance fold walks the
+// cells once for every condensate that covers the hit, more of them the more coordinates; all, only once.  4 x 200k hits,
+// distance fold, 125 cells: 4 coordinates 1.47 ms by cell and 1.09 against all, 6 19.1 and 12.8; 216 cells: 4 2.22 and
+// 2.20, 6 27.4 and 29.5.
+__device__ __forceinline__ bool assigns_by_cell(int n_cells, int dims, bool by_max_beta)
+{
+    return n_cells >= (by_max_beta || dims <= 3 ? kMinCells : 150);
+}
 
 typedef unsigned long long u64;
 
@@ -600,7 +608,7 @@ claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max
 // Lists of an event's condensates: in priority order (alpha_idx, flags, the rank of masked ones) and by grid cell.
 template <int NR>
 __global__ void __launch_bounds__(1024)
-list_condensates_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int *__restrict__ n_condensates,
+list_condensates_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, bool by_max_beta, int *__restrict__ n_condensates,
                         int *__restrict__ alpha_out, unsigned char *__restrict__ is_cond, int *__restrict__ assignment)
 {
     pdl_begin();
@@ -609,7 +617,7 @@ list_condensates_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, i
     const int e = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const CondGrid grid = make_cond_grid(b.layout.grid, b.max_radius, dims, cells_per_dim);
     const int n_cells = grid.n[0] * grid.n[1] * grid.n[2];
-    const bool by_grid = *b.use_grid != 0;
+    const bool by_grid = *b.use_grid != 0, by_cell = assigns_by_cell(n_cells, dims, by_max_beta);
     const int off = b.row_splits_h[e], n_h = b.row_splits_h[e + 1] - off;
     const int word0 = off / 32 + e;
     int *__restrict__ cell_start = b.cell_count + (size_t)e * (cells_cap + 1);
@@ -684,11 +692,29 @@ list_condensates_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, i
         is_cond[id] = 1;
         Rec<NR> x;
         const int cell = cell_at(a, &x);
-        if (cell >= 0) atomicAdd(cell_start + cell, 1);
-        else assignment[id] = r;  // a masked hit is assigned to itself: picked up by assign_hits_kernel
+        if (cell < 0) assignment[id] = r;  // a masked hit is assigned to itself: picked up by assign_hits_kernel
+        else if (by_cell) atomicAdd(cell_start + cell, 1);
     }
     __syncthreads();
     carry = 0;
+    if (!by_cell) {  // those that cover others, in priority order
+        for (int base = 0; base < n_cond; base += 1024) {
+            const int r = base + t;
+            Rec<NR> x;
+            const bool covers = r < n_cond && cell_at(b.cl.subset_pos[off + r], &x) >= 0;
+            const int incl = block_scan(covers ? 1 : 0);
+            if (covers) {
+                store_rec<NR>(b.c_rec + (size_t)(off + carry + incl - 1) * NR, x);
+                b.c_rank[off + carry + incl - 1] = r;
+            }
+            __syncthreads();
+            if (t == 1023) s_base = carry + incl;
+            __syncthreads();
+            carry = s_base;
+        }
+        if (t == 0) cell_start[0] = carry;
+        return;
+    }
     for (int base = 0; base <= n_cells; base += 1024) {
         const int c = base + t;
         const int n = c < n_cells ? __ldcg(cell_start + c) : 0;
@@ -712,6 +738,8 @@ list_condensates_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, i
 // Every hit against the condensates of the cells around it.  Of those that cover it the first in priority order wins
 // (by_max_beta), or the reference's distance fold is applied to them in priority order
 // (binned_assign_to_condensates_kernel.cc:80-125).  A masked hit is only ever assigned to itself.
+// Where the cells around a hit hold most condensates, the hits of a block walk all of them in priority order instead,
+// through shared memory (assigns_by_cell): one walk does the fold, and by beta the first that covers the hit ends it.
 template <int NR>
 __global__ void __launch_bounds__(kThreads)
 assign_hits_kernel(Buffers b, const float *__restrict__ ccoords, const int *__restrict__ mask, int dims, int n_events,
@@ -723,8 +751,48 @@ assign_hits_kernel(Buffers b, const float *__restrict__ ccoords, const int *__re
     HitTile t;
     if (!find_tile(b.layout, n_events, blockIdx.x / (b.layout.tile / kThreads), &t)) return;
     const int i = (blockIdx.x % (b.layout.tile / kThreads)) * kThreads + threadIdx.x;
-    if (i >= t.n) return;
     const CondGrid grid = make_cond_grid(b.layout.grid, b.max_radius, dims, cells_per_dim);
+    if (!assigns_by_cell(grid.n[0] * grid.n[1] * grid.n[2], dims, by_max_beta) && t.event < n_events) {
+        __shared__ float4 s_rec[kThreads][NR];
+        const int off = b.row_splits_h[t.event], first = n_condensates[t.event];
+        const int n_cover = b.cell_count[(size_t)t.event * (cells_cap + 1)];
+        const bool live = i < t.n;
+        const int v = t.first + i, m = live && mask ? mask[v] : 0;
+        int found = live && m > 0 && is_cond[v] ? assignment[v] : -1;  // its own rank
+        Rec<NR> x;
+#pragma unroll
+        for (int d = 0; d < NR * 4; d++) x.v[d] = 0.f;
+#pragma unroll
+        for (int d = 0; d < rec_dims<NR>(); d++)
+            if (live && d < dims) x.v[d] = __fsub_rn(ccoords[(size_t)v * dims + d], b.layout.grid->all_min[d]);
+        bool done = !live || m != 0;
+        float min_distance = 10e20f;
+        for (int c0 = 0; c0 < n_cover; c0 += kThreads) {
+            if (__syncthreads_and(done ? 1 : 0)) break;
+            if (c0 + (int)threadIdx.x < n_cover)
+#pragma unroll
+                for (int u = 0; u < NR; u++) s_rec[threadIdx.x][u] = b.c_rec[(size_t)(off + c0 + threadIdx.x) * NR + u];
+            __syncthreads();
+            const int here = min(kThreads, n_cover - c0);
+            for (int c = 0; c < here && !done; c++) {
+                const Rec<NR> r = load_rec<NR>(s_rec[c]);
+                const float dsq = rec_distsq<NR>(r, x, dims), r2 = r.v[rec_r2_slot<NR>()];
+                if (!(dsq <= r2)) continue;
+                if (by_max_beta || __fmul_rn(min_distance, r2) >= dsq) {
+                    found = c0 + c;
+                    min_distance = dsq;
+                    done = by_max_beta;
+                }
+            }
+        }
+        if (m == 0 && found >= 0) found = b.c_rank[off + found];
+        if (live) {
+            assignment[v] = found;
+            association[v] = found >= 0 ? alpha[first + found] : -1;
+        }
+        return;
+    }
+    if (i >= t.n) return;
     const bool real = t.event < n_events;
     const int off = real ? b.row_splits_h[t.event] : 0, first_alpha = real ? n_condensates[t.event] : 0;
     const int n_cond = real ? n_condensates[t.event + 1] - first_alpha : 0;
@@ -915,7 +983,7 @@ int run_claims(const Buffers &b, const Plan &p, int dims, int num_rows, int tile
     if (int rc = launch_claim_windows(dims, b.h_ccoords, b.h_dist, b.h_mask, b.h_orig, b.row_splits_h, b.order, b.status_h,
                                       b.alpha_h, b.stage, b.cl, num_rows, b.use_grid, stream))
         return rc;
-    HGC_CUDA_TRY(launch_pdl(list_condensates_kernel<NR>, num_rows, 1024, 0, stream, b, dims, p.cells, p.cells_per_dim, n_condensates, alpha_idx,
+    HGC_CUDA_TRY(launch_pdl(list_condensates_kernel<NR>, num_rows, 1024, 0, stream, b, dims, p.cells, p.cells_per_dim, by_max_beta, n_condensates, alpha_idx,
                                                                is_cond, assignment));
     HGC_LAUNCH_CHECK();
     HGC_CUDA_TRY(launch_pdl(assign_hits_kernel<NR>, tiles * (b.layout.tile / kThreads), kThreads, 0, stream, b, ccoords, mask, dims, num_rows, p.cells,
