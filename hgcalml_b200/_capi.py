@@ -200,19 +200,22 @@ def set_order(idx: torch.Tensor, order: torch.Tensor):
 
 
 def noted_order(idx):
-    """What set_order noted, for a later order_of with another view of the same table."""
+    """What set_order noted, for a backward pass, which sees another view of the table."""
     return _noted(idx, "_hgc_order", RowOrder)
 
 
-def order_of(idx, n: int, note=None):
-    note = noted_order(idx) if note is None else note
+def order_of(idx, n: int):
+    note = noted_order(idx)
     return None if note is None else note.get(idx, n)
 
 
 def row_order(order, idx, n: int):
-    """The processing order the caller names, else the one noted with the neighbour table, if any."""
+    """The processing order the caller names (backward passes name the note of the forward pass), else the one noted
+    with the neighbour table, if any."""
     if order is None:
         return order_of(idx, n)
+    if type(order) is RowOrder:
+        return order.get(idx, n)
     require_cuda(order)
     if order.numel() != n or order.device != idx.device:
         raise HgcError(f"order must be a permutation of the {n} hits on {idx.device}, not {order.numel()} entries on "

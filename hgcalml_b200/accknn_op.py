@@ -81,11 +81,9 @@ class _AccumulateLinKnnFunction(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, weights, features, indices, mean_and_max, order):
-        if order is not None:
-            order = C.row_order(order, indices, indices.shape[0])
         out, maxidx = AccumulateLinKnn(weights, features, indices, mean_and_max=mean_and_max, order=order)
         ctx.save_for_backward(weights, features, indices, maxidx)
-        ctx.order, ctx.noted = order, C.noted_order(indices)
+        ctx.order = C.noted_order(indices) if order is None else order
         ctx.lists = C.noted_lists(indices) if ctx.needs_input_grad[0] else None  # else no search comes after
         ctx.mark_non_differentiable(maxidx)
         ctx.set_materialize_grads(False)  # no zeros for the arg-max output
@@ -96,8 +94,7 @@ class _AccumulateLinKnnFunction(torch.autograd.Function):
         if grad_out is None:
             return None, None, None, None, None
         weights, features, indices, maxidx = ctx.saved_tensors
-        order = C.order_of(indices, indices.shape[0], ctx.noted) if ctx.order is None else ctx.order
-        gw, gf = AccumulateKnnGrad(grad_out, weights, features, indices, maxidx, order=order, _lists=ctx.lists)
+        gw, gf = AccumulateKnnGrad(grad_out, weights, features, indices, maxidx, order=ctx.order, _lists=ctx.lists)
         return gw, gf, None, None, None
 
 

@@ -107,7 +107,7 @@ class _BinnedSelectKnnFunction(torch.autograd.Function):
         if grad_dist is None:
             return None, None, None, None, None, None
         coords, idx, dist = ctx.saved_tensors
-        return SelectKnnGrad(grad_dist, idx, dist, coords, order=C.order_of(idx, idx.shape[0], ctx.order),
+        return SelectKnnGrad(grad_dist, idx, dist, coords, order=ctx.order,
                              _lists=ctx.lists), None, None, None, None, None
 
 

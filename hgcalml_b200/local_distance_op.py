@@ -27,7 +27,7 @@ class _LocalDistanceFunction(torch.autograd.Function):
     def backward(ctx, grad_dist):
         coords, idx, dist = ctx.saved_tensors
         # the reference registers SelectKnnGrad as the gradient (modules/local_distance_op.py:27-40)
-        return SelectKnnGrad(grad_dist, idx, dist, coords, order=C.order_of(idx, idx.shape[0], ctx.order)), None
+        return SelectKnnGrad(grad_dist, idx, dist, coords, order=ctx.order), None
 
 
 def LocalDistance(coords, neighbour_idxs):

@@ -47,7 +47,7 @@ class _PushKnnFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad):
         w, f, nidx = ctx.saved_tensors
-        wg, fg = PushKnnGrad(grad, w, f, nidx, order=C.order_of(nidx, nidx.shape[0], ctx.order))
+        wg, fg = PushKnnGrad(grad, w, f, nidx, order=ctx.order)
         return wg, fg, None
 
 

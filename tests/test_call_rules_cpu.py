@@ -23,7 +23,7 @@ def test_a_noted_order_that_was_written_to_is_not_used():
     assert C.order_of(idx, 50) is order
     order += 1000
     assert C.order_of(idx, 50) is None
-    assert C.order_of(idx, 50, note) is None  # as a backward pass asks
+    assert C.row_order(note, idx, 50) is None  # as a backward pass asks
 
 
 def test_a_table_with_notes_can_be_saved_and_copied():
