@@ -32,12 +32,14 @@ sys.path.insert(0, ROOT)
 
 METRIC = "hits/sec for BinnedSelectKnn+AccumulateKnn at 200k-hit events"
 UNIT = "hits/s"
-# Counters of the two main kernels at K = F = 64, 4 coordinates, from one ncu capture of a 400k-hit
-# launch each (the DRAM traffic grows in proportion to the hits); this is their only copy.
+# Counters at K = F = 64, 4 coordinates, from ncu captures of 400k-hit launches (profiles/neighbour_path_400k.md; of the
+# op-level search profiles/op_level_search_400k.md).  DRAM traffic and instructions grow in proportion to the hits.
+# "binned_select_knn": all eight kernels of a call; its issue share is that of select_knn_tile_kernel, 94 % of them.
 NCU = {
-    "accumulate_knn": {"dram_bytes_per_hit": 1782, "algorithmic_bytes_per_hit": 1536},
-    "accumulate_knn_no_argmax": {"dram_bytes_per_hit": 1314, "algorithmic_bytes_per_hit": 1280},
-    "select_knn": {"dram_bytes_per_hit": 433, "issue_active_pct": 90.4, "warp_instructions_per_query": 5715},
+    "accumulate_knn": {"dram_bytes_per_hit": 1755, "algorithmic_bytes_per_hit": 1536},
+    "accumulate_knn_no_argmax": {"dram_bytes_per_hit": 1296, "algorithmic_bytes_per_hit": 1280},
+    "binned_select_knn": {"dram_bytes_per_hit": 530, "issue_active_pct": 73.7, "warp_instructions_per_query": 2110},
+    "select_knn_op_level": {"dram_bytes_per_hit": 433, "issue_active_pct": 90.4, "warp_instructions_per_query": 5715},
 }
 
 
@@ -357,22 +359,31 @@ def main():
             acc_na = dict(hbm(kt["accumulate_no_argmax_ms"], 8 * K + 12 * F,
                               NCU["accumulate_knn_no_argmax"]["dram_bytes_per_hit"]),
                           kernel="accumulate kernel, [mean | max] only (what the host-buffer entry runs)")
-            knn_hbm = hbm(kt["select_knn_ms"], 4 * 4 + 4 + 4 * 4 + 8 * K, NCU["select_knn"]["dram_bytes_per_hit"])
-            # The search is bound by instruction issue, not by memory: its roofline is the warp
-            # instructions it needs per query (ncu) against the issue slots of the SMs at the clock
-            # sampled during the run; the HBM view is kept beside it.
-            instr = NCU["select_knn"]["warp_instructions_per_query"]
+            # The search is bound by instruction issue and gathers that miss L1, not by memory: its roofline is the
+            # warp instructions it needs per query (ncu) against the issue slots of the SMs at the clock sampled
+            # during the run; the HBM view is kept beside it.
             issue_peak = sms * 4 * sm_mhz * 1e6 / 1e9
-            issue_ach = n * instr / (kt["select_knn_ms"] * 1e-3) / 1e9 if full else None
-            knn = {"kernel": "select_knn_kernel", "bound": "issue", "achieved": issue_ach, "peak": issue_peak,
-                   "unit": "G warp-instructions/s", "frac": issue_ach / issue_peak if full else None,
-                   "ms_per_launch": kt["select_knn_ms"],
-                   "ncu_issue_active_pct": NCU["select_knn"]["issue_active_pct"] if full else None,
-                   "ncu_warp_instructions_per_query": instr if full else None,
-                   "traffic": knn_hbm["traffic"], "hbm": knn_hbm}
-            dominant = knn if kt["select_knn_ms"] >= kt["accumulate_ms"] else acc
+
+            def issue(kernel, key, ms_, bytes_per_hit):
+                instr = NCU[key]["warp_instructions_per_query"]
+                ach = n * instr / (ms_ * 1e-3) / 1e9 if full else None
+                view = hbm(ms_, bytes_per_hit, NCU[key]["dram_bytes_per_hit"])
+                return {"kernel": kernel, "bound": "issue", "achieved": ach, "peak": issue_peak,
+                        "unit": "G warp-instructions/s", "frac": ach / issue_peak if full else None,
+                        "ms_per_launch": ms_, "ncu_issue_active_pct": NCU[key]["issue_active_pct"] if full else None,
+                        "ncu_warp_instructions_per_query": instr if full else None, "traffic": view["traffic"],
+                        "hbm": view}
+
+            # what a step runs: one BinnedSelectKnn call, timed as a whole
+            knn = issue("select_knn_tile_kernel, with the two orders and the packing before it (one BinnedSelectKnn "
+                        "call)", "binned_select_knn", kt["binned_select_knn_wrapper_ms"], 4 * 4 + 4 + 8 * K)
+            # the op-level entry, whose callers bring their own bins: not part of a step
+            op_level = issue("select_knn_kernel (op-level entry, not part of a step)", "select_knn_op_level",
+                             kt["select_knn_ms"], 4 * 4 + 4 + 4 * 4 + 8 * K)
+            dominant = knn if kt["binned_select_knn_wrapper_ms"] >= kt["accumulate_ms"] else acc
             line["roofline"] = dominant
-            line["roofline_kernels"] = {"select_knn": knn, "accumulate_knn": acc, "accumulate_knn_no_argmax": acc_na}
+            line["roofline_kernels"] = {"binned_select_knn": knn, "accumulate_knn": acc,
+                                        "accumulate_knn_no_argmax": acc_na, "select_knn_op_level": op_level}
             line["stage_ms"] = kt
             if "single_event" in extra:
                 line["single_event"] = extra["single_event"]
@@ -387,9 +398,9 @@ def main():
 
 
 def measure_kernels(torch, dev, coords, feats, rs, K, F, reps=3):
-    """Per-launch durations of the two main kernels with CUDA events on the launching stream:
-    AccumulateKnn is a single kernel; the search kernel is timed through the op-level entry on
-    bin-sorted inputs (its only other launches are the small packing and bounding-box kernels)."""
+    """Durations of the two calls of a step with CUDA events on the launching stream (AccumulateKnn is a single kernel),
+    and of the op-level search on bin-sorted inputs, which is not part of a step (its only other launches are the
+    small packing and bounding-box kernels)."""
     from hgcalml_b200.binned_select_knn_op import BinnedSelectKnn, _BinnedSelectKnn
     from hgcalml_b200.accknn_op import AccumulateKnn
     from hgcalml_b200.bin_by_coordinates_op import BinByCoordinates

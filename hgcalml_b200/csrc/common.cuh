@@ -50,10 +50,16 @@ int sm_count();
 // Launches a kernel that may start while the kernel before it in the stream is still finishing: its blocks become resident
 // and wait in pdl_begin(), which takes about a microsecond off every step from one kernel to the next.  Every kernel
 // launched this way begins with pdl_begin(), in all of its blocks, so that "the kernel before has completed" holds
-// through any chain of them.  700 hits: 75 -> 56 us a call, 20k 131 -> 105 us.
-// launch_overlapped does so up to kOverlapHits hits: blocks that become resident early take room from the kernel that is
-// still running and inherit its split between L1 and shared memory, which costs more than it gains where kernels are
-// long (400k hits: sort passes overlapped 1824 us a call, not overlapped 1788 us).
+// through any chain of them.
+// Kernels that are short at every size are always launched so: the condensate path, keep_noise, the epilogues of dense
+// layers, LocalDistance, the op-level sorts (4 x 200k hits condensed 460 -> 440 us, 100k 285 -> 266; two GravNet layers
+// with message passing on 200k hits 2864 -> 2848).
+// launch_overlapped is for the kernels whose length grows with the batch (search, orders, accumulation, backward ops): up to
+// kOverlapHits hits.  Blocks that become resident early take room from the kernel that is still running and inherit its
+// split between L1 and shared memory.  Search and accumulation, K = 16, F = 32, in us, not overlapped / overlapped: 20k hits
+// 154/135, 40k 196/185, 64k 254/239, 70k 274/280, 100k 340/325, 150k 453/457, 200k 595/590, 300k 760/787, 400k 918/946;
+// K = F = 64: 20k 195/184, 64k 455/449, 70k 480/487, 100k 625/623, 150k 882/893, 400k 1729/1776; a training step on 200k
+// hits 3390/3496.  Between 65k and 200k hits neither is always better; the line lies where the gain ends.
 template <typename... Params, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args &&...args)
 {
