@@ -26,8 +26,7 @@
 // bins).  64 events of 200k hits, K = 64, 4 coordinates: 68.0 -> 32.5 ms; 200k hits with coordinates N(0,1)-like in four
 // dimensions: 1.77 -> 0.88 ms.  5.7k -> 2.0k warp instructions per query: 18 chunk visits instead of 36 candidate steps,
 // one word sort instead of seven merges of 64-bit keys, and what finds the chunks is shared by a tile.
-// The kernel is bound by the latency of gathers that miss L1 (64 % hit) and by issue (74 % of the slots) together
-// (profiles/neighbour_path_400k.md).
+// The kernel is bound by the latency of gathers that miss L1 (64 % hit) and by issue (74 % of the slots) together.
 // It is therefore sensitive to everything that takes L1 away: spilled registers (a 144-byte frame: +35 %), shared
 // memory, more resident blocks (10 instead of 9 per SM: +7 %).  What depends on the tile only is kept in
 // shared memory rather than in registers for that reason.
