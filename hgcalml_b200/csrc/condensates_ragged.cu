@@ -428,6 +428,7 @@ claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max
     const int rank = (int)cluster.block_rank();
     const int g = rank * kClaimThreads + t;
     const int off = b.row_splits_h[e], n_h = b.row_splits_h[e + 1] - off;
+    if (n_h == 0) return;  // all blocks of the cluster
     const int n_steps = (n_h + kStep - 1) / kStep;
     const int word0 = off / 32 + e;
     const float4 *__restrict__ recs = b.p_rec + (size_t)off * NR;
@@ -465,7 +466,7 @@ claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max
     auto flat = [&grid](int at) { return (((at >> 16) & 127) * grid.n[1] + ((at >> 8) & 255)) * grid.n[2] + (at & 255); };
     const int slice = (n_cells + CB - 1) / CB;
 
-    for (int round = 0; round <= n_h; round++) {
+    for (int round = 0;; round++) {
         // first open hit of every cell, among this block's
         for (int w = 0; w * 32 < n_steps; w++) {
             unsigned u = w == 0 ? open0 : open_words[(size_t)w * kStep];
@@ -491,7 +492,9 @@ claim_grid_kernel(Buffers b, int dims, int cells_cap, int cells_per_dim, int max
             int total = 0;
 #pragma unroll
             for (int r = 0; r < CB; r++) total += s_left[(round - 1) & 1][r];
-            if (total == 0) break;  // the same in every block of the cluster; nobody looks at another block from here on
+            // the same in every block of the cluster, and nobody looks at another block from here on: a block that leaves
+            // while others may still write to its shared memory faults them.  (A round settles a hit at least.)
+            if (total == 0 || round > n_h) break;
         }
         // merged, for all blocks
         for (int c = rank * slice + t; c < min((rank + 1) * slice, n_cells); c += kClaimThreads) {

@@ -102,3 +102,13 @@ def test_a_block_per_event(cuda, oracle, dims):
     beta[:] = rng.uniform(0.05, 1., beta.shape)  # nearly all are high
     mask = rng.choice([0] * 30 + [1, -1], beta.shape).astype(np.int32)
     _check(cuda, oracle, cc, beta, np.full_like(beta, 0.5), rs, mask=mask, modes=(True,))
+
+
+@pytest.mark.parametrize("n_events", [1, 4, 18, 19])
+def test_events_without_high_hits(cuda, oracle, n_events):
+    """Nothing to settle: the blocks of an event's cluster must still leave together."""
+    cc, beta, rs, rng = _batch([300] * n_events, 3, 37)
+    beta *= 0.05
+    beta[:300:100] = 0.9 if n_events > 1 else 0.  # the first of several events has some
+    for _ in range(20):
+        _check(cuda, oracle, cc, beta, np.full_like(beta, 0.2), rs, thr=0.3, modes=(True,))
