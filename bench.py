@@ -32,7 +32,8 @@ sys.path.insert(0, ROOT)
 
 METRIC = "hits/sec for BinnedSelectKnn+AccumulateKnn at 200k-hit events"
 UNIT = "hits/s"
-# Counters at K = F = 64, 4 coordinates, from ncu captures of 400k-hit launches (summaries in profiles/).  DRAM traffic and instructions grow in proportion to the hits.
+# Counters at K = F = 64, 4 coordinates, from ncu captures of 400k-hit launches (summaries in profiles/).  DRAM
+# traffic and instructions grow in proportion to the hits.
 # "binned_select_knn": all eight kernels of a call; its issue share is that of select_knn_tile_kernel, 94 % of them.
 NCU = {
     "accumulate_knn": {"dram_bytes_per_hit": 1755, "algorithmic_bytes_per_hit": 1536},

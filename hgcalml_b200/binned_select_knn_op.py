@@ -60,8 +60,11 @@ def BinnedSelectKnn(K: int, coords, row_splits, direction=None, n_bins=None, max
     del max_radius, name
     C.require_cuda(coords, row_splits, direction)
     coords, row_splits = C.f32(coords), C.i32(row_splits)
+    n, _ = coords.shape
     if direction is not None:
         direction = C.i32(direction)
+        if direction.numel() < n:
+            raise C.HgcError("BinnedSelectKnn needs a direction tensor with length nvert.")
     C.check_device(coords)
     idx, dist, sorting, rc = C.native.select_knn(coords, row_splits, direction, K, -1 if n_bins is None else int(n_bins),
                                                  int(max_bin_dims), bool(tf_compatible))
@@ -81,8 +84,9 @@ def SelectKnnGrad(grad_distances, indices, distances, coordinates, order=None, _
     C.require_cuda(grad_distances, indices, coordinates)
     g, idx, coords = C.f32(grad_distances), C.i32(indices), C.f32(coordinates)
     del distances  # an input of the op that is never read
+    n, _ = idx.shape
     C.check_device(coords)
-    order = C.row_order(order, indices, idx.shape[0])
+    order = C.row_order(order, indices, n)
     out, rc = C.native.select_knn_grad(g, idx, coords, order, None if _lists is None else _lists.take())
     C.check(rc, "SelectKnnGrad")
     return out

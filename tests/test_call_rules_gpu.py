@@ -138,3 +138,19 @@ def test_kept_noise_needs_events_that_are_all_hits(cuda, splits):
     rs, dist = torch.tensor(splits, dtype=torch.int32, device=cuda), torch.full((900, 1), .1, device=cuda)
     with pytest.raises(C.HgcError):
         BuildAndAssignCondensatesBinned(x, beta, dist, rs, .9, assign_by_max_beta=True, keep_noise=True)
+
+
+def test_tensors_of_more_dimensions_are_refused(cuda):
+    from hgcalml_b200 import _capi as C
+    from hgcalml_b200.accknn_op import AccumulateKnn, AccumulateKnnGrad
+    from hgcalml_b200.binned_select_knn_op import BinnedSelectKnn, SelectKnnGrad
+    from hgcalml_b200.push_knn_op import PushKnn, PushKnnGrad
+    c, rs = torch.rand((40, 3), device=cuda), torch.tensor([0, 40], dtype=torch.int32, device=cuda)
+    idx, d2 = BinnedSelectKnn(5, c, rs)
+    x = torch.randn((40, 4), device=cuda)
+    for call in (lambda: BinnedSelectKnn(5, c[:, :, None].repeat(1, 1, 2), rs), lambda: BinnedSelectKnn(5, c[:, 0], rs),
+                 lambda: BinnedSelectKnn(5, c, rs, direction=rs), lambda: SelectKnnGrad(d2, idx[:, :, None], None, c),
+                 lambda: AccumulateKnn(d2, x, idx[:, :, None]), lambda: PushKnn(d2, x, idx[:, :, None]),
+                 lambda: AccumulateKnnGrad(x, d2, x, idx[:, :, None], None), lambda: PushKnnGrad(x, d2, x, idx[:, :, None])):
+        with pytest.raises((C.HgcError, ValueError, IndexError, RuntimeError)):
+            call()
