@@ -165,7 +165,7 @@ int hgc_index_replacer(
  * maximum wins, accumulate_knn_kernel.cc:65).  Two corners differ from the CPU loop: a NaN product
  * is ignored by the maximum (the CPU op keeps one that sits in slot 0), and when the maximum is a
  * zero reached by products of both signs its sign bit may differ (+0 here, the later product's
- * there); neither occurs with finite, non-negative weights and features without NaN and -0.
+ * there; weights that underflow to 0 give such products).
  * Without d_out_maxidxs the arg-max bookkeeping is not run at all (about a third faster).
  * ------------------------------------------------------------------------------------- */
 int hgc_accumulate_knn(
