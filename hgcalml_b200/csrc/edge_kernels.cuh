@@ -1,103 +1,184 @@
 // Kernels over the edges of a neighbour table that the backward ops and PushKnn have in common.
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace hgc {
 
+// (ax * bx, ay * by), rounded one by one.  Sums stay with __fadd_rn: ptxas contracts a packed addition of a packed product
+// to a fused one although both ask for rounding.
+__device__ __forceinline__ float2 mul2(float ax, float ay, float bx, float by)
+{
+    float2 r;
+    asm("{ .reg .b64 ra, rb, rr; mov.b64 ra, {%2,%3}; mov.b64 rb, {%4,%5}; mul.rn.f32x2 rr, ra, rb; mov.b64 {%0,%1}, rr; }"
+        : "=f"(r.x), "=f"(r.y) : "f"(ax), "f"(ay), "f"(bx), "f"(by));
+    return r;
+}
 enum EdgeSum {
     kSumPlain,    // x[i,f] * w[e]
     kSumMean,     // (x[i,f] / K) * w[e]
     kSumMeanMax   // the same plus, where the target is the maximum of (i, f), x[i,F+f] * w[e]
 };
 
-// out[m,f] = sum over the edges e = (i, slot) that point at m, in ascending order.  One warp per target, lanes over
-// a slab of up to 32 * FPL features starting at f0.  Every lane fetches one edge with its weight and flags, then
-// the warp walks the 32 edges, the rows of 8 of them in flight.  The terms are added one by one, in edge
-// order.  Which features of a source have the target as their maximum comes as bits (arg_flags_kernel): reading
-// the arg-max row of every edge instead doubled the gathered bytes.
-// 12.8 M edges, F = 64, hits in the search's order: 0.91 ms.  Half of the gathered lines miss L1, and the registers of 8 rows
-// in flight leave 24 warps per SM to hide that; 60 % of the issue slots.
-// POW2: K is a power of two, so that the division is an exact scaling.
-template <int FPL, int MODE, bool POW2>
-__global__ void __launch_bounds__(256)
-edge_sum_kernel(const float *__restrict__ x, int ldx, const float *__restrict__ weights,
-                const unsigned *__restrict__ flags, const int *__restrict__ nidx, const int *__restrict__ bounds,
-                const int *__restrict__ edges, float *__restrict__ out, int n_vert, int K, int F, int f0,
-                const int *__restrict__ order)
+template <int VW> struct EdgeVec { float v[VW]; };
+template <int VW>
+__device__ __forceinline__ EdgeVec<VW> load_edge_vec(const float *p)
+{
+    EdgeVec<VW> r;
+    if constexpr (VW == 4) {
+        const float4 q = __ldg(reinterpret_cast<const float4 *>(p));
+        r.v[0] = q.x; r.v[1] = q.y; r.v[2] = q.z; r.v[3] = q.w;
+    } else {
+        static_assert(VW == 2, "vectors of two or four");
+        const float2 q = __ldg(reinterpret_cast<const float2 *>(p));
+        r.v[0] = q.x; r.v[1] = q.y;
+    }
+    return r;
+}
+
+// The same if any bit of `wanted` is set; otherwise, and (not WHOLE) in places whose bit is not set, the values do not count.
+template <int VW, bool WHOLE>
+__device__ __forceinline__ EdgeVec<VW> load_edge_vec_if(const float *p, unsigned wanted)
+{
+    EdgeVec<VW> r;
+#pragma unroll
+    for (int v = 0; v < VW; v++) r.v[v] = 0.f;
+    if constexpr (WHOLE && VW == 4) {
+        asm volatile("{ .reg .pred q; setp.ne.u32 q, %5, 0; @q ld.global.nc.v4.f32 {%0,%1,%2,%3}, [%4]; }"
+                     : "+f"(r.v[0]), "+f"(r.v[1]), "+f"(r.v[2]), "+f"(r.v[3]) : "l"(p), "r"(wanted));
+    } else {
+#pragma unroll
+        for (int v = 0; v < VW; v++)
+            if ((wanted >> v) & 1u) r.v[v] = __ldg(p + v);
+    }
+    return r;
+}
+
+// out[m,f] = sum over the edges e = (i, slot) that point at m, in ascending order, for the features f0 .. f0 + LPT * VW - 1.
+// LPT lanes work on one target, VW neighbouring features each; a warp has 32 / LPT targets.  Every lane fetches one edge with
+// its weight and flags and puts them into shared memory, from where all lanes read them with one broadcast load per edge
+// (four shuffles before); the rows of two edges are in flight.  The terms are added one by one, in edge order.
+// Rows lie `ldr` floats apart in `rows`, whole vectors in every row; SCALE multiplies them with 1 / K.  In the mode kSumMeanMax
+// `maxima` (rows `ldm` floats apart, HVEC: whole vectors) holds what goes to the maximum alone.  Which features of a source
+// have the target as their maximum comes as bits (arg_flags_kernel): reading the arg-max row of every edge instead doubled
+// the gathered bytes.
+// 12.8 M edges, F = 64, hits in the search's order: 0.57 ms; a warp per target with 4-byte loads and 8 rows in flight took
+// 0.91, its 77 registers leaving 24 warps per SM.  Half of the gathered lines miss L1 and resident warps hide that better than
+// rows in flight: 16 lanes x 4 features with 2 rows and 40 warps per SM beat 4 rows (+1 %), 8 rows (+20 %), a warp x 2 features
+// (+10 %), and 64 warps, which spill (+27 %).  PushKnn, 200k hits, K = 40, F = 32: 433 -> 341 us.
+template <int LPT, int VW, int MODE, bool SCALE, bool HVEC>
+__global__ void __launch_bounds__(256, 5)
+edge_sum_kernel(const float *__restrict__ rows, int ldr, const float *__restrict__ maxima, int ldm,
+                const float *__restrict__ weights, const unsigned *__restrict__ flags, const int *__restrict__ nidx,
+                const int *__restrict__ bounds, const int *__restrict__ edges, float *__restrict__ out, int n_vert, int K, int F,
+                int f0, const int *__restrict__ order)
 {
     pdl_begin();
-    constexpr int U = 8;
-    const int lane = threadIdx.x & 31;
-    const int slot = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (slot >= n_vert) return;
-    const int m = order ? order[slot] : slot;  // processing order only: every target is visited once
-    const int begin = bounds[m], end = bounds[m + 1];
-    const float kf = (float)K, inv = 1.f / kf;
-    float acc[FPL];
-    bool mine[FPL];
-#pragma unroll
-    for (int u = 0; u < FPL; u++) {
-        acc[u] = 0.f;
-        mine[u] = f0 + u * 32 + lane < F;
+    constexpr int T = 32 / LPT;  // targets of a warp
+    __shared__ uint4 s_edge[8][32];  // source, weight, flags
+    const int lane = threadIdx.x & 31, hl = lane & (LPT - 1);
+    uint4 *__restrict__ mine = s_edge[threadIdx.x >> 5] + (lane & ~(LPT - 1));
+    const int slot = (blockIdx.x * 8 + (threadIdx.x >> 5)) * T + lane / LPT;
+    int m = 0, begin = 0, end = 0;
+    if (slot < n_vert) {
+        m = order ? order[slot] : slot;  // processing order only: every target is visited once
+        begin = bounds[m];
+        end = bounds[m + 1];
     }
-    const float *__restrict__ xl = x + f0 + lane;
-    for (int p = begin; p < end; p += 32) {
-        const int e = p + lane < end ? edges[p + lane] : 0;
-        const int my_i = e / K;
-        float my_w = 0.f;
-        unsigned my_flag[FPL];
+    const float inv = 1.f / (float)K;
+    const int f = hl * VW;
+    const bool have = f0 + f < F;
+    const float *__restrict__ row0 = rows + (have ? f : 0);
+    const float *__restrict__ max0 = MODE == kSumMeanMax ? maxima + (have ? f : 0) : nullptr;
+    const unsigned flag_mask = f0 + f + VW <= F ? (1u << VW) - 1u : (1u << (have ? F - f0 - f : 0)) - 1u;
+    float acc[VW];
 #pragma unroll
-        for (int u = 0; u < FPL; u++) my_flag[u] = 0u;
-        if (p + lane < end) {
-            my_w = weights[e];
+    for (int v = 0; v < VW; v++) acc[v] = 0.f;
+    for (int p = begin; __any_sync(0xffffffffu, p < end); p += LPT) {
+        const int n_here = min(LPT, end - p);  // may be below zero where another target's list is longer
+        __syncwarp();
+        if (hl < n_here) {
+            const int e = edges[p + hl], i = e / K;
+            uint4 ed = make_uint4((unsigned)i, __float_as_uint(weights[e]), 0u, 0u);
             if (MODE == kSumMeanMax) {
                 bool counts = true;
-                if (my_i == m) {
+                if (i == m) {
                     // the hit is its own neighbour: only its first occurrence in the row counts for the maximum
-                    for (int k = e - my_i * K - 1; k >= 0; k--) counts = counts && nidx[(size_t)my_i * K + k] != m;
+                    for (int k = e - i * K - 1; k >= 0; k--) counts = counts && nidx[(size_t)i * K + k] != m;
                 }
                 if (counts) {
                     const uint2 b = *reinterpret_cast<const uint2 *>(flags + 2 * (size_t)e);
-                    my_flag[0] = b.x;
-                    if (FPL > 1) my_flag[FPL - 1] = b.y;
+                    ed.z = b.x;
+                    ed.w = b.y;
                 }
             }
+            mine[hl] = ed;
         }
-        const int n_here = min(32, end - p);
-        for (int q0 = 0; q0 < n_here; q0 += U) {
-            float g[U][FPL], h[U][FPL], w[U];
+        __syncwarp();
+        // two rows at a time; while every target of the warp has two more edges, without a test per target
+        auto two = [&](int q0, auto tail) {
+            EdgeVec<VW> g[2], h[2];
+            float w[2];
+            unsigned b[2];
 #pragma unroll
-            for (int q = 0; q < U; q++) {
-                // beyond the last edge: i = 0 with weight 0, not added below
-                const int i = __shfl_sync(0xffffffffu, my_i, (q0 + q) & 31);
-                w[q] = __shfl_sync(0xffffffffu, my_w, (q0 + q) & 31);
-                const float *row = xl + (size_t)i * ldx;
-#pragma unroll
-                for (int u = 0; u < FPL; u++) {
-                    g[q][u] = mine[u] ? __ldg(row + u * 32) : 0.f;
-                    h[q][u] = 0.f;
+            for (int q = 0; q < 2; q++) {
+                const uint4 ed = mine[q0 + q];
+                w[q] = __uint_as_float(ed.y);
+                b[q] = 0u;
+                if (!tail.value || q0 + q < n_here) {
+                    g[q] = load_edge_vec<VW>(row0 + (size_t)ed.x * ldr);
                     if (MODE == kSumMeanMax) {
-                        const unsigned b = __shfl_sync(0xffffffffu, my_flag[u], (q0 + q) & 31);
-                        if ((b >> lane) & 1u) h[q][u] = __ldg(row + F + u * 32);
+                        b[q] = ((LPT * VW > 32 && f >= 32 ? ed.w : ed.z) >> (f & 31)) & flag_mask;
+                        h[q] = load_edge_vec_if<VW, HVEC>(max0 + (size_t)ed.x * ldm, b[q]);
                     }
                 }
             }
 #pragma unroll
-            for (int q = 0; q < U; q++) {
-                if (q0 + q >= n_here) break;  // uniform
+            for (int q = 0; q < 2; q++) {
+                if (!tail.value || q0 + q < n_here) {
+                    float t[VW];
 #pragma unroll
-                for (int u = 0; u < FPL; u++) {
-                    float t = MODE == kSumPlain ? g[q][u] : POW2 ? __fmul_rn(g[q][u], inv) : __fdiv_rn(g[q][u], kf);
-                    t = __fmul_rn(t, w[q]);
-                    if (MODE == kSumMeanMax && h[q][u] != 0.f) t = __fadd_rn(t, __fmul_rn(h[q][u], w[q]));
-                    acc[u] = __fadd_rn(acc[u], t);
+                    for (int v = 0; v < VW; v += 2) {
+                        float2 r = make_float2(g[q].v[v], g[q].v[v + 1]);
+                        if (SCALE) r = mul2(r.x, r.y, inv, inv);
+                        r = mul2(r.x, r.y, w[q], w[q]);
+                        t[v] = r.x;
+                        t[v + 1] = r.y;
+                        if (MODE == kSumMeanMax) {
+                            r = mul2(h[q].v[v], h[q].v[v + 1], w[q], w[q]);
+                            if (b[q] & (1u << v)) t[v] = __fadd_rn(t[v], r.x);
+                            if (b[q] & (2u << v)) t[v + 1] = __fadd_rn(t[v + 1], r.y);
+                        }
+                    }
+#pragma unroll
+                    for (int v = 0; v < VW; v++) acc[v] = __fadd_rn(acc[v], t[v]);
                 }
             }
-        }
+        };
+        const int n_all = T == 1 ? n_here : max(0, __reduce_min_sync(0xffffffffu, n_here));
+        const int n_max = T == 1 ? n_here : __reduce_max_sync(0xffffffffu, n_here);
+        int q0 = 0;
+        for (; q0 + 2 <= n_all; q0 += 2) two(q0, std::false_type());
+        for (; q0 < n_max; q0 += 2) two(q0, std::true_type());
     }
+    if (have && slot < n_vert) {
+        float *dst = out + (size_t)m * F + f0 + f;
 #pragma unroll
-    for (int u = 0; u < FPL; u++)
-        if (mine[u]) out[(size_t)m * F + f0 + u * 32 + lane] = acc[u];
+        for (int v = 0; v < VW; v++)
+            if (f0 + f + v < F) dst[v] = acc[v];
+    }
+}
+
+// dst[i, 0 .. ld - 1] = x[i, 0 .. n - 1] / k, zeros behind: rows of whole vectors for edge_sum_kernel.  k == 1 copies.
+// Dividing every row once instead of once per edge: both gradients of 200k hits, K = 40, F = 32 918 -> 718 us.
+static __global__ void __launch_bounds__(256)
+edge_rows_kernel(const float *__restrict__ x, int ldx, int n, float k, float *__restrict__ dst, int ld, int n_vert)
+{
+    pdl_begin();
+    const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
+    const int i = (int)(t / ld), f = (int)(t - (long long)i * ld);
+    if (i < n_vert) dst[t] = f < n ? __fdiv_rn(x[(size_t)i * ldx + f], k) : 0.f;
 }
 
 // flags[e][2]: for every edge e = (i, slot) with target m, the features f0 .. f0 + 63 of hit i whose arg-max is m.
@@ -133,14 +214,16 @@ arg_flags_kernel(const int *__restrict__ arg, const int *__restrict__ nidx, unsi
 // through the features one by one; the rows of the warp's 32 neighbours are read coalesced, 32 features at
 // a time, into shared memory, from where every lane reads its own (rows 36 floats apart: no bank conflicts).
 // A lane reading its row from global memory directly touched 32 lines with every load.
-// 12.8 M edges, F = 64: 0.84 ms, bound by issue (80 % of the slots) and the L1 data stage (79 %): 32 loads, shuffles and
-// shared-memory stores per warp and 32 features.
+// VEC: rows are whole 16-byte vectors (F % 4 == 0, bases aligned), which cp.async puts into shared memory past the registers
+// and L1.  12.8 M edges, F = 64: 0.85 ms with 4-byte loads and stores and a test of every feature for the maximum, bound by
+// issue (80 % of the slots) and the L1 data stage (79 %); 0.62 with 16-byte loads and stores, packed products and the
+// maxima taken from the bits; 0.51 with cp.async (cached in L1 as well 0.53; MAX without the bound on registers 0.56).
 // MAX also writes the edge's bits for edge_sum_kernel (features 0 .. 63), which it compares for anyway.
-template <bool GRAD, bool MAX>
-__global__ void __launch_bounds__(256)
+template <bool GRAD, bool MAX, bool VEC>
+__global__ void __launch_bounds__(256, MAX ? 5 : 6)
 edge_dot_kernel(const float *__restrict__ own, int ld_own, const float *__restrict__ x, const int *__restrict__ arg,
                 const int *__restrict__ nidx, float *__restrict__ out, long long n_edges, int n_vert, int K, int F,
-                bool vec4, const int *__restrict__ order, unsigned *__restrict__ flags)
+                const int *__restrict__ order, unsigned *__restrict__ flags)
 {
     pdl_begin();
     constexpr int kRow = 36;
@@ -153,7 +236,7 @@ edge_dot_kernel(const float *__restrict__ own, int ld_own, const float *__restri
     int i = 0, m = -1;
     long long e = 0;
     if (t < n_edges) {
-        const int row = (int)(t / K);
+        const int row = n_edges <= 0xffffffffLL ? (int)((unsigned)t / (unsigned)K) : (int)(t / K);
         i = order ? order[row] : row;  // processing order only
         e = (long long)i * K + (t - (long long)row * K);
         m = nidx[e];
@@ -161,16 +244,31 @@ edge_dot_kernel(const float *__restrict__ own, int ld_own, const float *__restri
     }
     const float *__restrict__ g = own + (size_t)i * ld_own;
     const int *__restrict__ am = MAX ? arg + (size_t)i * F : nullptr;
+    const int arg_m = m >= 0 ? m : (int)0x80000000;  // no neighbour is nobody's maximum
     float mean_part = 0.f, max_part = 0.f;
     uint2 bits = make_uint2(0u, 0u);
     for (int f0 = 0; f0 < F; f0 += 32) {
         unsigned hit = 0u;
         __syncwarp();
-        const bool in = f0 + lane < F;
+        if (VEC) {
+            const int c = (lane & 7) * 4;
+            const bool in = f0 + c < F;
+#pragma unroll
+            for (int q = 0; q < 32; q += 4) {
+                const int mq = __shfl_sync(0xffffffffu, m, q + (lane >> 3));
+                const int bytes = in && mq >= 0 ? 16 : 0;  // the rest of the 16 bytes is filled with zeros
+                const unsigned dst = (unsigned)__cvta_generic_to_shared(s + (q + (lane >> 3)) * kRow + c);
+                const float *src = x + (bytes ? (size_t)mq * F + f0 + c : 0);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(bytes) : "memory");
+            }
+            asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+        } else {
+            const bool in = f0 + lane < F;
 #pragma unroll 8
-        for (int q = 0; q < 32; q++) {
-            const int mq = __shfl_sync(0xffffffffu, m, q);
-            s[q * kRow + lane] = in && mq >= 0 ? __ldg(x + (size_t)mq * F + f0 + lane) : 0.f;
+            for (int q = 0; q < 32; q++) {
+                const int mq = __shfl_sync(0xffffffffu, m, q);
+                s[q * kRow + lane] = in && mq >= 0 ? __ldg(x + (size_t)mq * F + f0 + lane) : 0.f;
+            }
         }
         __syncwarp();
 #pragma unroll
@@ -179,11 +277,11 @@ edge_dot_kernel(const float *__restrict__ own, int ld_own, const float *__restri
             const float4 xv = *reinterpret_cast<const float4 *>(s + lane * kRow + c);
             float4 gv = make_float4(0.f, 0.f, 0.f, 0.f);
             int4 av = make_int4(-1, -1, -1, -1);
-            const int left = F - f0 - c;
-            if (vec4) {
+            if (VEC) {
                 gv = __ldg(reinterpret_cast<const float4 *>(g + f0 + c));
                 if (MAX) av = __ldg(reinterpret_cast<const int4 *>(am + f0 + c));
             } else {
+                const int left = F - f0 - c;
                 gv.x = g[f0 + c];
                 if (left > 1) gv.y = g[f0 + c + 1];
                 if (left > 2) gv.z = g[f0 + c + 2];
@@ -196,21 +294,28 @@ edge_dot_kernel(const float *__restrict__ own, int ld_own, const float *__restri
                 }
             }
             // features beyond the last are zeros on both sides and change nothing
-            mean_part = __fadd_rn(mean_part, __fmul_rn(gv.x, xv.x));
-            mean_part = __fadd_rn(mean_part, __fmul_rn(gv.y, xv.y));
-            mean_part = __fadd_rn(mean_part, __fmul_rn(gv.z, xv.z));
-            mean_part = __fadd_rn(mean_part, __fmul_rn(gv.w, xv.w));
-            if (MAX && m >= 0) {
-                const float *h = g + F + f0 + c;
-                hit |= (av.x == m ? 1u : 0u) << c | (av.y == m ? 2u : 0u) << c | (av.z == m ? 4u : 0u) << c | (av.w == m ? 8u : 0u) << c;
-                if (av.x == m) max_part = __fadd_rn(max_part, __fmul_rn(h[0], xv.x));
-                if (av.y == m) max_part = __fadd_rn(max_part, __fmul_rn(h[1], xv.y));
-                if (av.z == m) max_part = __fadd_rn(max_part, __fmul_rn(h[2], xv.z));
-                if (av.w == m) max_part = __fadd_rn(max_part, __fmul_rn(h[3], xv.w));
+            const float2 p01 = mul2(gv.x, gv.y, xv.x, xv.y), p23 = mul2(gv.z, gv.w, xv.z, xv.w);
+            mean_part = __fadd_rn(mean_part, p01.x);
+            mean_part = __fadd_rn(mean_part, p01.y);
+            mean_part = __fadd_rn(mean_part, p23.x);
+            mean_part = __fadd_rn(mean_part, p23.y);
+            if (MAX) {
+                if (av.x == arg_m) hit |= 1u << c;
+                if (av.y == arg_m) hit |= 2u << c;
+                if (av.z == arg_m) hit |= 4u << c;
+                if (av.w == arg_m) hit |= 8u << c;
             }
         }
-        if (f0 == 0) bits.x = hit;
-        if (f0 == 32) bits.y = hit;
+        if (MAX) {
+            // a feature's maximum lies in one slot, so a lane has F / K of them on average
+            const float *__restrict__ gm = g + F + f0;
+            for (unsigned left = hit; left != 0u; left &= left - 1u) {
+                const int f = __ffs(left) - 1;
+                max_part = __fadd_rn(max_part, __fmul_rn(__ldg(gm + f), s[lane * kRow + f]));
+            }
+            if (f0 == 0) bits.x = hit;
+            if (f0 == 32) bits.y = hit;
+        }
     }
     if (t >= n_edges) return;
     if (MAX && flags) *reinterpret_cast<uint2 *>(flags + 2 * (size_t)e) = bits;
@@ -224,17 +329,33 @@ edge_dot_kernel(const float *__restrict__ own, int ld_own, const float *__restri
     }
 }
 
-// Features per lane and division mode of edge_sum_kernel; slabs of 64 features.
+// One slab of up to 64 features of edge_sum_kernel.  `scratch`: room for n_vert rows of a slab.  Lanes per target: as many as
+// the width needs at four features each, so that narrow rows share a warp (200k hits, K = 16, F = 16: PushKnn 220 -> 146 us).
 template <int MODE>
 int launch_edge_sum_slab(const float *x, int ldx, const float *weights, const unsigned *flags, const int *nidx,
                          const int *bounds, const int *edges, float *out, int n_vert, int K, int F, int f0,
-                         const int *order, cudaStream_t stream)
+                         const int *order, float *scratch, cudaStream_t stream)
 {
-    const int blocks = div_up(n_vert, 8);
-#define HGC_SUM(FPL, P) HGC_CUDA_TRY(launch_overlapped(n_vert, edge_sum_kernel<FPL, MODE, P>, blocks, 256, 0, stream, x, ldx, weights, flags, nidx, bounds, edges, out, n_vert, K, F, f0, order))
-    const bool pow2 = MODE == kSumPlain || (K & (K - 1)) == 0;
-    if (F - f0 <= 32) { if (pow2) HGC_SUM(1, true); else HGC_SUM(1, false); }
-    else              { if (pow2) HGC_SUM(2, true); else HGC_SUM(2, false); }
+    const int width = F - f0 < 64 ? F - f0 : 64;
+    // rows are read where they lie if they are whole vectors and the division by K is an exact scaling
+    const bool whole = F % 4 == 0 && ldx % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+    const bool exact = MODE == kSumPlain || (K & (K - 1)) == 0;
+    const float *rows = x + f0;
+    int ldr = ldx;
+    if (!whole || !exact) {
+        ldr = (width + 3) / 4 * 4;
+        HGC_CUDA_TRY(launch_overlapped(n_vert, edge_rows_kernel, div_up((long long)n_vert * ldr, 256), 256, 0, stream, x + f0, ldx, width,
+                                       MODE == kSumPlain ? 1.f : (float)K, scratch, ldr, n_vert));
+        HGC_LAUNCH_CHECK();
+        rows = scratch;
+    }
+    const bool scale = MODE != kSumPlain && rows != scratch;  // only rows that are whole vectors are scaled
+#define HGC_SUM(LPT, VW, S, H) HGC_CUDA_TRY(launch_overlapped(n_vert, edge_sum_kernel<LPT, VW, MODE, S, H>, div_up(n_vert, 8 * (32 / LPT)), 256, 0, stream, rows, ldr, x + F + f0, ldx, weights, flags, nidx, bounds, edges, out, n_vert, K, F, f0, order))
+#define HGC_SUM_W(S, H) do { if (width > 32) HGC_SUM(16, 4, S, H); else if (width > 16) HGC_SUM(8, 4, S, H); else HGC_SUM(4, 4, S, H); } while (0)
+    if constexpr (MODE == kSumPlain) HGC_SUM_W(false, false);
+    else if constexpr (MODE == kSumMean) { if (scale) HGC_SUM_W(true, false); else HGC_SUM_W(false, false); }
+    else { if (scale) HGC_SUM_W(true, true); else if (whole) HGC_SUM_W(false, true); else HGC_SUM_W(false, false); }
+#undef HGC_SUM_W
 #undef HGC_SUM
     HGC_LAUNCH_CHECK();
     return HGC_OK;

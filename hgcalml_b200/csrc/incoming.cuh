@@ -15,6 +15,7 @@ struct Incoming {
     int *edges;           // [n_edges] edge ids e = hit * n_neigh + slot
     int *place;           // [n_edges] place of an edge in its target's list; scratch of the long sort afterwards
     unsigned *flags;      // [n_edges][2] scratch of the op: one bit per feature of a slab of 64
+    float *rows;          // [n_vert][64] scratch of the op: rows of a slab (edge_rows_kernel)
 };
 
 template <typename W>
@@ -28,6 +29,7 @@ Incoming incoming_layout(W &ws, int n_vert, int n_neigh)
     b.edges = ws.template take<int>(ne);
     b.place = ws.template take<int>(ne);
     b.flags = ws.template take<unsigned>(2 * ne);
+    b.rows = ws.template take<float>(64 * n);
     return b;
 }
 

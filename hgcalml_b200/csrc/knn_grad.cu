@@ -144,13 +144,12 @@ extern "C" int hgc_accumulate_knn_grad_ordered(
     const bool mm = mean_and_max != 0;
     const long long ne = (long long)n_vert * n_neigh;
     auto aligned16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
-    const bool vec4 = n_feat % 4 == 0 && aligned16(d_grad_from_out_features) && (!mm || aligned16(d_max_feat_indices));
-    if (mm)
-        HGC_CUDA_TRY(launch_overlapped(n_vert, edge_dot_kernel<true, true>, div_up(ne, 256), 256, 0, stream, d_grad_from_out_features, n_grad_from_out_feat, d_feat, d_max_feat_indices, d_neigh_indices,
-                d_out_grad_distances, ne, n_vert, n_neigh, n_feat, vec4, d_order, b.flags));
-    else
-        HGC_CUDA_TRY(launch_overlapped(n_vert, edge_dot_kernel<true, false>, div_up(ne, 256), 256, 0, stream, d_grad_from_out_features, n_grad_from_out_feat, d_feat, nullptr, d_neigh_indices, d_out_grad_distances, ne,
-                n_vert, n_neigh, n_feat, vec4, d_order, nullptr));
+    const bool vec4 = n_feat % 4 == 0 && aligned16(d_feat) && aligned16(d_grad_from_out_features) && (!mm || aligned16(d_max_feat_indices));
+    HGC_CUDA_TRY(launch_overlapped(n_vert, mm ? vec4 ? edge_dot_kernel<true, true, true> : edge_dot_kernel<true, true, false>
+                                              : vec4 ? edge_dot_kernel<true, false, true> : edge_dot_kernel<true, false, false>,
+                                   div_up(ne, 256), 256, 0, stream, d_grad_from_out_features, n_grad_from_out_feat, d_feat,
+                                   mm ? d_max_feat_indices : nullptr, d_neigh_indices, d_out_grad_distances, ne, n_vert, n_neigh,
+                                   n_feat, d_order, mm ? b.flags : nullptr));
     HGC_LAUNCH_CHECK();
     for (int f0 = 0; f0 < n_feat; f0 += 64) {
         if (mm && f0 > 0) {  // the bits of the first slab are a by-product of the weights' gradient
@@ -160,10 +159,10 @@ extern "C" int hgc_accumulate_knn_grad_ordered(
         }
         const int rc = mm ? launch_edge_sum_slab<kSumMeanMax>(d_grad_from_out_features, n_grad_from_out_feat, d_distances,
                                                               b.flags, d_neigh_indices, b.bounds, b.edges,
-                                                              d_out_grad_features, n_vert, n_neigh, n_feat, f0, d_order, stream)
+                                                              d_out_grad_features, n_vert, n_neigh, n_feat, f0, d_order, b.rows, stream)
                           : launch_edge_sum_slab<kSumMean>(d_grad_from_out_features, n_grad_from_out_feat, d_distances,
                                                            nullptr, d_neigh_indices, b.bounds, b.edges,
-                                                           d_out_grad_features, n_vert, n_neigh, n_feat, f0, d_order, stream);
+                                                           d_out_grad_features, n_vert, n_neigh, n_feat, f0, d_order, b.rows, stream);
         if (rc) return rc;
     }
     return HGC_OK;

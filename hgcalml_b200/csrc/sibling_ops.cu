@@ -105,13 +105,14 @@ extern "C" int hgc_push_knn_grad_ordered(
         HGC_LAUNCH_CHECK();
     }
     if (ne > 0) {
-        const bool vec4 = n_feat % 4 == 0 && (reinterpret_cast<uintptr_t>(d_feat) & 15u) == 0;
+        const bool vec4 = n_feat % 4 == 0 && ((reinterpret_cast<uintptr_t>(d_feat) | reinterpret_cast<uintptr_t>(d_grad)) & 15u) == 0;
         if (n_feat < kNarrow)
             HGC_CUDA_TRY(launch_overlapped(n_vert, push_grad_weights_kernel, div_up(ne, 256), 256, 0, stream, d_grad, d_feat, d_idxs, d_w_grad, ne,
                                            n_vert, n_neigh, n_feat, d_order));
         else
-            HGC_CUDA_TRY(launch_overlapped(n_vert, edge_dot_kernel<false, false>, div_up(ne, 256), 256, 0, stream, d_feat, n_feat, d_grad, nullptr, d_idxs, d_w_grad,
-                                                                          ne, n_vert, n_neigh, n_feat, vec4, d_order, nullptr));
+            HGC_CUDA_TRY(launch_overlapped(n_vert, vec4 ? edge_dot_kernel<false, false, true> : edge_dot_kernel<false, false, false>,
+                                           div_up(ne, 256), 256, 0, stream, d_feat, n_feat, d_grad, nullptr, d_idxs, d_w_grad,
+                                           ne, n_vert, n_neigh, n_feat, d_order, nullptr));
         HGC_LAUNCH_CHECK();
     }
     return HGC_OK;
@@ -163,7 +164,7 @@ extern "C" int hgc_push_knn_ordered(
     if (int rc = build_incoming(d_idxs, n_vert, n_neigh, b, ws.status(), stream)) return rc;
     for (int f0 = 0; f0 < n_feat; f0 += 64)
         if (int rc = launch_edge_sum_slab<kSumPlain>(d_feat, n_feat, d_weights, nullptr, nullptr, b.bounds, b.edges, d_out_feat,
-                                                     n_vert, n_neigh, n_feat, f0, d_order, stream))
+                                                     n_vert, n_neigh, n_feat, f0, d_order, b.rows, stream))
             return rc;
     return HGC_OK;
 }

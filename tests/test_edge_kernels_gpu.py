@@ -131,3 +131,31 @@ def test_push_knn_grad_around_the_narrow_rows(cuda, oracle, F):
     for o in (None, T(rng.permutation(n).astype(np.int32), cuda)):
         gw, gf = PushKnnGrad(T(g, cuda), T(w, cuda), T(f, cuda), T(idx, cuda), order=o)
         assert np.array_equal(bits(N(gw)), bits(rw)) and np.array_equal(bits(N(gf)), bits(rf))
+
+
+@pytest.mark.parametrize("K", [8, 11])
+@pytest.mark.parametrize("F", [2, 4, 16, 20, 36, 66, 68, 128])
+def test_rows_of_whole_and_of_part_vectors(cuda, oracle, K, F):
+    """Lanes per target change with the width (16, 32, 64); rows that are no whole vectors, lie off a 16-byte boundary or are
+    divided by a K that is no power of two are copied first."""
+    from hgcalml_b200.accknn_op import AccumulateKnnGrad, AccumulateLinKnn
+    from hgcalml_b200.push_knn_op import PushKnn, PushKnnGrad
+    n = 700
+    idx, rng = _table(n, K, F)
+    feat, grad = rng.standard_normal((n, F), dtype=np.float32), rng.standard_normal((n, 2 * F), dtype=np.float32)
+    w = rng.random((n, K), dtype=np.float32)
+
+    def shifted(a):
+        flat = torch.empty(a.size + 1, dtype=torch.float32, device=cuda)
+        return flat[1:].view(a.shape).copy_(T(a, cuda))
+    table = T(idx, cuda)
+    for put in (lambda a: T(a, cuda), shifted):
+        _, maxidx = AccumulateLinKnn(T(w, cuda), T(feat, cuda), table)
+        gw, gf = AccumulateKnnGrad(put(grad), put(w), put(feat), table, maxidx)
+        rw, rf = oracle.op_accumulate_knn_grad(grad, w, feat, idx, N(maxidx))
+        assert np.array_equal(bits(N(gw)), bits(rw)) and np.array_equal(bits(N(gf)), bits(rf))
+        assert np.array_equal(bits(N(PushKnn(put(w), put(feat), table))), bits(oracle.op_push_knn(w, feat, idx)))
+        g1 = np.ascontiguousarray(grad[:, :F])
+        rw, rf = oracle.op_push_knn_grad(g1, w, feat, idx)
+        gw, gf = PushKnnGrad(put(g1), put(w), put(feat), table)
+        assert np.array_equal(bits(N(gw)), bits(rw)) and np.array_equal(bits(N(gf)), bits(rf))
