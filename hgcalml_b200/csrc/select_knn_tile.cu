@@ -6,23 +6,50 @@
 namespace hgc {
 namespace {
 
-// A block per super-chunk, a thread per hit: the 1024 hits of a super-chunk, consecutive on the curve, are
-// split five times at the median of the coordinate in which the part is widest, which leaves parts of 32 hits:
-// the chunks.  Their boxes do not overlap, and a ball of 64 hits in four dimensions meets a third fewer of
-// them than of runs of 32 hits along the curve.  A part is split by sorting words of the quantised position
-// in the part (22 bits) and the hit's number (10 bits), a network of shuffles and a few exchanges through
-// shared memory; the split need not be exact.  Padding sorts last at every level, so the real hits
-// stay in front.
-constexpr int kPackThreads = 1024;
+// A block per super-chunk of 1024 hits that are consecutive on the curve, a warp per 128 of them, which it splits twice at the
+// median of the coordinate in which the part is widest: that leaves parts of 32 hits, the chunks.  Their boxes do not
+// overlap, and a ball of 64 hits in four dimensions meets fewer of them than of runs of 32 hits along the curve.  A part is
+// split by sorting words of the quantised position in the part (25 bits) and the hit's place (7 bits), four words per lane, by
+// a network of shuffles; the split need not be exact.  Padding sorts last, so the real hits stay in front.
+// Five splits of the whole super-chunk, a thread per hit, took 18 us for one block and 57 us for 400k hits, most of it in
+// shuffles and barriers, and gave chunks that are no better: search and packing, 400k hits in four dimensions, K = 64, from
+// parts of 1024 1202 us, 512 1180, 256 1188, 128 1168, 32 (no split) 1192.  This kernel: 18 us for 400k hits, 10 for one block.
+constexpr int kPackThreads = 256;
+constexpr int kSuper = 1024;
+constexpr int kPart = 128;
 constexpr int kSplitDims = 8;  // coordinates that splits look at
 
-__device__ __forceinline__ unsigned exchange_u32(unsigned v, unsigned *s_x, int partner, bool lower)
+__device__ __forceinline__ void order_pair(unsigned &a, unsigned &b)
 {
-    __syncthreads();  // the previous exchange has been read
-    s_x[threadIdx.x] = v;
-    __syncthreads();
-    const unsigned o = s_x[partner];
-    return lower ? min(v, o) : max(v, o);
+    const unsigned lo = min(a, b);
+    b = max(a, b);
+    a = lo;
+}
+
+// Ascending sort of every group of N words (N / 4 lanes, four consecutive words each).
+template <int N>
+__device__ __forceinline__ void sort_parts(unsigned (&w)[4], int lane)
+{
+    order_pair(w[0], w[1]); order_pair(w[2], w[3]);
+    order_pair(w[0], w[3]); order_pair(w[1], w[2]);
+    order_pair(w[0], w[1]); order_pair(w[2], w[3]);
+#pragma unroll
+    for (int k = 8; k <= N; k <<= 1) {
+        unsigned o[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) o[r] = __shfl_xor_sync(0xffffffffu, w[3 - r], (k >> 2) - 1);
+#pragma unroll
+        for (int r = 0; r < 4; r++) w[r] = (lane & (k >> 3)) == 0 ? min(w[r], o[r]) : max(w[r], o[r]);
+#pragma unroll
+        for (int j = k >> 4; j > 0; j >>= 1)
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const unsigned v = __shfl_xor_sync(0xffffffffu, w[r], j);
+                w[r] = (lane & j) == 0 ? min(w[r], v) : max(w[r], v);
+            }
+        order_pair(w[0], w[2]); order_pair(w[1], w[3]);
+        order_pair(w[0], w[1]); order_pair(w[2], w[3]);
+    }
 }
 
 __global__ void __launch_bounds__(kPackThreads)
@@ -32,11 +59,10 @@ pack_tiles_kernel(const float *__restrict__ coords, int C, const int *__restrict
 {
     pdl_begin();
     extern __shared__ float s_c[];  // [min(C, kSplitDims)][1024] coordinates in curve order
-    __shared__ float s_lo[32][16], s_hi[32][16];
-    __shared__ unsigned s_x[kPackThreads];
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    __shared__ float s_lo[kPackThreads / 32][16], s_hi[kPackThreads / 32][16];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sup = blockIdx.x;
-    if (sup == 0 && warp == 31) {  // the chunk that holds no hits
+    if (sup == 0 && warp == 7) {  // the chunk that holds no hits
         s.ranks[nobody + lane] = 0;
         for (int u = 0; u < nv4; u++)
             s.pts[(size_t)(nobody + lane) * nv4 + u] = make_float4(NAN, NAN, NAN, NAN);
@@ -49,97 +75,136 @@ pack_tiles_kernel(const float *__restrict__ coords, int C, const int *__restrict
     }
     const int e = lo_e;
     const int chunk0 = o.event_chunk[e], chunk1 = o.event_chunk[e + 1];
-    const int local0 = (sup - o.event_super[e]) * kPackThreads;
+    const int local0 = (sup - o.event_super[e]) * kSuper + warp * kPart;
     const int pos0 = o.event_pos[e] + local0;
-    const int n_here = min(o.event_pos[e + 1] - pos0, kPackThreads);
+    const int n_here = min(o.event_pos[e + 1] - pos0, kPart);  // below one: nothing for this warp
     const int cd = min(C, kSplitDims);
-    {
-        const int id = t < n_here ? perm[pos0 + t] : -1;
-        for (int c = 0; c < cd; c++) s_c[c * kPackThreads + t] = id >= 0 ? coords[(size_t)id * C + c] : 0.f;
+    float *__restrict__ s_w = s_c + warp * kPart;
+    int id[4], li[4];  // hit and place in the part, of the four places lane * 4 ..
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        li[r] = lane * 4 + r;
+        id[r] = li[r] < n_here ? perm[pos0 + li[r]] : -1;
     }
-    __syncthreads();
-    int li = t;  // hit (in curve order) at this thread's place
-    for (int size = kPackThreads; size > 32; size >>= 1) {
-        if (n_here <= 32) break;
-        // extents of the part this warp belongs to
-        const bool real = li < n_here;
-        for (int c = 0; c < cd; c++) {
-            const float x = s_c[c * kPackThreads + li];
-            const float lo = warp_min_f32(real ? x : INFINITY), hi = warp_max_f32(real ? x : -INFINITY);
-            if (lane == 0) { s_lo[warp][c] = lo; s_hi[warp][c] = hi; }
+#pragma unroll
+    for (int r = 0; r < 4; r++)
+        for (int c = 0; c < cd; c++) s_w[c * kSuper + li[r]] = id[r] >= 0 ? coords[(size_t)id[r] * C + c] : 0.f;
+    __syncwarp();
+    if (n_here > 32) {
+#pragma unroll
+        for (int level = 0; level < 2; level++) {
+            // extents of the part, or of its lower and upper half
+            const bool upper = level == 1 && lane >= 16;
+            float best_lo = 0.f, best_ext = -1.f;
+            int dim = 0;
+            for (int c = 0; c < cd; c++) {
+                float lo = INFINITY, hi = -INFINITY;
+#pragma unroll
+                for (int r = 0; r < 4; r++)
+                    if (li[r] < n_here) {
+                        const float x = s_w[c * kSuper + li[r]];
+                        lo = fminf(lo, x);
+                        hi = fmaxf(hi, x);
+                    }
+                if (level == 0) {
+                    lo = warp_min_f32(lo);
+                    hi = warp_max_f32(hi);
+                } else {
+                    const float lo0 = warp_min_f32(upper ? INFINITY : lo), lo1 = warp_min_f32(upper ? lo : INFINITY);
+                    const float hi0 = warp_max_f32(upper ? -INFINITY : hi), hi1 = warp_max_f32(upper ? hi : -INFINITY);
+                    lo = upper ? lo1 : lo0;
+                    hi = upper ? hi1 : hi0;
+                }
+                if (hi - lo > best_ext) { best_ext = hi - lo; best_lo = lo; dim = c; }
+            }
+            const float scale = best_ext > 0.f ? 33554426.f / best_ext : 0.f;
+            unsigned w[4];
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                w[r] = 0x1ffffffu;
+                if (li[r] < n_here)
+                    w[r] = (unsigned)fminf(fmaxf((s_w[dim * kSuper + li[r]] - best_lo) * scale, 0.f), 33554426.f);
+                w[r] = (w[r] << 7) | (unsigned)li[r];
+            }
+            if (level == 0) sort_parts<kPart>(w, lane); else sort_parts<kPart / 2>(w, lane);
+#pragma unroll
+            for (int r = 0; r < 4; r++) li[r] = (int)(w[r] & 127u);
         }
-        __syncthreads();
-        const int w0 = warp & ~(size / 32 - 1);
-        float best_lo = 0.f, best_ext = -1.f;
-        int dim = 0;
-        for (int c = 0; c < cd; c++) {
-            const bool in = lane < size / 32;
-            const float lo = warp_min_f32(in ? s_lo[w0 + lane][c] : INFINITY);
-            const float hi = warp_max_f32(in ? s_hi[w0 + lane][c] : -INFINITY);
-            if (hi - lo > best_ext) { best_ext = hi - lo; best_lo = lo; dim = c; }
-        }
-        const float scale = best_ext > 0.f ? 4194302.f / best_ext : 0.f;
-        unsigned w = 0x3fffffu;
-        if (real) w = (unsigned)fminf(fmaxf((s_c[dim * kPackThreads + li] - best_lo) * scale, 0.f), 4194302.f);
-        w = (w << 10) | (unsigned)li;
-        // ascending sort of every part of `size` threads
-        w = warp_sort_u32(w, lane);
-        for (int k = 64; k <= size; k <<= 1) {
-            w = exchange_u32(w, s_x, t ^ (k - 1), (t & (k >> 1)) == 0);
-            for (int j = k >> 2; j >= 32; j >>= 1) w = exchange_u32(w, s_x, t ^ j, (t & j) == 0);
-            w = warp_bitonic_merge_u32(w, lane);
-        }
-        li = (int)(w & 1023u);
+#pragma unroll
+        for (int r = 0; r < 4; r++) id[r] = li[r] < n_here ? perm[pos0 + li[r]] : -1;
     }
 
-    const int chunk = chunk0 + local0 / 32 + warp;
+    // eight lanes hold a chunk now
+    const int chunk = chunk0 + local0 / 32 + (lane >> 3);
     const bool have = chunk < chunk1;
-    const int id = li < n_here ? perm[pos0 + li] : -1;
+    const size_t at = (size_t)chunk * 32 + (lane & 7) * 4;
+    bool usable[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        usable[r] = id[r] >= 0;
+        if (direction != nullptr && usable[r]) {
+            const int d = direction[id[r]];
+            usable[r] = !(d == 1 || d == 2);  // may not be anybody's neighbour
+        }
+    }
     if (have) {
-        s.ids[(size_t)chunk * 32 + lane] = id;
-        s.ranks[(size_t)chunk * 32 + lane] = id >= 0 ? rank_of[id] : 0;
-        if (lane == 0) {
+        int rank[4];
+#pragma unroll
+        for (int r = 0; r < 4; r++) rank[r] = id[r] >= 0 ? rank_of[id[r]] : 0;
+        *reinterpret_cast<int4 *>(s.ids + at) = make_int4(id[0], id[1], id[2], id[3]);
+        *reinterpret_cast<int4 *>(s.ranks + at) = make_int4(rank[0], rank[1], rank[2], rank[3]);
+        if ((lane & 7) == 0) {
             // hits beyond the last event take part in nothing
             const bool none = e == n_events;
             s.chunk_info[chunk] = make_int4(chunk0, none ? chunk0 : chunk1, o.event_super[e], o.event_super[e + 1]);
         }
     }
-    bool usable = id >= 0;
-    if (direction != nullptr && usable) {
-        const int d = direction[id];
-        usable = !(d == 1 || d == 2);  // may not be anybody's neighbour
-    }
     const float nan = __int_as_float(0x7fffffff);
-    __syncthreads();  // s_lo, s_hi are used again
     for (int u = 0; u < nv4; u++) {
-        float c[4], lo[4], hi[4];
+        float p[4][4], lo[4], hi[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const int d = u * 4 + k;
-            c[k] = 0.f;
-            if (d < C && usable) c[k] = coords[(size_t)id * C + d];
-            lo[k] = warp_min_f32(usable ? c[k] : INFINITY);
-            hi[k] = warp_max_f32(usable ? c[k] : -INFINITY);
-            if (!usable) c[k] = nan;
+            lo[k] = INFINITY;
+            hi[k] = -INFINITY;
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                p[r][k] = 0.f;
+                if (d < C && id[r] >= 0) p[r][k] = d < cd ? s_w[d * kSuper + li[r]] : coords[(size_t)id[r] * C + d];
+                if (usable[r]) {
+                    lo[k] = fminf(lo[k], p[r][k]);
+                    hi[k] = fmaxf(hi[k], p[r][k]);
+                } else {
+                    p[r][k] = nan;
+                }
+            }
+#pragma unroll
+            for (int j = 1; j < 8; j <<= 1) {
+                lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], j));
+                hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], j));
+            }
         }
         if (have) {
-            s.pts[((size_t)chunk * 32 + lane) * nv4 + u] = make_float4(c[0], c[1], c[2], c[3]);
-            if (lane == 0) {
+#pragma unroll
+            for (int r = 0; r < 4; r++) s.pts[(at + r) * nv4 + u] = make_float4(p[r][0], p[r][1], p[r][2], p[r][3]);
+            if ((lane & 7) == 0) {
                 s.chunk_box[((size_t)chunk * nv4 + u) * 2] = make_float4(lo[0], lo[1], lo[2], lo[3]);
                 s.chunk_box[((size_t)chunk * nv4 + u) * 2 + 1] = make_float4(hi[0], hi[1], hi[2], hi[3]);
             }
         }
-        if (lane == 0)
 #pragma unroll
-            for (int k = 0; k < 4; k++) { s_lo[warp][u * 4 + k] = lo[k]; s_hi[warp][u * 4 + k] = hi[k]; }
+        for (int k = 0; k < 4; k++) {
+            const float l = warp_min_f32(lo[k]), h = warp_max_f32(hi[k]);
+            if (lane == 0) { s_lo[warp][u * 4 + k] = l; s_hi[warp][u * 4 + k] = h; }
+        }
     }
     __syncthreads();
     if (warp < nv4) {
         float lo[4], hi[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            lo[k] = warp_min_f32(s_lo[lane][warp * 4 + k]);
-            hi[k] = warp_max_f32(s_hi[lane][warp * 4 + k]);
+            lo[k] = warp_min_f32(s_lo[lane & 7][warp * 4 + k]);
+            hi[k] = warp_max_f32(s_hi[lane & 7][warp * 4 + k]);
         }
         if (lane == 0) {
             s.super_box[((size_t)sup * nv4 + warp) * 2] = make_float4(lo[0], lo[1], lo[2], lo[3]);
@@ -154,7 +219,7 @@ int build_tiles(const float *coords, int n_coords, const int *curve_perm, const 
                 int n_events, const int *direction, const TileScratch &s, int n_vert, cudaStream_t stream)
 {
     if (n_vert <= 0) return HGC_OK;
-    const size_t smem = sizeof(float) * kPackThreads * (n_coords < kSplitDims ? n_coords : kSplitDims);
+    const size_t smem = sizeof(float) * kSuper * (n_coords < kSplitDims ? n_coords : kSplitDims);
     HGC_CUDA_TRY(launch_overlapped(n_vert, pack_tiles_kernel, (int)tile_supers_cap(n_vert, n_events), kPackThreads, smem, stream, coords, n_coords, curve_perm, rank_of, direction, n_events, o, s, (n_coords + 3) / 4,
             (int)(tile_chunks_cap(n_vert, n_events) * 32)));
     HGC_LAUNCH_CHECK();
