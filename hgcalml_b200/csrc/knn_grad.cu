@@ -57,9 +57,9 @@ select_grad_kernel(const float *__restrict__ grad_dist, const int *__restrict__ 
 #pragma unroll
         for (int u = 0; u < U; u++)
             if (j[u] >= 0) {
+                // the reference rounds val - (2 g) d in double, and to float; the products of floats are exact in double
                 const float d = __fsub_rn(x[u], xm);
-                // separately rounded double operations, as the host compiler evaluates the reference expression
-                val = (float)__dsub_rn((double)val, __dmul_rn(__dmul_rn(2.0, (double)g[u]), (double)d));
+                val = (float)__fma_rn(-2.0 * (double)g[u], (double)d, (double)val);
             }
     }
     const int end = bounds[m + 1];
@@ -74,8 +74,9 @@ select_grad_kernel(const float *__restrict__ grad_dist, const int *__restrict__ 
 #pragma unroll
         for (int u = 0; u < U; u++)
             if (p + u < end) {
+                // (2 g) d, exact in double, rounded to float: the float product, and doubling is exact
                 const float d = __fsub_rn(xm, x[u]);
-                val = __fadd_rn(val, (float)__dmul_rn(__dmul_rn(2.0, (double)g[u]), (double)d));
+                val = __fadd_rn(val, __fmul_rn(g[u], d + d));
             }
     }
     grad_coord[(size_t)m * C + c] = val;
