@@ -97,9 +97,11 @@ __device__ __forceinline__ float count_bound(const float (&v)[N], int target, in
 struct Pruned { knn_key thr; int cnt; };
 
 // Sorts the parked hits and keeps exactly the `keep` smallest, in order; returns the largest of them.  For rows
-// whose distances tie so that counting cannot part them; rare, so kept out of line.
+// whose distances tie so that counting cannot part them; rare.  Out of line for the long lists, whose networks are most of the
+// kernel's code otherwise (200k hits, K = 100: 1020 -> 975 us); a call costs the short ones more in spills than it saves (K = 64
+// +2 %).
 template <int L>
-__device__ __forceinline__ knn_key keep_smallest(knn_key *buf, int cnt, int keep, int lane)
+__device__ __forceinline__ knn_key keep_smallest_inline(knn_key *buf, int cnt, int keep, int lane)
 {
     knn_key list[L];
 #pragma unroll
@@ -114,8 +116,19 @@ __device__ __forceinline__ knn_key keep_smallest(knn_key *buf, int cnt, int keep
     return shfl_key(list_reg<L>(list, (keep - 1) / 32), (keep - 1) & 31);
 }
 
-// Reduces the parked hits to at most `limit` (>= want) of the smallest and tightens the bound.  Not inlined:
-// it needs more registers than the code around it and is called once or twice per query.
+template <int L>
+__device__ __noinline__ knn_key keep_smallest_call(knn_key *buf, int cnt, int keep, int lane)
+{
+    return keep_smallest_inline<L>(buf, cnt, keep, lane);
+}
+template <int L>
+__device__ __forceinline__ knn_key keep_smallest(knn_key *buf, int cnt, int keep, int lane)
+{
+    if constexpr (L > 2) return keep_smallest_call<L>(buf, cnt, keep, lane);
+    else return keep_smallest_inline<L>(buf, cnt, keep, lane);
+}
+
+// Reduces the parked hits to at most `limit` (>= want) of the smallest and tightens the bound.
 template <int L>
 __device__ __forceinline__ Pruned prune_parked(knn_key *buf, int cnt, int want, int window, int limit, knn_key thr,
                                             float expo, int lane)
@@ -235,8 +248,7 @@ struct TileQuery {
     {
         const knn_key key = make_key(ds, rank);
         const bool pass = ok && key <= thr;
-        const unsigned m = __ballot_sync(0xffffffffu, pass);
-        if (m == 0u) return;
+        const unsigned m = __ballot_sync(0xffffffffu, pass);  // (leaving early where it is empty: 400k hits +1 %)
         if (pass) buf[cnt + __popc(m & ((1u << lane) - 1u))] = key;
         cnt += __popc(m);
     }
