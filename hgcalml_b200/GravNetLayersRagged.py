@@ -99,13 +99,18 @@ class _Dense(torch.nn.Module):
         self.activation = _activation(activation)
 
     def forward(self, x):
-        y = x @ self.kernel
-        bias = self.bias
+        kernel, bias = self.kernel, self.bias
+        # one kernel where only the values count; bias and activation over the library's y in one pass, in place, where that
+        # is the faster way and the bias is one dense row beside y; every other form takes the tensor operations
+        relu = self.activation is torch.relu
+        plain = relu or self.activation is _linear
+        if plain and type(x) in _PLAIN and type(kernel) in _PLAIN and (bias is None or type(bias) in _PLAIN) and x.is_cuda:
+            y = C.native.dense(x, kernel, bias, relu)
+            if y is not None:
+                return y
+        y = x @ kernel
         if bias is not None:
-            # bias and activation go over y in one pass, in place, where only the values count and the bias is one dense
-            # row beside y; every other form takes the tensor operations
-            relu = self.activation is torch.relu
-            if (relu or self.activation is _linear) and y.is_cuda and type(y) in _PLAIN and type(bias) in _PLAIN:
+            if plain and y.is_cuda and type(y) in _PLAIN and type(bias) in _PLAIN:
                 rc = C.native.bias_act(y, bias, relu)
                 if rc != C.NOT_TAKEN:
                     C.check(rc, "dense layer")

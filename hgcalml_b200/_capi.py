@@ -49,6 +49,7 @@ def _load():
         "hgc_accumulate_knn_ordered": (I, [P] * 5 + [I] * 6 + [P, P]),
         "hgc_accumulate_knn_exp": (I, [P] * 5 + [I] * 5 + [ctypes.c_float, P, P]),
         "hgc_gravnet_collect": (I, [P, P, I, I, I, P, P, I, P, I, I, ctypes.c_float, I, P, P]),
+        "hgc_dense": (I, [P] * 4 + [I] * 4 + [P]),
         "hgc_bias_act": (I, [P, P, I, I, I, P]),
         "hgc_copy_columns": (I, [P, P, I, I, I, P]),
         "hgc_binned_select_knn_ragged_workspace_bytes": (S, [I] * 6),

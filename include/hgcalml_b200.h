@@ -212,6 +212,11 @@ int hgc_gravnet_collect(
         int n_vert, int n_feat, float distance_scale, int subtract_self, const int *d_order,
         hgc_stream_t stream);
 
+/* A dense layer in float32: y[n, n_out] = x[n, n_in] w[n_in, n_out], plus bias[n_out] unless NULL, then max(y, 0) when relu is
+ * set.  n_in: a multiple of 4, at most 512, d_x on a 16-byte boundary; HGC_ERR_UNSUPPORTED otherwise. */
+int hgc_dense(const float *d_x, const float *d_w, const float *d_bias, float *d_y, int n, int n_in, int n_out, int relu,
+              hgc_stream_t stream);
+
 /* Around the dense layers of the GravNet layers: y[n, n_feat] += bias in place, then max(y, 0) when relu is set;
  * and d_src[n, n_feat] copied into columns of a row-major buffer with row stride ld_dst floats (d_dst points at the
  * first of them). */

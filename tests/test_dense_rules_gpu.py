@@ -87,3 +87,41 @@ def test_the_sign_of_zero_is_that_of_the_operations(cuda):
         want = torch.relu(y + b) if relu else y + b
         C.check(C.lib.hgc_bias_act(C.ptr(y), C.ptr(b), 1, 4, relu, C.stream_of(y)), "bias_act")
         assert torch.equal(torch.signbit(y)[:, :3], torch.signbit(want)[:, :3]) and y[0, 3].isnan(), (relu, y, want)
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 127, 2049, 49153])
+@pytest.mark.parametrize("n_in,n_out", [(4, 1), (12, 4), (64, 5), (132, 8), (16, 9), (20, 16), (48, 17), (32, 32), (36, 33), (64, 64), (192, 65), (512, 130)])
+def test_dense_kernel_at_the_edges_of_its_tiles(cuda, n, n_in, n_out):
+    from hgcalml_b200 import _capi as C
+    g = torch.Generator(device=cuda).manual_seed(n + n_in)
+    x, w = torch.randn((n, n_in), generator=g, device=cuda), torch.randn((n_in, n_out), generator=g, device=cuda)
+    b = torch.randn(n_out, generator=g, device=cuda)
+    for bias, relu in ((None, 0), (b, 0), (b, 1)):
+        y = torch.full((n + 1, n_out), 7., device=cuda)
+        C.check(C.lib.hgc_dense(C.ptr(x), C.ptr(w), C.ptr(bias), C.ptr(y), n, n_in, n_out, relu, C.stream_of(x)), "dense")
+        want = x.double() @ w.double()
+        size = x.double().abs() @ w.double().abs()
+        if bias is not None:
+            want, size = want + b, size + b.abs()
+        if relu:
+            want = want.clamp_min(0.)
+        # n_in fused multiply-adds and one addition, each off by half an ulp of at most the sum of the terms' sizes
+        assert ((y[:n].double() - want).abs() <= (n_in + 1) * 2. ** -24 * size).all()
+        assert (y[n] == 7.).all()
+
+
+def test_precisions_that_the_caller_chose_are_the_library_s(cuda):
+    layer, x = _layer(cuda, n_in=64, n_out=64)
+    layer.requires_grad_(False)
+    x = torch.randn((3000, 64), generator=torch.Generator(device=cuda).manual_seed(2), device=cuda)
+    want = torch.relu(x @ layer.kernel + layer.bias)
+    assert torch.equal(layer(x), want)
+    with torch.autocast("cuda", dtype=torch.float16):
+        half = layer(x)
+        assert torch.equal(half, torch.relu(x @ layer.kernel + layer.bias))
+    assert not torch.equal(half.float(), want)
+    torch.backends.cuda.matmul.allow_tf32 = True
+    try:
+        assert torch.equal(layer(x), torch.relu(x @ layer.kernel + layer.bias))
+    finally:
+        torch.backends.cuda.matmul.allow_tf32 = False
