@@ -41,43 +41,13 @@ __device__ __forceinline__ void range_of_block(const float *__restrict__ coords,
     }
 }
 
-// One block: finishes the min/max reduction and derives the grid exactly as the Python wrappers do
-// (modules/bin_by_coordinates_op.py:49-71, modules/binned_select_knn_op.py:57-63), in float32.
-__device__ __forceinline__ void grid_from_partials(const float *partial, int n_partials, int n_dims, int n_all,
-                  const int *__restrict__ row_splits, int n_rs, int n_bins_arg, int n_neigh,
-                  int pre_normalized, GridParams *__restrict__ g)
+// The grid from the range of the batch, exactly as the Python wrappers derive it
+// (modules/bin_by_coordinates_op.py:49-71, modules/binned_select_knn_op.py:57-63), in float32.  One warp; lane c holds minimum
+// and maximum of coordinate c, zeros beyond n_all.
+__device__ __forceinline__ void grid_from_range(float mn, float mx, int n_dims, int n_all, const int *__restrict__ row_splits, int n_rs,
+                                                int n_bins_arg, int n_neigh, int pre_normalized, GridParams *__restrict__ g)
 {
-    // min / max over the per-block partial results: thread t looks at coordinate t % 8 of every
-    // (kGridSetupThreads / 8)-th partial; shuffles combine the lanes of a coordinate, shared memory the warps
-    static_assert(kMaxBinDims == 8 && kGridSetupThreads % 32 == 0, "layout of the reduction");
-    constexpr int kGridWarps = kGridSetupThreads / 32;
-    __shared__ float s_mn[kGridWarps][8], s_mx[kGridWarps][8];
-    {
-        const int cc = threadIdx.x & 7;
-        float a = INFINITY, b = -INFINITY;
-        for (int p = threadIdx.x >> 3; p < n_partials; p += kGridSetupThreads / 8) {
-            a = fminf(a, __ldcg(partial + ((size_t)p * 2 + 0) * kMaxBinDims + cc));  // perhaps written in this launch
-            b = fmaxf(b, __ldcg(partial + ((size_t)p * 2 + 1) * kMaxBinDims + cc));
-        }
-#pragma unroll
-        for (int o = 8; o < 32; o <<= 1) {
-            a = fminf(a, __shfl_xor_sync(0xffffffffu, a, o));
-            b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, o));
-        }
-        if ((threadIdx.x & 31) < 8) { s_mn[threadIdx.x >> 5][cc] = a; s_mx[threadIdx.x >> 5][cc] = b; }
-    }
-    __syncthreads();
-    if (threadIdx.x >= 32) return;  // the rest is one warp's work
-    const int c = threadIdx.x;
-    float mn = 0.f, mx = 0.f;
-    if (c < n_all) {
-        mn = INFINITY; mx = -INFINITY;
-#pragma unroll
-        for (int w = 0; w < kGridWarps; w++) {
-            mn = fminf(mn, s_mn[w][c]);
-            mx = fmaxf(mx, s_mx[w][c]);
-        }
-    }
+    const int c = threadIdx.x & 31;
     // The wrapper shifts by the minimum first; x -> x - mn is monotone, so the shifted extremes
     // are the extremes shifted.
     const float shift = pre_normalized ? 0.f : mn;
@@ -132,6 +102,45 @@ __device__ __forceinline__ void grid_from_partials(const float *partial, int n_p
             cell *= 0.5f;
         }
     }
+}
+
+// One block: finishes the min/max reduction and derives the grid.
+__device__ __forceinline__ void grid_from_partials(const float *partial, int n_partials, int n_dims, int n_all,
+                  const int *__restrict__ row_splits, int n_rs, int n_bins_arg, int n_neigh,
+                  int pre_normalized, GridParams *__restrict__ g)
+{
+    // min / max over the per-block partial results: thread t looks at coordinate t % 8 of every
+    // (kGridSetupThreads / 8)-th partial; shuffles combine the lanes of a coordinate, shared memory the warps
+    static_assert(kMaxBinDims == 8 && kGridSetupThreads % 32 == 0, "layout of the reduction");
+    constexpr int kGridWarps = kGridSetupThreads / 32;
+    __shared__ float s_mn[kGridWarps][8], s_mx[kGridWarps][8];
+    {
+        const int cc = threadIdx.x & 7;
+        float a = INFINITY, b = -INFINITY;
+        for (int p = threadIdx.x >> 3; p < n_partials; p += kGridSetupThreads / 8) {
+            a = fminf(a, __ldcg(partial + ((size_t)p * 2 + 0) * kMaxBinDims + cc));  // perhaps written in this launch
+            b = fmaxf(b, __ldcg(partial + ((size_t)p * 2 + 1) * kMaxBinDims + cc));
+        }
+#pragma unroll
+        for (int o = 8; o < 32; o <<= 1) {
+            a = fminf(a, __shfl_xor_sync(0xffffffffu, a, o));
+            b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, o));
+        }
+        if ((threadIdx.x & 31) < 8) { s_mn[threadIdx.x >> 5][cc] = a; s_mx[threadIdx.x >> 5][cc] = b; }
+    }
+    __syncthreads();
+    if (threadIdx.x >= 32) return;  // the rest is one warp's work
+    float mn = 0.f, mx = 0.f;
+    const int c = threadIdx.x;
+    if (c < n_all) {
+        mn = INFINITY; mx = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < kGridWarps; w++) {
+            mn = fminf(mn, s_mn[w][c]);
+            mx = fmaxf(mx, s_mx[w][c]);
+        }
+    }
+    grid_from_range(mn, mx, n_dims, n_all, row_splits, n_rs, n_bins_arg, n_neigh, pre_normalized, g);
 }
 
 // Position on a Hilbert curve: J. Skilling, "Programming the Hilbert curve", AIP Conf. Proc. 707 (2004) 381.
