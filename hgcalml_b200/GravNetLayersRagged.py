@@ -72,10 +72,9 @@ def collect_neighbours(features, neighbour_indices, distancesq, *, first_slot: i
     maxidx = torch.empty((n, f), dtype=torch.int32, device=feat.device) if with_max_idxs else None
     order = C.row_order(order, neighbour_indices, n)
     view = out[:, out_column:out_column + 2 * f]
-    C.check(C.lib.hgc_gravnet_collect(C.ptr(dist), C.ptr(idx), ld, first_slot, k, C.ptr(feat),
-                                      view.data_ptr() if n else None, out.stride(0), C.ptr(maxidx), n, f,
-                                      float(distance_scale), int(bool(subtract_self)), C.ptr(order),
-                                      C.stream_of(feat)), "gravnet_collect")
+    C.check_device(feat)
+    C.check(C.native.collect(dist, idx, first_slot, k, feat, view, maxidx, float(distance_scale), bool(subtract_self), order),
+            "gravnet_collect")
     return view, maxidx
 
 

@@ -65,28 +65,14 @@ def merge_noise_as_indiv_cp(assignment, asso_idx, alpha_idx, is_cond, n_condensa
     return _merge_noise(assignment, asso_idx, alpha_idx, is_cond, n_condensates, row_splits)
 
 
-def _host_int():
-    # page-locked, so that the copy that fills it needs no staging
-    return torch.empty((1,), dtype=torch.int32, pin_memory=True)
-
-
 def _merge_noise(assignment, asso, alpha, is_cond, n_condensates, row_splits):
     # alpha may be longer than the list of condensates: its length is n_condensates[-1]
-    dev, n, n_rs = assignment.device, assignment.shape[0], row_splits.shape[0]
-    new = torch.empty((4, n), dtype=torch.int32, device=dev)  # assignment, association, alpha (up to 2 n)
-    cond = torch.empty((n,), dtype=torch.bool, device=dev)
-    n_cond = torch.empty((n_rs,), dtype=torch.int32, device=dev)
-    ws = C.workspace(C.lib.hgc_merge_noise_workspace_bytes(n, n_rs), dev)
-    n_alpha = _host_int()
-    if alpha.shape[0] == 0:
-        alpha = new  # nothing is read from it
-    C.check(C.lib.hgc_merge_noise(
-        C.ptr(assignment), C.ptr(asso), C.ptr(alpha), C.ptr(is_cond), C.ptr(n_condensates), C.ptr(row_splits),
-        new[0].data_ptr(), new[1].data_ptr(), new[2].data_ptr(), C.ptr(cond), C.ptr(n_cond), n_alpha.data_ptr(),
-        n, n_rs, C.ptr(ws), ws.numel(), C.stream_of(assignment)), "merge_noise_as_indiv_cp")
-    if n_alpha.item() < 0:
+    C.check_device(assignment)
+    new, cond, n_cond, n_alpha, rc = C.native.merge_noise(assignment, asso, alpha, is_cond, n_condensates, row_splits)
+    C.check(rc, "merge_noise_as_indiv_cp")
+    if n_alpha < 0:
         raise C.HgcError("merge_noise_as_indiv_cp: the row splits must ascend and cover all hits")
-    return new[0][:, None], new[1], new[2:].reshape(-1)[:n_alpha.item()], cond[:, None], n_cond
+    return new[0][:, None], new[1], new[2:].reshape(-1)[:n_alpha], cond[:, None], n_cond
 
 
 def _segment_ids_to_row_splits(ids, num_segments):
@@ -119,22 +105,15 @@ def BuildAndAssignCondensatesBinned(ccoords, betas, dist, row_splits, beta_thres
     mask = None
     if no_condensation_mask is not None:
         mask = C.i32(no_condensation_mask, dev).reshape(-1)
-    assignment = torch.empty((n,), dtype=torch.int32, device=dev)
-    asso = torch.empty((n,), dtype=torch.int32, device=dev)
-    alpha = torch.empty((n,), dtype=torch.int32, device=dev)
-    is_cond = torch.empty((n,), dtype=torch.bool, device=dev)
-    n_condensates = torch.empty((n_rs,), dtype=torch.int32, device=dev)
-    ws = C.workspace(C.lib.hgc_build_and_assign_condensates_workspace_bytes(n, dims, n_rs, nbin_dims), dev)
-    n_alpha = None if keep_noise else _host_int()  # the number of condensates is not needed in between
-    C.check(C.lib.hgc_build_and_assign_condensates(
-        C.ptr(ccoords), C.ptr(betas), C.ptr(dist), C.ptr(mask), C.ptr(row_splits),
-        C.ptr(assignment), C.ptr(asso), C.ptr(alpha), C.ptr(is_cond), C.ptr(n_condensates),
-        C.ptr(n_alpha), n, dims, n_rs, float(beta_threshold), float(distance_threshold),
-        int(bool(assign_by_max_beta)), nbin_dims, C.ptr(ws), ws.numel(), C.stream_of(ccoords)),
-        "BuildAndAssignCondensatesBinned")
+    C.check_device(ccoords)
+    # the number of condensates is not needed in between when the noise comes after
+    assignment, asso, alpha, is_cond, n_condensates, n_alpha, rc = C.native.condensates(
+        ccoords, betas, dist, mask, row_splits, float(beta_threshold), float(distance_threshold), bool(assign_by_max_beta),
+        nbin_dims, not keep_noise)
+    C.check(rc, "BuildAndAssignCondensatesBinned")
     if keep_noise:
         return _merge_noise(assignment, asso, alpha, is_cond, n_condensates, row_splits)
-    return assignment[:, None], asso, alpha[:n_alpha.item()], is_cond[:, None], n_condensates
+    return assignment[:, None], asso, alpha[:n_alpha], is_cond[:, None], n_condensates
 
 
 def BuildAndAssignCondensatesBinnedStepwise(ccoords, betas, dist, row_splits, beta_threshold,

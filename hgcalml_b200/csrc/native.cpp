@@ -2,6 +2,7 @@
 // mirrors check and convert their arguments and call these with dense CUDA tensors of the right types; the status code
 // of the C ABI comes back as the last element.  A call costs the host about 15 us less than the same steps through
 // ctypes (of 52 us for a search of nine launches).
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/utils/pybind.h>
 #include <ATen/ATen.h>
 #include <ATen/PythonTorchFunctionTLS.h>
@@ -96,6 +97,92 @@ std::tuple<Tensor, int> select_knn_grad(const Tensor &grad, const Tensor &indice
     return {out, rc};
 }
 
+// (squared distances, status)
+std::tuple<Tensor, int> local_distance(const Tensor &indices, const Tensor &coords)
+{
+    Tensor out = like(coords, indices.sizes(), at::kFloat);
+    const int rc = hgc_local_distance(data<int>(indices), data<float>(coords), data<float>(out), (int)coords.size(1),
+                                      (int)coords.size(0), (int)indices.size(0), (int)indices.size(1), stream_of(coords));
+    return {out, rc};
+}
+
+// (features, status)
+std::tuple<Tensor, int> push_knn(const Tensor &weights, const Tensor &features, const Tensor &indices, const MaybeTensor &order)
+{
+    const int n = (int)indices.size(0), k = (int)indices.size(1), f = (int)features.size(1);
+    Tensor out = like(features, features.sizes(), at::kFloat);
+    Tensor ws = workspace(features, hgc_knn_grad_workspace_bytes(n, k));
+    const int rc = hgc_push_knn_ordered(data<float>(weights), data<float>(features), data<int>(indices), data<float>(out), n, k, f,
+                                        data<int>(order), ws.data_ptr(), (size_t)ws.numel(), stream_of(features));
+    return {out, rc};
+}
+
+// (gradient of the weights, gradient of the features, status)
+std::tuple<Tensor, Tensor, int> push_knn_grad(const Tensor &grad, const Tensor &weights, const Tensor &features,
+                                              const Tensor &indices, const MaybeTensor &order)
+{
+    const int n = (int)indices.size(0), k = (int)indices.size(1), f = (int)features.size(1);
+    Tensor gw = like(weights, weights.sizes(), at::kFloat), gf = like(features, features.sizes(), at::kFloat);
+    const int rc = hgc_push_knn_grad_ordered(data<float>(grad), data<float>(weights), data<float>(features), data<int>(indices),
+                                             data<float>(gf), data<float>(gw), n, k, f, data<int>(order), stream_of(features));
+    return {gw, gf, rc};
+}
+
+// status; `out`: the columns that take the collected features
+int collect(const Tensor &dist, const Tensor &indices, int first_slot, int k, const Tensor &features, const Tensor &out,
+            const MaybeTensor &max_idx, float scale, bool subtract_self, const MaybeTensor &order)
+{
+    const int n = (int)indices.size(0);
+    return hgc_gravnet_collect(data<float>(dist), data<int>(indices), (int)indices.size(1), first_slot, k, data<float>(features),
+                               n > 0 ? data<float>(out) : nullptr, (int)out.stride(0), data<int>(max_idx), n, (int)features.size(1),
+                               scale, subtract_self, data<int>(order), stream_of(features));
+}
+
+Tensor host_int()  // page-locked, so that the copy that fills it needs no staging
+{
+    return at::empty({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+}
+
+// (assignment, association, condensates, flags, condensates before every event, number of condensates or -1, status); with
+// `counted` the call waits for the number
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, int, int> condensates(const Tensor &coords, const Tensor &betas, const Tensor &dist,
+                                                                         const MaybeTensor &mask, const Tensor &row_splits,
+                                                                         double beta_threshold, double distance_threshold,
+                                                                         bool by_max_beta, int nbin_dims, bool counted)
+{
+    const int n = (int)coords.size(0), dims = (int)coords.size(1), n_rs = (int)row_splits.size(0);
+    Tensor assignment = like(coords, {n}, at::kInt), association = like(coords, {n}, at::kInt), alpha = like(coords, {n}, at::kInt);
+    Tensor flags = like(coords, {n}, at::kBool), counts = like(coords, {n_rs}, at::kInt);
+    Tensor ws = workspace(coords, hgc_build_and_assign_condensates_workspace_bytes(n, dims, n_rs, nbin_dims));
+    Tensor n_alpha;
+    if (counted) n_alpha = host_int();
+    const int rc = hgc_build_and_assign_condensates(
+            data<float>(coords), data<float>(betas), data<float>(dist), data<int>(mask), data<int>(row_splits), data<int>(assignment),
+            data<int>(association), data<int>(alpha), static_cast<unsigned char *>(flags.data_ptr()), data<int>(counts),
+            counted ? data<int>(n_alpha) : nullptr, n, dims, n_rs, (float)beta_threshold, (float)distance_threshold, by_max_beta,
+            nbin_dims, ws.data_ptr(), (size_t)ws.numel(), stream_of(coords));
+    return {assignment, association, alpha, flags, counts, counted && rc == HGC_OK ? *data<int>(n_alpha) : -1, rc};
+}
+
+// (assignment, association, and condensates, rows of one tensor; flags; condensates before every event; their number, status).
+// `alpha` may be longer than the list of condensates.
+std::tuple<Tensor, Tensor, Tensor, int, int> merge_noise(const Tensor &assignment, const Tensor &association, const Tensor &alpha,
+                                                         const Tensor &flags, const Tensor &counts, const Tensor &row_splits)
+{
+    const int64_t n = assignment.size(0);
+    const int n_rs = (int)row_splits.size(0);
+    Tensor all = like(assignment, {4, n}, at::kInt);  // the condensates take up to two rows
+    Tensor new_flags = like(assignment, {n}, at::kBool), new_counts = like(assignment, {n_rs}, at::kInt), n_alpha = host_int();
+    Tensor ws = workspace(assignment, hgc_merge_noise_workspace_bytes((int)n, n_rs));
+    int *rows = data<int>(all);
+    const int rc = hgc_merge_noise(
+            data<int>(assignment), data<int>(association), alpha.numel() > 0 ? data<int>(alpha) : rows,
+            static_cast<unsigned char *>(flags.data_ptr()), data<int>(counts), data<int>(row_splits), rows, rows + n, rows + 2 * n,
+            static_cast<unsigned char *>(new_flags.data_ptr()), data<int>(new_counts), data<int>(n_alpha), (int)n, n_rs, ws.data_ptr(),
+            (size_t)ws.numel(), stream_of(assignment));
+    return {all, new_flags, new_counts, rc == HGC_OK ? *data<int>(n_alpha) : 0, rc};
+}
+
 // Whether a kernel on raw pointers may stand in for a tensor operation: no function transform, dispatch mode or trace is
 // to see the operation ..
 bool operations_are_seen()
@@ -173,12 +260,22 @@ int copy_columns(const Tensor &x, const Tensor &out, int column)
 
 PYBIND11_MODULE(_native, m)
 {
+    // what goes wrong inside torch (memory that runs out, say) keeps its Python type
+    pybind11::register_local_exception_translator([](std::exception_ptr p) {
+        if (p) torch::translate_exception_to_python(p);
+    });
     // other Python threads run while a call enqueues, as they do during a ctypes call
     const auto unlocked = pybind11::call_guard<pybind11::gil_scoped_release>();
     m.def("select_knn", &select_knn, unlocked);
     m.def("accumulate", &accumulate, unlocked);
     m.def("accumulate_grad", &accumulate_grad, unlocked);
     m.def("select_knn_grad", &select_knn_grad, unlocked);
+    m.def("local_distance", &local_distance, unlocked);
+    m.def("push_knn", &push_knn, unlocked);
+    m.def("push_knn_grad", &push_knn_grad, unlocked);
+    m.def("collect", &collect, unlocked);
+    m.def("condensates", &condensates, unlocked);
+    m.def("merge_noise", &merge_noise, unlocked);
     m.def("dense", &dense, unlocked);
     m.def("bias_act", &bias_act, unlocked);
     m.def("copy_columns", &copy_columns, unlocked);

@@ -9,9 +9,9 @@ from .binned_select_knn_op import SelectKnnGrad
 
 def _local_distance(neighbour_idxs, coordinates):
     idx, coords = C.i32(neighbour_idxs), C.f32(coordinates)
-    out = torch.empty(idx.shape, dtype=torch.float32, device=coords.device)
-    C.check(C.lib.hgc_local_distance(C.ptr(idx), C.ptr(coords), C.ptr(out), coords.shape[1], coords.shape[0],
-                                     idx.shape[0], idx.shape[1], C.stream_of(coords)), "LocalDistance")
+    C.check_device(coords)
+    out, rc = C.native.local_distance(idx, coords)
+    C.check(rc, "LocalDistance")
     return out
 
 

@@ -12,13 +12,12 @@ def _push_knn(w, f, nidx, order=None):
     Contributions are summed in (i, k) order, so the result does not change from run to run."""
     C.require_cuda(w, f, nidx)
     w, f, nidx = C.f32(w), C.f32(f), C.i32(nidx)
-    n, k = nidx.shape
+    n, _ = nidx.shape
     if w.shape != nidx.shape or f.shape[0] != n:
         raise C.HgcError("PushKnn expects weights and indices of equal shape and one feature row per vertex")
-    out = torch.empty_like(f)
-    ws = C.workspace(C.lib.hgc_knn_grad_workspace_bytes(n, k), f.device)
-    C.check(C.lib.hgc_push_knn_ordered(C.ptr(w), C.ptr(f), C.ptr(nidx), C.ptr(out), n, k, f.shape[1], C.ptr(order),
-                                       C.ptr(ws), ws.numel(), C.stream_of(f)), "PushKnn")
+    C.check_device(f)
+    out, rc = C.native.push_knn(w, f, nidx, order)
+    C.check(rc, "PushKnn")
     return out
 
 
@@ -28,12 +27,10 @@ def PushKnnGrad(grad, weights, features, indices, order=None):
     sets the order in which hits are processed."""
     C.require_cuda(grad, weights, features, indices)
     g, w, f, idx = C.f32(grad), C.f32(weights), C.f32(features), C.i32(indices)
-    n, k = idx.shape
-    wg = torch.empty_like(w)
-    fg = torch.empty_like(f)
-    order = C.row_order(order, indices, n)
-    C.check(C.lib.hgc_push_knn_grad_ordered(C.ptr(g), C.ptr(w), C.ptr(f), C.ptr(idx), C.ptr(fg), C.ptr(wg),
-                                            n, k, f.shape[1], C.ptr(order), C.stream_of(f)), "PushKnnGrad")
+    n, _ = idx.shape
+    C.check_device(f)
+    wg, fg, rc = C.native.push_knn_grad(g, w, f, idx, C.row_order(order, indices, n))
+    C.check(rc, "PushKnnGrad")
     return wg, fg
 
 
