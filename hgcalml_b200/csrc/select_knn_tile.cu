@@ -240,12 +240,15 @@ int search_tiles(const TileScratch &s, const HitOrder &o, const int *rank_to_id,
     a.n_coords = n_coords; a.K = K; a.tf_compat = tf_compat;
     a.expo = 2.f / (float)n_coords;
     a.guess = powf(1.6f, a.expo);  // 60 % more hits, at equal density: measured flat from 1.3 to 1.8
-    // Queries per block: whole chunks share the list of one tile among most queries; small batches are cut
-    // finer, so that every SM has work.
-    const long long chunks = (long long)tile_chunks_cap(n_vert, n_events);
-    const long long fill = (long long)sm_count() * 8;
+    // Queries per block: whole chunks share the list of one tile among most queries; smaller batches are cut finer, so that
+    // every SM has work to the end.  A list costs little beside the queries in four dimensions and less in more, so the cut
+    // goes on there while blocks are few rounds of what is resident (9 to 6 per SM).  us with 8 blocks per SM wanted everywhere /
+    // with this rule, showers: 4 dimensions, K = 64, 25k hits 158 / 148, 50k 254 / 223, 80k 372 / 341, 130k 530 / 503; K = 32 50k 211 / 186; 5
+    // dimensions, K = 48, 20k 180 / 162, 50k 387 / 328, 130k 861 / 817.  3 dimensions lose by it: 20k uniform hits 86 / 96.
+    const long long chunks = (long long)tile_chunks_cap(n_vert, n_events), sms = sm_count();
+    const long long whole = sms * (n_coords <= 3 ? 8 : n_coords == 4 ? 30 : 40), cut = sms * (n_coords <= 3 ? 8 : n_coords == 4 ? (K < 24 ? 10 : 18) : 40);
     a.tile = 32;
-    while (a.tile > 4 && chunks * (32 / a.tile) < fill) a.tile >>= 1;
+    while (a.tile > 4 && chunks * (32 / a.tile) < (a.tile == 32 ? whole : cut)) a.tile >>= 1;
     const long long tiles = chunks * (32 / a.tile);
     if (tiles > 0x7fffffffLL) return HGC_ERR_UNSUPPORTED;
     switch ((n_coords + 3) / 4) {
