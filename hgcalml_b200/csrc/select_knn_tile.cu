@@ -6,17 +6,15 @@
 namespace hgc {
 namespace {
 
-// A block per super-chunk of 1024 hits that are consecutive on the curve, a warp per 128 of them, which it splits twice at the
-// median of the coordinate in which the part is widest: that leaves parts of 32 hits, the chunks.  Their boxes do not
+// A block per super-chunk of 1024 hits that are consecutive on the curve, a warp per 32 W of them (128 or 256), which it splits two
+// or three times at the median of the coordinate in which the part is widest: that leaves parts of 32 hits, the chunks.  Their boxes do not
 // overlap, and a ball of 64 hits in four dimensions meets fewer of them than of runs of 32 hits along the curve.  A part is
-// split by sorting words of the quantised position in the part (25 bits) and the hit's place (7 bits), four words per lane, by
-// a network of shuffles; the split need not be exact.  Padding sorts last, so the real hits stay in front.
+// split by sorting words of the quantised position in the part (25 bits) and the hit's place (7 bits), W words per lane, by a
+// network of shuffles; the split need not be exact.  Padding sorts last, so the real hits stay in front.
 // Five splits of the whole super-chunk, a thread per hit, took 18 us for one block and 57 us for 400k hits, most of it in
 // shuffles and barriers, and gave chunks that are no better: search and packing, 400k hits in four dimensions, K = 64, from
 // parts of 1024 1202 us, 512 1180, 256 1188, 128 1168, 32 (no split) 1192.  This kernel: 18 us for 400k hits, 10 for one block.
-constexpr int kPackThreads = 256;
 constexpr int kSuper = 1024;
-constexpr int kPart = 128;
 constexpr int kSplitDims = 8;  // coordinates that splits look at
 
 __device__ __forceinline__ void order_pair(unsigned &a, unsigned &b)
@@ -26,43 +24,100 @@ __device__ __forceinline__ void order_pair(unsigned &a, unsigned &b)
     a = lo;
 }
 
-// Ascending sort of every group of N words (N / 4 lanes, four consecutive words each).
-template <int N>
-__device__ __forceinline__ void sort_parts(unsigned (&w)[4], int lane)
+// Ascending sort of every group of N words (N / W lanes, W consecutive words each).
+template <int N, int W>
+__device__ __forceinline__ void sort_parts(unsigned (&w)[W], int lane)
 {
-    order_pair(w[0], w[1]); order_pair(w[2], w[3]);
-    order_pair(w[0], w[3]); order_pair(w[1], w[2]);
-    order_pair(w[0], w[1]); order_pair(w[2], w[3]);
+    // compares the words of a lane whose numbers differ in the bits of m
+    auto inside = [&](int m) {
 #pragma unroll
-    for (int k = 8; k <= N; k <<= 1) {
-        unsigned o[4];
+        for (int r = 0; r < W; r++)
+            if ((r ^ m) > r) order_pair(w[r], w[r ^ m]);
+    };
 #pragma unroll
-        for (int r = 0; r < 4; r++) o[r] = __shfl_xor_sync(0xffffffffu, w[3 - r], (k >> 2) - 1);
+    for (int k = 2; k <= N; k <<= 1) {
+        if (k <= W) {
+            inside(k - 1);
+        } else {
+            unsigned o[W];
 #pragma unroll
-        for (int r = 0; r < 4; r++) w[r] = (lane & (k >> 3)) == 0 ? min(w[r], o[r]) : max(w[r], o[r]);
+            for (int r = 0; r < W; r++) o[r] = __shfl_xor_sync(0xffffffffu, w[W - 1 - r], k / W - 1);
 #pragma unroll
-        for (int j = k >> 4; j > 0; j >>= 1)
+            for (int r = 0; r < W; r++) w[r] = (lane & (k / (2 * W))) == 0 ? min(w[r], o[r]) : max(w[r], o[r]);
+        }
 #pragma unroll
-            for (int r = 0; r < 4; r++) {
-                const unsigned v = __shfl_xor_sync(0xffffffffu, w[r], j);
-                w[r] = (lane & j) == 0 ? min(w[r], v) : max(w[r], v);
+        for (int j = k / 4; j > 0; j >>= 1) {
+            if (j < W) {
+                inside(j);
+            } else {
+#pragma unroll
+                for (int r = 0; r < W; r++) {
+                    const unsigned v = __shfl_xor_sync(0xffffffffu, w[r], j / W);
+                    w[r] = (lane & (j / W)) == 0 ? min(w[r], v) : max(w[r], v);
+                }
             }
-        order_pair(w[0], w[2]); order_pair(w[1], w[3]);
-        order_pair(w[0], w[1]); order_pair(w[2], w[3]);
+        }
     }
 }
 
-__global__ void __launch_bounds__(kPackThreads)
+// One split: the places of a part of kPart >> LEVEL hits in the order of the coordinate in which it is widest.
+template <int LEVEL, int W>
+__device__ __forceinline__ void split_part(const float *__restrict__ s_w, int cd, int n_here, int lane, int (&li)[W])
+{
+    constexpr int kLanes = 32 >> LEVEL;  // that hold the part
+    constexpr int kPlaceBits = W == 4 ? 7 : 8;
+    constexpr unsigned kTop = (1u << (32 - kPlaceBits)) - 1u;
+    const float span = W == 4 ? 33554426.f : 16777212.f;  // below kTop
+    static_assert(W == 4 || W == 8, "parts of 128 or 256");
+    float best_lo = 0.f, best_ext = -1.f;
+    int dim = 0;
+    for (int c = 0; c < cd; c++) {
+        float lo = INFINITY, hi = -INFINITY;
+#pragma unroll
+        for (int r = 0; r < W; r++)
+            if (li[r] < n_here) {
+                const float x = s_w[c * kSuper + li[r]];
+                lo = fminf(lo, x);
+                hi = fmaxf(hi, x);
+            }
+        if (LEVEL == 0) {
+            lo = warp_min_f32(lo);
+            hi = warp_max_f32(hi);
+        } else {
+#pragma unroll
+            for (int o = 1; o < kLanes; o <<= 1) {
+                lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+                hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+            }
+        }
+        if (hi - lo > best_ext) { best_ext = hi - lo; best_lo = lo; dim = c; }
+    }
+    const float scale = best_ext > 0.f ? span / best_ext : 0.f;
+    unsigned w[W];
+#pragma unroll
+    for (int r = 0; r < W; r++) {
+        w[r] = kTop;
+        if (li[r] < n_here) w[r] = (unsigned)fminf(fmaxf((s_w[dim * kSuper + li[r]] - best_lo) * scale, 0.f), span);
+        w[r] = (w[r] << kPlaceBits) | (unsigned)li[r];
+    }
+    sort_parts<kLanes * W, W>(w, lane);
+#pragma unroll
+    for (int r = 0; r < W; r++) li[r] = (int)(w[r] & ((1u << kPlaceBits) - 1u));
+}
+
+template <int W>
+__global__ void __launch_bounds__(kSuper / W)
 pack_tiles_kernel(const float *__restrict__ coords, int C, const int *__restrict__ perm,
                   const int *__restrict__ rank_of,
                   const int *__restrict__ direction, int n_events, HitOrder o, TileScratch s, int nv4, int nobody)
 {
     pdl_begin();
+    constexpr int kPart = 32 * W, kWarpsHere = kSuper / kPart;
     extern __shared__ float s_c[];  // [min(C, kSplitDims)][1024] coordinates in curve order
-    __shared__ float s_lo[kPackThreads / 32][16], s_hi[kPackThreads / 32][16];
+    __shared__ float s_lo[kWarpsHere][16], s_hi[kWarpsHere][16];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sup = blockIdx.x;
-    if (sup == 0 && warp == 7) {  // the chunk that holds no hits
+    if (sup == 0 && warp == kWarpsHere - 1) {  // the chunk that holds no hits
         s.ranks[nobody + lane] = 0;
         for (int u = 0; u < nv4; u++)
             s.pts[(size_t)(nobody + lane) * nv4 + u] = make_float4(NAN, NAN, NAN, NAN);
@@ -80,67 +135,32 @@ pack_tiles_kernel(const float *__restrict__ coords, int C, const int *__restrict
     const int n_here = min(o.event_pos[e + 1] - pos0, kPart);  // below one: nothing for this warp
     const int cd = min(C, kSplitDims);
     float *__restrict__ s_w = s_c + warp * kPart;
-    int id[4], li[4];  // hit and place in the part, of the four places lane * 4 ..
+    int id[W], li[W];  // hit and place in the part, of the places lane * W ..
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
-        li[r] = lane * 4 + r;
+    for (int r = 0; r < W; r++) {
+        li[r] = lane * W + r;
         id[r] = li[r] < n_here ? perm[pos0 + li[r]] : -1;
     }
 #pragma unroll
-    for (int r = 0; r < 4; r++)
+    for (int r = 0; r < W; r++)
         for (int c = 0; c < cd; c++) s_w[c * kSuper + li[r]] = id[r] >= 0 ? coords[(size_t)id[r] * C + c] : 0.f;
     __syncwarp();
     if (n_here > 32) {
+        split_part<0, W>(s_w, cd, n_here, lane, li);
+        split_part<1, W>(s_w, cd, n_here, lane, li);
+        if constexpr (W >= 8) split_part<2, W>(s_w, cd, n_here, lane, li);
 #pragma unroll
-        for (int level = 0; level < 2; level++) {
-            // extents of the part, or of its lower and upper half
-            const bool upper = level == 1 && lane >= 16;
-            float best_lo = 0.f, best_ext = -1.f;
-            int dim = 0;
-            for (int c = 0; c < cd; c++) {
-                float lo = INFINITY, hi = -INFINITY;
-#pragma unroll
-                for (int r = 0; r < 4; r++)
-                    if (li[r] < n_here) {
-                        const float x = s_w[c * kSuper + li[r]];
-                        lo = fminf(lo, x);
-                        hi = fmaxf(hi, x);
-                    }
-                if (level == 0) {
-                    lo = warp_min_f32(lo);
-                    hi = warp_max_f32(hi);
-                } else {
-                    const float lo0 = warp_min_f32(upper ? INFINITY : lo), lo1 = warp_min_f32(upper ? lo : INFINITY);
-                    const float hi0 = warp_max_f32(upper ? -INFINITY : hi), hi1 = warp_max_f32(upper ? hi : -INFINITY);
-                    lo = upper ? lo1 : lo0;
-                    hi = upper ? hi1 : hi0;
-                }
-                if (hi - lo > best_ext) { best_ext = hi - lo; best_lo = lo; dim = c; }
-            }
-            const float scale = best_ext > 0.f ? 33554426.f / best_ext : 0.f;
-            unsigned w[4];
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-                w[r] = 0x1ffffffu;
-                if (li[r] < n_here)
-                    w[r] = (unsigned)fminf(fmaxf((s_w[dim * kSuper + li[r]] - best_lo) * scale, 0.f), 33554426.f);
-                w[r] = (w[r] << 7) | (unsigned)li[r];
-            }
-            if (level == 0) sort_parts<kPart>(w, lane); else sort_parts<kPart / 2>(w, lane);
-#pragma unroll
-            for (int r = 0; r < 4; r++) li[r] = (int)(w[r] & 127u);
-        }
-#pragma unroll
-        for (int r = 0; r < 4; r++) id[r] = li[r] < n_here ? perm[pos0 + li[r]] : -1;
+        for (int r = 0; r < W; r++) id[r] = li[r] < n_here ? perm[pos0 + li[r]] : -1;
     }
 
-    // eight lanes hold a chunk now
-    const int chunk = chunk0 + local0 / 32 + (lane >> 3);
+    // 32 / W lanes hold a chunk now
+    constexpr int kLanes = 32 / W;
+    const int chunk = chunk0 + local0 / 32 + lane / kLanes;
     const bool have = chunk < chunk1;
-    const size_t at = (size_t)chunk * 32 + (lane & 7) * 4;
-    bool usable[4];
+    const size_t at = (size_t)chunk * 32 + (lane % kLanes) * W;
+    bool usable[W];
 #pragma unroll
-    for (int r = 0; r < 4; r++) {
+    for (int r = 0; r < W; r++) {
         usable[r] = id[r] >= 0;
         if (direction != nullptr && usable[r]) {
             const int d = direction[id[r]];
@@ -148,12 +168,15 @@ pack_tiles_kernel(const float *__restrict__ coords, int C, const int *__restrict
         }
     }
     if (have) {
-        int rank[4];
+        int rank[W];
 #pragma unroll
-        for (int r = 0; r < 4; r++) rank[r] = id[r] >= 0 ? rank_of[id[r]] : 0;
-        *reinterpret_cast<int4 *>(s.ids + at) = make_int4(id[0], id[1], id[2], id[3]);
-        *reinterpret_cast<int4 *>(s.ranks + at) = make_int4(rank[0], rank[1], rank[2], rank[3]);
-        if ((lane & 7) == 0) {
+        for (int r = 0; r < W; r++) rank[r] = id[r] >= 0 ? rank_of[id[r]] : 0;
+#pragma unroll
+        for (int r = 0; r < W; r += 4) {
+            *reinterpret_cast<int4 *>(s.ids + at + r) = make_int4(id[r], id[r + 1], id[r + 2], id[r + 3]);
+            *reinterpret_cast<int4 *>(s.ranks + at + r) = make_int4(rank[r], rank[r + 1], rank[r + 2], rank[r + 3]);
+        }
+        if (lane % kLanes == 0) {
             // hits beyond the last event take part in nothing
             const bool none = e == n_events;
             s.chunk_info[chunk] = make_int4(chunk0, none ? chunk0 : chunk1, o.event_super[e], o.event_super[e + 1]);
@@ -161,14 +184,14 @@ pack_tiles_kernel(const float *__restrict__ coords, int C, const int *__restrict
     }
     const float nan = __int_as_float(0x7fffffff);
     for (int u = 0; u < nv4; u++) {
-        float p[4][4], lo[4], hi[4];
+        float p[W][4], lo[4], hi[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const int d = u * 4 + k;
             lo[k] = INFINITY;
             hi[k] = -INFINITY;
 #pragma unroll
-            for (int r = 0; r < 4; r++) {
+            for (int r = 0; r < W; r++) {
                 p[r][k] = 0.f;
                 if (d < C && id[r] >= 0) p[r][k] = d < cd ? s_w[d * kSuper + li[r]] : coords[(size_t)id[r] * C + d];
                 if (usable[r]) {
@@ -179,15 +202,15 @@ pack_tiles_kernel(const float *__restrict__ coords, int C, const int *__restrict
                 }
             }
 #pragma unroll
-            for (int j = 1; j < 8; j <<= 1) {
+            for (int j = 1; j < kLanes; j <<= 1) {
                 lo[k] = fminf(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], j));
                 hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], j));
             }
         }
         if (have) {
 #pragma unroll
-            for (int r = 0; r < 4; r++) s.pts[(at + r) * nv4 + u] = make_float4(p[r][0], p[r][1], p[r][2], p[r][3]);
-            if ((lane & 7) == 0) {
+            for (int r = 0; r < W; r++) s.pts[(at + r) * nv4 + u] = make_float4(p[r][0], p[r][1], p[r][2], p[r][3]);
+            if (lane % kLanes == 0) {
                 s.chunk_box[((size_t)chunk * nv4 + u) * 2] = make_float4(lo[0], lo[1], lo[2], lo[3]);
                 s.chunk_box[((size_t)chunk * nv4 + u) * 2 + 1] = make_float4(hi[0], hi[1], hi[2], hi[3]);
             }
@@ -199,16 +222,16 @@ pack_tiles_kernel(const float *__restrict__ coords, int C, const int *__restrict
         }
     }
     __syncthreads();
-    if (warp < nv4) {
+    for (int u = warp; u < nv4; u += kWarpsHere) {
         float lo[4], hi[4];
 #pragma unroll
         for (int k = 0; k < 4; k++) {
-            lo[k] = warp_min_f32(s_lo[lane & 7][warp * 4 + k]);
-            hi[k] = warp_max_f32(s_hi[lane & 7][warp * 4 + k]);
+            lo[k] = warp_min_f32(s_lo[lane % kWarpsHere][u * 4 + k]);
+            hi[k] = warp_max_f32(s_hi[lane % kWarpsHere][u * 4 + k]);
         }
         if (lane == 0) {
-            s.super_box[((size_t)sup * nv4 + warp) * 2] = make_float4(lo[0], lo[1], lo[2], lo[3]);
-            s.super_box[((size_t)sup * nv4 + warp) * 2 + 1] = make_float4(hi[0], hi[1], hi[2], hi[3]);
+            s.super_box[((size_t)sup * nv4 + u) * 2] = make_float4(lo[0], lo[1], lo[2], lo[3]);
+            s.super_box[((size_t)sup * nv4 + u) * 2 + 1] = make_float4(hi[0], hi[1], hi[2], hi[3]);
         }
     }
 }
@@ -220,8 +243,14 @@ int build_tiles(const float *coords, int n_coords, const int *curve_perm, const 
 {
     if (n_vert <= 0) return HGC_OK;
     const size_t smem = sizeof(float) * kSuper * (n_coords < kSplitDims ? n_coords : kSplitDims);
-    HGC_CUDA_TRY(launch_overlapped(n_vert, pack_tiles_kernel, (int)tile_supers_cap(n_vert, n_events), kPackThreads, smem, stream, coords, n_coords, curve_perm, rank_of, direction, n_events, o, s, (n_coords + 3) / 4,
-            (int)(tile_chunks_cap(n_vert, n_events) * 32)));
+#define HGC_PACK(W) HGC_CUDA_TRY(launch_overlapped(n_vert, pack_tiles_kernel<W>, (int)tile_supers_cap(n_vert, n_events), kSuper / W, smem, stream, coords, n_coords, curve_perm, rank_of, direction, n_events, o, s, (n_coords + 3) / 4, (int)(tile_chunks_cap(n_vert, n_events) * 32)))
+    // Parts of 256 where an event has many more hits than the curve has cells (6 bits per coordinate or fewer), which leaves runs
+    // of 128 without an order of their own; elsewhere the longer chain per warp costs more.  Search and orders, us with parts of 128 /
+    // 256: 300k hits 5 dimensions K = 12 1678 / 1633, 6 dimensions K = 64 3218 / 3181, 1 M 16138 / 15806; 100k 5 dimensions K = 12
+    // 488 / 508; 300k 3 dimensions 499 / 499; 700 hits 36 / 43.
+    if (n_coords >= 5 && n_vert / n_events >= 150000) HGC_PACK(8);
+    else HGC_PACK(4);
+#undef HGC_PACK
     HGC_LAUNCH_CHECK();
     return HGC_OK;
 }

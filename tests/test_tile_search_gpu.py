@@ -98,3 +98,23 @@ def test_small_batches_have_the_order_of_large_ones(cuda, dims, sizes):
     i1, d1, s1 = BinnedSelectKnn(9, T(np.concatenate([c, more]), cuda), T(np.append(rs, n + 5000).astype(np.int32), cuda), **kw)
     assert np.array_equal(N(s0), N(s1)[:n])
     assert np.array_equal(N(i0), N(i1)[:n]) and np.array_equal(N(d0).view(np.uint32), N(d1)[:n].view(np.uint32))
+
+
+def test_a_large_event_in_five_dimensions(cuda, oracle):
+    """Parts of 256 hits are split into chunks where events hold 150k hits and more; brute force for a sample."""
+    from hgcalml_b200.binned_select_knn_op import BinnedSelectKnn
+    import torch
+    n, K = 150211, 20
+    c, _, rs = synth.shower_batch([n], dims=5, n_feat=0, with_features=False, seed=3)
+    idx, d2, sorting = BinnedSelectKnn(K, T(c, cuda), T(rs, cuda), return_sorting=True)
+    assert torch.equal(sorting.sort().values, torch.arange(n, dtype=torch.int32, device=cuda))
+    x = T(c, cuda)
+    rows = torch.arange(0, n, 997, device=cuda)
+    d = torch.zeros((len(rows), n), device=cuda)
+    for k in range(5):  # in coordinate order, unfused, as the op sums
+        t = x[rows, k][:, None] - x[:, k][None]
+        d = d + t * t
+    d[torch.arange(len(rows), device=cuda), rows] = -1.
+    want, _ = torch.topk(d, K, largest=False)
+    assert torch.equal(want.sort(dim=1).values[:, 1:], d2[rows][:, 1:]) and torch.equal(idx[rows, 0].long(), rows)
+    assert torch.equal(torch.gather(d, 1, idx[rows].long())[:, 1:], d2[rows][:, 1:])
