@@ -38,7 +38,7 @@ UNIT = "hits/s"
 NCU = {
     "accumulate_knn": {"dram_bytes_per_hit": 1755, "algorithmic_bytes_per_hit": 1536},
     "accumulate_knn_no_argmax": {"dram_bytes_per_hit": 1296, "algorithmic_bytes_per_hit": 1280},
-    "binned_select_knn": {"dram_bytes_per_hit": 530, "issue_active_pct": 73.7, "warp_instructions_per_query": 2110},
+    "binned_select_knn": {"dram_bytes_per_hit": 530, "issue_active_pct": 75.4, "warp_instructions_per_query": 2080},
     "select_knn_op_level": {"dram_bytes_per_hit": 433, "issue_active_pct": 90.4, "warp_instructions_per_query": 5715},
 }
 

@@ -2,7 +2,7 @@
 // code; instantiated per coordinate width in select_knn_tile_nv*.cu).
 //
 // Layout (hit_order.cu, pack_tiles_kernel).  The hits of an event follow a Hilbert curve through all their
-// coordinates; runs of 1024 (super-chunks) are cut by medians into chunks of 32 hits.  A chunk never
+// coordinates; parts of 128 or 256 are cut by medians into chunks of 32 hits, 1024 make a super-chunk.  A chunk never
 // straddles events (the last one of an event is padded with NaN points, which no comparison accepts).  Chunks and
 // super-chunks have bounding boxes over all coordinates.
 //
