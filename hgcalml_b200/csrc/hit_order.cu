@@ -250,27 +250,29 @@ __device__ __forceinline__ unsigned equal_digits(unsigned digit, bool ok)
 // Small batches: range, grid, event layout and both orders in one launch, a block per event and order, the sort inside its
 // shared memory.  Each block finds the range of the whole batch for itself, which is a few loads per thread.
 // A chain of six launches is mostly launches and first touches here; search with both orders, us with the chain / with this
-// kernel: 700 hits 53 / 34, 2048 55 / 43, 4096 59 / 54, 31 events of 100 50 / 34.  4096 hits are what a block's shared memory holds
-// without asking for more, and where the gain ends; one block per event of any size because the host does not know the sizes,
-// and no more events than a warp lays out.
-constexpr int kSmallHits = 4096, kSmallEvents = 31, kSmallThreads = 512, kSmallWarps = kSmallThreads / kWarp;
-constexpr int kSmallItems = kSmallHits / kSmallThreads;
+// kernel: 700 hits 53 / 34, 2048 55 / 43, 4096 59 / 54, 31 events of 100 50 / 34, 30 of 200 52 / 39, three of 2000 to 3000 66 / 60.  One
+// block per event of any size because the host does not know the sizes, so that more than 4096 hits (512 threads, eight hits each)
+// take it, with 1024 threads, only where the events are small on average: one event of 8192 hits 82 / 88.  No more events than a
+// warp lays out.
+constexpr int kSmallHits = 8192, kSmallMean = 2800, kSmallEvents = 31, kSmallItems = 8;
 constexpr int kSmallBits = 9, kSmallDigits = 1 << kSmallBits;
 
-template <int D, int B>
+template <int D, int B, int kSmallThreads>
 __global__ void __launch_bounds__(kSmallThreads)
 order_small_kernel(const float *__restrict__ coords, int C, int n_dims, int n_vert, const int *__restrict__ row_splits, int n_rs,
                    int n_bins, int n_neigh, HitOrder o, int *__restrict__ bin_perm, int *__restrict__ rank,
                    int *__restrict__ curve_perm, unsigned *status)
 {
     pdl_begin();
+    constexpr int kSmallWarps = kSmallThreads / kWarp, kHits = kSmallThreads * kSmallItems;
     __shared__ GridParams s_grid;
     __shared__ float s_mn[kSmallWarps][D], s_mx[kSmallWarps][D];
     __shared__ int s_first, s_end, s_warp[kSmallDigits / 64];
-    __shared__ unsigned s_count[kSmallWarps][kSmallDigits / 2];  // two digits per word: places of a digit in the warps before
+    extern __shared__ unsigned s_small[];
+    unsigned (*s_count)[kSmallDigits / 2] = reinterpret_cast<unsigned (*)[kSmallDigits / 2]>(s_small);  // two digits per word: places of a digit in the warps before
     __shared__ int s_start[kSmallDigits];
-    __shared__ unsigned s_key[kSmallHits];
-    __shared__ unsigned short s_hit[kSmallHits];
+    unsigned *s_key = s_small + kSmallWarps * (kSmallDigits / 2);
+    unsigned short *s_hit = reinterpret_cast<unsigned short *>(s_key + kHits);
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int order = blockIdx.x & 1, e = blockIdx.x >> 1, n_events = n_rs - 1;
     float mn[D], mx[D];
@@ -319,7 +321,7 @@ order_small_kernel(const float *__restrict__ coords, int C, int n_dims, int n_ve
     if (e == n_events && t == 0) flag_status(status, HGC_STATUS_FLAT_BIN_OVERFLOW);
     // keys: scratch of the locality code lies where the counts will be
     unsigned short (*frac)[kSmallThreads] = reinterpret_cast<unsigned short (*)[kSmallThreads]>(&s_count[0][0]);
-    static_assert(sizeof(s_count) >= sizeof(unsigned short) * kMaxBinDims * kSmallThreads, "");
+    static_assert(sizeof(unsigned) * kSmallWarps * (kSmallDigits / 2) >= sizeof(unsigned short) * kMaxBinDims * kSmallThreads, "");
     for (int i = t; i < n; i += kSmallThreads) {
         float x[D];
 #pragma unroll
@@ -398,6 +400,20 @@ order_small_kernel(const float *__restrict__ coords, int C, int n_dims, int n_ve
     }
 }
 
+template <int D, int B, int T>
+int launch_small(const float *coords, int n_coords, int n_bin_dims, int n_vert, const int *row_splits, int n_rs, int n_bins, int n_neigh,
+                 const HitOrder &o, int *bin_perm, int *rank, int *curve_perm, unsigned *status, cudaStream_t stream)
+{
+    const auto kernel = order_small_kernel<D, B, T>;
+    const size_t smem = sizeof(unsigned) * (T / kWarp) * (kSmallDigits / 2) + (sizeof(unsigned) + sizeof(unsigned short)) * T * kSmallItems;
+    // (set on every call: the setting belongs to the current device)
+    if (T > 512) HGC_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    HGC_CUDA_TRY(launch_pdl(kernel, 2 * n_rs, T, smem, stream, coords, n_coords, n_bin_dims, n_vert, row_splits, n_rs, n_bins, n_neigh, o,
+                            bin_perm, rank, curve_perm, status));
+    HGC_LAUNCH_CHECK();
+    return HGC_OK;
+}
+
 }  // namespace
 
 int range_and_layout(const float *coords, int n_coords, int n_bin_dims, const int *row_splits, int n_rs, int n_bins,
@@ -417,9 +433,10 @@ int order_hits(const float *coords, int n_coords, int n_bin_dims, const int *row
     if (bin_bits + kSubBits > 32) return HGC_ERR_UNSUPPORTED;
     const int n_events = n_rs - 1;
     const int n_all = n_coords < kMaxBinDims ? n_coords : kMaxBinDims;
-    if (n_vert <= kSmallHits && n_events <= kSmallEvents && bin_bits > 0) {
+    if (n_vert <= (n_vert / n_events <= kSmallMean ? kSmallHits : kSmallHits / 2) && n_events <= kSmallEvents && bin_bits > 0) {
 #define HGC_SMALL(D, B)                                                                                            \
-    case D: HGC_CUDA_TRY(launch_pdl(order_small_kernel<D, B>, 2 * n_rs, kSmallThreads, 0, stream, coords, n_coords, n_bin_dims, n_vert, row_splits, n_rs, n_bins, n_neigh, o, bin_perm, rank, curve_perm, status)); break
+    case D: if (int rc = n_vert <= 512 * kSmallItems ? launch_small<D, B, 512>(coords, n_coords, n_bin_dims, n_vert, row_splits, n_rs, n_bins, n_neigh, o, bin_perm, rank, curve_perm, status, stream) \
+                                                     : launch_small<D, B, 1024>(coords, n_coords, n_bin_dims, n_vert, row_splits, n_rs, n_bins, n_neigh, o, bin_perm, rank, curve_perm, status, stream)) return rc; break
         switch (n_all) {
             HGC_SMALL(2, 13);
             HGC_SMALL(3, 9);
@@ -431,7 +448,6 @@ int order_hits(const float *coords, int n_coords, int n_bin_dims, const int *row
             default: return HGC_ERR_UNSUPPORTED;
         }
 #undef HGC_SMALL
-        HGC_LAUNCH_CHECK();
         return HGC_OK;
     }
     if (int rc = range_and_layout(coords, n_coords, n_bin_dims, row_splits, n_rs, n_bins, n_neigh, n_vert, o, status, stream))

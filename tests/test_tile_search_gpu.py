@@ -83,19 +83,19 @@ def test_coinciding_points(cuda, oracle, K):
 
 
 @pytest.mark.parametrize("dims", [2, 3, 4, 5, 6, 7, 8])
-@pytest.mark.parametrize("sizes", [[1], [33, 0, 479], [512], [513], [2049, 1, 30], [4096], [100] * 31])
+@pytest.mark.parametrize("sizes", [[1], [33, 0, 479], [512], [513], [2049, 1, 30], [4096], [100, 8000, 92], [1, 8190, 0, 1], [100] * 31, [264] * 31])
 def test_small_batches_have_the_order_of_large_ones(cuda, dims, sizes):
-    """Batches of up to 4096 hits in 31 events are ordered by one kernel; the same hits in front of others, which leave the
+    """Batches of up to 8192 hits in 31 events are ordered by one kernel; the same hits in front of others, which leave the
     range of the batch as it is, by the chain of kernels for any size."""
     from hgcalml_b200.binned_select_knn_op import BinnedSelectKnn
     rng = np.random.default_rng(dims + len(sizes))
     n = sum(sizes)
     c = rng.standard_normal((n, dims), dtype=np.float32)
-    more = c[rng.integers(0, n, 5000)]
+    more = c[rng.integers(0, n, 9000)]
     rs = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int32)
     kw = dict(n_bins=7, return_sorting=True)
     i0, d0, s0 = BinnedSelectKnn(9, T(c, cuda), T(rs, cuda), **kw)
-    i1, d1, s1 = BinnedSelectKnn(9, T(np.concatenate([c, more]), cuda), T(np.append(rs, n + 5000).astype(np.int32), cuda), **kw)
+    i1, d1, s1 = BinnedSelectKnn(9, T(np.concatenate([c, more]), cuda), T(np.append(rs, n + 9000).astype(np.int32), cuda), **kw)
     assert np.array_equal(N(s0), N(s1)[:n])
     assert np.array_equal(N(i0), N(i1)[:n]) and np.array_equal(N(d0).view(np.uint32), N(d1)[:n].view(np.uint32))
 
