@@ -74,9 +74,12 @@ select_grad_kernel(const float *__restrict__ grad_dist, const int *__restrict__ 
 #pragma unroll
         for (int u = 0; u < U; u++)
             if (p + u < end) {
-                // (2 g) d, exact in double, rounded to float: the float product, and doubling is exact
+                // (2 g) d, exact in double, rounded to float: the float product with one factor doubled, which is exact as long
+                // as it does not overflow.  d is doubled below one, g above: where 2 g overflows then, so does the product.
                 const float d = __fsub_rn(xm, x[u]);
-                val = __fadd_rn(val, __fmul_rn(g[u], d + d));
+                const bool near = fabsf(d) < 1.f;
+                const float a = near ? d : g[u], b = near ? g[u] : d;
+                val = __fadd_rn(val, __fmul_rn(a + a, b));
             }
     }
     grad_coord[(size_t)m * C + c] = val;

@@ -159,3 +159,23 @@ def test_rows_of_whole_and_of_part_vectors(cuda, oracle, K, F):
         rw, rf = oracle.op_push_knn_grad(g1, w, feat, idx)
         gw, gf = PushKnnGrad(put(g1), put(w), put(feat), table)
         assert np.array_equal(bits(N(gw)), bits(rw)) and np.array_equal(bits(N(gf)), bits(rf))
+
+
+@pytest.mark.parametrize("K", [1, 6, 8])
+def test_select_knn_grad_over_the_range_of_floats(cuda, oracle, K):
+    """Differences whose double is no float any more, subnormal ones, and gradients at both ends and of zero."""
+    from hgcalml_b200.binned_select_knn_op import SelectKnnGrad
+    n = 600
+    rng = np.random.default_rng(K)
+    idx = rng.integers(-1, n, (n, K)).astype(np.int32)
+    powers = np.float32(2.) ** rng.integers(-149, 128, (2, n, max(K, 4))).astype(np.float32)
+    c = (powers[0, :, :4] * rng.uniform(-1., 1., (n, 4))).astype(np.float32)
+    c[::5], c[1::5] = np.float32(1.6e38), np.float32(-1.6e38)
+    g = (powers[1, :, :K] * rng.uniform(-1., 1., (n, K))).astype(np.float32)
+    g[::3] *= np.float32(1e-30)
+    g[1::3] = 0.
+    ref = oracle.op_select_knn_grad(g, idx, c)
+    assert np.isfinite(ref).any() and (ref != 0.).any()
+    got = N(SelectKnnGrad(T(g, cuda), T(idx, cuda), None, T(c, cuda)))
+    nan = np.isnan(ref)
+    assert np.array_equal(nan, np.isnan(got)) and np.array_equal(bits(got[~nan]), bits(ref[~nan]))
