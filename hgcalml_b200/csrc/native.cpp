@@ -225,14 +225,22 @@ int bias_act(const Tensor &y, const Tensor &bias, bool relu)
     return hgc_bias_act(data<float>(y), data<float>(bias), (int)y.size(0), (int)y.size(1), relu, stream_of(y));
 }
 
+// Products of float32 in float32.  (allowTF32CuBLAS() asks the same, but throws where the caller chose the precision through
+// torch.backends.fp32_precision or torch.backends.cuda.matmul.fp32_precision.)
+bool full_precision()
+{
+    const at::Float32Precision p = at::globalContext().float32Precision(at::Float32Backend::CUDA, at::Float32Op::MATMUL);
+    return p == at::Float32Precision::NONE || p == at::Float32Precision::IEEE;
+}
+
 // act(x kernel + bias) in one kernel, or None where the tensor operations would do more than that or the library's GEMM is
 // the faster one
 MaybeTensor dense(const Tensor &x, const Tensor &kernel, const MaybeTensor &bias, bool relu)
 {
     if (operations_are_seen() || at::impl::torch_function_mode_enabled() ||
-        at::autocast::is_autocast_enabled(at::kCUDA) || at::globalContext().allowTF32CuBLAS() ||
+        at::autocast::is_autocast_enabled(at::kCUDA) ||
         !values_only(x) || !values_only(kernel) || x.dim() != 2 || kernel.dim() != 2 || !x.is_contiguous() ||
-        !kernel.is_contiguous() || x.size(1) != kernel.size(0))
+        !kernel.is_contiguous() || x.size(1) != kernel.size(0) || !full_precision())
         return std::nullopt;
     if (bias.has_value() && (!values_only(*bias) || bias->dim() != 1 || bias->size(0) != kernel.size(1) || !bias->is_contiguous()))
         return std::nullopt;

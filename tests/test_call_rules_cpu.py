@@ -5,6 +5,7 @@ import io
 import threading
 import weakref
 
+import pytest
 import torch
 
 
@@ -76,3 +77,17 @@ def test_pipelines_given_up_by_the_garbage_collector_wait_for_nothing(monkeypatc
     gc.collect()
     idle = [s for pool in P._idle_streams.values() for s in pool]
     assert len(set(map(id, idle))) == len(idle)  # no triple is there twice
+
+
+@pytest.mark.parametrize("precision", ["tf32", "ieee", "none"])
+@pytest.mark.parametrize("where", [torch.backends, torch.backends.cuda.matmul], ids=["everywhere", "products"])
+def test_a_precision_chosen_by_the_caller_is_no_error(where, precision):
+    """Asked about a layer, the host binding leaves it to the tensor operations and raises nothing."""
+    from hgcalml_b200 import _capi as C
+    before = where.fp32_precision
+    try:
+        where.fp32_precision = precision
+        got = C.native.dense(torch.ones((8, 4)), torch.ones((4, 4)), None, True)
+    finally:
+        where.fp32_precision = before
+    assert got is None

@@ -125,3 +125,27 @@ def test_precisions_that_the_caller_chose_are_the_library_s(cuda):
         assert torch.equal(layer(x), torch.relu(x @ layer.kernel + layer.bias))
     finally:
         torch.backends.cuda.matmul.allow_tf32 = False
+
+
+@pytest.mark.parametrize("setting", ["ieee", "tf32", "tf32 everywhere", "high"])
+def test_precisions_chosen_through_any_of_torch_s_settings(cuda, setting):
+    layer, _ = _layer(cuda, n_in=64, n_out=64)
+    layer.requires_grad_(False)
+    x = torch.randn((3000, 64), generator=torch.Generator(device=cuda).manual_seed(2), device=cuda)
+    plain = torch.relu(x @ layer.kernel + layer.bias)
+    try:
+        if setting == "high":
+            torch.set_float32_matmul_precision("high")
+        elif setting == "tf32 everywhere":
+            torch.backends.fp32_precision = "tf32"
+        else:
+            torch.backends.cuda.matmul.fp32_precision = setting
+        want, got = torch.relu(x @ layer.kernel + layer.bias), layer(x)
+        layer.requires_grad_(True)
+        trained = layer(x)
+    finally:
+        torch.set_float32_matmul_precision("highest")
+        torch.backends.fp32_precision = "none"
+        torch.backends.cuda.matmul.fp32_precision = "none"
+    assert torch.equal(got, want) and torch.equal(trained, want)
+    assert torch.equal(want, plain) == (setting == "ieee")
