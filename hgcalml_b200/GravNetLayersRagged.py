@@ -104,8 +104,9 @@ class _Dense(torch.nn.Module):
         relu = self.activation is torch.relu
         plain = relu or self.activation is _linear
         if plain and type(x) in _PLAIN and type(kernel) in _PLAIN and (bias is None or type(bias) in _PLAIN) and x.is_cuda:
-            y = C.native.dense(x, kernel, bias, relu)
-            if y is not None:
+            y, rc = C.native.dense(x, kernel, bias, relu)
+            if rc != C.NOT_TAKEN:
+                C.check(rc, "dense layer")
                 return y
         y = x @ kernel
         if bias is not None:

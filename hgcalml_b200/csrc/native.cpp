@@ -25,6 +25,8 @@ typedef std::optional<Tensor> MaybeTensor;
 template <typename T> T *data(const Tensor &t) { return static_cast<T *>(t.data_ptr()); }
 template <typename T> T *data(const MaybeTensor &t) { return t.has_value() ? static_cast<T *>(t->data_ptr()) : nullptr; }
 
+bool aligned16(const Tensor &t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0; }
+
 hgc_stream_t stream_of(const Tensor &t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
 
 Tensor like(const Tensor &t, at::IntArrayRef sizes, at::ScalarType type) { return at::empty(sizes, t.options().dtype(type)); }
@@ -233,24 +235,24 @@ bool full_precision()
     return p == at::Float32Precision::NONE || p == at::Float32Precision::IEEE;
 }
 
-// act(x kernel + bias) in one kernel, or None where the tensor operations would do more than that or the library's GEMM is
-// the faster one
-MaybeTensor dense(const Tensor &x, const Tensor &kernel, const MaybeTensor &bias, bool relu)
+// (act(x kernel + bias), status) in one kernel; kNotTaken where the tensor operations would do more than that, hgc_dense does not
+// take the rows (whole 16-byte vectors) or the library's GEMM is the faster one
+std::tuple<MaybeTensor, int> dense(const Tensor &x, const Tensor &kernel, const MaybeTensor &bias, bool relu)
 {
+    const std::tuple<MaybeTensor, int> not_taken{std::nullopt, kNotTaken};
     if (operations_are_seen() || at::impl::torch_function_mode_enabled() ||
         at::autocast::is_autocast_enabled(at::kCUDA) ||
         !values_only(x) || !values_only(kernel) || x.dim() != 2 || kernel.dim() != 2 || !x.is_contiguous() ||
         !kernel.is_contiguous() || x.size(1) != kernel.size(0) || !full_precision())
-        return std::nullopt;
+        return not_taken;
     if (bias.has_value() && (!values_only(*bias) || bias->dim() != 1 || bias->size(0) != kernel.size(1) || !bias->is_contiguous()))
-        return std::nullopt;
+        return not_taken;
     const int64_t n = x.size(0), n_in = x.size(1), n_out = kernel.size(1);
-    if (!dense_is_faster(n, n_in, n_out)) return std::nullopt;
+    if (n_in % 4 != 0 || !aligned16(x) || !dense_is_faster(n, n_in, n_out)) return not_taken;
     Tensor y = like(x, {n, n_out}, at::kFloat);
     const int rc = hgc_dense(data<float>(x), data<float>(kernel), data<float>(bias), data<float>(y), (int)n, (int)n_in, (int)n_out, relu,
                              stream_of(x));
-    if (rc != HGC_OK) return std::nullopt;  // shapes that it does not take
-    return y;
+    return {y, rc};
 }
 
 // out[:, column:] = x, likewise

@@ -87,7 +87,7 @@ def test_a_precision_chosen_by_the_caller_is_no_error(where, precision):
     before = where.fp32_precision
     try:
         where.fp32_precision = precision
-        got = C.native.dense(torch.ones((8, 4)), torch.ones((4, 4)), None, True)
+        got, rc = C.native.dense(torch.ones((8, 4)), torch.ones((4, 4)), None, True)
     finally:
         where.fp32_precision = before
-    assert got is None
+    assert got is None and rc == C.NOT_TAKEN

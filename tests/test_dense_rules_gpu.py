@@ -149,3 +149,39 @@ def test_precisions_chosen_through_any_of_torch_s_settings(cuda, setting):
         torch.backends.cuda.matmul.fp32_precision = "none"
     assert torch.equal(got, want) and torch.equal(trained, want)
     assert torch.equal(want, plain) == (setting == "ieee")
+
+
+def test_a_failed_launch_is_no_reason_for_the_library(cuda, monkeypatch):
+    from hgcalml_b200 import _capi as C
+    layer, x = _layer(cuda)
+    native = C.native
+
+    class Failing:
+        def __getattr__(self, name):
+            return getattr(native, name)
+
+        def dense(self, *args):
+            return None, -4  # HGC_ERR_CUDA
+    monkeypatch.setattr(C, "native", Failing())
+    with torch.no_grad(), pytest.raises(C.HgcError):
+        layer(x)
+
+
+@pytest.mark.parametrize("n,n_in,n_out,own", [(3000, 64, 64, 1), (20, 64, 64, 1), (3000, 22, 8, 0), (3000, 512, 512, 0)])
+def test_which_layers_take_the_kernel(cuda, n, n_in, n_out, own):
+    """The kernel alone where it is taken; elsewhere the library's product and one pass for bias and activation."""
+    from hgcalml_b200 import _capi as C
+    layer, _ = _layer(cuda, n_in=n_in, n_out=n_out)
+    x = torch.randn((n, n_in), generator=torch.Generator(device=cuda).manual_seed(4), device=cuda)
+    with torch.no_grad():
+        before = C.lib.hgc_launch_count()
+        y, rc = C.native.dense(x, layer.kernel, layer.bias, True)
+        assert C.lib.hgc_launch_count() - before == own and rc == (C.HGC_OK if own else C.NOT_TAKEN)
+        before = C.lib.hgc_launch_count()
+        z = layer(x)
+        assert C.lib.hgc_launch_count() - before == 1
+        if own:
+            assert torch.equal(y, z)
+            shifted = torch.empty(x.numel() + 1, device=cuda)[1:].view(x.shape).copy_(x)
+            assert C.native.dense(shifted, layer.kernel, layer.bias, True)[1] == C.NOT_TAKEN
+            assert torch.allclose(layer(shifted), z, rtol=1e-5, atol=1e-5)
