@@ -191,9 +191,8 @@ template <int TM, int TN, bool RELU>
 int launch_rows(const float *x, int K, const float *w, int n_out, const float *bias, float *y, int n_rows, cudaStream_t stream)
 {
     const auto kernel = dense_kernel<TM, TN, RELU>;
-    const size_t smem = sizeof(float) * kStages * (16 * TM * kPitch + kDepth * 8 * TN);
-    // (set on every call: the setting belongs to the current device)
-    if (smem > 48 * 1024) HGC_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr size_t smem = sizeof(float) * kStages * (16 * TM * kPitch + kDepth * 8 * TN);
+    static_assert(smem <= 48 * 1024, "more needs cudaFuncSetAttribute");
     const bool vec_out = n_out % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & 15u) == 0;
     HGC_CUDA_TRY(launch_pdl(kernel, dim3(div_up(n_rows, 16 * TM), div_up(n_out, 8 * TN)), kThreads, smem, stream, x, K, w, n_out, bias, y, n_rows,
                             n_out % 4 == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0, vec_out));
@@ -236,8 +235,8 @@ extern "C" int hgc_dense(const float *d_x, const float *d_w, const float *d_bias
     if (n < 0 || n_in < 1 || n_out < 0) return HGC_ERR_INVALID_ARGUMENT;
     if (n == 0 || n_out == 0) return HGC_OK;
     if (!d_x || !d_w || !d_y) return HGC_ERR_INVALID_ARGUMENT;
-    // rows of whole 16-byte vectors, and w for 64 columns inside a block's shared memory
-    if (n_in % 4 != 0 || (reinterpret_cast<uintptr_t>(d_x) & 15u) != 0 || n_in > 512) return HGC_ERR_UNSUPPORTED;
+    // rows of whole 16-byte vectors, which is how they are staged
+    if (n_in % 4 != 0 || (reinterpret_cast<uintptr_t>(d_x) & 15u) != 0) return HGC_ERR_UNSUPPORTED;
     return relu ? run_dense<true>(d_x, n_in, d_w, n_out, d_bias, d_y, n, stream)
                 : run_dense<false>(d_x, n_in, d_w, n_out, d_bias, d_y, n, stream);
 }

@@ -213,7 +213,7 @@ int hgc_gravnet_collect(
         hgc_stream_t stream);
 
 /* A dense layer in float32: y[n, n_out] = x[n, n_in] w[n_in, n_out], plus bias[n_out] unless NULL, then max(y, 0) when relu is
- * set.  n_in: a multiple of 4, at most 512, d_x on a 16-byte boundary; HGC_ERR_UNSUPPORTED otherwise. */
+ * set.  n_in: a multiple of 4, d_x on a 16-byte boundary; HGC_ERR_UNSUPPORTED otherwise. */
 int hgc_dense(const float *d_x, const float *d_w, const float *d_bias, float *d_y, int n, int n_in, int n_out, int relu,
               hgc_stream_t stream);
 

@@ -185,3 +185,17 @@ def test_which_layers_take_the_kernel(cuda, n, n_in, n_out, own):
             shifted = torch.empty(x.numel() + 1, device=cuda)[1:].view(x.shape).copy_(x)
             assert C.native.dense(shifted, layer.kernel, layer.bias, True)[1] == C.NOT_TAKEN
             assert torch.allclose(layer(shifted), z, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("n", [50, 49200])
+@pytest.mark.parametrize("n_out", [3, 7, 12, 30, 70])
+def test_dense_kernel_with_long_rows(cuda, n, n_out):
+    from hgcalml_b200 import _capi as C
+    n_in = 516
+    g = torch.Generator(device=cuda).manual_seed(n + n_out)
+    x, w = torch.randn((n, n_in), generator=g, device=cuda), torch.randn((n_in, n_out), generator=g, device=cuda)
+    y = torch.empty((n, n_out), device=cuda)
+    C.check(C.lib.hgc_dense(C.ptr(x), C.ptr(w), None, C.ptr(y), n, n_in, n_out, 0, C.stream_of(x)), "dense")
+    # n_in fused multiply-adds, each off by half an ulp of at most the sum of the terms' sizes
+    assert ((y.double() - x.double() @ w.double()).abs() <= n_in * 2. ** -24 * (x.double().abs() @ w.double().abs())).all()
+    assert C.lib.hgc_dense(C.ptr(x), C.ptr(w), None, C.ptr(y), n, 514, n_out, 0, C.stream_of(x)) == -3
