@@ -21,30 +21,20 @@ enum EdgeSum {
     kSumMeanMax   // the same plus, where the target is the maximum of (i, f), x[i,F+f] * w[e]
 };
 
-template <int VW> struct EdgeVec { float v[VW]; };
-template <int VW>
-__device__ __forceinline__ EdgeVec<VW> load_edge_vec(const float *p)
+constexpr int VW = 4;  // features per lane of edge_sum_kernel
+struct EdgeVec { float v[VW]; };
+__device__ __forceinline__ EdgeVec load_edge_vec(const float *p)
 {
-    EdgeVec<VW> r;
-    if constexpr (VW == 4) {
-        const float4 q = __ldg(reinterpret_cast<const float4 *>(p));
-        r.v[0] = q.x; r.v[1] = q.y; r.v[2] = q.z; r.v[3] = q.w;
-    } else {
-        static_assert(VW == 2, "vectors of two or four");
-        const float2 q = __ldg(reinterpret_cast<const float2 *>(p));
-        r.v[0] = q.x; r.v[1] = q.y;
-    }
-    return r;
+    const float4 q = __ldg(reinterpret_cast<const float4 *>(p));
+    return {{q.x, q.y, q.z, q.w}};
 }
 
 // The same if any bit of `wanted` is set; otherwise, and (not WHOLE) in places whose bit is not set, the values do not count.
-template <int VW, bool WHOLE>
-__device__ __forceinline__ EdgeVec<VW> load_edge_vec_if(const float *p, unsigned wanted)
+template <bool WHOLE>
+__device__ __forceinline__ EdgeVec load_edge_vec_if(const float *p, unsigned wanted)
 {
-    EdgeVec<VW> r;
-#pragma unroll
-    for (int v = 0; v < VW; v++) r.v[v] = 0.f;
-    if constexpr (WHOLE && VW == 4) {
+    EdgeVec r = {{0.f, 0.f, 0.f, 0.f}};
+    if constexpr (WHOLE) {
         asm volatile("{ .reg .pred q; setp.ne.u32 q, %5, 0; @q ld.global.nc.v4.f32 {%0,%1,%2,%3}, [%4]; }"
                      : "+f"(r.v[0]), "+f"(r.v[1]), "+f"(r.v[2]), "+f"(r.v[3]) : "l"(p), "r"(wanted));
     } else {
@@ -67,7 +57,7 @@ __device__ __forceinline__ EdgeVec<VW> load_edge_vec_if(const float *p, unsigned
 // 0.91, its 77 registers leaving 24 warps per SM.  Half of the gathered lines miss L1 and resident warps hide that better than
 // rows in flight: 16 lanes x 4 features with 2 rows and 40 warps per SM beat 4 rows (+1 %), 8 rows (+20 %), a warp x 2 features
 // (+10 %), and 64 warps, which spill (+27 %).  PushKnn, 200k hits, K = 40, F = 32: 433 -> 341 us.
-template <int LPT, int VW, int MODE, bool SCALE, bool HVEC>
+template <int LPT, int MODE, bool SCALE, bool HVEC>
 __global__ void __launch_bounds__(256, 5)
 edge_sum_kernel(const float *__restrict__ rows, int ldr, const float *__restrict__ maxima, int ldm,
                 const float *__restrict__ weights, const unsigned *__restrict__ flags, const int *__restrict__ nidx,
@@ -118,7 +108,7 @@ edge_sum_kernel(const float *__restrict__ rows, int ldr, const float *__restrict
         __syncwarp();
         // two rows at a time; while every target of the warp has two more edges, without a test per target
         auto two = [&](int q0, auto tail) {
-            EdgeVec<VW> g[2], h[2];
+            EdgeVec g[2], h[2];
             float w[2];
             unsigned b[2];
 #pragma unroll
@@ -127,10 +117,10 @@ edge_sum_kernel(const float *__restrict__ rows, int ldr, const float *__restrict
                 w[q] = __uint_as_float(ed.y);
                 b[q] = 0u;
                 if (!tail.value || q0 + q < n_here) {
-                    g[q] = load_edge_vec<VW>(row0 + (size_t)ed.x * ldr);
+                    g[q] = load_edge_vec(row0 + (size_t)ed.x * ldr);
                     if (MODE == kSumMeanMax) {
                         b[q] = ((LPT * VW > 32 && f >= 32 ? ed.w : ed.z) >> (f & 31)) & flag_mask;
-                        h[q] = load_edge_vec_if<VW, HVEC>(max0 + (size_t)ed.x * ldm, b[q]);
+                        h[q] = load_edge_vec_if<HVEC>(max0 + (size_t)ed.x * ldm, b[q]);
                     }
                 }
             }
@@ -156,8 +146,7 @@ edge_sum_kernel(const float *__restrict__ rows, int ldr, const float *__restrict
                 }
             }
         };
-        const int n_all = T == 1 ? n_here : max(0, __reduce_min_sync(0xffffffffu, n_here));
-        const int n_max = T == 1 ? n_here : __reduce_max_sync(0xffffffffu, n_here);
+        const int n_all = max(0, __reduce_min_sync(0xffffffffu, n_here)), n_max = __reduce_max_sync(0xffffffffu, n_here);
         int q0 = 0;
         for (; q0 + 2 <= n_all; q0 += 2) two(q0, std::false_type());
         for (; q0 < n_max; q0 += 2) two(q0, std::true_type());
@@ -350,8 +339,8 @@ int launch_edge_sum_slab(const float *x, int ldx, const float *weights, const un
         rows = scratch;
     }
     const bool scale = MODE != kSumPlain && rows != scratch;  // only rows that are whole vectors are scaled
-#define HGC_SUM(LPT, VW, S, H) HGC_CUDA_TRY(launch_overlapped(n_vert, edge_sum_kernel<LPT, VW, MODE, S, H>, div_up(n_vert, 8 * (32 / LPT)), 256, 0, stream, rows, ldr, x + F + f0, ldx, weights, flags, nidx, bounds, edges, out, n_vert, K, F, f0, order))
-#define HGC_SUM_W(S, H) do { if (width > 32) HGC_SUM(16, 4, S, H); else if (width > 16) HGC_SUM(8, 4, S, H); else HGC_SUM(4, 4, S, H); } while (0)
+#define HGC_SUM(LPT, S, H) HGC_CUDA_TRY(launch_overlapped(n_vert, edge_sum_kernel<LPT, MODE, S, H>, div_up(n_vert, 8 * (32 / LPT)), 256, 0, stream, rows, ldr, x + F + f0, ldx, weights, flags, nidx, bounds, edges, out, n_vert, K, F, f0, order))
+#define HGC_SUM_W(S, H) do { if (width > 32) HGC_SUM(16, S, H); else if (width > 16) HGC_SUM(8, S, H); else HGC_SUM(4, S, H); } while (0)
     if constexpr (MODE == kSumPlain) HGC_SUM_W(false, false);
     else if constexpr (MODE == kSumMean) { if (scale) HGC_SUM_W(true, false); else HGC_SUM_W(false, false); }
     else { if (scale) HGC_SUM_W(true, true); else if (whole) HGC_SUM_W(false, true); else HGC_SUM_W(false, false); }
