@@ -2,7 +2,7 @@
 directly on the kNN + accumulation path: ``RaggedGravNet`` (:3102-3288) and
 ``DistanceWeightedMessagePassing`` (:3540-3612), as inference-time torch modules on CUDA tensors.
 
-The dense layers are plain library GEMMs (``torch.nn.functional.linear``); everything between them --
+The dense layers are ``hgc_dense`` or library GEMMs, whichever is faster; everything between them --
 neighbour search, the slice that drops the self slot, ``10.*distsq``, ``exp``, the weighted mean / max,
 the subtraction of the hit's own features and the concatenation -- is the library's
 ``hgc_binned_select_knn_ragged`` and ``hgc_gravnet_collect``: the collected features are written

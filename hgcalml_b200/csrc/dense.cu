@@ -1,7 +1,7 @@
 // Dense layers in one pass: y = act(x w + bias) in float32.
 //
-// Every product goes into its sum with one fused multiply-add, k ascending, and the bias is added to the rounded sum: what a
-// plain float32 GEMM and the operations behind it compute.
+// Every product goes into its sum with one fused multiply-add, k ascending, and the bias is added to the rounded sum.  A float32
+// GEMM of the library that does not split k gives the same bits.
 #include "common.cuh"
 
 namespace hgc {

@@ -63,9 +63,10 @@ inline size_t hit_order_zeroed_bytes(int n_vert, int n_events)
 int range_and_layout(const float *coords, int n_coords, int n_bin_dims, const int *row_splits, int n_rs, int n_bins,
                      int n_neigh, int n_vert, const HitOrder &o, unsigned *status, cudaStream_t stream);
 
-// Grid of the batch, event layout, and both orders:
+// Event layout and both orders:
 //   bin_perm[p]: hit at position p of the order by (event, bin, locality code, hit number); rank[hit] is its inverse
 //   curve_perm[p]: hit at position p of the order by (event, position on a Hilbert curve, hit number)
+// `o.grid` is of use afterwards only with bin_bits 0: the one kernel that orders small batches keeps the grid to itself.
 // The sort clears nothing: `o`'s histograms and `status` must be zero.  bin_bits: bits of a bin number inside
 // an event, at most 16; 0 for grids that need more, whose order by bin is left to the caller (bin_perm and rank are
 // not written).

@@ -7,10 +7,12 @@ namespace hgc {
 namespace {
 
 // A block per super-chunk of 1024 hits that are consecutive on the curve, a warp per 32 W of them (128 or 256), which it splits two
-// or three times at the median of the coordinate in which the part is widest: that leaves parts of 32 hits, the chunks.  Their boxes do not
-// overlap, and a ball of 64 hits in four dimensions meets fewer of them than of runs of 32 hits along the curve.  A part is
-// split by sorting words of the quantised position in the part (25 bits) and the hit's place (7 bits), W words per lane, by a
-// network of shuffles; the split need not be exact.  Padding sorts last, so the real hits stay in front.
+// or three times at the median of the coordinate in which the part is widest: that leaves parts of 32 hits, the chunks.  The boxes of a
+// warp's chunks overlap only where hits tie or differ by less than the quantisation (those of two warps may: nothing
+// separates runs of the curve), and a ball of 64 hits in four dimensions meets fewer of them than of runs of 32 hits along the
+// curve.  A part is split by sorting words of the quantised position in the part (25 bits for W = 4, 24 for W = 8) and the
+// hit's place (7 or 8 bits), W words per lane, by a network of shuffles; the split need not be exact.  Padding sorts last, so
+// the real hits stay in front.
 // Five splits of the whole super-chunk, a thread per hit, took 18 us for one block and 57 us for 400k hits, most of it in
 // shuffles and barriers, and gave chunks that are no better: search and packing, 400k hits in four dimensions, K = 64, from
 // parts of 1024 1202 us, 512 1180, 256 1188, 128 1168, 32 (no split) 1192.  This kernel: 18 us for 400k hits, 10 for one block.
