@@ -3,6 +3,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "incoming.cuh"
 
 namespace hgc {
 
@@ -45,6 +46,49 @@ __device__ __forceinline__ EdgeVec load_edge_vec_if(const float *p, unsigned wan
     return r;
 }
 
+// Source, weight and (kSumMeanMax) the two words of flags of an edge that points at m.
+template <int MODE>
+__device__ __forceinline__ uint4 edge_record(int e, int m, int K, const float *__restrict__ weights,
+                                             const unsigned *__restrict__ flags, const int *__restrict__ nidx)
+{
+    const int i = e / K;
+    uint4 ed = make_uint4((unsigned)i, __float_as_uint(weights[e]), 0u, 0u);
+    if (MODE == kSumMeanMax) {
+        bool counts = true;
+        if (i == m) {
+            // the hit is its own neighbour: only its first occurrence in the row counts for the maximum
+            for (int k = e - i * K - 1; k >= 0; k--) counts = counts && nidx[(size_t)i * K + k] != m;
+        }
+        if (counts) {
+            const uint2 b = *reinterpret_cast<const uint2 *>(flags + 2 * (size_t)e);
+            ed.z = b.x;
+            ed.w = b.y;
+        }
+    }
+    return ed;
+}
+
+// What an edge adds to VW features: g, times 1 / K where SCALE, and h where a bit of b is set, both times the weight.
+template <int MODE, bool SCALE>
+__device__ __forceinline__ EdgeVec edge_terms(const EdgeVec &g, const EdgeVec &h, float w, unsigned b, float inv)
+{
+    EdgeVec t;
+#pragma unroll
+    for (int v = 0; v < VW; v += 2) {
+        float2 r = make_float2(g.v[v], g.v[v + 1]);
+        if (SCALE) r = mul2(r.x, r.y, inv, inv);
+        r = mul2(r.x, r.y, w, w);
+        t.v[v] = r.x;
+        t.v[v + 1] = r.y;
+        if (MODE == kSumMeanMax) {
+            r = mul2(h.v[v], h.v[v + 1], w, w);
+            if (b & (1u << v)) t.v[v] = __fadd_rn(t.v[v], r.x);
+            if (b & (2u << v)) t.v[v + 1] = __fadd_rn(t.v[v + 1], r.y);
+        }
+    }
+    return t;
+}
+
 // out[m,f] = sum over the edges e = (i, slot) that point at m, in ascending order, for the features f0 .. f0 + LPT * VW - 1.
 // LPT lanes work on one target, VW neighbouring features each; a warp has 32 / LPT targets.  Every lane fetches one edge with
 // its weight and flags and puts them into shared memory, from where all lanes read them with one broadcast load per edge
@@ -57,62 +101,123 @@ __device__ __forceinline__ EdgeVec load_edge_vec_if(const float *p, unsigned wan
 // 0.91, its 77 registers leaving 24 warps per SM.  Half of the gathered lines miss L1 and resident warps hide that better than
 // rows in flight: 16 lanes x 4 features with 2 rows and 40 warps per SM beat 4 rows (+1 %), 8 rows (+20 %), a warp x 2 features
 // (+10 %), and 64 warps, which spill (+27 %).  PushKnn, 200k hits, K = 40, F = 32: 433 -> 341 us.
-template <int LPT, int MODE, bool SCALE, bool HVEC>
-__global__ void __launch_bounds__(256, 5)
+// Wide lists (wide_list) are worked on by whole blocks, before their other targets: every LPT lanes fetch rows of their own, two
+// at a time, whose terms go through shared memory to one thread per feature that adds them in edge order.  The other targets of a
+// block are dealt out again, those without edges last, so that warps are whole where most hits are nobody's neighbours.
+// us with every target in a group of lanes of its own / so, 200k hits, K = F = 64, one hit in 100 a neighbour: PushKnn 3075 / 1417,
+// gradient of the accumulation 5078 / 2450; one neighbour of all hits: 56500 / 9060, 81600 / 17300; searched tables as before.
+// R: rows in flight per target, eight where the targets are too few to fill the chip (gradient on 2000 hits, K = 16 27.7 / 25.1).
+template <int LPT, int R, int MODE, bool SCALE, bool HVEC>
+__global__ void __launch_bounds__(256, R == 2 ? 5 : 2)
 edge_sum_kernel(const float *__restrict__ rows, int ldr, const float *__restrict__ maxima, int ldm,
                 const float *__restrict__ weights, const unsigned *__restrict__ flags, const int *__restrict__ nidx,
-                const int *__restrict__ bounds, const int *__restrict__ edges, float *__restrict__ out, int n_vert, int K, int F,
-                int f0, const int *__restrict__ order)
+                const int *__restrict__ bounds, const int *__restrict__ edges, WideLists wide, float *__restrict__ out,
+                int n_vert, int K, int F, int f0, const int *__restrict__ order)
 {
     pdl_begin();
     constexpr int T = 32 / LPT;  // targets of a warp
-    __shared__ uint4 s_edge[8][32];  // source, weight, flags
+    __shared__ uint4 s_edge[256];  // source, weight, flags; terms of wide lists
+    __shared__ int s_target[8 * T][3];  // hit, first edge, end; those with edges in front, for every 32
+    constexpr int G = 256 / LPT;  // rows of a block
     const int lane = threadIdx.x & 31, hl = lane & (LPT - 1);
-    uint4 *__restrict__ mine = s_edge[threadIdx.x >> 5] + (lane & ~(LPT - 1));
-    const int slot = (blockIdx.x * 8 + (threadIdx.x >> 5)) * T + lane / LPT;
-    int m = 0, begin = 0, end = 0;
-    if (slot < n_vert) {
-        m = order ? order[slot] : slot;  // processing order only: every target is visited once
-        begin = bounds[m];
-        end = bounds[m + 1];
-    }
     const float inv = 1.f / (float)K;
     const int f = hl * VW;
     const bool have = f0 + f < F;
     const float *__restrict__ row0 = rows + (have ? f : 0);
     const float *__restrict__ max0 = MODE == kSumMeanMax ? maxima + (have ? f : 0) : nullptr;
     const unsigned flag_mask = f0 + f + VW <= F ? (1u << VW) - 1u : (1u << (have ? F - f0 - f : 0)) - 1u;
+
+    if (threadIdx.x < 8 * T) {
+        const int slot = blockIdx.x * (8 * T) + threadIdx.x;
+        int m = -1, begin = 0, end = 0;
+        if (slot < n_vert) {
+            m = order ? order[slot] : slot;  // processing order only: every target is visited once
+            begin = bounds[m];
+            end = bounds[m + 1];
+            if (end - begin > wide.limit) {
+                m = -1;
+                end = begin;
+            }
+        }
+        constexpr unsigned kAll = 8 * T < 32 ? (1u << (8 * T)) - 1u : 0xffffffffu;
+        const unsigned busy = __ballot_sync(kAll, end > begin), before = (1u << lane) - 1u;
+        const int at = end > begin ? __popc(busy & before) : __popc(busy) + __popc(~busy & kAll & before);
+        int *t = s_target[(threadIdx.x & ~31) + at];
+        t[0] = m;
+        t[1] = begin;
+        t[2] = end;
+    }
+    __syncthreads();
+
+    const int n_long = wide.counts[0], n_wide = n_long + wide.counts[1];
+    for (int l = blockIdx.x; l < n_wide; l += gridDim.x) {
+        const float *__restrict__ s_term = reinterpret_cast<const float *>(s_edge);
+        const int m = wide.hits[l < n_long ? l : wide.room - 1 - (l - n_long)], end = bounds[m + 1], mine = threadIdx.x / LPT;
+        int p = bounds[m];
+        float acc = 0.f;
+        int e[2];
+#pragma unroll
+        for (int q = 0; q < 2; q++) e[q] = p + q * G + mine < end ? edges[p + q * G + mine] : -1;
+        for (; p < end; p += 2 * G) {
+            EdgeVec g[2], h[2];
+            float w[2];
+            unsigned b[2];
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                w[q] = 0.f;
+                b[q] = 0u;
+                if (e[q] >= 0) {
+                    const uint4 ed = edge_record<MODE>(e[q], m, K, weights, flags, nidx);
+                    w[q] = __uint_as_float(ed.y);
+                    g[q] = load_edge_vec(row0 + (size_t)ed.x * ldr);
+                    if (MODE == kSumMeanMax) {
+                        b[q] = ((LPT * VW > 32 && f >= 32 ? ed.w : ed.z) >> (f & 31)) & flag_mask;
+                        h[q] = load_edge_vec_if<HVEC>(max0 + (size_t)ed.x * ldm, b[q]);
+                    }
+                }
+                const int next = p + (2 + q) * G + mine;
+                e[q] = next < end ? edges[next] : -1;
+            }
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const int n_here = min(G, end - p - q * G);
+                if (mine < n_here) {
+                    const EdgeVec t = edge_terms<MODE, SCALE>(g[q], h[q], w[q], b[q], inv);
+                    s_edge[threadIdx.x] = make_uint4(__float_as_uint(t.v[0]), __float_as_uint(t.v[1]), __float_as_uint(t.v[2]), __float_as_uint(t.v[3]));
+                }
+                __syncthreads();
+                if (threadIdx.x < LPT * VW) {
+                    if (n_here == G) {
+#pragma unroll 16
+                        for (int k = 0; k < G; k++) acc = __fadd_rn(acc, s_term[k * (LPT * VW) + threadIdx.x]);
+                    } else {
+                        for (int k = 0; k < n_here; k++) acc = __fadd_rn(acc, s_term[k * (LPT * VW) + threadIdx.x]);
+                    }
+                }
+                __syncthreads();
+            }
+        }
+        if (threadIdx.x < LPT * VW && f0 + (int)threadIdx.x < F) out[(size_t)m * F + f0 + threadIdx.x] = acc;
+    }
+
+    uint4 *__restrict__ mine = s_edge + (threadIdx.x & ~(LPT - 1));
+    const int *t = s_target[threadIdx.x / LPT];
+    const int m = t[0], begin = t[1], end = t[2];
     float acc[VW];
 #pragma unroll
     for (int v = 0; v < VW; v++) acc[v] = 0.f;
     for (int p = begin; __any_sync(0xffffffffu, p < end); p += LPT) {
         const int n_here = min(LPT, end - p);  // may be below zero where another target's list is longer
         __syncwarp();
-        if (hl < n_here) {
-            const int e = edges[p + hl], i = e / K;
-            uint4 ed = make_uint4((unsigned)i, __float_as_uint(weights[e]), 0u, 0u);
-            if (MODE == kSumMeanMax) {
-                bool counts = true;
-                if (i == m) {
-                    // the hit is its own neighbour: only its first occurrence in the row counts for the maximum
-                    for (int k = e - i * K - 1; k >= 0; k--) counts = counts && nidx[(size_t)i * K + k] != m;
-                }
-                if (counts) {
-                    const uint2 b = *reinterpret_cast<const uint2 *>(flags + 2 * (size_t)e);
-                    ed.z = b.x;
-                    ed.w = b.y;
-                }
-            }
-            mine[hl] = ed;
-        }
+        if (hl < n_here) mine[hl] = edge_record<MODE>(edges[p + hl], m, K, weights, flags, nidx);
         __syncwarp();
-        // two rows at a time; while every target of the warp has two more edges, without a test per target
-        auto two = [&](int q0, auto tail) {
-            EdgeVec g[2], h[2];
-            float w[2];
-            unsigned b[2];
+        // R rows at a time; while every target of the warp has as many more edges, without a test per target
+        auto some = [&](int q0, auto tail) {
+            EdgeVec g[R], h[R];
+            float w[R];
+            unsigned b[R];
 #pragma unroll
-            for (int q = 0; q < 2; q++) {
+            for (int q = 0; q < R; q++) {
                 const uint4 ed = mine[q0 + q];
                 w[q] = __uint_as_float(ed.y);
                 b[q] = 0u;
@@ -125,33 +230,20 @@ edge_sum_kernel(const float *__restrict__ rows, int ldr, const float *__restrict
                 }
             }
 #pragma unroll
-            for (int q = 0; q < 2; q++) {
+            for (int q = 0; q < R; q++) {
                 if (!tail.value || q0 + q < n_here) {
-                    float t[VW];
+                    const EdgeVec t = edge_terms<MODE, SCALE>(g[q], h[q], w[q], b[q], inv);
 #pragma unroll
-                    for (int v = 0; v < VW; v += 2) {
-                        float2 r = make_float2(g[q].v[v], g[q].v[v + 1]);
-                        if (SCALE) r = mul2(r.x, r.y, inv, inv);
-                        r = mul2(r.x, r.y, w[q], w[q]);
-                        t[v] = r.x;
-                        t[v + 1] = r.y;
-                        if (MODE == kSumMeanMax) {
-                            r = mul2(h[q].v[v], h[q].v[v + 1], w[q], w[q]);
-                            if (b[q] & (1u << v)) t[v] = __fadd_rn(t[v], r.x);
-                            if (b[q] & (2u << v)) t[v + 1] = __fadd_rn(t[v + 1], r.y);
-                        }
-                    }
-#pragma unroll
-                    for (int v = 0; v < VW; v++) acc[v] = __fadd_rn(acc[v], t[v]);
+                    for (int v = 0; v < VW; v++) acc[v] = __fadd_rn(acc[v], t.v[v]);
                 }
             }
         };
         const int n_all = max(0, __reduce_min_sync(0xffffffffu, n_here)), n_max = __reduce_max_sync(0xffffffffu, n_here);
         int q0 = 0;
-        for (; q0 + 2 <= n_all; q0 += 2) two(q0, std::false_type());
-        for (; q0 < n_max; q0 += 2) two(q0, std::true_type());
+        for (; q0 + R <= n_all; q0 += R) some(q0, std::false_type());
+        for (; q0 < n_max; q0 += R) some(q0, std::true_type());
     }
-    if (have && slot < n_vert) {
+    if (have && m >= 0) {
         float *dst = out + (size_t)m * F + f0 + f;
 #pragma unroll
         for (int v = 0; v < VW; v++)
@@ -318,13 +410,14 @@ edge_dot_kernel(const float *__restrict__ own, int ld_own, const float *__restri
     }
 }
 
-// One slab of up to 64 features of edge_sum_kernel.  `scratch`: room for n_vert rows of a slab.  Lanes per target: as many as
+// One slab of up to 64 features of edge_sum_kernel.  Lanes per target: as many as
 // the width needs at four features each, so that narrow rows share a warp (200k hits, K = 16, F = 16: PushKnn 220 -> 146 us).
 template <int MODE>
 int launch_edge_sum_slab(const float *x, int ldx, const float *weights, const unsigned *flags, const int *nidx,
-                         const int *bounds, const int *edges, float *out, int n_vert, int K, int F, int f0,
-                         const int *order, float *scratch, cudaStream_t stream)
+                         const Incoming &lists, float *out, int n_vert, int K, int F, int f0, const int *order,
+                         cudaStream_t stream)
 {
+    float *const scratch = lists.rows;
     const int width = F - f0 < 64 ? F - f0 : 64;
     // rows are read where they lie if they are whole vectors and the division by K is an exact scaling
     const bool whole = F % 4 == 0 && ldx % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
@@ -338,9 +431,10 @@ int launch_edge_sum_slab(const float *x, int ldx, const float *weights, const un
         HGC_LAUNCH_CHECK();
         rows = scratch;
     }
+    const bool few = div_up(n_vert, 16) <= 2 * sm_count();
     const bool scale = MODE != kSumPlain && rows != scratch;  // only rows that are whole vectors are scaled
-#define HGC_SUM(LPT, S, H) HGC_CUDA_TRY(launch_overlapped(n_vert, edge_sum_kernel<LPT, MODE, S, H>, div_up(n_vert, 8 * (32 / LPT)), 256, 0, stream, rows, ldr, x + F + f0, ldx, weights, flags, nidx, bounds, edges, out, n_vert, K, F, f0, order))
-#define HGC_SUM_W(S, H) do { if (width > 32) HGC_SUM(16, S, H); else if (width > 16) HGC_SUM(8, S, H); else HGC_SUM(4, S, H); } while (0)
+#define HGC_SUM(LPT, R, S, H) HGC_CUDA_TRY(launch_overlapped(n_vert, edge_sum_kernel<LPT, R, MODE, S, H>, div_up(n_vert, 8 * (32 / LPT)), 256, 0, stream, rows, ldr, x + F + f0, ldx, weights, flags, nidx, lists.bounds, lists.edges, lists.wide, out, n_vert, K, F, f0, order))
+#define HGC_SUM_W(S, H) do { if (few) HGC_SUM(16, 8, S, H); else if (width > 32) HGC_SUM(16, 2, S, H); else if (width > 16) HGC_SUM(8, 2, S, H); else HGC_SUM(4, 2, S, H); } while (0)
     if constexpr (MODE == kSumPlain) HGC_SUM_W(false, false);
     else if constexpr (MODE == kSumMean) { if (scale) HGC_SUM_W(true, false); else HGC_SUM_W(false, false); }
     else { if (scale) HGC_SUM_W(true, true); else if (whole) HGC_SUM_W(false, true); else HGC_SUM_W(false, false); }

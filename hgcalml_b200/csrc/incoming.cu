@@ -85,7 +85,7 @@ __device__ __forceinline__ void sort_list(int *list, int n, int lane)
 // but with the 48 registers that they would take the short lists wait longer (K = 16, 200k hits: 95 -> 104 us).
 // Lists of 129 to 512 edges, a block each before: K = 96, 200k hits 4.4 -> 0.8 ms, K = 128 8.1 -> 1.1 ms for SelectKnnGrad.
 __global__ void __launch_bounds__(256, 8)
-sort_lists_kernel(const int *__restrict__ bounds, int *__restrict__ edges, int n_vert, int *__restrict__ long_lists)
+sort_lists_kernel(const int *__restrict__ bounds, int *__restrict__ edges, int n_vert, WideLists wide)
 {
     pdl_begin();
     const int m = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -97,20 +97,22 @@ sort_lists_kernel(const int *__restrict__ bounds, int *__restrict__ edges, int n
     else if (n <= 128) sort_list<4>(edges + begin, n, lane);
     else if (n <= 256) sort_list<8>(edges + begin, n, lane);
     else if (n <= kWarpList) sort_list<16>(edges + begin, n, lane);
-    else if (lane == 0) long_lists[1 + atomicAdd(long_lists, 1)] = m;
+    if (n > wide.limit && lane == 0) {
+        if (n > kWarpList) wide.hits[atomicAdd(wide.counts, 1)] = m;
+        else wide.hits[wide.room - 1 - atomicAdd(wide.counts + 1, 1)] = m;
+    }
 }
 
 // Lists of more than kWarpList edges: a block per list, radix sort of 8-bit digits through global memory.
 __global__ void __launch_bounds__(256)
-sort_long_lists_kernel(const int *__restrict__ bounds, int *edges, int *tmp, const int *__restrict__ long_lists,
-                       int n_passes)
+sort_long_lists_kernel(const int *__restrict__ bounds, int *edges, int *tmp, WideLists wide, int n_passes)
 {
     pdl_begin();
     __shared__ int s_run[256], s_count[8][256], s_warp[8];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int n_long = long_lists[0];
+    const int n_long = wide.counts[0];
     for (int l = blockIdx.x; l < n_long; l += gridDim.x) {
-        const int m = long_lists[1 + l], begin = bounds[m], n = bounds[m + 1] - begin;
+        const int m = wide.hits[l], begin = bounds[m], n = bounds[m + 1] - begin;
         int *src = edges + begin, *dst = tmp + begin;
         for (int p = 0; p < n_passes; p++) {
             const int shift = 8 * p;
@@ -163,14 +165,14 @@ sort_long_lists_kernel(const int *__restrict__ bounds, int *edges, int *tmp, con
 int build_incoming(const int *nidx, int n_vert, int n_neigh, const Incoming &b, unsigned *status, cudaStream_t stream)
 {
     const long long ne = (long long)n_vert * n_neigh;
-    // the status word, the counts (bounds) and the number of long lists lie one after another
-    HGC_CUDA_TRY(cudaMemsetAsync(status, 0, (size_t)(reinterpret_cast<char *>(b.long_lists + 1) - reinterpret_cast<char *>(status)), stream));
+    // the status word, the counts (bounds) and those of wide lists lie one after another
+    HGC_CUDA_TRY(cudaMemsetAsync(status, 0, (size_t)(reinterpret_cast<char *>(b.wide.counts + 2) - reinterpret_cast<char *>(status)), stream));
     HGC_CUDA_TRY(launch_overlapped(n_vert, count_targets_kernel, div_up(ne, 256), 256, 0, stream, nidx, ne, n_vert, b.bounds, b.place));
     HGC_LAUNCH_CHECK();
     if (int rc = exclusive_scan_ints(b.bounds, n_vert + 1, b.scan, stream)) return rc;
     HGC_CUDA_TRY(launch_overlapped(n_vert, place_edges_kernel, div_up(ne, 256), 256, 0, stream, nidx, b.place, ne, n_vert, b.bounds, b.edges));
     HGC_LAUNCH_CHECK();
-    HGC_CUDA_TRY(launch_overlapped(n_vert, sort_lists_kernel, div_up(n_vert, 8), 256, 0, stream, b.bounds, b.edges, n_vert, b.long_lists));
+    HGC_CUDA_TRY(launch_overlapped(n_vert, sort_lists_kernel, div_up(n_vert, 8), 256, 0, stream, b.bounds, b.edges, n_vert, b.wide));
     HGC_LAUNCH_CHECK();
     if (ne > kWarpList) {
         // Eight blocks per SM where there are edges enough: 60k hits, K = 500, 44 % of the lists longer than this:
@@ -178,7 +180,7 @@ int build_incoming(const int *nidx, int n_vert, int n_neigh, const Incoming &b, 
         // table would notice (1 M edges: 38 -> 40 us), so no more than one for every four of the longest warp lists.
         const long long want = ne / (4 * kWarpList), resident = 8 * sm_count();
         const int blocks = (int)(want < 1 ? 1 : want < resident ? want : resident);
-        HGC_CUDA_TRY(launch_pdl(sort_long_lists_kernel, blocks, 256, 0, stream, b.bounds, b.edges, b.place, b.long_lists, (bits_for(ne) + 7) / 8));
+        HGC_CUDA_TRY(launch_pdl(sort_long_lists_kernel, blocks, 256, 0, stream, b.bounds, b.edges, b.place, b.wide, (bits_for(ne) + 7) / 8));
         HGC_LAUNCH_CHECK();
     }
     return HGC_OK;

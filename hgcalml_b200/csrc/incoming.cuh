@@ -8,9 +8,28 @@ namespace hgc {
 
 constexpr int kWarpList = 512;  // longest list that a warp sorts in registers
 
+// Lists longer than this are wide, and whole blocks of edge_sum_kernel work on them: five or six times what a hit receives on
+// average, which hardly any does whose neighbours are looked for among all hits.  (Up to 32768 hits such a list is what the
+// others wait for.)  us without / with wide lists, PushKnn: 200k hits, K = 16, F = 32, one hit in 25 a neighbour 512 / 232, one in 10
+// 306 / 260 (only lists of more than 512 edges: 532, 298); one in 4, where three times K for a line took 302, 243 / 186.  9000 hits, 20 of
+// them neighbours of all others 114 / 46.  200k hits, K = 64, F = 64, one hit in 8 a neighbour 1136 / 1230 with 6 K, 1188 with 512.
+inline int wide_list(int n_vert, int n_neigh)
+{
+    if (n_neigh > (n_vert <= (1 << 15) ? 102 : 42)) return kWarpList;
+    return n_vert <= (1 << 15) ? (n_neigh <= 16 ? 80 : 5 * n_neigh) : (n_neigh <= 21 ? 127 : 6 * n_neigh);
+}
+
+// The hits with wide lists: those of more than kWarpList edges from the front, the others from the back.
+struct WideLists {
+    int limit;    // wide_list
+    int *counts;  // [2] of more than kWarpList, of the others
+    int *hits;
+    int room;
+};
+
 struct Incoming {
     int *bounds;          // [n_vert + 2] incoming edges of hit m are edges[bounds[m] .. bounds[m + 1])
-    int *long_lists;      // [1 + n_edges / (kWarpList + 1) + 1] number of hits with more than kWarpList incoming edges, and the hits
+    WideLists wide;
     int *scan;            // scratch of the prefix sum
     int *edges;           // [n_edges] edge ids e = hit * n_neigh + slot
     int *place;           // [n_edges] place of an edge in its target's list; scratch of the long sort afterwards
@@ -23,8 +42,11 @@ Incoming incoming_layout(W &ws, int n_vert, int n_neigh)
 {
     const size_t n = n_vert > 0 ? n_vert : 0, ne = n * (size_t)(n_neigh > 0 ? n_neigh : 0);
     Incoming b;
-    b.bounds = ws.template take<int>(n + 2);  // first, with long_lists: one memset clears both and the status word
-    b.long_lists = ws.template take<int>(ne / (kWarpList + 1) + 2);
+    b.bounds = ws.template take<int>(n + 2);  // first, with the counts: one memset clears both and the status word
+    b.wide.limit = wide_list((int)n, n_neigh);
+    b.wide.room = (int)(ne / ((size_t)b.wide.limit + 1)) + 1;
+    b.wide.counts = ws.template take<int>(2 + (size_t)b.wide.room);
+    b.wide.hits = b.wide.counts + 2;
     b.scan = ws.template take<int>(scan_scratch_ints((int)n + 1));
     b.edges = ws.template take<int>(ne);
     b.place = ws.template take<int>(ne);

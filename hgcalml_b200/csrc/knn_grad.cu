@@ -162,11 +162,11 @@ extern "C" int hgc_accumulate_knn_grad_ordered(
             HGC_LAUNCH_CHECK();
         }
         const int rc = mm ? launch_edge_sum_slab<kSumMeanMax>(d_grad_from_out_features, n_grad_from_out_feat, d_distances,
-                                                              b.flags, d_neigh_indices, b.bounds, b.edges,
-                                                              d_out_grad_features, n_vert, n_neigh, n_feat, f0, d_order, b.rows, stream)
+                                                              b.flags, d_neigh_indices, b, d_out_grad_features, n_vert, n_neigh, n_feat, f0,
+                                                              d_order, stream)
                           : launch_edge_sum_slab<kSumMean>(d_grad_from_out_features, n_grad_from_out_feat, d_distances,
-                                                           nullptr, d_neigh_indices, b.bounds, b.edges,
-                                                           d_out_grad_features, n_vert, n_neigh, n_feat, f0, d_order, b.rows, stream);
+                                                           nullptr, d_neigh_indices, b, d_out_grad_features, n_vert, n_neigh, n_feat, f0,
+                                                           d_order, stream);
         if (rc) return rc;
     }
     return HGC_OK;

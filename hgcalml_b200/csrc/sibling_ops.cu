@@ -163,8 +163,8 @@ extern "C" int hgc_push_knn_ordered(
     const Incoming b = incoming_layout(ws, n_vert, n_neigh);
     if (int rc = build_incoming(d_idxs, n_vert, n_neigh, b, ws.status(), stream)) return rc;
     for (int f0 = 0; f0 < n_feat; f0 += 64)
-        if (int rc = launch_edge_sum_slab<kSumPlain>(d_feat, n_feat, d_weights, nullptr, nullptr, b.bounds, b.edges, d_out_feat,
-                                                     n_vert, n_neigh, n_feat, f0, d_order, b.rows, stream))
+        if (int rc = launch_edge_sum_slab<kSumPlain>(d_feat, n_feat, d_weights, nullptr, nullptr, b, d_out_feat, n_vert, n_neigh, n_feat, f0,
+                                                     d_order, stream))
             return rc;
     return HGC_OK;
 }

@@ -179,3 +179,53 @@ def test_select_knn_grad_over_the_range_of_floats(cuda, oracle, K):
     got = N(SelectKnnGrad(T(g, cuda), T(idx, cuda), None, T(c, cuda)))
     nan = np.isnan(ref)
     assert np.array_equal(nan, np.isnan(got)) and np.array_equal(bits(got[~nan]), bits(ref[~nan]))
+
+
+def _check_sums(cuda, oracle, idx, F, rng):
+    from hgcalml_b200.accknn_op import AccumulateKnnGrad, AccumulateLinKnn
+    from hgcalml_b200.push_knn_op import PushKnn
+    n, K = idx.shape
+    feat, grad = rng.standard_normal((n, F), dtype=np.float32), rng.standard_normal((n, 2 * F), dtype=np.float32)
+    w = rng.random((n, K), dtype=np.float32)
+    table, order = T(idx, cuda), T(rng.permutation(n).astype(np.int32), cuda)
+    _, arg = AccumulateLinKnn(T(w, cuda), T(feat, cuda), table)
+    for g, a in ((grad, arg), (np.ascontiguousarray(grad[:, F:]), None)):
+        rw, rf = oracle.op_accumulate_knn_grad(g, w, feat, idx, N(arg))
+        for o in (None, order):
+            gw, gf = AccumulateKnnGrad(T(g, cuda), T(w, cuda), T(feat, cuda), table, a, order=o)
+            assert np.array_equal(bits(N(gw)), bits(rw)) and np.array_equal(bits(N(gf)), bits(rf))
+    assert np.array_equal(bits(N(PushKnn(T(w, cuda), T(feat, cuda), table))), bits(oracle.op_push_knn(w, feat, idx)))
+
+
+def _hits(cuda, few):
+    """On either side of the number of targets that fill the chip with two rows in flight each."""
+    return 1300 if few else 2 * 16 * torch.cuda.get_device_properties(cuda).multi_processor_count + 17
+
+
+@pytest.mark.parametrize("K,F", [(5, 16), (21, 64), (30, 32), (64, 6), (200, 66)])
+@pytest.mark.parametrize("few", [True, False])
+def test_sums_over_lists_that_whole_blocks_work_on(cuda, oracle, K, F, few):
+    """Lists of more than 80, 127, five or six times K and 512 edges among shorter ones; the other targets of a block are dealt
+    out again."""
+    n, rng = _hits(cuda, few), np.random.default_rng(K)
+    counts = [31, 80, 81, 5 * K, 5 * K + 1, 112, 113, 511, 512, 513, 527, 528, 529, 700]
+    flat = rng.integers(-1, n, n * K).astype(np.int32)
+    flat[np.isin(flat, rng.choice(n, n // 2, replace=False))] = -1  # half of the hits are nobody's neighbours
+    flat[(flat >= 40) & (flat < 40 + 7 * len(counts))] = -1
+    at = rng.permutation(flat.size)
+    for i, count in enumerate(counts):  # between hits with short lists
+        flat[at[:count]] = 40 + 7 * i
+        at = at[count:]
+    idx = flat.reshape(n, K)
+    idx[40, 0] = idx[40, K - 1] = 40  # the hit itself twice
+    _check_sums(cuda, oracle, idx, F, rng)
+
+
+@pytest.mark.parametrize("K,F,every", [(40, 16, 4), (16, 32, 10), (16, 64, 6), (64, 64, 12), (64, 20, 12), (64, 16, 60), (24, 70, 50)])
+@pytest.mark.parametrize("few", [True, False])
+def test_sums_where_few_hits_are_neighbours(cuda, oracle, K, F, every, few):
+    """Wide lists of both kinds, more of them than blocks, and blocks with few targets that have edges."""
+    n, rng = _hits(cuda, few), np.random.default_rng(K + F)
+    idx = rng.integers(0, n // every, (n, K)).astype(np.int32) * every
+    idx[rng.random(idx.shape) < 0.05] = -1
+    _check_sums(cuda, oracle, idx, F, rng)
