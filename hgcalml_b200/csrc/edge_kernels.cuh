@@ -390,9 +390,15 @@ edge_dot_kernel(const float *__restrict__ own, int ld_own, const float *__restri
         if (MAX) {
             // a feature's maximum lies in one slot, so a lane has F / K of them on average
             const float *__restrict__ gm = g + F + f0;
-            for (unsigned left = hit; left != 0u; left &= left - 1u) {
-                const int f = __ffs(left) - 1;
-                max_part = __fadd_rn(max_part, __fmul_rn(__ldg(gm + f), s[lane * kRow + f]));
+            // (two loads at a time: a table of few edges waits for them)
+            for (unsigned left = hit; left != 0u;) {
+                const int a = __ffs(left) - 1;
+                left &= left - 1u;
+                const int b = left != 0u ? __ffs(left) - 1 : a;
+                const float ga = __ldg(gm + a), gb = __ldg(gm + b);
+                max_part = __fadd_rn(max_part, __fmul_rn(ga, s[lane * kRow + a]));
+                if (left != 0u) max_part = __fadd_rn(max_part, __fmul_rn(gb, s[lane * kRow + b]));
+                left &= left - 1u;
             }
             if (f0 == 0) bits.x = hit;
             if (f0 == 32) bits.y = hit;
