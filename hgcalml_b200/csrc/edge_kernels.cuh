@@ -426,11 +426,10 @@ int launch_edge_sum_slab(const float *x, int ldx, const float *weights, const un
     float *const scratch = lists.rows;
     const int width = F - f0 < 64 ? F - f0 : 64;
     // rows are read where they lie if they are whole vectors and the division by K is an exact scaling
-    const bool whole = F % 4 == 0 && ldx % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
-    const bool exact = MODE == kSumPlain || (K & (K - 1)) == 0;
+    const bool whole = copied_row(F, aligned16(x), false) == 0;
     const float *rows = x + f0;
     int ldr = ldx;
-    if (!whole || !exact) {
+    if (copied_row(F, aligned16(x), MODE != kSumPlain && !power_of_two(K)) > 0) {
         ldr = (width + 3) / 4 * 4;
         HGC_CUDA_TRY(launch_overlapped(n_vert, edge_rows_kernel, div_up((long long)n_vert * ldr, 256), 256, 0, stream, x + f0, ldx, width,
                                        MODE == kSumPlain ? 1.f : (float)K, scratch, ldr, n_vert));

@@ -32,13 +32,25 @@ struct Incoming {
     WideLists wide;
     int *scan;            // scratch of the prefix sum
     int *edges;           // [n_edges] edge ids e = hit * n_neigh + slot
-    int *place;           // [n_edges] place of an edge in its target's list; scratch of the long sort afterwards
     unsigned *flags;      // [n_edges][2] scratch of the op: one bit per feature of a slab of 64
-    float *rows;          // [n_vert][64] scratch of the op: rows of a slab (edge_rows_kernel)
+    int *place;           // [n_edges] place of an edge in its target's list; scratch of the long sort afterwards
+    float *rows;          // scratch of the op: rows of a slab (edge_rows_kernel)
 };
 
+// Floats per hit that an op copies its rows into, a slab of up to 64 features at a time: none where rows are whole 16-byte vectors
+// that need no division.
+inline int copied_row(int n_feat, bool aligned, bool divided)
+{
+    if (n_feat % 4 == 0 && aligned && !divided) return 0;
+    return n_feat < 64 ? (n_feat + 3) / 4 * 4 : 64;
+}
+inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+inline bool power_of_two(int k) { return (k & (k - 1)) == 0; }
+
+// `row`: floats per hit of the copied rows.  They take the place of `place`, which the finished lists do not need, that of `flags`
+// in an op without flags, and what they are longer than that behind it.
 template <typename W>
-Incoming incoming_layout(W &ws, int n_vert, int n_neigh)
+Incoming incoming_layout(W &ws, int n_vert, int n_neigh, int row = 0, bool with_flags = true)
 {
     const size_t n = n_vert > 0 ? n_vert : 0, ne = n * (size_t)(n_neigh > 0 ? n_neigh : 0);
     Incoming b;
@@ -49,9 +61,11 @@ Incoming incoming_layout(W &ws, int n_vert, int n_neigh)
     b.wide.hits = b.wide.counts + 2;
     b.scan = ws.template take<int>(scan_scratch_ints((int)n + 1));
     b.edges = ws.template take<int>(ne);
-    b.place = ws.template take<int>(ne);
     b.flags = ws.template take<unsigned>(2 * ne);
-    b.rows = ws.template take<float>(64 * n);
+    b.place = ws.template take<int>(ne);
+    b.rows = with_flags ? reinterpret_cast<float *>(b.place) : reinterpret_cast<float *>(b.flags);
+    const size_t room = with_flags ? ne : 3 * ne, want = n * (size_t)row;
+    if (want > room) ws.template take<float>(want - room);
     return b;
 }
 
@@ -59,6 +73,12 @@ struct IncomingSizer {
     Sizer s;
     template <typename T> T *take(size_t n) { s.take<T>(n); return nullptr; }
 };
+inline size_t incoming_bytes(int n_vert, int n_neigh, int row = 0, bool with_flags = true)
+{
+    IncomingSizer w;
+    incoming_layout(w, n_vert, n_neigh, row, with_flags);
+    return w.s.used;
+}
 
 // Builds the lists; also clears the workspace's status word.
 int build_incoming(const int *nidx, int n_vert, int n_neigh, const Incoming &b, unsigned *status, cudaStream_t stream);

@@ -93,9 +93,19 @@ using namespace hgc;
 
 extern "C" size_t hgc_knn_grad_workspace_bytes(int n_vert, int n_neigh)
 {
-    IncomingSizer w;
-    incoming_layout(w, n_vert, n_neigh);
-    return w.s.used;
+    return incoming_bytes(n_vert, n_neigh, 64);  // the widest rows beside flags
+}
+
+extern "C" size_t hgc_select_knn_grad_workspace_bytes(int n_vert, int n_neigh) { return incoming_bytes(n_vert, n_neigh); }
+
+static size_t accumulate_grad_bytes(int n_vert, int n_neigh, int n_feat, int mean_and_max, bool aligned)
+{
+    return incoming_bytes(n_vert, n_neigh, copied_row(n_feat, aligned, !power_of_two(n_neigh)), mean_and_max);
+}
+
+extern "C" size_t hgc_accumulate_knn_grad_workspace_bytes(int n_vert, int n_neigh, int n_feat, int mean_and_max)
+{
+    return accumulate_grad_bytes(n_vert, n_neigh, n_feat, mean_and_max, true);
 }
 
 static int check_edge_count(int n_vert, int n_neigh)
@@ -134,10 +144,11 @@ extern "C" int hgc_accumulate_knn_grad_ordered(
                        (mean_and_max && !d_max_feat_indices)))
         return HGC_ERR_INVALID_ARGUMENT;
     if (n_neigh > 0 && (!d_distances || !d_neigh_indices || !d_out_grad_distances)) return HGC_ERR_INVALID_ARGUMENT;
-    const size_t need = hgc_knn_grad_workspace_bytes(n_vert, n_neigh);
+    const bool mm = mean_and_max != 0;
+    const size_t need = accumulate_grad_bytes(n_vert, n_neigh, n_feat, mm, aligned16(d_grad_from_out_features));
     if (int rc = check_workspace(workspace, workspace_bytes, need)) return rc;
     Carver ws(workspace);
-    const Incoming b = incoming_layout(ws, n_vert, n_neigh);
+    const Incoming b = incoming_layout(ws, n_vert, n_neigh, 0, mm);
     if (n_neigh == 0) {
         HGC_CUDA_TRY(cudaMemsetAsync(ws.status(), 0, kAlign, stream));
         if (n_feat > 0)
@@ -145,9 +156,7 @@ extern "C" int hgc_accumulate_knn_grad_ordered(
         return HGC_OK;
     }
     if (int rc = build_incoming(d_neigh_indices, n_vert, n_neigh, b, ws.status(), stream)) return rc;
-    const bool mm = mean_and_max != 0;
     const long long ne = (long long)n_vert * n_neigh;
-    auto aligned16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
     const bool vec4 = n_feat % 4 == 0 && aligned16(d_feat) && aligned16(d_grad_from_out_features) && (!mm || aligned16(d_max_feat_indices));
     HGC_CUDA_TRY(launch_overlapped(n_vert, mm ? vec4 ? edge_dot_kernel<true, true, true> : edge_dot_kernel<true, true, false>
                                               : vec4 ? edge_dot_kernel<true, false, true> : edge_dot_kernel<true, false, false>,
@@ -191,7 +200,7 @@ static int select_knn_grad(const float *d_grad_dist, const int *d_indices, const
     if (n_coords < 0) return HGC_ERR_INVALID_ARGUMENT;
     if (n_vert == 0 || n_coords == 0) return HGC_OK;
     if (!d_coord || !d_grad_coord || (n_neigh > 0 && (!d_grad_dist || !d_indices))) return HGC_ERR_INVALID_ARGUMENT;
-    const size_t need = hgc_knn_grad_workspace_bytes(n_vert, n_neigh);
+    const size_t need = hgc_select_knn_grad_workspace_bytes(n_vert, n_neigh);
     if (int rc = check_workspace(workspace, workspace_bytes, need)) return rc;
     Carver ws(workspace);
     const Incoming b = incoming_layout(ws, n_vert, n_neigh);

@@ -78,7 +78,7 @@ std::tuple<Tensor, Tensor, Tensor, int> accumulate_grad(const Tensor &grad, cons
 {
     const int n = (int)indices.size(0), k = (int)indices.size(1), f = (int)features.size(1), g = (int)grad.size(1);
     Tensor gw = like(features, {n, k}, at::kFloat), gf = like(features, {n, f}, at::kFloat);
-    Tensor ws = workspace(features, hgc_knn_grad_workspace_bytes(n, k));
+    Tensor ws = workspace(features, aligned16(grad) ? hgc_accumulate_knn_grad_workspace_bytes(n, k, f, g > f) : hgc_knn_grad_workspace_bytes(n, k));
     const int rc = hgc_accumulate_knn_grad_ordered(
             data<float>(grad), data<float>(weights), data<float>(features), data<int>(max_idx), data<int>(indices),
             data<float>(gw), data<float>(gf), n, k, f, g, 0, g > f, data<int>(order), ws.data_ptr(), (size_t)ws.numel(),
@@ -92,7 +92,7 @@ std::tuple<Tensor, int> select_knn_grad(const Tensor &grad, const Tensor &indice
 {
     const int n = (int)indices.size(0), k = (int)indices.size(1), c = (int)coords.size(1);
     Tensor out = like(coords, coords.sizes(), at::kFloat);
-    const Tensor ws = lists.has_value() ? *lists : workspace(coords, hgc_knn_grad_workspace_bytes(n, k));
+    const Tensor ws = lists.has_value() ? *lists : workspace(coords, hgc_select_knn_grad_workspace_bytes(n, k));
     const auto run = lists.has_value() ? hgc_select_knn_grad_after : hgc_select_knn_grad_ordered;
     const int rc = run(data<float>(grad), data<int>(indices), nullptr, data<float>(coords), data<float>(out), n, k, c,
                        data<int>(order), ws.data_ptr(), (size_t)ws.numel(), stream_of(coords));
@@ -113,7 +113,7 @@ std::tuple<Tensor, int> push_knn(const Tensor &weights, const Tensor &features, 
 {
     const int n = (int)indices.size(0), k = (int)indices.size(1), f = (int)features.size(1);
     Tensor out = like(features, features.sizes(), at::kFloat);
-    Tensor ws = workspace(features, hgc_knn_grad_workspace_bytes(n, k));
+    Tensor ws = workspace(features, aligned16(features) ? hgc_push_knn_workspace_bytes(n, k, f) : hgc_knn_grad_workspace_bytes(n, k));
     const int rc = hgc_push_knn_ordered(data<float>(weights), data<float>(features), data<int>(indices), data<float>(out), n, k, f,
                                         data<int>(order), ws.data_ptr(), (size_t)ws.numel(), stream_of(features));
     return {out, rc};

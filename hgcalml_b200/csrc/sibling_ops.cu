@@ -134,6 +134,13 @@ extern "C" int hgc_local_distance(
     return HGC_OK;
 }
 
+static size_t push_bytes(int n_vert, int n_neigh, int n_feat, bool aligned)
+{
+    return incoming_bytes(n_vert, n_neigh, copied_row(n_feat, aligned, false), false);
+}
+
+extern "C" size_t hgc_push_knn_workspace_bytes(int n_vert, int n_neigh, int n_feat) { return push_bytes(n_vert, n_neigh, n_feat, true); }
+
 extern "C" int hgc_push_knn(
         const float *d_weights, const float *d_feat, const int *d_idxs, float *d_out_feat,
         int n_vert, int n_neigh, int n_feat, void *workspace, size_t workspace_bytes, hgc_stream_t stream)
@@ -155,12 +162,12 @@ extern "C" int hgc_push_knn_ordered(
         HGC_CUDA_TRY(cudaMemsetAsync(d_out_feat, 0, sizeof(float) * (size_t)n_vert * n_feat, stream));
         return HGC_OK;
     }
-    const size_t need = hgc_knn_grad_workspace_bytes(n_vert, n_neigh);
+    const size_t need = push_bytes(n_vert, n_neigh, n_feat, aligned16(d_feat));
     if (int rc = check_workspace(workspace, workspace_bytes, need)) return rc;
     Carver ws(workspace);
     // sums in (hit, slot) order (modules/compiled/push_knn_kernel.cc:35-71; the reference's GPU kernel scatters with
     // atomicAdd, push_knn_kernel.cu.cc:61)
-    const Incoming b = incoming_layout(ws, n_vert, n_neigh);
+    const Incoming b = incoming_layout(ws, n_vert, n_neigh, 0, false);
     if (int rc = build_incoming(d_idxs, n_vert, n_neigh, b, ws.status(), stream)) return rc;
     for (int f0 = 0; f0 < n_feat; f0 += 64)
         if (int rc = launch_edge_sum_slab<kSumPlain>(d_feat, n_feat, d_weights, nullptr, nullptr, b, d_out_feat, n_vert, n_neigh, n_feat, f0,

@@ -213,7 +213,7 @@ public:
         Tensor *out;
         OP_REQUIRES_OK(ctx, ctx->allocate_output(0, {n_vert, C}, &out));
         Workspace ws;
-        OP_REQUIRES_OK(ctx, ws.Allocate(ctx, hgc_knn_grad_workspace_bytes(n_vert, K)));
+        OP_REQUIRES_OK(ctx, ws.Allocate(ctx, hgc_select_knn_grad_workspace_bytes(n_vert, K)));
         OP_REQUIRES_OK(ctx, FromHgc(hgc_select_knn_grad(
             g.flat<float>().data(), idx.flat<int>().data(), dist.flat<float>().data(), coord.flat<float>().data(),
             out->flat<float>().data(), n_vert, K, C, ws.ptr, ws.bytes, StreamOf(ctx)), "SelectKnnGrad"));

@@ -327,10 +327,13 @@ int hgc_merge_noise(
  * coordinates, d_grad_coord [n_vert, n_coords]; d_dist is accepted and not read, as in the
  * reference.  Deterministic for the same reason.
  *
- * Both take a workspace of hgc_knn_grad_workspace_bytes (about 16 bytes per (hit, slot) pair) and
- * need n_vert * n_neigh < 2^31.
+ * Both take a workspace of hgc_knn_grad_workspace_bytes (about 16 bytes per (hit, slot) pair, and 4 (64 - n_neigh) per hit
+ * where n_neigh is below 64) and need n_vert * n_neigh < 2^31.  The queries of the single ops ask for no more than the op uses, which for
+ * most widths is the first part alone; that of hgc_accumulate_knn_grad goes for d_grad_from_out_features on a 16-byte boundary.
  * ------------------------------------------------------------------------------------- */
 size_t hgc_knn_grad_workspace_bytes(int n_vert, int n_neigh);
+size_t hgc_accumulate_knn_grad_workspace_bytes(int n_vert, int n_neigh, int n_feat, int mean_and_max);
+size_t hgc_select_knn_grad_workspace_bytes(int n_vert, int n_neigh);
 int hgc_accumulate_knn_grad(
         const float *d_grad_from_out_features, const float *d_distances, const float *d_feat,
         const int *d_max_feat_indices, const int *d_neigh_indices,
@@ -376,11 +379,12 @@ int hgc_select_knn_grad_after(
  * PushKnn -- replaces PushKnnOpFunctor (modules/compiled/push_knn_kernel.h):
  * d_out_feat[m,f] = sum over all (i,k) with d_idxs[i,k] == m of d_feat[i,f] * d_weights[i,k], summed
  * in (i,k) order without atomics (bit-identical to the reference's CPU loop).  Workspace:
- * hgc_knn_grad_workspace_bytes(n_vert, n_neigh).
+ * hgc_knn_grad_workspace_bytes(n_vert, n_neigh), or hgc_push_knn_workspace_bytes for d_feat on a 16-byte boundary.
  * ------------------------------------------------------------------------------------- */
 int hgc_local_distance(
         const int *d_neigh_idxs, const float *d_coords, float *d_distances,
         int n_coords, int n_in_vert, int n_out_vert, int n_neigh, hgc_stream_t stream);
+size_t hgc_push_knn_workspace_bytes(int n_vert, int n_neigh, int n_feat);
 int hgc_push_knn(
         const float *d_weights, const float *d_feat, const int *d_idxs, float *d_out_feat,
         int n_vert, int n_neigh, int n_feat, void *workspace, size_t workspace_bytes, hgc_stream_t stream);

@@ -151,3 +151,21 @@ def _build_c_user(out_path):
 def test_plain_c_user_of_the_abi_compiles_and_links(tmp_path):
     """The header is C (not C++) and the library links into a program that knows nothing of Python or torch."""
     _build_c_user(str(tmp_path / "knn_from_c"))
+
+
+@pytest.mark.parametrize("K", [1, 3, 8, 12, 40, 64, 100])
+def test_workspaces_of_the_backward_ops(K):
+    """16 bytes per edge hold lists and flags; rows of features lie in what the lists no longer need, and take more only where
+    they are longer than that."""
+    from hgcalml_b200 import _capi as C
+    L, n = C.lib, 100000
+    lists = L.hgc_select_knn_grad_workspace_bytes(n, K)
+    assert 16 * n * K <= lists <= 16 * n * K + 6 * n + 8192
+    assert L.hgc_knn_grad_workspace_bytes(n, K) <= lists + 4 * n * max(0, 64 - K) + 256
+    for F in (1, 4, 22, 32, 64, 66, 128):
+        ops = [L.hgc_push_knn_workspace_bytes(n, K, F)] + [L.hgc_accumulate_knn_grad_workspace_bytes(n, K, F, mm) for mm in (0, 1)]
+        assert lists <= min(ops) and max(ops) <= L.hgc_knn_grad_workspace_bytes(n, K)
+        if F % 4 == 0:
+            assert ops[0] == lists
+            if K & (K - 1) == 0:
+                assert ops == [lists] * 3

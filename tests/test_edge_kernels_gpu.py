@@ -229,3 +229,36 @@ def test_sums_where_few_hits_are_neighbours(cuda, oracle, K, F, every, few):
     idx = rng.integers(0, n // every, (n, K)).astype(np.int32) * every
     idx[rng.random(idx.shape) < 0.05] = -1
     _check_sums(cuda, oracle, idx, F, rng)
+
+
+@pytest.mark.parametrize("K", [1, 5, 8, 24])
+@pytest.mark.parametrize("F", [3, 16, 30, 64, 70])
+def test_no_op_leaves_its_workspace(cuda, oracle, K, F):
+    from hgcalml_b200 import _capi as C
+    from hgcalml_b200.accknn_op import AccumulateLinKnn
+    n, L = 2100, C.lib
+    idx, rng = _table(n, max(K, 2), F)
+    idx = np.ascontiguousarray(idx[:, :K])
+    feat, grad, w = (rng.standard_normal(s, dtype=np.float32) for s in ((n, F), (n, 2 * F), (n, K)))
+    x, go, wt, table = T(feat, cuda), T(grad, cuda), T(w, cuda), T(idx, cuda)
+    g1 = go[:, :F].contiguous()
+    _, arg = AccumulateLinKnn(wt, x, table)
+    coords = T(grad[:, :2].copy(), cuda)
+
+    def call(need, fn, *outs):
+        ws = torch.full((need + 4096,), 0xa5, dtype=torch.uint8, device=cuda)
+        outs = [torch.empty(s, device=cuda) for s in outs]
+        C.check(fn(ws, need, *[C.ptr(o) for o in outs], C.stream_of(ws)), "op")
+        assert (ws[need:] == 0xa5).all()
+        return [N(o) for o in outs]
+    for mm, g in ((1, go), (0, g1)):
+        gw, gf = call(L.hgc_accumulate_knn_grad_workspace_bytes(n, K, F, mm), lambda ws, b, gw, gf, s: L.hgc_accumulate_knn_grad(
+            C.ptr(g), C.ptr(wt), C.ptr(x), C.ptr(arg) if mm else None, C.ptr(table), gw, gf, n, K, F, g.shape[1], 0, mm, C.ptr(ws), b, s), (n, K), (n, F))
+        rw, rf = oracle.op_accumulate_knn_grad(N(g), w, feat, idx, N(arg))
+        assert np.array_equal(bits(gw), bits(rw)) and np.array_equal(bits(gf), bits(rf))
+    (out,) = call(L.hgc_push_knn_workspace_bytes(n, K, F), lambda ws, b, o, s: L.hgc_push_knn(
+        C.ptr(wt), C.ptr(x), C.ptr(table), o, n, K, F, C.ptr(ws), b, s), (n, F))
+    assert np.array_equal(bits(out), bits(oracle.op_push_knn(w, feat, idx)))
+    (gc,) = call(L.hgc_select_knn_grad_workspace_bytes(n, K), lambda ws, b, o, s: L.hgc_select_knn_grad(
+        C.ptr(wt), C.ptr(table), None, C.ptr(coords), o, n, K, 2, C.ptr(ws), b, s), (n, 2))
+    assert np.array_equal(bits(gc), bits(oracle.op_select_knn_grad(w, idx, N(coords))))
