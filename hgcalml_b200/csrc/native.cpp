@@ -17,6 +17,8 @@
 
 #include "../../include/hgcalml_b200.h"
 
+namespace hgc { int sm_count(); }  // of the library
+
 namespace {
 
 using at::Tensor;
@@ -205,17 +207,27 @@ bool values_only(const Tensor &t)
 
 constexpr int kNotTaken = 1;
 
-// Where hgc_dense is at least as fast as the library's GEMM with the bias and activation kernel behind it (float32, us,
-// library / hgc_dense): 200k rows 64 x 4 31 / 13, 64 x 64 68 / 55, 192 x 64 129 / 123, 128 x 128 184 / 172, 288 x 96 273 / 335; 20k rows
-// 64 x 6 8.4 / 5.3, 96 x 32 9.0 / 8.0, 64 x 64 10.6 / 9.6, 192 x 64 19 / 23, 128 x 128 24 / 28; 4000 rows 64 x 6 3.9 / 4.3, 48 x 16 4.9 / 2.7,
-// 64 x 64 5.3 / 4.9.
+// Where hgc_dense is at least as fast as the library's GEMM with the bias and activation kernel behind it: time over the library's
+// (float32, 24 batches of 1 to 1M rows for each of 30 shapes).
+//   up to 8 columns: 0.33 to 0.9; at 60k rows 256 x 8 1.06, so that long rows of more than four columns start above that
+//   9 to 32: 0.44 to 0.95; 128 x 24 and 128 x 12 1.04 and 1.06 at 49k
+//   33 to 64: up to 64 inputs 0.44 to 1.00, but 64 x 48 1.06 at 80k, where blocks of 128 rows leave a second round of the chip nearly
+//     empty; likewise at 160k in the third round 192 x 64 1.06 and 128 x 48 1.05 (128 x 64 0.98); else 128 x 64 0.88 to 0.93,
+//     192 x 64 0.93 to 0.98, 128 x 48 0.93 to 0.98, 192 x 48 1.00 to 1.04, from 131k on
+//   65 to 128, 64 at a time: 64 x 72 and 64 x 96 below 1.00, 96 x 96 0.90 to 1.00, 128 x 120 and 128 x 128 0.93 to 0.99; 96 x 80 1.03,
+//     128 x 72 and 128 x 96 1.02 to 1.14, 128 x 104 1.02
 bool dense_is_faster(int64_t n, int64_t n_in, int64_t n_out)
 {
     if (n < 1 || n > 0x7fffffff || n_in < 4 || n_out < 1) return false;
-    if (n_out <= 8) return n_in <= 32 || (n_in <= 64 && n >= 10000) || (n_in <= 256 && n >= 32768);
-    if (n_out <= 32) return n_in <= 96 || (n_in <= 128 && n >= 49152);
-    if (n_out <= 64) return n_in <= 64 || (n_in <= 192 && n >= 131072);
-    return n_out <= 128 && n_in <= 128 && n >= 131072;
+    if (n_out <= 8) return n_in <= 32 || (n_in <= 64 && n >= 10000) || (n_in <= 256 && n >= (n_in > 128 && n_out > 4 ? 65536 : 32768));
+    if (n_out <= 32) return n_in <= 96 || (n_in <= 128 && n >= 57344);
+    if (n_out <= 64) {
+        const int64_t blocks = (n + 127) / 128, round = 4 * (int64_t)hgc::sm_count(), last = blocks % round;
+        const bool tail = blocks > round && blocks < 3 * round && last > 0 && last * 6 < round;
+        if (n_in <= 64) return n_in <= 32 || n_out > 56 || !tail || blocks > 2 * round;
+        return n >= 131072 && (n_out > 56 ? n_in <= 128 || (n_in <= 192 && !tail) : n_in <= 128 && !tail);
+    }
+    return n_out <= 128 && n_in <= (n_out > 112 ? 128 : n_out > 88 ? 96 : 64) && n >= 131072;
 }
 
 // y = act(y + bias) in place; kNotTaken where the tensor operations would do more than that
