@@ -53,7 +53,9 @@ int sm_count();
 // through any chain of them.
 // Kernels that are short at every size are always launched so: the condensate path, keep_noise, the epilogues of dense
 // layers, LocalDistance, the op-level sorts (4 x 200k hits condensed 460 -> 440 us, 100k 285 -> 266; two GravNet layers
-// with message passing on 200k hits 2864 -> 2848).
+// with message passing on 200k hits 2864 -> 2848).  So are the dense layers themselves, which gain by it at every size (us, launched
+// so up to 65536 rows only / always: six layers of 64 x 64, 64 x 4 and 192 x 64 on 70k rows 149.5 / 140.2, 200k 363.6 / 362.1, 400k 705.0 /
+// 698.4; 64 x 4 on 400k 26.7 / 23.9): their blocks share nothing through L1 with the kernel before.
 // launch_overlapped is for the kernels whose length grows with the batch (search, orders, accumulation, backward ops): up to
 // kOverlapHits hits.  Blocks that become resident early take room from the kernel that is still running and inherit its
 // split between L1 and shared memory.  Search and accumulation, K = 16, F = 32, in us, not overlapped / overlapped: 20k hits
