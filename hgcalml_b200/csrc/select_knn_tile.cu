@@ -275,10 +275,12 @@ int search_tiles(const TileScratch &s, const HitOrder &o, const int *rank_to_id,
     // every SM has work to the end.  A list costs little beside the queries in four dimensions and less in more, so the cut
     // goes on there while blocks are few rounds of what is resident (9 to 6 per SM).  us with 8 blocks per SM wanted everywhere /
     // with this rule, showers: 4 dimensions, K = 64, 25k hits 158 / 148, 50k 254 / 223, 80k 372 / 341, 130k 530 / 503; K = 32 50k 211 / 186; 5
-    // dimensions, K = 48, 20k 180 / 162, 50k 387 / 328, 130k 861 / 817.  3 dimensions lose by it: 20k uniform hits 86 / 96.  4 dimensions, K < 24,
-    // wanted 8 / 10, 18: 20k showers, K = 16 116 / 103 / 102, 50k 178 / 165 / 177.  K = 24 to 64, wanted 18 / 16: 20k K = 64 showers 132 / 126,
-    // uniform 146 / 137, normal 170 / 165; 38k showers K = 24 to 64 154 / 161 to 188 / 191, uniform 160 / 152 to 211 / 199.  7 and more
-    // dimensions, 8 wanted / 40: 8 dimensions, K = 16, 30k showers 0.63 of the time, uniform 0.85, normal 0.79; 50k 0.67, 0.95, 0.91; 70k 0.75, 1.08, 1.05.
+    // dimensions, K = 48, 20k 180 / 162, 50k 387 / 328, 130k 861 / 817.  3 dimensions lose by it: 20k uniform hits 86 / 96.  4 dimensions, K < 24, 50k
+    // showers in tiles of 32 / 16 (whole): K = 4 160 / 147, 16 178 / 165; 20k hits, K = 4 and 16, wanted 10 / 18: showers 96.8 / 95.4, 102.6 / 102.5,
+    // uniform 98.4 / 97.9, 106.5 / 109.6, normal 115 / 108, 124 / 125.  K = 24 to 64, wanted 18 / 16: 20k K = 64 showers 132 / 126, uniform 146 /
+    // 137, normal 170 / 165; 38k showers K = 24 to 64 154 / 161 to 188 / 191, uniform 160 / 152 to 211 / 199.  7 and more dimensions, of the time with 8
+    // wanted (and chunks from parts of 1024): 8 dimensions, K = 16, 30k showers 0.63, uniform 0.85, normal 0.79; 50k 0.67, 0.95, 0.91; 70k 0.75,
+    // 1.08, 1.05.
     const long long chunks = (long long)tile_chunks_cap(n_vert, n_events), sms = sm_count();
     const long long whole = sms * (n_coords <= 3 ? 8 : n_coords == 4 ? 30 : 40), cut = sms * (n_coords <= 3 ? 8 : n_coords == 4 ? (K < 24 ? 10 : 16) : 40);
     a.tile = 32;
