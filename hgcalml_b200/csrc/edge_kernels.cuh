@@ -97,7 +97,7 @@ __device__ __forceinline__ EdgeVec edge_terms(const EdgeVec &g, const EdgeVec &h
 // `maxima` (rows `ldm` floats apart, HVEC: whole vectors) holds what goes to the maximum alone.  Which features of a source
 // have the target as their maximum comes as bits (arg_flags_kernel): reading the arg-max row of every edge instead doubled
 // the gathered bytes.
-// 12.8 M edges, F = 64, hits in the search's order: 0.57 ms; a warp per target with 4-byte loads and 8 rows in flight took
+// 12.8 M edges, F = 64, hits in the search's order: 0.55 ms; a warp per target with 4-byte loads and 8 rows in flight took
 // 0.91, its 77 registers leaving 24 warps per SM.  Half of the gathered lines miss L1 and resident warps hide that better than
 // rows in flight: 16 lanes x 4 features with 2 rows and 40 warps per SM beat 4 rows (+1 %), 8 rows (+20 %), a warp x 2 features
 // (+10 %), and 64 warps, which spill (+27 %).  PushKnn, 200k hits, K = 40, F = 32: 433 -> 341 us.
@@ -298,7 +298,7 @@ arg_flags_kernel(const int *__restrict__ arg, const int *__restrict__ nidx, unsi
 // VEC: rows are whole 16-byte vectors (F % 4 == 0, bases aligned), which cp.async puts into shared memory past the registers
 // and L1.  12.8 M edges, F = 64: 0.85 ms with 4-byte loads and stores and a test of every feature for the maximum, bound by
 // issue (80 % of the slots) and the L1 data stage (79 %); 0.62 with 16-byte loads and stores, packed products and the
-// maxima taken from the bits; 0.51 with cp.async (cached in L1 as well 0.53; MAX without the bound on registers 0.56).
+// maxima taken from the bits; 0.50 with cp.async (cached in L1 as well 0.53; MAX without the bound on registers 0.56).
 // MAX also writes the edge's bits for edge_sum_kernel (features 0 .. 63), which it compares for anyway.
 template <bool GRAD, bool MAX, bool VEC>
 __global__ void __launch_bounds__(256, MAX ? 5 : 6)
